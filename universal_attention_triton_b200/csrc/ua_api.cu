@@ -942,9 +942,16 @@ int ua_decode_step(const UaDims* dims, int dtype, int gate_dtype, int t, const v
   p.BH = s.B * s.H; p.R = s.R; p.D = s.D; p.C = s.C; p.Lcap = s.L; p.t = t;
   p.kcache = k_cache; p.vcache = v_cache; p.src = src_cache; p.q = q_t; p.dest = dest_t; p.state = decay_state;
   p.out = out_t; p.lse = lse_t;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (ua::decode::step_mma_takes(p, dtype == UA_BF16)) {
+    const int nt = t / s.C + 1;
+    bool ok;
+    if (s.D == 64) ok = gate_dtype == UA_F32 ? ua::decode::launch_step_mma_c<64, float>(p, nt, st) : ua::decode::launch_step_mma_c<64, bf16>(p, nt, st);
+    else ok = gate_dtype == UA_F32 ? ua::decode::launch_step_mma_c<128, float>(p, nt, st) : ua::decode::launch_step_mma_c<128, bf16>(p, nt, st);
+    return ok && cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  }
   const size_t smem = ua::decode::smem_bytes(p);
   if (smem > 48 * 1024) return UA_ERR_UNSUPPORTED;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const dim3 grid((unsigned)p.BH, (unsigned)(t / s.C + 1));
   if (dtype == UA_F32) ua::decode::step_kernel<float, float><<<grid, s.C, smem, st>>>(p);
   else if (gate_dtype == UA_F32) ua::decode::step_kernel<bf16, float><<<grid, s.C, smem, st>>>(p);
