@@ -98,147 +98,183 @@ struct MkCtx {
   __device__ __forceinline__ int srow(int j) const { return r0 + (j - jb) * 128; }
 };
 
+// Small dense products of the prep and finish kernels: mma.sync on tiles that sit in shared memory as [rows][D + 8] bf16 (the
+// padding makes every ldmatrix conflict free).  A block has 128 x D x D multiply-adds to do, so what counts is how soon it is
+// done, not the rate; the tcgen05 path would spend longer on its set-up than this takes.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <int D> struct MkDense {
+  static constexpr int kStride = D + 8;                  // elements per row of a padded tile
+  static constexpr int kTile = 128 * kStride * 2;        // bytes
+};
+
 // ------------------------------------------------------------------ prep kernel --
 // One block per chunk: ksum / 128 (bf16), M^T / 128 (bf16, in the swizzled layout the sweep kernel's MMAs read), and the
-// chunk's N / w / u accumulators set to zero.
+// chunk's N / w / u accumulators set to zero.  M = K^T V - ksum (x) vsum / 128 from exact bf16 products with fp32 sums.
 template <int D>
 __global__ void __launch_bounds__(256) masked_prep_kernel(const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                                                           MaskedParams p) {
+  using Dn = MkDense<D>;
   extern __shared__ __align__(16) uint8_t prep_smem[];
   __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(prep_smem);
-  __nv_bfloat16* sV = sK + 128 * D;
-  float* sSum = reinterpret_cast<float*>(sV + 128 * D);
+  __nv_bfloat16* sV = sK + 128 * Dn::kStride;
+  float* sSum = reinterpret_cast<float*>(sV + 128 * Dn::kStride);
   const size_t chunk = blockIdx.x;
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   float* nacc = p.nacc + chunk * (size_t)kNaccRows<D>() * D;
-  for (int x = t; x < (D + 2) * D / 4; x += 256) reinterpret_cast<float4*>(nacc)[x] = make_float4(0.f, 0.f, 0.f, 0.f);
   const uint4* gk = reinterpret_cast<const uint4*>(kc + chunk * 128 * D);
   const uint4* gv = reinterpret_cast<const uint4*>(vc + chunk * 128 * D);
+#pragma unroll
   for (int x = t; x < 128 * D / 8; x += 256) {
-    reinterpret_cast<uint4*>(sK)[x] = gk[x];
-    reinterpret_cast<uint4*>(sV)[x] = gv[x];
+    const int row = x / (D / 8), col = (x % (D / 8)) * 8;
+    *reinterpret_cast<uint4*>(sK + row * Dn::kStride + col) = gk[x];
+    *reinterpret_cast<uint4*>(sV + row * Dn::kStride + col) = gv[x];
   }
+  for (int x = t; x < (D + 2) * D / 4; x += 256) reinterpret_cast<float4*>(nacc)[x] = make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
   if (t < 2 * D) {
     const __nv_bfloat16* src = (t < D) ? sK + t : sV + (t - D);
     float acc = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < 128; ++k) acc += __bfloat162float(src[k * D]);
+#pragma unroll 16
+    for (int k = 0; k < 128; ++k) acc += __bfloat162float(src[k * Dn::kStride]);
     sSum[t] = acc;
     if (t < D) p.ksum[chunk * D + t] = __float2bfloat16_rn(acc * (1.0f / 128.0f));
     else nacc[(size_t)(D + 2) * D + (t - D)] = acc * (1.0f / 128.0f);
   }
+  // M^T: warp = 16 rows d' x kCols columns d
+  constexpr int kMT = D / 16, kSplit = 8 / kMT, kCols = D / kSplit;
+  const int m0 = (warp % kMT) * 16, n0 = (warp / kMT) * kCols;
+  float acc[kCols / 8][4];
+#pragma unroll
+  for (int n = 0; n < kCols / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  const uint32_t aK = smem_u32(sK) + 2 * (((lane >> 4) * 8 + (lane & 7)) * Dn::kStride + m0 + ((lane >> 3) & 1) * 8);
+  const uint32_t aV = smem_u32(sV) + 2 * ((lane & 15) * Dn::kStride + n0 + (lane >> 4) * 8);
+#pragma unroll
+  for (int k = 0; k < 128; k += 16) {
+    uint32_t a[4];
+    ldmatrix_x4_trans(a, aK + 2 * k * Dn::kStride);
+#pragma unroll
+    for (int n = 0; n < kCols; n += 16) {
+      uint32_t b[4];
+      ldmatrix_x4_trans(b, aV + 2 * (k * Dn::kStride + n));
+      mma_16816(acc[n / 8], a, b[0], b[1]);
+      mma_16816(acc[n / 8 + 1], a, b[2], b[3]);
+    }
+  }
   __syncthreads();
   uint8_t* img = p.mt + chunk * (size_t)(D * D * 2);
-  // each thread: four rows d' (dp0 .. dp0 + 3) x eight columns d0 .. d0 + 7 of M^T, so that a value tile row is converted once per four rows
-  for (int o = t; o < D * D / 32; o += 256) {
-    const int dp0 = (o / (D / 8)) * 4, d0 = (o % (D / 8)) * 8;
-    float acc[4][8];
 #pragma unroll
-    for (int y = 0; y < 4; ++y)
+  for (int h = 0; h < 2; ++h) {
+    const int dp = m0 + (lane >> 2) + 8 * h, half = dp >> 6, row = dp & 63;
+    const float ks = sSum[dp] * (1.0f / 128.0f);
 #pragma unroll
-      for (int x = 0; x < 8; ++x) acc[y][x] = 0.f;
-#pragma unroll 2
-    for (int k = 0; k < 128; ++k) {
-      const uint2 kraw = *reinterpret_cast<const uint2*>(sK + k * D + dp0);
-      const float kv[4] = {__uint_as_float(kraw.x << 16), __uint_as_float(kraw.x & 0xffff0000u), __uint_as_float(kraw.y << 16),
-                           __uint_as_float(kraw.y & 0xffff0000u)};
-      const uint4 raw = *reinterpret_cast<const uint4*>(sV + k * D + d0);
-      const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-      float vv[8];
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        vv[2 * x] = __uint_as_float(rw[x] << 16);
-        vv[2 * x + 1] = __uint_as_float(rw[x] & 0xffff0000u);
-      }
-#pragma unroll
-      for (int y = 0; y < 4; ++y)
-#pragma unroll
-        for (int x = 0; x < 8; ++x) acc[y][x] = fmaf(kv[y], vv[x], acc[y][x]);
-    }
-#pragma unroll
-    for (int y = 0; y < 4; ++y) {
-      const int dp = dp0 + y;
-      const float ks = sSum[dp] * (1.0f / 128.0f);
-      uint32_t w4[4];
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        __nv_bfloat162 hh = __floats2bfloat162_rn((acc[y][2 * x] - ks * sSum[D + d0 + 2 * x]) * (1.0f / 128.0f),
-                                                  (acc[y][2 * x + 1] - ks * sSum[D + d0 + 2 * x + 1]) * (1.0f / 128.0f));
-        w4[x] = *reinterpret_cast<uint32_t*>(&hh);
-      }
-      const int half = dp >> 6, row = dp & 63, box = d0 >> 6, chunk16 = (d0 & 63) >> 3;
-      *reinterpret_cast<uint4*>(img + ((size_t)(half * (D / 64) + box) * 64 + row) * 128 + (((chunk16 ^ row) & 7) << 4)) =
-          make_uint4(w4[0], w4[1], w4[2], w4[3]);
+    for (int n = 0; n < kCols / 8; ++n) {
+      const int d = n0 + 8 * n + (lane & 3) * 2, box = d >> 6, piece = (d & 63) >> 3;
+      const __nv_bfloat162 v = __floats2bfloat162_rn((acc[n][2 * h] - ks * sSum[D + d]) * (1.0f / 128.0f),
+                                                     (acc[n][2 * h + 1] - ks * sSum[D + d + 1]) * (1.0f / 128.0f));
+      *reinterpret_cast<__nv_bfloat162*>(img + ((size_t)(half * (D / 64) + box) * 64 + row) * 128 + (((piece ^ row) & 7) << 4) +
+                                         (d & 7) * 2) = v;
     }
   }
 }
 
 // ---------------------------------------------------------------- finish kernel --
-// One block per chunk i >= 1 (thread = key): dK_i += ((V_i - vbar) N_i + 1 (x) w_i) / 128.  (dV_i = 1 (x) u_i / 128 is the same row
-// for every key: the main backward kernel adds it from the chunk's u row when it writes dV_i.)
+// One block per chunk i >= 1: dK_i += ((V_i - vbar) N_i + 1 (x) w_i) / 128 = (V_i N_i + 1 (x) (w_i - vbar N_i)) / 128.  (dV_i =
+// 1 (x) u_i / 128 is the same row for every key: the main backward kernel adds it from the chunk's u row when it writes dV_i.)
+// N_i is fp32 and enters as the sum of three bf16 values (24 bits), V_i is bf16 as it is, sums in fp32: the product keeps fp32
+// precision on the tensor cores.  Warp = 2 D / 16 .. columns d' of all 128 keys, so that N_i is read and split once.
 template <int D>
-__global__ void __launch_bounds__(128) masked_finish_kernel(const __nv_bfloat16* __restrict__ vc, MaskedParams p) {
-  __shared__ __align__(16) float sN[32 * D];          // 32 rows d' of N^T at a time
-  __shared__ float sW[D];
+__global__ void __launch_bounds__(256) masked_finish_kernel(const __nv_bfloat16* __restrict__ vc, MaskedParams p) {
+  using Dn = MkDense<D>;
+  extern __shared__ __align__(16) uint8_t fin_smem[];
+  __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(fin_smem);
+  float* sVbar = reinterpret_cast<float*>(fin_smem + Dn::kTile);
   const int N = p.s.N;
   const size_t chunk = blockIdx.x;
   if (chunk % N == 0) return;           // no rows before the first chunk
-  const int key = threadIdx.x;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const float* nacc = p.nacc + chunk * (size_t)kNaccRows<D>() * D;
-  const float* vbar = nacc + (size_t)(D + 2) * D;
-  float vcen[D];
-  {
-    const uint4* gv = reinterpret_cast<const uint4*>(vc + (chunk * 128 + key) * D);
+  const uint4* gv = reinterpret_cast<const uint4*>(vc + chunk * 128 * D);
 #pragma unroll
-    for (int x = 0; x < D / 8; ++x) {
-      const uint4 raw = gv[x];
-      const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162*>(&rw[y]);
-        vcen[8 * x + 2 * y] = __bfloat162float(hv.x) - vbar[8 * x + 2 * y];
-        vcen[8 * x + 2 * y + 1] = __bfloat162float(hv.y) - vbar[8 * x + 2 * y + 1];
-      }
-    }
-  }
-  for (int x = key; x < D; x += 128) sW[x] = nacc[(size_t)D * D + x];
-  float* dk = p.acc_dk + (chunk * 128 + key) * D;
+  for (int x = t; x < 128 * D / 8; x += 256)
+    *reinterpret_cast<uint4*>(sV + (x / (D / 8)) * Dn::kStride + (x % (D / 8)) * 8) = gv[x];
+  if (t < D) sVbar[t] = nacc[(size_t)(D + 2) * D + t];
+  __syncthreads();
   if (p.acc_dv) {                       // row ranges: the same row u / 128 for every key, added to the shared fp32 buffer
-    const float* u = nacc + (size_t)(D + 1) * D;
-    float4* dv = reinterpret_cast<float4*>(p.acc_dv + (chunk * 128 + key) * D);
-#pragma unroll 4
-    for (int x = 0; x < D / 4; ++x) {
+    const float4* u = reinterpret_cast<const float4*>(nacc + (size_t)(D + 1) * D);
+    float4* dv = reinterpret_cast<float4*>(p.acc_dv + chunk * 128 * D);
+    for (int x = t; x < 128 * D / 4; x += 256) {
+      const float4 add = u[x % (D / 4)];
       float4 cur = dv[x];
-      cur.x += u[4 * x] * (1.0f / 128.0f); cur.y += u[4 * x + 1] * (1.0f / 128.0f);
-      cur.z += u[4 * x + 2] * (1.0f / 128.0f); cur.w += u[4 * x + 3] * (1.0f / 128.0f);
+      cur.x += add.x * (1.0f / 128.0f); cur.y += add.y * (1.0f / 128.0f);
+      cur.z += add.z * (1.0f / 128.0f); cur.w += add.w * (1.0f / 128.0f);
       dv[x] = cur;
     }
   }
-#pragma unroll 1
-  for (int blk = 0; blk < D / 32; ++blk) {
-    __syncthreads();
-    for (int x = key; x < 32 * D / 4; x += 128) reinterpret_cast<float4*>(sN)[x] = reinterpret_cast<const float4*>(nacc + (size_t)blk * 32 * D)[x];
-    __syncthreads();
-#pragma unroll 1
-    for (int q = 0; q < 32; q += 4) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  constexpr int kNW = D / 64;           // column tiles of 8 per warp
+  const int n0 = warp * 8 * kNW;
+  float acc[kNW][8][4], vb[kNW];
 #pragma unroll
-      for (int d = 0; d < D; d += 4) {
+  for (int n = 0; n < kNW; ++n) {
+    vb[n] = 0.f;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const float4 nv = *reinterpret_cast<const float4*>(sN + (q + x) * D + d);
-          acc[x] = fmaf(vcen[d], nv.x, fmaf(vcen[d + 1], nv.y, fmaf(vcen[d + 2], nv.z, fmaf(vcen[d + 3], nv.w, acc[x]))));
+    for (int m = 0; m < 8; ++m) acc[n][m][0] = acc[n][m][1] = acc[n][m][2] = acc[n][m][3] = 0.f;
+  }
+  const uint32_t aV = smem_u32(sV) + 2 * ((lane & 15) * Dn::kStride + (lane >> 4) * 8);
+  const float* nrow = nacc + (size_t)(n0 + (lane >> 2)) * D + (lane & 3) * 2;       // N^T[d'][d]
+#pragma unroll 2
+  for (int k = 0; k < D; k += 16) {
+    uint32_t b[kNW][3][2];
+#pragma unroll
+    for (int n = 0; n < kNW; ++n)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float2 v = *reinterpret_cast<const float2*>(nrow + (size_t)n * 8 * D + k + 8 * h);
+        vb[n] = fmaf(v.x, sVbar[k + 8 * h + (lane & 3) * 2], fmaf(v.y, sVbar[k + 8 * h + (lane & 3) * 2 + 1], vb[n]));
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const __nv_bfloat162 hi = __floats2bfloat162_rn(v.x, v.y);
+          b[n][q][h] = *reinterpret_cast<const uint32_t*>(&hi);
+          v.x -= __bfloat162float(hi.x); v.y -= __bfloat162float(hi.y);
         }
       }
-      float4* dst = reinterpret_cast<float4*>(dk + blk * 32 + q);
-      float4 cur = *dst;
-      cur.x += (acc[0] + sW[blk * 32 + q]) * (1.0f / 128.0f);
-      cur.y += (acc[1] + sW[blk * 32 + q + 1]) * (1.0f / 128.0f);
-      cur.z += (acc[2] + sW[blk * 32 + q + 2]) * (1.0f / 128.0f);
-      cur.w += (acc[3] + sW[blk * 32 + q + 3]) * (1.0f / 128.0f);
-      *dst = cur;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      uint32_t a[4];
+      ldmatrix_x4(a, aV + 2 * (m * 16 * Dn::kStride + k));
+#pragma unroll
+      for (int n = 0; n < kNW; ++n)
+#pragma unroll
+        for (int q = 2; q >= 0; --q) mma_16816(acc[n][m], a, b[n][q][0], b[n][q][1]);
     }
+  }
+#pragma unroll
+  for (int n = 0; n < kNW; ++n) {
+    // vbar . N[:, d'] for d' = n0 + 8 n + lane / 4, over the four lanes that hold its pieces; handed to the lanes that own the columns
+    vb[n] += __shfl_xor_sync(0xffffffffu, vb[n], 1);
+    vb[n] += __shfl_xor_sync(0xffffffffu, vb[n], 2);
+    const int dp = n0 + 8 * n + (lane & 3) * 2;
+    const float c0 = nacc[(size_t)D * D + dp] - __shfl_sync(0xffffffffu, vb[n], (lane & 3) * 8);
+    const float c1 = nacc[(size_t)D * D + dp + 1] - __shfl_sync(0xffffffffu, vb[n], (lane & 3) * 8 + 4);
+    float* dk = p.acc_dk + (chunk * 128 + (lane >> 2)) * D + dp;
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float2* at = reinterpret_cast<float2*>(dk + (size_t)(m * 16 + 8 * h) * D);
+        float2 cur = *at;
+        cur.x += (acc[n][m][2 * h] + c0) * (1.0f / 128.0f);
+        cur.y += (acc[n][m][2 * h + 1] + c1) * (1.0f / 128.0f);
+        *at = cur;
+      }
   }
 }
 

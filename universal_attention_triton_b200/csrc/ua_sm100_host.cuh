@@ -210,14 +210,14 @@ int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* 
   if (p.items_per_bh == 0) return UA_OK;
   const auto* k16 = static_cast<const __nv_bfloat16*>(kc);
   const auto* v16 = static_cast<const __nv_bfloat16*>(vc);
-  const int prep_smem = 2 * 128 * D * 2 + 2 * D * 4;
+  const int prep_smem = 2 * MkDense<D>::kTile + 2 * D * 4, finish_smem = MkDense<D>::kTile + D * 4;
   auto prep = masked_prep_kernel<D>;
   if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem) != cudaSuccess) return UA_ERR_CUDA;
   prep<<<(unsigned)(BH * s.N), 256, prep_smem, st>>>(k16, v16, p);
   auto sweep = masked_sweep_kernel<D>;
   if (cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
   sweep<<<(unsigned)(BH * p.items_per_bh * Cfg::kKB), 384, Cfg::kSmemBytes, st>>>(tmQ, tmG, tmDQ, p);
-  masked_finish_kernel<D><<<(unsigned)(BH * s.N), 128, 0, st>>>(v16, p);
+  masked_finish_kernel<D><<<(unsigned)(BH * s.N), 256, finish_smem, st>>>(v16, p);      // (at most 35 KB: no opt-in needed)
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
 
