@@ -74,6 +74,7 @@ SIGNATURES = {
 PREP_NORMALIZE_KEYS, PREP_SIGMOID_GATES = 1, 2
 
 _lib = None
+_native = None
 
 
 def load():
@@ -92,6 +93,22 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def native():
+    """The extension module with the tensor plumbing (``csrc/ua_torch.cpp``), which calls the same library."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _ua_torch
+        except ImportError as e:
+            raise UaLibraryError(f"the extension module beside {LIB_PATH} does not load ({e}): build it with "
+                                 "`python -m universal_attention_triton_b200.build`") from e
+        from .ops import plain
+        _ua_torch.bind(UaLibraryError, plain)
+        _native = _ua_torch
+    return _native
 
 
 def check(code: int, what: str):

@@ -1,4 +1,4 @@
-"""In-tree build of libua_b200.so (sm_100a only) with nvcc.
+"""In-tree build of libua_b200.so (sm_100a only) with nvcc, and of the extension module _ua_torch.so above it.
 
     python -m universal_attention_triton_b200.build [--verbose]
 
@@ -16,6 +16,9 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libua_b200.so")
 SOURCES = ["ua_api.cu"]
+# the tensor plumbing above the library: an extension module, host code only
+TORCH_SOURCE = "ua_torch.cpp"
+TORCH_PATH = os.path.join(PKG_DIR, "_ua_torch.so")
 # developer micro-benchmark (stand-alone executable, not loaded by the package): `--tools` builds it next to the library
 TOOL_SOURCE = "mma_timing.cu"
 TOOL_PATH = os.path.join(PKG_DIR, "mma_timing.bin")
@@ -33,9 +36,9 @@ def _nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(TORCH_PATH):
         return True
-    t = os.path.getmtime(LIB_PATH)
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(TORCH_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(os.path.dirname(PKG_DIR), "include", "ua_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
@@ -52,7 +55,27 @@ def build(force: bool = False, verbose: bool = False) -> str:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed building libua_b200.so")
+    _build_torch_module()
     return LIB_PATH
+
+
+def _build_torch_module() -> None:
+    """The extension module that holds the tensor plumbing; links the library by its place beside it."""
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda_inc = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for inc in include_paths() + [cuda_inc, sysconfig.get_paths()["include"]]:
+        cmd += ["-isystem", inc]
+    cmd += [os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_PATH, "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-L" + torch_lib,
+            "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("the C++ compiler failed building _ua_torch.so")
 
 
 def build_tools() -> str:

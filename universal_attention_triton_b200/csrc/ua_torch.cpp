@@ -1,0 +1,321 @@
+// Tensor plumbing of the package in native code: argument checks, allocations, the current stream and the calls into
+// libua_b200.so.  ops.py documents each function under its own name; this file holds what used to be Python there, because
+// at the small sizes the host path was the whole cost (a training step of B1 H8 R4 L1024 spent 790 us of which 318 on the GPU).
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <optional>
+#include <string>
+#include <tuple>
+
+#include "../../include/ua_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+// set once at import and never released (the interpreter is gone when static objects are destroyed)
+py::handle g_error;      // _lib.UaLibraryError
+py::handle g_unwrap;     // ops.plain: takes functorch's wrappers off a tensor
+
+[[noreturn]] void raise(py::handle type, const std::string& msg) {
+  PyErr_SetString(type.ptr(), msg.c_str());
+  throw py::error_already_set();
+}
+void check(int code, const char* what) {
+  if (code != UA_OK)
+    raise(g_error, std::string(what) + " failed: " + ua_error_string(code) + " (code " + std::to_string(code) + ")");
+}
+
+// the tensor with storage: functorch's wrappers (torch.func.grad) taken off where there are any
+Tensor plain(const Tensor& t) {
+  return t.key_set().has(c10::DispatchKey::FuncTorchGradWrapper) ? g_unwrap(t).cast<Tensor>() : t;
+}
+template <typename... Ts> void require_cuda(const Ts&... ts) {
+  if (!(ts.is_cuda() && ...))
+    raise(PyExc_RuntimeError, "Universal Attention has no CPU path: tensors must live on a CUDA device");
+}
+int code_of(at::ScalarType t) {
+  if (t == at::kFloat) return UA_F32;
+  if (t == at::kBFloat16) return UA_BF16;
+  raise(PyExc_TypeError, std::string("Universal Attention kernels support float32 and bfloat16, got ") + c10::toString(t));
+}
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+// With UA_CHECK_STATUS=1 every call synchronises and reads the kernels' status word (a bounded device-side wait that ran
+// out): for tests and debugging.
+void check_status(const Tensor& ws, void* stream, const char* what) {
+  const char* e = std::getenv("UA_CHECK_STATUS");
+  if (e && std::strcmp(e, "1") == 0) check(ua_workspace_status(ptr(ws), stream), (std::string(what) + " (device status)").c_str());
+}
+
+struct Gates { Tensor src, dest; };
+// the kernels take gates either in the q/k/v dtype or in fp32, both the same
+Gates gates(const Tensor& s, const Tensor& d, at::ScalarType dt) {
+  auto cast = [&](const Tensor& g) { return (g.scalar_type() == dt || g.scalar_type() == at::kFloat) ? g.contiguous() : g.to(at::kFloat).contiguous(); };
+  Gates g{cast(s), cast(d)};
+  if (g.src.scalar_type() != g.dest.scalar_type()) g = Gates{g.src.to(at::kFloat), g.dest.to(at::kFloat)};
+  return g;
+}
+
+struct Problem {
+  UaDims dims;
+  int64_t b, h, r, n, c, d, L;
+  at::ScalarType dt;
+  int code;
+};
+Problem problem(const Tensor& kc, const Tensor& xq) {
+  Problem p;
+  TORCH_CHECK(kc.dim() == 5, "keys are (b, h, n, c, d)");
+  p.b = kc.size(0); p.h = kc.size(1); p.n = kc.size(2); p.c = kc.size(3); p.d = kc.size(4);
+  p.r = xq.size(2); p.L = p.n * p.c;
+  p.dt = xq.scalar_type(); p.code = code_of(p.dt);
+  p.dims = UaDims{(int)p.b, (int)p.h, (int)p.r, (int)p.n, (int)p.c, (int)p.d};
+  return p;
+}
+struct Inputs { Tensor kc, vc, q; Gates g; };
+Inputs inputs(const Problem& p, const Tensor& kc, const Tensor& vc, const Tensor& xq, const Tensor& ss, const Tensor& sd) {
+  const int64_t keys = p.b * p.h * p.L;
+  TORCH_CHECK(vc.sizes() == kc.sizes() && xq.numel() == keys * p.r * p.d && ss.numel() == keys && sd.numel() == keys,
+              "shapes of the operator's inputs do not fit together");
+  TORCH_CHECK(kc.scalar_type() == p.dt && vc.scalar_type() == p.dt, "keys, values and queries share one dtype");
+  return Inputs{kc.contiguous(), vc.contiguous(), xq.contiguous(), gates(ss, sd, p.dt)};
+}
+
+// (out_cm, lse_cm, denom_cm, carry or None)
+std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_cm(const Tensor& kc_, const Tensor& vc_, const Tensor& xq_, const Tensor& ss_,
+                                                         const Tensor& sd_, int flags, bool keep_carry) {
+  require_cuda(kc_, vc_, xq_, ss_, sd_);
+  const Tensor kc = plain(kc_), xq = plain(xq_);
+  const Problem p = problem(kc, xq);
+  const c10::cuda::CUDAGuard guard(kc.device());
+  const Inputs in = inputs(p, kc, plain(vc_), xq, plain(ss_), plain(sd_));
+  const auto opt = kc.options().requires_grad(false);
+  Tensor out = at::empty({p.b, p.h, p.n, p.r, p.L, p.d}, opt.dtype(p.dt));
+  Tensor lse = at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(at::kFloat));
+  Tensor denom = p.code == UA_F32 ? lse : at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(p.dt));
+  const size_t ws_bytes = std::max<size_t>(ua_fwd_workspace_bytes(&p.dims, p.code, flags), 256);
+  Tensor ws = at::empty({(int64_t)ws_bytes}, opt.dtype(at::kByte));
+  OptTensor carry;
+  if (keep_carry) {
+    if (const size_t bytes = ua_carry_bytes(&p.dims, p.code, flags)) carry = at::empty({(int64_t)(bytes / 4)}, opt.dtype(at::kFloat));
+  }
+  void* st = stream_of(kc);
+  check(ua_fwd_keep(&p.dims, p.code, code_of(in.g.src.scalar_type()), ptr(in.kc), ptr(in.vc), ptr(in.q), ptr(in.g.src), ptr(in.g.dest),
+                    ptr(out), static_cast<float*>(ptr(lse)), p.code == UA_F32 ? nullptr : ptr(denom), carry ? ptr(*carry) : nullptr,
+                    ptr(ws), ws_bytes, flags, st), "ua_fwd");
+  check_status(ws, st, "ua_fwd");
+  return {out, lse, denom, carry};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> backward_cm(const Tensor& kc_, const Tensor& vc_, const Tensor& xq_, const Tensor& ss_,
+                                                               const Tensor& sd_, const Tensor& g_out_, const Tensor& g_denom_, int flags,
+                                                               const OptTensor& carry_, const OptTensor& lse_, const OptTensor& out_) {
+  require_cuda(kc_, vc_, xq_, ss_, sd_, g_out_, g_denom_);
+  const Tensor kc = plain(kc_), vc = plain(vc_), xq = plain(xq_), ss = plain(ss_), sd = plain(sd_);
+  const Problem p = problem(kc, xq);
+  const c10::cuda::CUDAGuard guard(kc.device());
+  const Inputs in = inputs(p, kc, vc, xq, ss, sd);
+  const Tensor g_out = plain(g_out_).to(p.dt).contiguous();
+  Tensor g_denom = plain(g_denom_);
+  if (g_denom.scalar_type() != at::kFloat && g_denom.scalar_type() != p.dt) g_denom = g_denom.to(at::kFloat);
+  g_denom = g_denom.contiguous();
+  const int64_t rows = p.b * p.h * p.n * p.r * p.L;
+  TORCH_CHECK(g_out.numel() == rows * p.d && g_denom.numel() == rows, "upstream gradients do not have the outputs' shape");
+  Tensor carry, lse, out;
+  if (carry_) {
+    carry = plain(*carry_);
+    if ((size_t)carry.numel() * 4 != ua_carry_bytes(&p.dims, p.code, flags)) carry = Tensor();
+  }
+  if (lse_) {
+    lse = plain(*lse_);
+    if (lse.scalar_type() != at::kFloat || lse.sizes() != at::IntArrayRef({p.b, p.h, p.n, p.r, p.L}) || !lse.is_cuda())
+      raise(PyExc_ValueError, "lse must be the fp32 chunk-major (b,h,n,r,L) log-sum-exp of the forward");
+    lse = lse.contiguous();
+  }
+  if (out_) {
+    out = plain(*out_);
+    if (!(out.is_cuda() && out.scalar_type() == p.dt && out.is_contiguous() && out.sizes() == at::IntArrayRef({p.b, p.h, p.n, p.r, p.L, p.d})))
+      out = Tensor();
+  }
+  const auto opt = kc.options().requires_grad(false);
+  Tensor dk = at::empty(kc.sizes(), opt), dv = at::empty(kc.sizes(), opt), dq = at::empty(xq.sizes(), opt.dtype(p.dt));
+  Tensor dss = at::empty(ss.sizes(), opt.dtype(in.g.src.scalar_type())), dsd = at::empty(sd.sizes(), opt.dtype(in.g.src.scalar_type()));
+  const size_t ws_bytes = std::max<size_t>(ua_bwd_workspace_bytes(&p.dims, p.code, flags), 256);
+  Tensor ws = at::empty({(int64_t)ws_bytes}, opt.dtype(at::kByte));
+  void* st = stream_of(kc);
+  check(ua_bwd_saved(&p.dims, p.code, code_of(in.g.src.scalar_type()), ptr(in.kc), ptr(in.vc), ptr(in.q), ptr(in.g.src), ptr(in.g.dest),
+                     ptr(g_out), ptr(g_denom), code_of(g_denom.scalar_type()), ptr(carry), static_cast<float*>(ptr(lse)), ptr(out), ptr(dk),
+                     ptr(dv), ptr(dq), ptr(dss), ptr(dsd), ptr(ws), ws_bytes, flags, st), "ua_bwd");
+  check_status(ws, st, "ua_bwd");
+  if (dss.scalar_type() != ss.scalar_type()) dss = dss.to(ss.scalar_type());
+  if (dsd.scalar_type() != sd.scalar_type()) dsd = dsd.to(sd.scalar_type());
+  return {dk, dv, dq, dss, dsd};
+}
+
+UaDims merge_dims(const Tensor& out_cm) {
+  TORCH_CHECK(out_cm.dim() == 6, "outputs are (b, h, n, r, L, d)");
+  const int64_t n = out_cm.size(2), L = out_cm.size(4);
+  return UaDims{(int)out_cm.size(0), (int)out_cm.size(1), (int)out_cm.size(3), (int)n, (int)(L / n), (int)out_cm.size(5)};
+}
+// merged (b,h,r,L,d) and, on request, the rows' log-sum-exp over all chunks
+std::tuple<Tensor, OptTensor> merge_fwd_cm(const Tensor& out_, const Tensor& lse_, bool stats) {
+  require_cuda(out_, lse_);
+  const Tensor out = plain(out_).contiguous(), lse = plain(lse_).to(at::kFloat).contiguous();
+  const UaDims dims = merge_dims(out);
+  const c10::cuda::CUDAGuard guard(out.device());
+  TORCH_CHECK(lse.numel() * out.size(5) == out.numel(), "log-sum-exp does not fit the outputs");
+  const auto opt = out.options().requires_grad(false);
+  Tensor merged = at::empty({out.size(0), out.size(1), out.size(3), out.size(4), out.size(5)}, opt);
+  OptTensor row_lse;
+  if (stats) row_lse = at::empty({out.size(0), out.size(1), out.size(3), out.size(4)}, opt.dtype(at::kFloat));
+  check(ua_merge_fwd_stats(&dims, code_of(out.scalar_type()), ptr(out), static_cast<float*>(ptr(lse)), ptr(merged),
+                           row_lse ? static_cast<float*>(ptr(*row_lse)) : nullptr, stream_of(out)), stats ? "ua_merge_fwd_stats" : "ua_merge_fwd");
+  return {merged, row_lse};
+}
+std::tuple<Tensor, Tensor> merge_bwd_cm(const Tensor& out_, const Tensor& lse_, const Tensor& g_, bool skip_zero_weight_blocks) {
+  require_cuda(out_, lse_, g_);
+  const Tensor out = plain(out_).contiguous(), lse = plain(lse_).to(at::kFloat).contiguous();
+  const Tensor g = plain(g_).to(out.scalar_type()).contiguous();
+  const UaDims dims = merge_dims(out);
+  const c10::cuda::CUDAGuard guard(out.device());
+  TORCH_CHECK(lse.numel() * out.size(5) == out.numel() && g.numel() * out.size(2) == out.numel(), "gradient or log-sum-exp does not fit the outputs");
+  const auto opt = out.options().requires_grad(false);
+  Tensor g_out = at::empty(out.sizes(), opt), g_lse = at::empty(lse.sizes(), opt.dtype(at::kFloat));
+  check(ua_merge_bwd(&dims, code_of(out.scalar_type()), ptr(out), static_cast<float*>(ptr(lse)), ptr(g), ptr(g_out), static_cast<float*>(ptr(g_lse)),
+                     skip_zero_weight_blocks ? UA_FLAG_SKIP_MASKED_FILL : 0, stream_of(out)), "ua_merge_bwd");
+  return {g_out, g_lse};
+}
+
+// ---- layout: chunk-major storage <-> the reference's shapes --------------------------------------------------------
+Tensor relayout(const Tensor& t_, int64_t inner, bool to_reference) {
+  require_cuda(t_);
+  const Tensor src = plain(t_).contiguous();
+  if (src.element_size() != 2 && src.element_size() != 4) raise(PyExc_TypeError, "relayout handles 2- and 4-byte elements");
+  const bool six = src.dim() == 6;
+  const int64_t b = src.size(0), h = src.size(1);
+  const int64_t n = to_reference ? src.size(2) : src.size(-1), r = src.size(to_reference ? 3 : 2), L = src.size(to_reference ? 4 : 3);
+  if (L % n) raise(PyExc_ValueError, "rows must be a multiple of the number of key chunks");
+  if (L / n % 16) raise(PyExc_ValueError, "chunk must be a multiple of 16");
+  // (chunk and head_dim are not used by the converter: only L = n * chunk matters)
+  const UaDims dims{(int)b, (int)h, (int)r, (int)n, (int)(L / n), 4};
+  const c10::cuda::CUDAGuard guard(src.device());
+  std::vector<int64_t> shape = to_reference ? std::vector<int64_t>{b, h, r, L} : std::vector<int64_t>{b, h, n, r, L};
+  if (six) shape.push_back(inner);
+  if (to_reference) shape.push_back(n);
+  Tensor dst = at::empty(shape, src.options().requires_grad(false));
+  check(ua_relayout(&dims, (int)inner, (int)src.element_size(), to_reference ? 1 : 0, ptr(src), ptr(dst), stream_of(src)), "ua_relayout");
+  return dst;
+}
+Tensor as_reference_out(const Tensor& t) { return t.permute({0, 1, 3, 4, 5, 2}); }
+Tensor as_reference_denom(const Tensor& t) { return t.permute({0, 1, 3, 4, 2}); }
+Tensor out_to_chunk_major(const Tensor& t_) {
+  const Tensor t = plain(t_), v = t.permute({0, 1, 5, 2, 3, 4});
+  return v.is_contiguous() ? v : relayout(t, t.size(4), false);
+}
+Tensor denom_to_chunk_major(const Tensor& t_) {
+  const Tensor t = plain(t_), v = t.permute({0, 1, 4, 2, 3});
+  return v.is_contiguous() ? v : relayout(t, 1, false);
+}
+
+// ---- incremental step ------------------------------------------------------------------------------------------------
+std::tuple<Tensor, Tensor> decode_step(int64_t t, const Tensor& k, const Tensor& v, const Tensor& src_, const Tensor& q_, const Tensor& dest_,
+                                       Tensor state, int64_t chunk) {
+  require_cuda(k, v, src_, q_, dest_, state);
+  const int64_t b = k.size(0), h = k.size(1), cap = k.size(2), d = k.size(3), r = q_.size(2);
+  const at::ScalarType dt = q_.scalar_type();
+  const int code = code_of(dt);
+  auto must = [](bool ok, const char* what) { if (!ok) raise(PyExc_AssertionError, what); };
+  must(state.scalar_type() == at::kFloat && state.is_contiguous() && state.sizes() == at::IntArrayRef({b, h, cap}), "decay_state is a contiguous fp32 (b, h, L_cap)");
+  must(k.is_contiguous() && v.is_contiguous() && v.sizes() == k.sizes() && cap % chunk == 0, "caches are contiguous (b, h, L_cap, d), whole chunks");
+  must(k.scalar_type() == dt && v.scalar_type() == dt && q_.numel() == b * h * r * d && src_.numel() == b * h * cap && dest_.numel() == b * h,
+       "shapes and dtypes of the step's inputs");
+  const c10::cuda::CUDAGuard guard(k.device());
+  const Gates g = gates(src_, dest_, dt);
+  const Tensor q = q_.contiguous();
+  const int64_t nt = t / chunk + 1;
+  const UaDims dims{(int)b, (int)h, (int)r, (int)(cap / chunk), (int)chunk, (int)d};
+  const auto opt = k.options().requires_grad(false);
+  Tensor out = at::empty({b, h, nt, r, d}, opt.dtype(dt)), lse = at::empty({b, h, nt, r}, opt.dtype(at::kFloat));
+  check(ua_decode_step(&dims, code, code_of(g.src.scalar_type()), (int)t, ptr(k), ptr(v), ptr(g.src), ptr(q), ptr(g.dest),
+                       static_cast<float*>(ptr(state)), ptr(out), static_cast<float*>(ptr(lse)), stream_of(k)), "ua_decode_step");
+  return {out.permute({0, 1, 3, 4, 2}), lse.permute({0, 1, 3, 2})};
+}
+
+// ---- input prologue ----------------------------------------------------------------------------------------------------
+// (kc, vc, xq, static_src, static_dest, key norms or None)
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> prepare_inputs(const Tensor& qs_, const Tensor& ks_, const Tensor& vs_, const Tensor& gs_,
+                                                                             int64_t chunk, int flags) {
+  require_cuda(qs_, ks_, vs_, gs_);
+  const at::ScalarType dt = qs_.scalar_type();
+  const c10::cuda::CUDAGuard guard(qs_.device());
+  const Tensor qs = plain(qs_).contiguous(), ks = plain(ks_).to(dt).contiguous(), vs = plain(vs_).to(dt).contiguous(), gs = plain(gs_).to(dt).contiguous();
+  const int64_t b = qs.size(0), s = qs.size(1), n = qs.size(2), d = qs.size(3), kv = ks.size(2);
+  auto must = [](bool ok) { if (!ok) raise(PyExc_AssertionError, "shapes of the projections do not fit together"); };
+  must(ks.sizes() == at::IntArrayRef({b, s, kv, d}) && vs.sizes() == ks.sizes() && gs.numel() == b * s * 2 * kv && n % kv == 0 && s % chunk == 0);
+  const auto opt = qs.options().requires_grad(false);
+  Tensor xq = at::empty({b, kv, n / kv, s, d}, opt), kc = at::empty({b, kv, s / chunk, chunk, d}, opt), vc = at::empty({b, kv, s / chunk, chunk, d}, opt);
+  Tensor src = at::empty({b, kv, s / chunk, chunk}, opt), dest = at::empty({b, kv, s}, opt);
+  OptTensor norm;
+  if (flags & UA_PREP_NORMALIZE_KEYS) norm = at::empty({b, kv, s}, opt.dtype(at::kFloat));
+  check(ua_prepare_inputs((int)b, (int)s, (int)n, (int)kv, (int)d, code_of(dt), flags, ptr(qs), ptr(ks), ptr(vs), ptr(gs), ptr(xq), ptr(kc), ptr(vc),
+                          ptr(src), ptr(dest), norm ? static_cast<float*>(ptr(*norm)) : nullptr, stream_of(qs)), "ua_prepare_inputs");
+  return {kc, vc, xq, src, dest, norm};
+}
+// gradients of the projections; an undefined upstream gradient counts as zeros
+std::tuple<Tensor, Tensor, Tensor, Tensor> prepare_inputs_bwd(const OptTensor& g_kc, const OptTensor& g_vc, const OptTensor& g_xq, const OptTensor& g_src,
+                                                              const OptTensor& g_dest, const Tensor& kc_, const Tensor& src_, const Tensor& dest_,
+                                                              const OptTensor& norm, int64_t n, int flags) {
+  const Tensor kc = plain(kc_), src = plain(src_), dest = plain(dest_);
+  const int64_t b = kc.size(0), kv = kc.size(1), s = kc.size(2) * kc.size(3), d = kc.size(4);
+  const at::ScalarType dt = kc.scalar_type();
+  const c10::cuda::CUDAGuard guard(kc.device());
+  const auto opt = kc.options().requires_grad(false);
+  auto full = [&](const OptTensor& g, at::IntArrayRef shape) { return g ? plain(*g).to(dt).contiguous() : at::zeros(shape, opt); };
+  const Tensor gk = full(g_kc, kc.sizes()), gv = full(g_vc, kc.sizes()), gq = full(g_xq, {b, kv, n / kv, s, d});
+  const Tensor gs = full(g_src, src.sizes()), gd = full(g_dest, dest.sizes());
+  require_cuda(gk, gv, gq, gs, gd);
+  TORCH_CHECK(gk.numel() == kc.numel() && gv.numel() == kc.numel() && gq.numel() == b * n * s * d && gs.numel() == src.numel() && gd.numel() == dest.numel(),
+              "upstream gradients do not have the outputs' shape");
+  Tensor dq = at::empty({b, s, n, d}, opt), dk = at::empty({b, s, kv, d}, opt), dv = at::empty({b, s, kv, d}, opt), dg = at::empty({b, s, 2, kv}, opt);
+  check(ua_prepare_inputs_bwd((int)b, (int)s, (int)n, (int)kv, (int)d, code_of(dt), flags, ptr(gq), ptr(gk), ptr(gv), ptr(gs), ptr(gd), ptr(kc),
+                              norm ? static_cast<float*>(ptr(plain(*norm))) : nullptr, ptr(src), ptr(dest), ptr(dq), ptr(dk), ptr(dv), ptr(dg), stream_of(kc)),
+        "ua_prepare_inputs_bwd");
+  return {dq, dk, dv, dg};
+}
+
+// Under a functorch transform every at:: call would wrap its result again; these functions work on plain tensors throughout.
+template <typename R, typename... A>
+auto outside_functorch(R (*f)(A...)) {
+  return [f](A... a) -> R {
+    const c10::impl::ExcludeDispatchKeyGuard guard(c10::DispatchKeySet({c10::DispatchKey::FuncTorchDynamicLayerFrontMode,
+                                                                       c10::DispatchKey::FuncTorchDynamicLayerBackMode,
+                                                                       c10::DispatchKey::FuncTorchGradWrapper}));
+    return f(std::forward<A>(a)...);
+  };
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_ua_torch, m) {
+  m.def("bind", [](py::object error, py::object unwrap) { g_error = error.release(); g_unwrap = unwrap.release(); });
+  m.def("forward_cm", outside_functorch(&forward_cm));
+  m.def("backward_cm", outside_functorch(&backward_cm));
+  m.def("merge_fwd_cm", outside_functorch(&merge_fwd_cm));
+  m.def("merge_bwd_cm", outside_functorch(&merge_bwd_cm));
+  m.def("relayout", outside_functorch(&relayout));
+  m.def("as_reference_out", outside_functorch(&as_reference_out));
+  m.def("as_reference_denom", outside_functorch(&as_reference_denom));
+  m.def("out_to_chunk_major", outside_functorch(&out_to_chunk_major));
+  m.def("denom_to_chunk_major", outside_functorch(&denom_to_chunk_major));
+  m.def("decode_step", outside_functorch(&decode_step));
+  m.def("prepare_inputs", outside_functorch(&prepare_inputs));
+  m.def("prepare_inputs_bwd", outside_functorch(&prepare_inputs_bwd));
+}

@@ -26,23 +26,26 @@ def _dtype_code(t: torch.dtype) -> int:
     raise TypeError(f"Universal Attention kernels support float32 and bfloat16, got {t}")
 
 
+try:
+    from torch._C._functorch import get_unwrapped, maybe_get_level, unwrap_if_dead
+except ImportError:      # pragma: no cover
+    maybe_get_level = None
+
+
+def _plain1(t):
+    if maybe_get_level is not None and isinstance(t, torch.Tensor):
+        for _ in range(16):
+            if maybe_get_level(t) == -1:
+                break
+            u = unwrap_if_dead(t)
+            t = u if u is not t else get_unwrapped(t)
+    return t
+
+
 def plain(*tensors):
     """Strips functorch wrappers (``torch.func.grad`` hands the backward its gradients and saved tensors wrapped, alive
     or already dead) so that the kernels get tensors with storage; first-order transforms only."""
-    try:
-        from torch._C._functorch import get_unwrapped, maybe_get_level, unwrap_if_dead
-    except ImportError:      # pragma: no cover
-        return tensors if len(tensors) != 1 else tensors[0]
-    out = []
-    for t in tensors:
-        if isinstance(t, torch.Tensor):
-            for _ in range(16):
-                if maybe_get_level(t) == -1:
-                    break
-                u = unwrap_if_dead(t)
-                t = u if u is not t else get_unwrapped(t)
-        out.append(t)
-    return tuple(out) if len(out) != 1 else out[0]
+    return tuple(_plain1(t) for t in tensors) if len(tensors) != 1 else _plain1(tensors[0])
 
 
 def _ptr(t):
@@ -83,39 +86,8 @@ def forward_cm(kc, vc, xq, static_src, static_dest, flags: int = 0, keep_carry: 
     """Returns (out_cm, lse_cm fp32, denom_cm).  ``denom_cm`` is ``lse_cm`` itself in fp32 mode.
     With ``keep_carry`` a fourth value is returned: the decay-prefix table for ``backward_cm(carry=...)``
     (``None`` for shapes whose backward does not use one)."""
-    _require_cuda(kc, vc, xq, static_src, static_dest)
-    lib = _lib.load()
-    b, h, n, c, d = kc.shape
-    r = xq.shape[2]
-    L = n * c
-    dt = xq.dtype
-    code = _dtype_code(dt)
-    kc, vc = kc.contiguous(), vc.contiguous()
-    q = xq.reshape(b, h, r, L, d).contiguous()
-    ss = _gate_cast(static_src.reshape(b, h, L), dt)
-    sd = _gate_cast(static_dest.reshape(b, h, L), dt)
-    if ss.dtype != sd.dtype:
-        ss, sd = ss.float(), sd.float()
-    dims = UaDims(b, h, r, n, c, d)
-    with torch.cuda.device(kc.device):
-        out_cm = torch.empty(b, h, n, r, L, d, dtype=dt, device=kc.device)
-        lse_cm = torch.empty(b, h, n, r, L, dtype=torch.float32, device=kc.device)
-        denom_cm = lse_cm if dt == torch.float32 else torch.empty(b, h, n, r, L, dtype=dt, device=kc.device)
-        ws_bytes = lib.ua_fwd_workspace_bytes(ctypes.byref(dims), code, flags)
-        ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=kc.device)
-        carry = None
-        if keep_carry:
-            cbytes = lib.ua_carry_bytes(ctypes.byref(dims), code, flags)
-            if cbytes:
-                carry = torch.empty(cbytes // 4, dtype=torch.float32, device=kc.device)
-        rc = lib.ua_fwd_keep(ctypes.byref(dims), code, _dtype_code(ss.dtype), _ptr(kc), _ptr(vc), _ptr(q), _ptr(ss), _ptr(sd),
-                             _ptr(out_cm), _ptr(lse_cm), _ptr(None if denom_cm is lse_cm else denom_cm), _ptr(carry),
-                             _ptr(ws), ws_bytes, flags, _stream())
-        _lib.check(rc, "ua_fwd")
-        _check_status(lib, ws, "ua_fwd")
-    if keep_carry:
-        return out_cm, lse_cm, denom_cm, carry
-    return out_cm, lse_cm, denom_cm
+    res = _lib.native().forward_cm(kc, vc, xq, static_src, static_dest, flags, keep_carry)
+    return res if keep_carry else res[:3]
 
 
 def backward_cm(kc, vc, xq, static_src, static_dest, g_out_cm, g_denom_cm, flags: int = 0, carry=None, lse=None, out_cm=None):
@@ -124,48 +96,7 @@ def backward_cm(kc, vc, xq, static_src, static_dest, g_out_cm, g_denom_cm, flags
     ``lse``: the fp32 ``lse_cm (b,h,n,r,L)`` of the same forward (lets the tensor-core backward skip its row max / sum).
     ``out_cm``: the output tiles ``(b,h,n,r,L,d)`` of the same forward, when the caller still holds them (``ua_bwd_saved``:
     the softmax gradient's row term comes from them instead of a sum over the keys)."""
-    _require_cuda(kc, vc, xq, static_src, static_dest, g_out_cm, g_denom_cm)
-    lib = _lib.load()
-    b, h, n, c, d = kc.shape
-    r = xq.shape[2]
-    L = n * c
-    dt = xq.dtype
-    code = _dtype_code(dt)
-    kcc, vcc = kc.contiguous(), vc.contiguous()
-    q = xq.reshape(b, h, r, L, d).contiguous()
-    ss = _gate_cast(static_src.reshape(b, h, L), dt)
-    sd = _gate_cast(static_dest.reshape(b, h, L), dt)
-    if ss.dtype != sd.dtype:
-        ss, sd = ss.float(), sd.float()
-    g_out_cm = g_out_cm.to(dt).contiguous()
-    if g_denom_cm.dtype not in (torch.float32, dt):
-        g_denom_cm = g_denom_cm.float()
-    g_denom_cm = g_denom_cm.contiguous()
-    dims = UaDims(b, h, r, n, c, d)
-    with torch.cuda.device(kc.device):
-        dkc = torch.empty_like(kcc)
-        dvc = torch.empty_like(vcc)
-        dxq = torch.empty_like(q)
-        dss = torch.empty_like(ss)
-        dsd = torch.empty_like(sd)
-        ws_bytes = lib.ua_bwd_workspace_bytes(ctypes.byref(dims), code, flags)
-        ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=kc.device)
-        if carry is not None and carry.numel() * 4 != lib.ua_carry_bytes(ctypes.byref(dims), code, flags):
-            carry = None
-        if lse is not None:
-            if lse.dtype != torch.float32 or tuple(lse.shape) != (b, h, n, r, L) or not lse.is_cuda:
-                raise ValueError("lse must be the fp32 chunk-major (b,h,n,r,L) log-sum-exp of the forward")
-            lse = lse.contiguous()
-        if out_cm is not None and not (out_cm.is_cuda and out_cm.dtype == dt and out_cm.is_contiguous()
-                                       and tuple(out_cm.shape) == (b, h, n, r, L, d)):
-            out_cm = None
-        rc = lib.ua_bwd_saved(ctypes.byref(dims), code, _dtype_code(ss.dtype), _ptr(kcc), _ptr(vcc), _ptr(q), _ptr(ss), _ptr(sd),
-                        _ptr(g_out_cm), _ptr(g_denom_cm), _dtype_code(g_denom_cm.dtype), _ptr(carry), _ptr(lse), _ptr(out_cm),
-                        _ptr(dkc), _ptr(dvc), _ptr(dxq), _ptr(dss), _ptr(dsd), _ptr(ws), ws_bytes, flags, _stream())
-        _lib.check(rc, "ua_bwd")
-        _check_status(lib, ws, "ua_bwd")
-    return (dkc.view(kc.shape), dvc.view(vc.shape), dxq.view(xq.shape),
-            dss.to(static_src.dtype).view(static_src.shape), dsd.to(static_dest.dtype).view(static_dest.shape))
+    return _lib.native().backward_cm(kc, vc, xq, static_src, static_dest, g_out_cm, g_denom_cm, flags, carry, lse, out_cm)
 
 
 def as_reference_out(out_cm):
@@ -180,42 +111,16 @@ def as_reference_denom(denom_cm):
 
 def out_to_chunk_major(t):
     """Reference-shaped out / g_out (b,h,r,L,d,n), any strides -> contiguous (b,h,n,r,L,d)."""
-    v = t.permute(0, 1, 5, 2, 3, 4)
-    return v if v.is_contiguous() else _relayout(t, inner=t.shape[4], to_reference=False)
+    return _lib.native().out_to_chunk_major(t)
 
 
 def denom_to_chunk_major(t):
     """Reference-shaped denom / g_denom (b,h,r,L,n), any strides -> contiguous (b,h,n,r,L)."""
-    v = t.permute(0, 1, 4, 2, 3)
-    return v if v.is_contiguous() else _relayout(t, inner=1, to_reference=False)
+    return _lib.native().denom_to_chunk_major(t)
 
 
 def _relayout(t, inner: int, to_reference: bool):
-    _require_cuda(t)
-    lib = _lib.load()
-    if t.element_size() not in (2, 4):
-        raise TypeError("relayout handles 2- and 4-byte elements")
-    if to_reference:      # t is chunk-major (b,h,n,r,L[,d])
-        b, h, n, r, L = t.shape[:5]
-        src = t.contiguous()
-        dst = torch.empty((b, h, r, L) + ((inner,) if t.dim() == 6 else ()) + (n,), dtype=t.dtype, device=t.device)
-    else:                 # t is reference-shaped (b,h,r,L[,d],n)
-        b, h, r, L = t.shape[:4]
-        n = t.shape[-1]
-        src = t.contiguous()
-        dst = torch.empty((b, h, n, r, L) + ((inner,) if t.dim() == 6 else ()), dtype=t.dtype, device=t.device)
-    dims = UaDims(b, h, r, n, 16, 4)      # chunk/head_dim are not used by the converter; only L = n*chunk matters
-    # the converter takes L through dims: encode L as n_chunks*chunk
-    if L % n:
-        raise ValueError("rows must be a multiple of the number of key chunks")
-    dims.chunk = L // n
-    if dims.chunk % 16:
-        raise ValueError("chunk must be a multiple of 16")
-    with torch.cuda.device(t.device):
-        rc = lib.ua_relayout(ctypes.byref(dims), inner, t.element_size(), 1 if to_reference else 0,
-                             _ptr(src), _ptr(dst), _stream())
-    _lib.check(rc, "ua_relayout")
-    return dst
+    return _lib.native().relayout(t, inner, to_reference)
 
 
 def to_reference_layout(out_cm, denom_cm):
@@ -226,34 +131,12 @@ def to_reference_layout(out_cm, denom_cm):
 
 def merge_fwd_cm(out_cm, lse_cm):
     """SMVecMatMul forward on chunk-major storage -> merged (b,h,r,L,d)."""
-    _require_cuda(out_cm, lse_cm)
-    lib = _lib.load()
-    b, h, n, r, L, d = out_cm.shape
-    dims = UaDims(b, h, r, n, L // n, d)
-    out_cm = out_cm.contiguous()
-    lse_cm = lse_cm.float().contiguous()
-    merged = torch.empty(b, h, r, L, d, dtype=out_cm.dtype, device=out_cm.device)
-    with torch.cuda.device(out_cm.device):
-        rc = lib.ua_merge_fwd(ctypes.byref(dims), _dtype_code(out_cm.dtype), _ptr(out_cm), _ptr(lse_cm), _ptr(merged), _stream())
-    _lib.check(rc, "ua_merge_fwd")
-    return merged
+    return _lib.native().merge_fwd_cm(out_cm, lse_cm, False)[0]
 
 
 def merge_fwd_stats_cm(out_cm, lse_cm):
     """``merge_fwd_cm`` that also returns the fp32 log-sum-exp of every row over ALL key chunks, (b,h,r,L)."""
-    _require_cuda(out_cm, lse_cm)
-    lib = _lib.load()
-    b, h, n, r, L, d = out_cm.shape
-    dims = UaDims(b, h, r, n, L // n, d)
-    out_cm = out_cm.contiguous()
-    lse_cm = lse_cm.float().contiguous()
-    merged = torch.empty(b, h, r, L, d, dtype=out_cm.dtype, device=out_cm.device)
-    row_lse = torch.empty(b, h, r, L, dtype=torch.float32, device=out_cm.device)
-    with torch.cuda.device(out_cm.device):
-        rc = lib.ua_merge_fwd_stats(ctypes.byref(dims), _dtype_code(out_cm.dtype), _ptr(out_cm), _ptr(lse_cm), _ptr(merged),
-                                    _ptr(row_lse), _stream())
-    _lib.check(rc, "ua_merge_fwd_stats")
-    return merged, row_lse
+    return _lib.native().merge_fwd_cm(out_cm, lse_cm, True)
 
 
 def forward_merged_lowmem(kc, vc, xq, static_src, static_dest):
@@ -347,21 +230,7 @@ def merge_bwd_cm(out_cm, lse_cm, g_merged, skip_zero_weight_blocks: bool = False
     """SMVecMatMul backward on chunk-major storage -> (g_out_cm, g_lse_cm fp32).
     ``skip_zero_weight_blocks``: leave the blocks whose merge weight is exactly zero unwritten
     (only valid when the consumer never reads them: backward with masked-block gradients skipped)."""
-    _require_cuda(out_cm, lse_cm, g_merged)
-    lib = _lib.load()
-    b, h, n, r, L, d = out_cm.shape
-    dims = UaDims(b, h, r, n, L // n, d)
-    out_cm = out_cm.contiguous()
-    lse_cm = lse_cm.float().contiguous()
-    g_merged = g_merged.to(out_cm.dtype).contiguous()
-    g_out_cm = torch.empty_like(out_cm)
-    g_lse_cm = torch.empty_like(lse_cm)
-    with torch.cuda.device(out_cm.device):
-        rc = lib.ua_merge_bwd(ctypes.byref(dims), _dtype_code(out_cm.dtype), _ptr(out_cm), _ptr(lse_cm), _ptr(g_merged),
-                              _ptr(g_out_cm), _ptr(g_lse_cm),
-                              _lib.FLAG_SKIP_MASKED_FILL if skip_zero_weight_blocks else 0, _stream())
-    _lib.check(rc, "ua_merge_bwd")
-    return g_out_cm, g_lse_cm
+    return _lib.native().merge_bwd_cm(out_cm, lse_cm, g_merged, skip_zero_weight_blocks)
 
 
 # ---- sequence-chunk sharding: forward / backward over a range of row tiles ---------------------------
@@ -534,24 +403,4 @@ def decode_step(t, k_cache, v_cache, src_cache, q_t, dest_t, decay_state, chunk)
     are the new row; ``decay_state (b,h,L_cap)`` fp32 is updated in place (zeros before ``t = 0``).  Returns
     ``(out_t (b,h,r,d,n_t), lse_t (b,h,r,n_t) fp32)`` as views with the key-chunk index last, i.e. row ``t`` of the
     operator's ``out`` / ``denom`` restricted to the ``n_t = t // chunk + 1`` chunks that hold keys ``<= t``."""
-    _require_cuda(k_cache, v_cache, src_cache, q_t, dest_t, decay_state)
-    lib = _lib.load()
-    b, h, Lcap, d = k_cache.shape
-    r = q_t.shape[2]
-    dt = q_t.dtype
-    assert decay_state.dtype == torch.float32 and decay_state.is_contiguous() and decay_state.shape == (b, h, Lcap)
-    assert k_cache.is_contiguous() and v_cache.is_contiguous() and Lcap % chunk == 0
-    src = _gate_cast(src_cache, dt).contiguous()
-    dst = _gate_cast(dest_t, dt).contiguous()
-    if src.dtype != dst.dtype:
-        src, dst = src.float(), dst.float()
-    nt = t // chunk + 1
-    dims = UaDims(b, h, r, Lcap // chunk, chunk, d)
-    with torch.cuda.device(k_cache.device):
-        out = torch.empty(b, h, nt, r, d, dtype=dt, device=k_cache.device)
-        lse = torch.empty(b, h, nt, r, dtype=torch.float32, device=k_cache.device)
-        rc = lib.ua_decode_step(ctypes.byref(dims), _dtype_code(dt), _dtype_code(src.dtype), int(t), _ptr(k_cache), _ptr(v_cache),
-                                _ptr(src), _ptr(q_t.contiguous()), _ptr(dst), _ptr(decay_state), _ptr(out), _ptr(lse), _stream())
-    _lib.check(rc, "ua_decode_step")
-    return out.permute(0, 1, 3, 4, 2), lse.permute(0, 1, 3, 2)
-
+    return _lib.native().decode_step(t, k_cache, v_cache, src_cache, q_t, dest_t, decay_state, chunk)
