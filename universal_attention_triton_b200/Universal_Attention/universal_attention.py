@@ -14,13 +14,24 @@ from .. import universal_attention_autograd as _ua
 
 class UniversalAttention(Function):
     @staticmethod
-    def forward(kc, vc, xq, static_src, static_dest):
+    def _check(kc, vc, xq, static_src, static_dest):
         b, h, r, _n, _c, d = xq.shape
         _, _, n_, c_, _ = kc.shape
         assert kc.shape == (b, h, n_, c_, d)
         assert vc.shape == (b, h, n_, c_, d)
         assert static_src.shape == (b, h, n_, c_)
         assert static_dest.shape == (b, h, _n, _c)
+
+    @classmethod
+    def apply(cls, kc, vc, xq, static_src, static_dest):
+        if _ua._transforms_active():
+            return super().apply(kc, vc, xq, static_src, static_dest)
+        cls._check(kc, vc, xq, static_src, static_dest)
+        return _ua._apply(kc, vc, xq, static_src, static_dest)
+
+    @staticmethod
+    def forward(kc, vc, xq, static_src, static_dest):
+        UniversalAttention._check(kc, vc, xq, static_src, static_dest)
         return _ua._forward(kc, vc, xq, static_src, static_dest)
 
     @staticmethod

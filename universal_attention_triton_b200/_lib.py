@@ -108,7 +108,21 @@ def native():
         from .ops import plain
         _ua_torch.bind(UaLibraryError, plain)
         _native = _ua_torch
+        for f in _on_native:
+            f(_native)
+        _on_native.clear()
     return _native
+
+
+_on_native = []
+
+
+def on_native(f):
+    """Runs ``f(module)`` on the extension module: now if it is loaded, else as soon as it is (a setting made before)."""
+    if _native is not None:
+        f(_native)
+    else:
+        _on_native.append(f)
 
 
 def check(code: int, what: str):

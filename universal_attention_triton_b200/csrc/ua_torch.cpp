@@ -4,10 +4,15 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <optional>
 #include <string>
 #include <tuple>
@@ -25,6 +30,7 @@ py::handle g_error;      // _lib.UaLibraryError
 py::handle g_unwrap;     // ops.plain: takes functorch's wrappers off a tensor
 
 [[noreturn]] void raise(py::handle type, const std::string& msg) {
+  const py::gil_scoped_acquire gil;
   PyErr_SetString(type.ptr(), msg.c_str());
   throw py::error_already_set();
 }
@@ -291,6 +297,193 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> prepare_inputs_bwd(const OptTensor& g
   return {dq, dk, dv, dg};
 }
 
+// ---- autograd nodes ------------------------------------------------------------------------------------------------------
+// The graph nodes behind ``UniversalAttention.apply``, ``SMVecMatMul.apply`` and ``prepare_inputs`` in eager mode.  They do what
+// the Python Functions of the same names do (forward, save, backward; those remain for functorch's transforms), without the
+// interpreter between the engine and the kernels: a Python node costs 35-60 us of host time each way.
+using torch::autograd::SavedVariable;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+bool g_strict_masked_grads = true;      // universal_attention_autograd.set_strict_masked_grads
+
+// Notes on gradient tensors whose part for the rows before each chunk is exactly zero (see _mark_masked_zero there): the tensor
+// itself, by weak reference, and its version counter, so that an in-place change voids the note and a tensor that autograd
+// builds from it does not carry it.  The last 64 are kept; a note that fell out only costs the shortcut.
+class MaskedZeroNotes {
+ public:
+  void add(const Tensor& t) {
+    const std::lock_guard<std::mutex> lock(m_);
+    slots_[next_++ % kSlots] = Note{c10::weak_intrusive_ptr<c10::TensorImpl>(t.getIntrusivePtr()), t._version()};
+  }
+  bool has(const Tensor& t) {
+    const std::lock_guard<std::mutex> lock(m_);
+    for (auto& n : slots_)
+      if (n && n->impl._unsafe_get_target() == t.unsafeGetTensorImpl() && !n->impl.expired()) return n->version == (uint32_t)t._version();
+    return false;
+  }
+ private:
+  static constexpr size_t kSlots = 64;
+  struct Note { c10::weak_intrusive_ptr<c10::TensorImpl> impl; uint32_t version; };
+  std::mutex m_;
+  std::optional<Note> slots_[kSlots];
+  size_t next_ = 0;
+};
+MaskedZeroNotes& notes() {
+  static auto* n = new MaskedZeroNotes;
+  return *n;
+}
+
+template <typename... Ts> bool wants_grad(const Ts&... ts) { return at::GradMode::is_enabled() && (ts.requires_grad() || ...); }
+template <typename N, typename... Ts> std::shared_ptr<N> make_node(const Ts&... ts) {
+  std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
+  n->set_next_edges(torch::autograd::collect_next_edges(ts...));
+  return n;
+}
+// errors of the calls above are Python exceptions: the engine's threads hold no interpreter lock when they run a node
+template <typename F> auto with_python(F f) {
+  try {
+    return f();
+  } catch (py::error_already_set& e) {
+    const py::gil_scoped_acquire gil;
+    throw std::runtime_error(e.what());
+  }
+}
+
+struct UaNode : torch::autograd::Node {
+  SavedVariable kc, vc, xq, ss, sd, lse, carry, out;
+  bool has_carry = false, has_out = false;
+  at::DimVector out_sizes, denom_sizes;
+  at::TensorOptions out_opt;
+  std::string name() const override { return "UniversalAttentionBackward"; }
+  void release_variables() override {
+    for (SavedVariable* v : {&kc, &vc, &xq, &ss, &sd, &lse, &carry, &out}) v->reset_data();
+  }
+  variable_list apply(variable_list&& g) override {
+    return with_python([&] {
+      const at::AutoDispatchBelowADInplaceOrView below;
+      const bool zero = g[0].defined() && g[1].defined() && notes().has(g[0]) && notes().has(g[1]);
+      const int flags = (g_strict_masked_grads && !zero) ? 0 : UA_FLAG_SKIP_MASKED_GRADS;
+      const Tensor g_out = out_to_chunk_major(g[0].defined() ? g[0] : at::zeros(out_sizes, out_opt));
+      const Tensor g_den = denom_to_chunk_major(g[1].defined() ? g[1] : at::zeros(denom_sizes, out_opt));
+      OptTensor c, o;
+      if (has_carry) c = carry.unpack();
+      if (has_out) o = out.unpack(shared_from_this()).permute({0, 1, 5, 2, 3, 4});      // the chunk-major storage behind the view
+      auto [a, b, d, e, f] = backward_cm(kc.unpack(), vc.unpack(), xq.unpack(), ss.unpack(), sd.unpack(), g_out, g_den, flags, c, lse.unpack(), o);
+      return variable_list{a, b, d, e, f};
+    });
+  }
+};
+
+std::tuple<Tensor, Tensor> ua_apply(const Tensor& kc, const Tensor& vc, const Tensor& xq, const Tensor& ss, const Tensor& sd, bool reference_layout,
+                                    bool save_output) {
+  const bool grad = wants_grad(kc, vc, xq, ss, sd);
+  Tensor out, denom, lse;
+  OptTensor carry;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    Tensor out_cm, denom_cm;
+    std::tie(out_cm, lse, denom_cm, carry) = forward_cm(kc, vc, xq, ss, sd, 0, grad);
+    if (reference_layout) {
+      out = relayout(out_cm, out_cm.size(5), true);
+      denom = relayout(denom_cm, 1, true);
+    } else {
+      out = as_reference_out(out_cm);
+      denom = as_reference_denom(denom_cm);
+    }
+  }
+  if (grad) {
+    auto n = make_node<UaNode>(kc, vc, xq, ss, sd);
+    n->kc = SavedVariable(kc, false); n->vc = SavedVariable(vc, false); n->xq = SavedVariable(xq, false);
+    n->ss = SavedVariable(ss, false); n->sd = SavedVariable(sd, false); n->lse = SavedVariable(lse, false);
+    if ((n->has_carry = carry.has_value())) n->carry = SavedVariable(*carry, false);
+    n->out_sizes = out.sizes(); n->denom_sizes = denom.sizes(); n->out_opt = out.options();
+    torch::autograd::set_history(out, n);
+    torch::autograd::set_history(denom, n);
+    if ((n->has_out = save_output && !reference_layout)) n->out = SavedVariable(out, true);
+  }
+  return {out, denom};
+}
+
+struct MergeNode : torch::autograd::Node {
+  SavedVariable mat, vec;
+  std::string name() const override { return "SMVecMatMulBackward"; }
+  void release_variables() override { mat.reset_data(); vec.reset_data(); }
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return variable_list(2);
+    return with_python([&] {
+      const at::AutoDispatchBelowADInplaceOrView below;
+      const Tensor m = mat.unpack(), v = vec.unpack();
+      auto [g_out, g_lse] = merge_bwd_cm(out_to_chunk_major(m), denom_to_chunk_major(v), g[0], !g_strict_masked_grads);
+      Tensor a = as_reference_out(g_out), b = as_reference_denom(g_lse);
+      if (b.scalar_type() != v.scalar_type()) b = b.to(v.scalar_type());
+      notes().add(a);
+      notes().add(b);
+      return variable_list{a, b};
+    });
+  }
+};
+
+Tensor merge_apply(const Tensor& mat, const Tensor& vec) {
+  const bool grad = wants_grad(mat, vec);
+  Tensor merged;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    merged = std::get<0>(merge_fwd_cm(out_to_chunk_major(mat), denom_to_chunk_major(vec), false));
+  }
+  if (grad) {
+    auto n = make_node<MergeNode>(mat, vec);
+    n->mat = SavedVariable(mat, false); n->vec = SavedVariable(vec, false);
+    torch::autograd::set_history(merged, n);
+  }
+  return merged;
+}
+
+struct PrepareNode : torch::autograd::Node {
+  SavedVariable kc, src, dest, norm;
+  bool has_norm = false;
+  int64_t heads = 0;
+  int flags = 0;
+  at::DimVector shapes[4];
+  std::string name() const override { return "_PrepareInputsBackward"; }
+  void release_variables() override {
+    for (SavedVariable* v : {&kc, &src, &dest, &norm}) v->reset_data();
+  }
+  variable_list apply(variable_list&& g) override {
+    return with_python([&] {
+      const at::AutoDispatchBelowADInplaceOrView below;
+      auto opt = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
+      OptTensor nrm;
+      if (has_norm) nrm = norm.unpack();
+      const auto self = shared_from_this();
+      auto [a, b, c, d] = prepare_inputs_bwd(opt(g[0]), opt(g[1]), opt(g[2]), opt(g[3]), opt(g[4]), kc.unpack(self), src.unpack(self), dest.unpack(self),
+                                             nrm, heads, flags);
+      return variable_list{a.view(shapes[0]), b.view(shapes[1]), c.view(shapes[2]), d.view(shapes[3])};
+    });
+  }
+};
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> prepare_apply(const Tensor& qs, const Tensor& ks, const Tensor& vs, const Tensor& gs, int64_t chunk,
+                                                                 int flags) {
+  const bool grad = wants_grad(qs, ks, vs, gs);
+  Tensor kc, vc, xq, src, dest;
+  OptTensor norm;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    std::tie(kc, vc, xq, src, dest, norm) = prepare_inputs(qs, ks, vs, gs, chunk, flags);
+  }
+  if (grad) {
+    auto n = make_node<PrepareNode>(qs, ks, vs, gs);
+    n->heads = qs.size(2); n->flags = flags;
+    const Tensor* in[4] = {&qs, &ks, &vs, &gs};
+    for (int i = 0; i < 4; ++i) n->shapes[i] = in[i]->sizes();
+    for (Tensor* t : {&kc, &vc, &xq, &src, &dest}) torch::autograd::set_history(*t, n);
+    n->kc = SavedVariable(kc, true); n->src = SavedVariable(src, true); n->dest = SavedVariable(dest, true);
+    if ((n->has_norm = norm.has_value())) n->norm = SavedVariable(*norm, false);
+  }
+  return {kc, vc, xq, src, dest};
+}
+
 // Under a functorch transform every at:: call would wrap its result again; these functions work on plain tensors throughout.
 template <typename R, typename... A>
 auto outside_functorch(R (*f)(A...)) {
@@ -306,6 +499,10 @@ auto outside_functorch(R (*f)(A...)) {
 
 PYBIND11_MODULE(_ua_torch, m) {
   m.def("bind", [](py::object error, py::object unwrap) { g_error = error.release(); g_unwrap = unwrap.release(); });
+  m.def("set_strict_masked_grads", [](bool on) { g_strict_masked_grads = on; });
+  m.def("ua_apply", &ua_apply);
+  m.def("merge_apply", &merge_apply);
+  m.def("prepare_apply", &prepare_apply);
   m.def("forward_cm", outside_functorch(&forward_cm));
   m.def("backward_cm", outside_functorch(&backward_cm));
   m.def("merge_fwd_cm", outside_functorch(&merge_fwd_cm));

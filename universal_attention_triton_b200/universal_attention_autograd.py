@@ -89,6 +89,7 @@ def set_strict_masked_grads(on: bool) -> None:
     consumes ``(out, denom)``; it is not for arbitrary upstream gradients."""
     global _STRICT_MASKED_GRADS
     _STRICT_MASKED_GRADS = bool(on)
+    _lib.on_native(lambda m: m.set_strict_masked_grads(_STRICT_MASKED_GRADS))
 
 
 def _forward(kc, vc, xq, static_src, static_dest):
@@ -139,6 +140,15 @@ def _masked_zero(t) -> bool:
     return v is not None and v == t._version
 
 
+_transforms_active = torch._C._are_functorch_transforms_active
+
+
+def _apply(kc, vc, xq, static_src, static_dest):
+    """``apply`` of the operator's Functions in eager mode: the same forward, saved tensors and backward as a graph node in
+    native code (``csrc/ua_torch.cpp``); functorch's transforms take the Python protocol."""
+    return _lib.native().ua_apply(kc, vc, xq, static_src, static_dest, _OUTPUT_LAYOUT == "reference", _SAVE_OUTPUT)
+
+
 def _backward(ctx, g_out, g_denom):
     # Upstream gradients that are known to vanish on the rows before each chunk contribute nothing there: the kernels of
     # those rows are skipped, with the same result.  Anything else takes the full path (unless strict mode is off).
@@ -167,13 +177,24 @@ class UniversalAttention(Function):
     (universal_attention_autograd.py:9, :41-44, :47)."""
 
     @staticmethod
-    def forward(kc, vc, xq, static_src, static_dest):
+    def _check(kc, vc, xq, static_src, static_dest):
         b, h, r, l, d = xq.shape
         _, _, n, c, _ = kc.shape
         assert kc.shape == (b, h, n, c, d) and n * c == l
         assert vc.shape == (b, h, n, c, d)
         assert static_src.shape == (b, h, n, c)
         assert static_dest.shape == (b, h, l)
+
+    @classmethod
+    def apply(cls, kc, vc, xq, static_src, static_dest):
+        if _transforms_active():
+            return super().apply(kc, vc, xq, static_src, static_dest)
+        cls._check(kc, vc, xq, static_src, static_dest)
+        return _apply(kc, vc, xq, static_src, static_dest)
+
+    @staticmethod
+    def forward(kc, vc, xq, static_src, static_dest):
+        UniversalAttention._check(kc, vc, xq, static_src, static_dest)
         return _forward(kc, vc, xq, static_src, static_dest)
 
     @staticmethod
@@ -191,13 +212,24 @@ class UniversalAttention2(Function):
     (universal_attention_autograd.py:104, :166-169, :172)."""
 
     @staticmethod
-    def forward(kc, vc, xq, static_src, static_dest):
+    def _check(kc, vc, xq, static_src, static_dest):
         b, h, r, _n, _c, d = xq.shape
         _, _, n_, c_, _ = kc.shape
         assert kc.shape == (b, h, n_, c_, d) and n_ * c_ == _n * _c
         assert vc.shape == (b, h, n_, c_, d)
         assert static_src.shape == (b, h, n_, c_)
         assert static_dest.shape == (b, h, _n, _c)
+
+    @classmethod
+    def apply(cls, kc, vc, xq, static_src, static_dest):
+        if _transforms_active():
+            return super().apply(kc, vc, xq, static_src, static_dest)
+        cls._check(kc, vc, xq, static_src, static_dest)
+        return _apply(kc, vc, xq, static_src, static_dest)
+
+    @staticmethod
+    def forward(kc, vc, xq, static_src, static_dest):
+        UniversalAttention2._check(kc, vc, xq, static_src, static_dest)
         return _forward(kc, vc, xq, static_src, static_dest)
 
     @staticmethod
@@ -214,8 +246,19 @@ class SMVecMatMul(Function):
     Takes the 6-D ``out`` and 5-D ``denom`` of the operator (any strides)."""
 
     @staticmethod
-    def forward(mat, vec):
+    def _check(mat, vec):
         assert mat.dim() == 6 and vec.dim() == 5 and mat.shape[:4] == vec.shape[:4] and mat.shape[-1] == vec.shape[-1]
+
+    @classmethod
+    def apply(cls, mat, vec):
+        if _transforms_active():
+            return super().apply(mat, vec)
+        cls._check(mat, vec)
+        return _lib.native().merge_apply(mat, vec)
+
+    @staticmethod
+    def forward(mat, vec):
+        SMVecMatMul._check(mat, vec)
         return ops.merge_fwd_cm(ops.out_to_chunk_major(mat), ops.denom_to_chunk_major(vec))
 
     @staticmethod
