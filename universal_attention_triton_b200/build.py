@@ -11,11 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libua_b200.so")
-SOURCES = ["ua_api.cu"]
+SOURCES = ["ua_bwd.cu", "ua_fwd.cu", "ua_api.cu"]      # compiled side by side
 # the tensor plumbing above the library: an extension module, host code only
 TORCH_SOURCE = "ua_torch.cpp"
 TORCH_PATH = os.path.join(PKG_DIR, "_ua_torch.so")
@@ -24,7 +26,7 @@ TOOL_SOURCE = "mma_timing.cu"
 TOOL_PATH = os.path.join(PKG_DIR, "mma_timing.bin")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared",
+    "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
 ]
 
 
@@ -33,6 +35,14 @@ def _nvcc() -> str:
     if not os.path.exists(exe):
         raise RuntimeError("nvcc not found; the CUDA library cannot be built")
     return exe
+
+
+def _run(cmd):
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("failed: " + " ".join(cmd[:1] + cmd[-4:]))
+    return res
 
 
 def _stale() -> bool:
@@ -48,13 +58,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     """Compile the library if it is missing or older than its sources; returns its path."""
     if not force and not _stale():
         return LIB_PATH
-    cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
-    cmd += [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB_PATH, "-lcuda"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed building libua_b200.so")
+    with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor() as pool:
+        objs = [os.path.join(tmp, src + ".o") for src in SOURCES]
+        extra = ["-Xptxas", "-v"] if verbose else []
+        for res in pool.map(lambda so: _run([_nvcc()] + NVCC_FLAGS + extra + ["-c", os.path.join(CSRC, so[0]), "-o", so[1]]), zip(SOURCES, objs)):
+            if verbose:
+                sys.stderr.write(res.stdout + res.stderr)
+        _run([_nvcc()] + NVCC_FLAGS + ["-shared"] + objs + ["-o", LIB_PATH, "-lcuda"])
     _build_torch_module()
     return LIB_PATH
 
@@ -72,20 +82,14 @@ def _build_torch_module() -> None:
         cmd += ["-isystem", inc]
     cmd += [os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_PATH, "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-L" + torch_lib,
             "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("the C++ compiler failed building _ua_torch.so")
+    _run(cmd)
 
 
 def build_tools() -> str:
     """Compile the stand-alone MMA timing micro-benchmark (run it on a B200: ``./mma_timing.bin 256``)."""
     cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--expt-relaxed-constexpr",
            os.path.join(CSRC, TOOL_SOURCE), "-o", TOOL_PATH, "-lcuda"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("nvcc failed building the MMA timing micro-benchmark")
+    _run(cmd)
     return TOOL_PATH
 
 

@@ -347,7 +347,12 @@ const char* ua_error_string(int code) {
 size_t ua_fwd_workspace_bytes(const UaDims* dims, int dtype, int flags) {
   if (check_dims(dims) == UA_OK) {
     ua::Shape s = to_shape(dims);
-    if (const int m = sub_chunks(s, dtype, flags)) return sub_layout(s, m, false, 256).total;
+    if (const int m = sub_chunks(s, dtype, flags)) {
+      const UaDims sd = sub_dims(dims, m);
+      return sub_layout(s, m, false, ua_fwd_workspace_bytes(&sd, dtype, flags)).total;
+    }
+    if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::fwd_supported(s, dtype) && ua::sm100::fwd_split(s))
+      return 256 + ua::sm100::fwd_totals_bytes(s);      // status word, tile totals of the segmented sweep
   }
   return 256;   // status word
 }
@@ -393,14 +398,15 @@ int ua_fwd_keep(const UaDims* dims, int dtype, int gate_dtype, const void* kc, c
   ua::Shape s = to_shape(dims);
   if (const int m = sub_chunks(s, dtype, flags)) {
     // sub-chunks of 128 keys, then the merge inside each chunk (see sub_chunks)
-    const SubWorkspace w = sub_layout(s, m, false, 256);
+    const UaDims sd = sub_dims(dims, m), gd = group_dims(dims, m);
+    const size_t inner = ua_fwd_workspace_bytes(&sd, dtype, flags);
+    const SubWorkspace w = sub_layout(s, m, false, inner);
     if (workspace_bytes < w.total) return UA_ERR_WORKSPACE;
     char* ws = static_cast<char*>(workspace);
-    const UaDims sd = sub_dims(dims, m), gd = group_dims(dims, m);
     void* out_sub = ws + w.off_out;
     float* lse_sub = reinterpret_cast<float*>(ws + w.off_lse);
     if ((e = ua_fwd_keep(&sd, dtype, gate_dtype, kc, vc, xq, static_src, static_dest, out_sub, lse_sub, nullptr, carry_out, workspace,
-                         256, flags & ~UA_FLAG_SKIP_MASKED_FILL, stream)))
+                         inner, flags & ~UA_FLAG_SKIP_MASKED_FILL, stream)))
       return e;
     if ((e = ua_merge_fwd_stats(&gd, dtype, out_sub, lse_sub, out_cm, lse_cm, stream))) return e;
     if (denom_cm) e = convert_any(dtype, lse_cm, denom_cm, (size_t)s.B * s.H * s.N * s.R * s.L, st);
@@ -415,7 +421,10 @@ int ua_fwd_keep(const UaDims* dims, int dtype, int gate_dtype, const void* kc, c
     fp.status = static_cast<int*>(workspace);
     fp.carry = ua_carry_bytes(dims, dtype, flags) ? static_cast<float*>(carry_out) : nullptr;
     ua::sm100::whole_sequence(fp);
-    return ua::sm100::launch_fwd<false>(s, gate_dtype, kc, vc, xq, fp, !(flags & UA_FLAG_SKIP_MASKED_FILL), st);
+    // (a caller whose workspace is from before the sweeps could be cut gets whole sweeps)
+    float* totals = workspace_bytes >= ua_fwd_workspace_bytes(dims, dtype, flags) && ua_fwd_workspace_bytes(dims, dtype, flags) > 256
+                        ? reinterpret_cast<float*>(static_cast<char*>(workspace) + 256) : nullptr;
+    return ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, !(flags & UA_FLAG_SKIP_MASKED_FILL), totals, st);
   }
 
   ua::simt::FwdParams p;
@@ -462,7 +471,7 @@ int ua_fwd_rows_keep(const UaDims* dims, int dtype, int gate_dtype, const UaRows
   if (!aligned16(kc) || !aligned16(vc) || !aligned16(xq_rows) || !aligned16(out_cm_rows)) return UA_ERR_ALIGNMENT;
   if (!workspace || workspace_bytes < 256 || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
   ua::Shape s = to_shape(dims);
-  if ((e = check_rows(s, ua::sm100::fwd_supported(s, dtype), rows))) return e;
+  if ((e = check_rows(s, ua::sm100::fwd_supported(s, dtype) && ua::sm100::chunk128(s), rows))) return e;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(workspace, 0, 256, st) != cudaSuccess) return UA_ERR_CUDA;
   ua::sm100::FwdParams fp{};
@@ -471,7 +480,7 @@ int ua_fwd_rows_keep(const UaDims* dims, int dtype, int gate_dtype, const UaRows
   fp.status = static_cast<int*>(workspace); fp.carry = carry_table_out;
   fp.j_begin = rows->tile_begin; fp.j_end = rows->tile_end; fp.Lr = rows->rows_total; fp.r0 = rows->row_offset;
   fp.carry_in = carry_in; fp.total_out = nullptr;
-  return ua::sm100::launch_fwd<false>(s, gate_dtype, kc, vc, xq_rows, fp, !(flags & UA_FLAG_SKIP_MASKED_FILL), st);
+  return ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq_rows, fp, !(flags & UA_FLAG_SKIP_MASKED_FILL), nullptr, st);
 }
 
 int ua_decay_totals_rows(const UaDims* dims, int dtype, int gate_dtype, const UaRows* rows, const void* kc,
@@ -484,7 +493,7 @@ int ua_decay_totals_rows(const UaDims* dims, int dtype, int gate_dtype, const Ua
   if (!aligned16(kc)) return UA_ERR_ALIGNMENT;
   if (!workspace || workspace_bytes < 256 || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
   ua::Shape s = to_shape(dims);
-  if ((e = check_rows(s, ua::sm100::fwd_supported(s, dtype), rows))) return e;
+  if ((e = check_rows(s, ua::sm100::fwd_supported(s, dtype) && ua::sm100::chunk128(s), rows))) return e;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(workspace, 0, 256, st) != cudaSuccess) return UA_ERR_CUDA;
   ua::sm100::FwdParams fp{};
@@ -492,7 +501,7 @@ int ua_decay_totals_rows(const UaDims* dims, int dtype, int gate_dtype, const Ua
   fp.status = static_cast<int*>(workspace); fp.carry = nullptr;
   fp.j_begin = rows->tile_begin; fp.j_end = rows->tile_end; fp.Lr = rows->rows_total; fp.r0 = rows->row_offset;
   fp.carry_in = carry_in; fp.total_out = total_out;
-  return ua::sm100::launch_fwd<true>(s, gate_dtype, kc, nullptr, nullptr, fp, false, st);
+  return ua::sm100::launch_fwd_carry(s, gate_dtype, kc, fp, st);
 }
 
 size_t ua_bwd_rows_workspace_bytes(const UaDims* dims, int dtype) {
@@ -570,7 +579,7 @@ int ua_bwd_rows_kept(const UaDims* dims, int dtype, int gate_dtype, const UaRows
     fp.status = status; fp.carry = tab;
     fp.j_begin = rows->tile_begin; fp.j_end = rows->tile_end; fp.Lr = rows->rows_total; fp.r0 = rows->row_offset;
     fp.carry_in = carry_in; fp.total_out = nullptr;
-    if ((e = ua::sm100::launch_fwd<false>(s, gate_dtype, kc, vc, xq_rows, fp, false, st))) return e;
+    if ((e = ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq_rows, fp, false, nullptr, st))) return e;
   }
   const float* gd32 = static_cast<const float*>(g_denom_cm_rows);
   if (g_denom_dtype != UA_F32) {
@@ -718,8 +727,8 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
       fp.status = reinterpret_cast<int*>(ws);
       fp.carry = carry_in ? nullptr : carry_tab;
       ua::sm100::whole_sequence(fp);
-      if (lse) e = ua::sm100::launch_fwd<true>(s, gate_dtype, kc, nullptr, nullptr, fp, false, st);      // decay-only pass
-      else e = ua::sm100::launch_fwd<false>(s, gate_dtype, kc, vc, xq, fp, false, st);
+      if (lse) e = ua::sm100::launch_fwd_carry(s, gate_dtype, kc, fp, st);      // decay-only pass
+      else e = ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, false, nullptr, st);
       if (e) return e;
       if (!lse) lse = fp.lse;
     }
@@ -997,7 +1006,7 @@ int ua_merge_fwd_stats(const UaDims* dims, int dtype, const void* out_cm, const 
 size_t ua_fwd_merged_workspace_bytes(const UaDims* dims, int dtype) {
   if (check_dims(dims) != UA_OK) return 0;
   ua::Shape s = to_shape(dims);
-  if (!ua::sm100::fwd_supported(s, dtype)) return 0;
+  if (!ua::sm100::fwd_supported(s, dtype) || !ua::sm100::chunk128(s)) return 0;
   const size_t BH = (size_t)s.B * s.H;
   return 256 + align_up(BH * s.N * (size_t)s.R * s.L * sizeof(float), 256) + align_up(BH * s.R * (size_t)s.L * s.D * sizeof(float), 256);
 }
@@ -1011,7 +1020,7 @@ int ua_fwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
   if (!kc || !vc || !xq || !static_src || !static_dest || !merged || !row_lse) return UA_ERR_NULL_POINTER;
   if (!aligned16(kc) || !aligned16(vc) || !aligned16(xq) || !aligned16(merged)) return UA_ERR_ALIGNMENT;
   ua::Shape s = to_shape(dims);
-  if (!ua::sm100::fwd_supported(s, dtype)) return UA_ERR_UNSUPPORTED;
+  if (!ua::sm100::fwd_supported(s, dtype) || !ua::sm100::chunk128(s)) return UA_ERR_UNSUPPORTED;
   const size_t need = ua_fwd_merged_workspace_bytes(dims, dtype);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1027,7 +1036,7 @@ int ua_fwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
   fp.status = reinterpret_cast<int*>(ws);
   fp.carry = ua_carry_bytes(dims, dtype, 0) ? static_cast<float*>(carry_out) : nullptr;
   ua::sm100::whole_sequence(fp);
-  if ((e = ua::sm100::launch_fwd<false>(s, gate_dtype, kc, vc, xq, fp, false, st))) return e;
+  if ((e = ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, false, nullptr, st))) return e;
   // the row's log-sum-exp over all key chunks
   row_lse_kernel<<<148 * 8, 256, 0, st>>>(lse_cm, row_lse, BH, s.N, s.R, s.L);
   if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
@@ -1085,7 +1094,7 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
     fp.s = s; fp.ssrc = static_src; fp.sdest = static_dest; fp.out = nullptr; fp.lse = nullptr; fp.denom = nullptr;
     fp.status = reinterpret_cast<int*>(ws); fp.carry = carry_tab;
     ua::sm100::whole_sequence(fp);
-    if ((e = ua::sm100::launch_fwd<true>(s, gate_dtype, kc, nullptr, nullptr, fp, false, st))) return e;
+    if ((e = ua::sm100::launch_fwd_carry(s, gate_dtype, kc, fp, st))) return e;
   }
   ua::sm100::Bwd2Params qp{};
   if (!aligned16(row_lse) || !aligned16(row_delta) || !aligned16(static_dest) || !aligned16(carry_tab)) return UA_ERR_ALIGNMENT;

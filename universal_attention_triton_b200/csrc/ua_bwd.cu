@@ -1,0 +1,116 @@
+// Launchers of the tensor-core backward.
+#include <cstdlib>
+
+#include "ua_sm100_host.cuh"
+
+namespace ua {
+namespace sm100 {
+namespace {
+
+// Columns of a half tile per worker thread: 16 (sixteen worker warps, 96 registers each) at head_dim 64, 32 (eight worker
+// warps, ~200 registers each) at head_dim 128.  At head_dim 64 sixteen warps (four per scheduler hide the TMEM and
+// shared-memory latencies) that hand dS over at once are 5-6 % faster than eight that defer the tail of a head, in every
+// build; sixteen that defer are slower than either (measured).
+#ifndef UA_BWD2_COLS_64
+#define UA_BWD2_COLS_64 16
+#endif
+#ifndef UA_BWD2_COLS_128
+#define UA_BWD2_COLS_128 32
+#endif
+template <int D> constexpr int bwd2_cols() { return D == 64 ? UA_BWD2_COLS_64 : UA_BWD2_COLS_128; }
+
+// Backward over the row tiles [p.j_begin, p.j_end) (the caller sets the range fields, e.g. with whole_sequence()).
+// With p.heads == 0 (correction pass) xq, g_out and p.acc_dq are not touched and may be null.
+template <int D, typename TG, int kMode>
+int launch_bwd2_t(const Shape& s, const void* kc, const void* vc, const void* xq, const void* g_out, const Bwd2Params& p,
+                  cudaStream_t st) {
+  using Cfg = Bwd2Cfg<D>;
+  CUtensorMap tmK, tmV, tmQ, tmG, tmDQ, tmDK;
+  const uint64_t BH = (uint64_t)s.B * s.H;
+  if (!make_rows_map(&tmK, kc, BH * s.L, D, 64) || !make_rows_map(&tmV, vc, BH * s.L, D, 64) ||
+      !make_f32_rows_map(&tmDK, p.acc_dkr, BH * s.L, D, 64))
+    return UA_ERR_CUDA;
+  if (p.heads == 0) {
+    tmQ = tmK; tmG = tmK; tmDQ = tmDK;       // never used
+  } else if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D, 64) ||
+             !make_rows_map(&tmG, g_out, (kMode == 2 ? BH : BH * s.N) * s.R * p.Lr, D, 64) ||
+             !make_f32_rows_map(&tmDQ, p.acc_dq, BH * s.R * p.Lr, D, 64)) {
+    return UA_ERR_CUDA;
+  }
+  constexpr int kCols = bwd2_cols<D>();
+  auto kern = p.heads > 0 ? bwd2_kernel<D, TG, kMode, kCols, true> : bwd2_kernel<D, TG, kMode, kCols, false>;
+  const int threads = 32 * (8 + 4 * (64 / kCols));
+  // the forward's output tiles at hand (per-chunk form, head_dim 64): the row term comes from them
+  CUtensorMap tmO = tmG;
+  if constexpr (kMode == 1 && Cfg::kOutTiles) {
+    if (p.heads > 0 && p.out_tiles != nullptr) {
+      if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
+      kern = bwd2_kernel<D, TG, 1, kCols, true, true>;
+    }
+  }
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
+  kern<<<(unsigned)(BH * s.N), threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
+  // the row-side dK joins the accumulator; d static_dest of the range's rows comes out of it
+  const int row_begin = p.j_begin * 128, row_end = p.j_end * 128;
+  const long long warps = (long long)BH * (row_end - row_begin);
+  if (warps > 0)
+    row_side_finish_kernel<D, TG><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+        static_cast<const __nv_bfloat16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dt, (int)BH, s.L, p.Lr,
+        p.r0, row_begin, row_end);
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+
+}  // namespace
+
+int launch_bwd2(const Shape& s, int gate_dtype, bool merged, const void* kc, const void* vc, const void* xq,
+                       const void* g_out, const Bwd2Params& p, cudaStream_t st) {
+#define UA_BWD2(D_, TG_) (merged ? launch_bwd2_t<D_, TG_, 2>(s, kc, vc, xq, g_out, p, st) : launch_bwd2_t<D_, TG_, 1>(s, kc, vc, xq, g_out, p, st))
+  if (s.D == 64) return gate_dtype == UA_F32 ? UA_BWD2(64, float) : UA_BWD2(64, __nv_bfloat16);
+  return gate_dtype == UA_F32 ? UA_BWD2(128, float) : UA_BWD2(128, __nv_bfloat16);
+#undef UA_BWD2
+}
+
+namespace {
+// Rows before a chunk over the row tiles [p.j_begin, p.j_end): prep (per-chunk constants), sweep (one pass over the upstream
+// gradient), finish (dK_i, and dV_i for a row range).  The caller has zeroed (or shares) acc_dq / acc_dk / acc_dv.
+template <int D>
+int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* xq, const void* g_out, float* acc_dq, MaskedParams p,
+                    cudaStream_t st) {
+  using Cfg = MkCfg<D>;
+  const uint64_t BH = (uint64_t)s.B * s.H;
+  CUtensorMap tmQ, tmG, tmDQ;
+  if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D) || !make_rows_map(&tmG, g_out, BH * s.N * s.R * p.Lr, D) ||
+      !make_f32_rows_map(&tmDQ, acc_dq, BH * s.R * p.Lr, D))
+    return UA_ERR_CUDA;
+  static const int jp_env = []() { const char* e = getenv("UA_MASKED_TILES"); return e ? atoi(e) : 0; }();
+  p.jp = jp_env > 0 ? jp_env : 8;
+  p.items_per_bh = 0;
+  const int jcap = (s.N - 1 < p.j_end) ? s.N - 1 : p.j_end;      // no row tile at or after the last chunk is before any chunk
+  for (int g = 0; g * Cfg::kG < s.N; ++g) {
+    int jmax = (((g + 1) * Cfg::kG < s.N) ? (g + 1) * Cfg::kG : s.N) - 1;
+    if (jmax > jcap) jmax = jcap;
+    if (jmax > p.j_begin) p.items_per_bh += (jmax - p.j_begin + p.jp - 1) / p.jp;
+  }
+  if (p.items_per_bh == 0) return UA_OK;
+  const auto* k16 = static_cast<const __nv_bfloat16*>(kc);
+  const auto* v16 = static_cast<const __nv_bfloat16*>(vc);
+  const int prep_smem = 2 * MkDense<D>::kTile + 2 * D * 4, finish_smem = MkDense<D>::kTile + D * 4;
+  auto prep = masked_prep_kernel<D>;
+  if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem) != cudaSuccess) return UA_ERR_CUDA;
+  prep<<<(unsigned)(BH * s.N), 256, prep_smem, st>>>(k16, v16, p);
+  auto sweep = masked_sweep_kernel<D>;
+  if (cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
+  sweep<<<(unsigned)(BH * p.items_per_bh * Cfg::kKB), 384, Cfg::kSmemBytes, st>>>(tmQ, tmG, tmDQ, p);
+  masked_finish_kernel<D><<<(unsigned)(BH * s.N), 256, finish_smem, st>>>(v16, p);      // (at most 35 KB: no opt-in needed)
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+
+}  // namespace
+
+int launch_masked(const Shape& s, const void* kc, const void* vc, const void* xq, const void* g_out, float* acc_dq,
+                         const MaskedParams& p, cudaStream_t st) {
+  return s.D == 64 ? launch_masked_t<64>(s, kc, vc, xq, g_out, acc_dq, p, st) : launch_masked_t<128>(s, kc, vc, xq, g_out, acc_dq, p, st);
+}
+
+}  // namespace sm100
+}  // namespace ua

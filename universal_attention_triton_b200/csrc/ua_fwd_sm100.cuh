@@ -1,8 +1,16 @@
 // Tensor-core forward of the Universal Attention operator for sm_100a.
 //
-// bf16 inputs, key chunk = 128, head_dim D in {64, 128}.  One thread block owns
-// one key chunk (b, h, i) and sweeps the row tiles j = i .. n-1 (128 rows each)
-// upwards, so the per-key decay prefix is carried in registers.
+// bf16 inputs, key chunk kC = 128 or 64, head_dim D in {64, 128}.  One thread block owns
+// one key chunk (b, h, i) and sweeps the 128-row tiles from the chunk's first row to the
+// end of the sequence upwards, so the per-key decay prefix is carried in registers.  Where
+// that leaves the chip idle (fewer blocks than SMs, or one long sweep among short ones) the
+// sweep of a chunk is cut into segments of p.seg tiles, one block each: tile_totals_kernel
+// first sums the log-retention of every (chunk, tile), and a segment starts from the sum of
+// the tiles before it (see fwd_split for when).
+//
+// kC = 64: tiles start at the chunk's own first row (so only the first one has masked
+// pairs; the last may be half a tile); the 64 keys are TMEM lanes 0..63 of G and columns
+// 0..63 of S, lanes 64..127 of G hold the next chunk's keys and are not looked at.
 //
 //   G    = K_i  K_j^T    tcgen05.mma  M = keys, N = rows   (keys on TMEM lanes)
 //   S_r  = Q_rj K_i^T    tcgen05.mma  M = rows, N = keys   (rows on TMEM lanes)
@@ -61,7 +69,11 @@ struct FwdParams {
   int r0;                  // row of the slab where the range starts (several ranges can share one slab)
   const float* carry_in;   // optional (b*h*n, 128): decay prefix of key k at its first row tile of the range
   float* total_out;        // optional (b*h*n, 128): decay prefix after the last row tile of the range
-  float* carry;          // optional (required in carry-only mode): (b*h*n, n, 2, 128) decay prefix of key k at the start of each 64-row half of row tile j
+  float* carry;          // optional: (b*h*n, L / 64, 128) decay prefix of key k at the start of every 64 rows
+  // segments (whole sequence only): row tiles per block, 0 = a block sweeps its whole chunk; with segments, tile_totals
+  // (b*h*n, tiles, 128) holds every key's log-retention sum over every row tile of its chunk's sweep
+  int seg, tiles;
+  const float* tile_totals;
   // merged-output mode (fwd_kernel<..., kMerge = true>): instead of writing `out`, every (chunk, row tile, head) adds its
   // share of the row's softmax over ALL keys, exp(m - row_lse) * (P~ V) with P~ = exp(s - m) unnormalised, to merged_acc
   float* merged_acc;     // (b,h,r,L,d) fp32, zeroed by the caller
@@ -148,7 +160,8 @@ struct FwdCtx {
   uint32_t tmem;
   volatile int* abort_flag;
   int i, bh, ntiles;
-  int j0;             // first row tile this block computes: max(i, j_begin)
+  int row0, srow0;    // first row of the block's first tile: in the sequence, and inside the slabs of row-indexed tensors
+  int t0;             // number of that tile in the chunk's sweep (0 unless the sweep is cut into segments)
   __device__ __forceinline__ uint32_t bar(int idx) const { return bars + 8u * idx; }
   __device__ __forceinline__ bool wait(int idx, uint32_t parity) const { return mbar_wait(bar(idx), parity & 1u, abort_flag); }
   // warp-collective forms for the decay and softmax groups
@@ -157,13 +170,13 @@ struct FwdCtx {
 };
 
 // ------------------------------------------------------------------ producer --
-template <int D, bool kCarryOnly>
+template <int D, int kC, bool kCarryOnly>
 __device__ __forceinline__ void fwd_producer(const FwdCtx<D>& c, const FwdParams& p, const CUtensorMap* tmK,
                                              const CUtensorMap* tmV, const CUtensorMap* tmQ) {
   using Cfg = FwdCfg<D>;
   const int L = p.s.L, R = p.s.R;
   const uint32_t sbase = smem_u32(c.smem);
-  const int krow = c.bh * L + c.i * 128;
+  const int krow = c.bh * L + c.i * kC;
   mbar_expect_tx(c.bar(kKvFull), (kCarryOnly ? 1 : 2) * Cfg::kTileBytes);
   for (int b = 0; b < Cfg::kBoxes; ++b) {
     tma_load_2d(sbase + Cfg::oKi + b * Cfg::kBoxBytes, tmK, b * 64, krow, c.bar(kKvFull));
@@ -174,7 +187,7 @@ __device__ __forceinline__ void fwd_producer(const FwdCtx<D>& c, const FwdParams
     if (u >= 1 && !c.wait(kKjEmpty + ks, u - 1)) return false;
     mbar_expect_tx(c.bar(kKjFull + ks), Cfg::kTileBytes);
     for (int b = 0; b < Cfg::kBoxes; ++b)
-      tma_load_2d(sbase + Cfg::oKj + ks * Cfg::kTileBytes + b * Cfg::kBoxBytes, tmK, b * 64, c.bh * L + (c.j0 + T) * 128,
+      tma_load_2d(sbase + Cfg::oKj + ks * Cfg::kTileBytes + b * Cfg::kBoxBytes, tmK, b * 64, c.bh * L + c.row0 + T * 128,
                   c.bar(kKjFull + ks));
     return true;
   };
@@ -192,19 +205,19 @@ __device__ __forceinline__ void fwd_producer(const FwdCtx<D>& c, const FwdParams
       mbar_expect_tx(c.bar(kQFull + qs), Cfg::kTileBytes);
       for (int b = 0; b < Cfg::kBoxes; ++b)
         tma_load_2d(sbase + Cfg::oQ + qs * Cfg::kTileBytes + b * Cfg::kBoxBytes, tmQ, b * 64,
-                    (c.bh * R + r) * p.Lr + p.r0 + (c.j0 + T - p.j_begin) * 128, c.bar(kQFull + qs));
+                    (c.bh * R + r) * p.Lr + c.srow0 + T * 128, c.bar(kQFull + qs));
       if (r == 0 && T + 1 < c.ntiles && !load_kj(T + 1)) return;
     }
   }
 }
 
 // ---------------------------------------------------------------- MMA issuer --
-template <int D, bool kCarryOnly, int kOut>
+template <int D, int kC, bool kCarryOnly, int kOut>
 __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) {
   using Cfg = FwdCfg<D>;
   const int R = p.s.R;
   const uint32_t sbase = smem_u32(c.smem);
-  constexpr uint32_t idesc_sq = idesc_bf16(128, 128, 0, 0);
+  constexpr uint32_t idesc_g = idesc_bf16(128, 128, 0, 0), idesc_s = idesc_bf16(128, kC, 0, 0);
   constexpr uint32_t idesc_pv = idesc_bf16(128, D, 0, 1);
   const uint32_t tS[2] = {c.tmem + Cfg::tS0, c.tmem + Cfg::tS1};
   const uint32_t tO[2] = {c.tmem + Cfg::tO0, c.tmem + (Cfg::kOBufs == 2 ? Cfg::tO1 : Cfg::tO0)};
@@ -212,12 +225,12 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
   // D[128 x 128] = A[128][D] * B[128][D]^T, both K-major.  Operands are passed as descriptor low words
   // (built once: shared-memory addresses never change); a k-step of 16 elements is +32 B (>>4 = 2), the
   // second 64-element box of a tile +16384 B (>>4 = 1024).
-  auto issue_kmajor = [&](uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo) {
-    mma_ss_c<false>(d_tmem, desc_from_lo(a_lo), desc_from_lo(b_lo), idesc_sq);
+  auto issue_kmajor = [&](uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+    mma_ss_c<false>(d_tmem, desc_from_lo(a_lo), desc_from_lo(b_lo), idesc);
 #pragma unroll
     for (int ks = 1; ks < D / 16; ++ks) {
       const uint32_t off = (ks >> 2) * 1024 + (ks & 3) * 2;
-      mma_ss_c<true>(d_tmem, desc_from_lo(a_lo + off), desc_from_lo(b_lo + off), idesc_sq);
+      mma_ss_c<true>(d_tmem, desc_from_lo(a_lo + off), desc_from_lo(b_lo + off), idesc);
     }
   };
   const uint32_t kKi = desc_lo(sbase + Cfg::oKi, 16);
@@ -227,7 +240,7 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
     if (!c.wait(kKjFull + ks, u)) return false;
     if (T >= 1 && !c.wait(kGFree, T - 1)) return false;
     tc_fence_after();
-    issue_kmajor(c.tmem + Cfg::tG, kKi, desc_lo(sbase + Cfg::oKj + ks * Cfg::kTileBytes, 16));
+    issue_kmajor(c.tmem + Cfg::tG, kKi, desc_lo(sbase + Cfg::oKj + ks * Cfg::kTileBytes, 16), idesc_g);
     tc_commit(c.bar(kGFull));
     tc_commit(c.bar(kKjEmpty + ks));
     return true;
@@ -246,7 +259,7 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
     tc_fence_after();
     mma_ts_c<false>(tO[ob], tS[sb], desc_from_lo(mVi), idesc_pv);
 #pragma unroll
-    for (int ks = 1; ks < 8; ++ks) mma_ts_c<true>(tO[ob], tS[sb] + ks * 8, desc_from_lo(mVi + ks * 128), idesc_pv);
+    for (int ks = 1; ks < kC / 16; ++ks) mma_ts_c<true>(tO[ob], tS[sb] + ks * 8, desc_from_lo(mVi + ks * 128), idesc_pv);
     tc_commit(c.bar(kOFull + sb));
     return true;
   };
@@ -264,7 +277,7 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
       const int qs = t & 1;
       if (!c.wait(kQFull + qs, t >> 1)) return;
       tc_fence_after();
-      issue_kmajor(tS[t & 1], desc_lo(sbase + Cfg::oQ + qs * Cfg::kTileBytes, 16), kKi);
+      issue_kmajor(tS[t & 1], desc_lo(sbase + Cfg::oQ + qs * Cfg::kTileBytes, 16), kKi, idesc_s);
       tc_commit(c.bar(kSFull + (t & 1)));
       tc_commit(c.bar(kQEmpty + qs));
       if (t >= 1 && !issue_pv(t - 1)) return;
@@ -275,37 +288,47 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
 }
 
 // --------------------------------------------------------------- decay group --
-template <int D, typename TG, bool kCarryOnly>
+template <int D, int kC, typename TG, bool kCarryOnly>
 __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p) {
   using Cfg = FwdCfg<D>;
   const int L = p.s.L;
   const int k = threadIdx.x & 127;
   const uint32_t lane_base = (uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16;
   const TG* ss = static_cast<const TG*>(p.ssrc) + (size_t)c.bh * L;
-  const TG* sd = static_cast<const TG*>(p.sdest) + (size_t)c.bh * p.Lr + p.r0 + (c.j0 - p.j_begin) * 128 + k;
-  const float s3 = cbrtf(Num<TG>::ld(ss + c.i * 128 + k));
-  float raw_next = Num<TG>::ld(sd);      // the gate value of the next tile is fetched one pass ahead: its latency hides behind the pass
+  const TG* sd = static_cast<const TG*>(p.sdest) + (size_t)c.bh * p.Lr + c.srow0 + k;
+  // (gate of row k of tile T; with chunks of 64 keys the last tile may reach beyond the sequence)
+  auto gate_at = [&](int T) -> float { return (kC == 128 || c.row0 + T * 128 + k < L) ? Num<TG>::ld(sd + T * 128) : 0.f; };
+  const bool live = k < kC;              // kC = 64: warps 6-7 hold no key and only fetch gates
+  const float s3 = live ? cbrtf(Num<TG>::ld(ss + c.i * kC + k)) : 0.f;
+  float raw_next = gate_at(0);           // the gate value of the next tile is fetched one pass ahead: its latency hides behind the pass
   float* sT3 = reinterpret_cast<float*>(c.smem + Cfg::oT3);
   uint8_t* sCs = c.smem + Cfg::oCs;
-  const size_t key_id = ((size_t)c.bh * p.s.N + c.i) * 128 + k;
+  const size_t chunk_id = (size_t)c.bh * p.s.N + c.i, key_id = chunk_id * 128 + k;
   // The prefix carried from tile to tile reaches -2e4 at L = 4096, where fp32 spacing is 2e-3: it is kept as an
   // unevaluated sum carry + carry_lo (the rounding error of every tile's addition is carried along), so that what a
   // row sees is one rounding away from the exact sum however many tiles came before it.
   float carry = p.carry_in ? p.carry_in[key_id] : 0.f, carry_lo = 0.f;
+  auto add_to_carry = [&](float tile) {      // carry + (carry_lo + tile) as an exact two-term sum
+    const float sum = carry + tile, bb = sum - carry;
+    carry_lo = (carry - (sum - bb)) + (tile - bb);
+    carry = sum;
+  };
+  if (live)
+    for (int T = 0; T < c.t0; ++T) add_to_carry(carry_lo + p.tile_totals[(chunk_id * p.tiles + T) * 128 + k]);
   UF_DECL
   for (int T = 0; T < c.ntiles; ++T) {
-    const int j = c.j0 + T;
     float* t3buf = sT3 + (T & 1) * 128;
     t3buf[k] = cbrtf(raw_next);
-    if (T + 1 < c.ntiles) raw_next = Num<TG>::ld(sd + (T + 1) * 128);
+    if (T + 1 < c.ntiles) raw_next = gate_at(T + 1);
     c.arrive_w(kT3Ready);
     if (!c.wait_w(kT3Ready, T)) return;
+    if (!live) continue;
     UF(0)
     if (!c.wait_w(kGFull, T)) return;
     UF(1)
     tc_fence_after();
-    const bool diag = (j == c.i);
-    float* carry_row = p.carry ? p.carry + (((size_t)c.bh * p.s.N + c.i) * p.s.N + j) * 256 + k : nullptr;
+    const bool diag = (c.row0 + T * 128 == c.i * kC);
+    float* carry_row = p.carry ? p.carry + (chunk_id * (L / 64) + (c.row0 + T * 128) / 64) * 128 + k : nullptr;
     if (carry_row) carry_row[0] = carry;
     // The prefix inside a tile is  carry + (carry_lo + sum of the totals of earlier 32-row blocks + scan inside the block).
     float tprev = carry_lo, cval = carry;
@@ -318,7 +341,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
         tc_fence_before();
         c.arrive_w(kGFree);
       }
-      if (cb == 2 && carry_row) carry_row[128] = cval;      // prefix after the first 64 rows of the tile
+      if (cb == 2 && carry_row && (kC == 128 || c.row0 + T * 128 + 64 < L)) carry_row[128] = cval;      // prefix after the first 64 rows of the tile
       float v[32], t3r[32];
 #pragma unroll
       for (int x = 0; x < 8; ++x) {
@@ -365,12 +388,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
         }
       }
     }
-    {
-      // carry + tprev (tprev = carry_lo + the tile's total) as an exact two-term sum
-      const float sum = carry + tprev, bb = sum - carry;
-      carry_lo = (carry - (sum - bb)) + (tprev - bb);
-      carry = sum;
-    }
+    add_to_carry(tprev);      // (tprev = carry_lo + the tile's total)
     if (!kCarryOnly) c.arrive_w(kCReady + T % Cfg::kCBufs);
     UF(2)
   }
@@ -379,7 +397,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
 }
 
 // ------------------------------------------------------------ softmax groups --
-template <int D, int kOut>
+template <int D, int kC, int kOut>
 __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams& p, int me) {
   constexpr bool kMerge = (kOut == kOutMerged);
   using Cfg = FwdCfg<D>;
@@ -416,7 +434,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
       // pass 1: s = S + C (written back to TMEM), row max.  64 columns per round trip: the two loads are in flight together.
       float m = -INFINITY;
 #pragma unroll 1
-      for (int cb = 0; cb < 2; ++cb) {
+      for (int cb = 0; cb < kC / 64; ++cb) {
         uint32_t s[64];
         tmem_ld32(tS + cb * 64, s);
         tmem_ld32(tS + cb * 64 + 32, s + 32);
@@ -442,7 +460,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
       const float2 kL2 = make_float2(kLog2e, kLog2e), nmb2 = make_float2(-mb, -mb);
       float2 l2 = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int cb = 0; cb < 2; ++cb) {
+      for (int cb = 0; cb < kC / 64; ++cb) {
         uint32_t s[64];
         tmem_ld32(tS + cb * 64, s);
         tmem_ld32(tS + cb * 64 + 32, s + 32);
@@ -464,7 +482,8 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
       tc_fence_before();
       c.arrive_w(kPReady + sb);
       UF(4)
-      const int qg = p.r0 + (c.j0 + T - p.j_begin) * 128 + row;      // row index inside the slab
+      const int qg = c.srow0 + T * 128 + row;                       // row index inside the slab
+      const bool in_range = kC == 128 || qg < p.Lr;                 // (kC = 64: the last tile may be half a tile)
       const float l = l2.x + l2.y;
       const float lse = m + lg2(l) * kLn2;
       const size_t orow = (chunk_id * R + r) * p.Lr + qg;
@@ -475,8 +494,8 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
         // to the unnormalised P~ V (the load's latency runs under the wait for the PV product)
         linv = ex2((m - p.row_lse[mrow]) * kLog2e);
       } else {
-        p.lse[orow] = lse;
-        if (p.denom) p.denom[orow] = __float2bfloat16_rn(lse);
+        if (in_range) p.lse[orow] = lse;
+        if (p.denom && in_range) p.denom[orow] = __float2bfloat16_rn(lse);
         linv = 1.0f / l;
       }
       UF(5)
@@ -502,7 +521,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
                        __uint_as_float(o[4 * u + 2]) * linv, __uint_as_float(o[4 * u + 3]) * linv);
           continue;
         }
-        if (!p.out) continue;                 // statistics-only run (the log-sum-exp for a backward that was not given one)
+        if (!p.out || !in_range) continue;    // statistics-only run (the log-sum-exp for a backward that was not given one)
 #ifdef UA_EXPERIMENT_NO_OUT_STORE
         if (cb >= 0) continue;
 #endif
@@ -526,39 +545,128 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
   UF_STORE(row == 0 && me == 0, 8)
 }
 
-// Rows before the key chunk (j < i): every score is -1e12 (fp32 absorbs k.q), the softmax is
-// uniform, so out = sum_k bf16(1/128) V_k and lse = -1e12 (universal_attention_autograd.py:28,
-// :154).  Pure HBM writes (i * 128 * R rows), done by warps 2-3 while the others compute the
-// n - i valid tiles: chunks with many masked rows have few tiles to compute.
-template <int D>
-__device__ __forceinline__ void fwd_fill_rows(const FwdCtx<D>& c, const FwdParams& p, __nv_bfloat16* vmean) {
+// Rows before key chunk `chunk`: every score is -1e12 (fp32 absorbs k.q), the softmax is
+// uniform, so out = sum_k bf16(1/kC) V_k and lse = -1e12 (universal_attention_autograd.py:28,
+// :154).  Pure HBM writes of the slab rows [row_lo, row_hi), done by warps 2-3 while the others
+// compute.  A block of a whole sweep writes its own chunk's rows (chunks with many of them have
+// few tiles to compute); a block of a segment of chunk i writes the same tiles' share of the
+// rows before chunk n-1-i, which has as many tiles to write as chunk i has to compute.
+template <int D, int kC>
+__device__ __forceinline__ void fwd_fill_rows(const FwdCtx<D>& c, const FwdParams& p, __nv_bfloat16* vmean, int chunk, int row_lo, int row_hi) {
+  if (row_lo >= row_hi) return;
   const int t = threadIdx.x - 64;                      // 0..63
   const int L = p.s.L, R = p.s.R, N = p.s.N;
-  const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.vc) + ((size_t)c.bh * L + (size_t)c.i * 128) * D;
-  const float w = 1.0f / 128.0f;
+  const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.vc) + ((size_t)c.bh * L + (size_t)chunk * kC) * D;
+  const float w = 1.0f / kC;
   for (int d = t; d < D; d += 64) {
     float acc = 0.f;
-    for (int k = 0; k < 128; ++k) acc = fmaf(w, __bfloat162float(v[(size_t)k * D + d]), acc);
+#pragma unroll 16
+    for (int k = 0; k < kC; ++k) acc = fmaf(w, __bfloat162float(v[(size_t)k * D + d]), acc);
     vmean[d] = __float2bfloat16_rn(acc);
   }
   named_bar_sync(2, 64);
-  const size_t chunk_id = (size_t)c.bh * N + c.i;
-  const int rows = ((c.i < p.j_end ? c.i : p.j_end) - p.j_begin) * 128;    // rows of the range that lie before the chunk
+  const size_t chunk_id = (size_t)c.bh * N + chunk;
+  const int rows = row_hi - row_lo;
   constexpr int kVecPerRow = D / 8;                    // 16-byte vectors
   const uint4 mine = reinterpret_cast<const uint4*>(vmean)[t % kVecPerRow];   // 64 % kVecPerRow == 0: fixed per thread
   for (int r = 0; r < R; ++r) {
-    uint4* o = reinterpret_cast<uint4*>(p.out + ((chunk_id * R + r) * p.Lr + p.r0) * D);
+    const size_t first = (chunk_id * R + r) * p.Lr + row_lo;
+    uint4* o = reinterpret_cast<uint4*>(p.out + first * D);
     const size_t nvec = (size_t)rows * kVecPerRow;
     for (size_t e = t; e < nvec; e += 64) o[e] = mine;
-    float* lr = p.lse + (chunk_id * R + r) * p.Lr + p.r0;
     for (int q = t; q < rows; q += 64) {
-      lr[q] = mask_value();
-      if (p.denom) p.denom[(chunk_id * R + r) * p.Lr + p.r0 + q] = __float2bfloat16_rn(mask_value());
+      p.lse[first + q] = mask_value();
+      if (p.denom) p.denom[first + q] = __float2bfloat16_rn(mask_value());
     }
   }
 }
 
-template <int D, typename TG, bool kCarryOnly, int kOut = kOutTiles>
+// ------------------------------------------------------- log-retention of a tile --
+// total[chunk][T][key] = sum of the log-retention of the key over the rows of tile T of its chunk's sweep: what the segments
+// of a cut sweep start from.  One block per (b, h, chunk, tile), 16 warps: warp % 4 = TMEM lane quadrant (keys), warp / 4 = 32 of
+// the 128 columns (rows).  Short by construction (one product of 128 x 128 x D and 32 elements per thread), so latency is all
+// that counts: B1 H8 L640 D64, 120 blocks: see fwd_split.
+template <int D, int kC, typename TG>
+__global__ void __launch_bounds__(512)
+tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles, const void* ssrc, const void* sdest, float* total, int* status) {
+  constexpr int kTile = 128 * D * 2, kBoxes = D / 64;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  float* t3 = reinterpret_cast<float*>(smem + 2 * kTile);
+  float* part = t3 + 128;                                // [3][128]
+  uint32_t* misc = reinterpret_cast<uint32_t*>(part + 384);      // [0] tmem base, [1] abort flag, [2..5] two barriers
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, BH = shp.B * shp.H, L = shp.L;
+  const int bh = blockIdx.x % BH;
+  int x = blockIdx.x / BH, i = 0;
+  for (;; ++i) {
+    const int nt = (L - i * kC + 127) / 128;
+    if (x < nt) break;
+    x -= nt;
+  }
+  const int row0 = i * kC + x * 128;
+  const uint32_t bar = smem_u32(misc + 2), sb = smem_u32(smem);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 1);
+  if (threadIdx.x == 0) {
+    misc[1] = 0;
+    mbar_init(bar, 1); mbar_init(bar + 8, 1);
+    mbar_init_fence();
+    mbar_expect_tx(bar, 2 * kTile);
+    for (int b = 0; b < kBoxes; ++b) {
+      tma_load_2d(sb + b * 16384, &tmK, b * 64, bh * L + i * kC, bar);
+      tma_load_2d(sb + kTile + b * 16384, &tmK, b * 64, bh * L + row0, bar);
+    }
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(misc), 128);
+    tmem_relinquish();
+  }
+  if (threadIdx.x >= 128 && threadIdx.x < 256) {
+    const int q = threadIdx.x - 128;
+    t3[q] = row0 + q < L ? cbrtf(Num<TG>::ld(static_cast<const TG*>(sdest) + (size_t)bh * L + row0 + q)) : 0.f;
+  }
+  const int quad = warp & 3, grp = warp >> 2, k = quad * 32 + lane;
+  const float s3 = k < kC ? cbrtf(Num<TG>::ld(static_cast<const TG*>(ssrc) + (size_t)bh * L + i * kC + k)) : 0.f;
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = misc[0];
+  if (threadIdx.x == 0 && mbar_wait(bar, 0, abort_flag)) {
+    constexpr uint32_t idesc = idesc_bf16(128, 128, 0, 0);
+    const uint32_t a = desc_lo(sb, 16), b = desc_lo(sb + kTile, 16);
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+      const uint32_t off = (ks >> 2) * 1024 + (ks & 3) * 2;
+      mma_ss(tmem, desc_from_lo(a + off), desc_from_lo(b + off), idesc, ks > 0);
+    }
+    tc_commit(bar + 8);
+  }
+  __syncwarp();
+  float local = 0.f;
+  if (mbar_wait_warp(bar + 8, 0, abort_flag)) {
+    tc_fence_after();
+    uint32_t g[32];
+    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + grp * 32, g);
+    tc_wait_ld();
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      float ell = log_retention(gated_affinity(gram_pow23(__uint_as_float(g[q])), s3, t3[grp * 32 + q]));
+      if (x == 0 && grp * 32 + q <= k) ell = 0.f;      // (only the first tile of a sweep has rows at or before the key)
+      local += ell;
+    }
+  }
+  if (grp) part[(grp - 1) * 128 + k] = local;
+  tc_fence_before();
+  __syncthreads();
+  if (grp == 0 && k < kC) total[(((size_t)bh * shp.N + i) * tiles + x) * 128 + k] = ((local + part[k]) + part[128 + k]) + part[256 + k];
+  if (*abort_flag) {
+    if (threadIdx.x == 0) atomicExch(status, 1);
+    for (int it = 0; it < 64; ++it) __nanosleep(2000);
+    __syncthreads();
+  }
+  if (warp == 1) tmem_dealloc(tmem, 128);
+}
+
+template <int D, int kC, typename TG, bool kCarryOnly, int kOut = kOutTiles>
 __global__ void __launch_bounds__(512, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
            const __grid_constant__ CUtensorMap tmQ, FwdParams p) {
@@ -573,17 +681,48 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   c.smem = smem;
   c.bars = smem_u32(smem + Cfg::oBar);
   c.abort_flag = reinterpret_cast<volatile int*>(misc + 1);
-  c.i = blockIdx.x / BH;                 // heavy chunks (small i: most row tiles) first
-  c.bh = blockIdx.x - c.i * BH;
-  c.j0 = c.i > p.j_begin ? c.i : p.j_begin;
-  c.ntiles = p.j_end - c.j0;            // <= 0: nothing to compute for this chunk in the row range (only the fill)
+  // heavy chunks (small i: most row tiles) first
+  int x = blockIdx.x / BH;
+  c.bh = blockIdx.x - x * BH;
+  int fill_chunk, fill_lo = 0, fill_hi;      // rows before which chunk this block writes, in slab rows
+  if (p.seg == 0) {
+    c.i = x;
+    c.t0 = 0;
+    if (kC == 128) {
+      const int j0 = c.i > p.j_begin ? c.i : p.j_begin;
+      c.row0 = j0 * 128;
+      c.ntiles = p.j_end - j0;              // <= 0: nothing to compute for this chunk in the row range (only the fill)
+    } else {
+      c.row0 = c.i * kC;
+      c.ntiles = (p.s.L - c.row0 + 127) / 128;
+    }
+    fill_chunk = c.i;
+    fill_lo = p.r0;
+    fill_hi = p.r0 + (kC == 128 ? ((c.i < p.j_end ? c.i : p.j_end) - p.j_begin) * 128 : c.i * kC);
+  } else {
+    int nt;
+    for (c.i = 0;; ++c.i) {
+      nt = (p.s.L - c.i * kC + 127) / 128;
+      const int ns = (nt + p.seg - 1) / p.seg;
+      if (x < ns) break;
+      x -= ns;
+    }
+    c.t0 = x * p.seg;
+    c.row0 = c.i * kC + c.t0 * 128;
+    c.ntiles = nt - c.t0 < p.seg ? nt - c.t0 : p.seg;
+    fill_chunk = p.s.N - 1 - c.i;
+    fill_lo = c.t0 * 128;
+    fill_hi = min(fill_lo + c.ntiles * 128, fill_chunk * kC);
+  }
+  c.srow0 = p.r0 + c.row0 - p.j_begin * 128;
 
   if (threadIdx.x == 0) {
     misc[1] = 0;
     for (int b = 0; b < kNumBars; ++b) {
       uint32_t count = 1;
       // one arrival per warp of the group that signals
-      if (b == kGFree || b == kCReady || b == kCReady + 1 || b == kT3Ready) count = 4;
+      if (b == kGFree || b == kCReady || b == kCReady + 1) count = kC / 32;
+      if (b == kT3Ready) count = 4;
       if (b == kCFree || b == kCFree + 1) count = 8;
       if (b == kPReady || b == kPReady + 1 || b == kOFree || b == kOFree + 1) count = 4;
       mbar_init(c.bar(b), count);
@@ -603,18 +742,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   c.tmem = misc[0];
 
   if (warp == 0) {
-    if (lane == 0 && c.ntiles > 0) fwd_producer<D, kCarryOnly>(c, p, &tmK, &tmV, &tmQ);
+    if (lane == 0 && c.ntiles > 0) fwd_producer<D, kC, kCarryOnly>(c, p, &tmK, &tmV, &tmQ);
   } else if (warp == 1) {
-    if (lane == 0 && c.ntiles > 0) fwd_mma<D, kCarryOnly, kOut>(c, p);
+    if (lane == 0 && c.ntiles > 0) fwd_mma<D, kC, kCarryOnly, kOut>(c, p);
   } else if (warp >= 4 && warp < 8) {
-    if (c.ntiles > 0) fwd_decay<D, TG, kCarryOnly>(c, p);
+    if (c.ntiles > 0) fwd_decay<D, kC, TG, kCarryOnly>(c, p);
     else if (p.total_out)      // no row of the range sees this chunk: its prefix does not move
       p.total_out[((size_t)c.bh * p.s.N + c.i) * 128 + (threadIdx.x & 127)] =
           p.carry_in ? p.carry_in[((size_t)c.bh * p.s.N + c.i) * 128 + (threadIdx.x & 127)] : 0.f;
   } else if (warp >= 8 && !kCarryOnly) {
-    if (c.ntiles > 0) fwd_softmax<D, kOut>(c, p, (warp - 8) >> 2);
-  } else if ((warp == 2 || warp == 3) && !kCarryOnly && p.fill_masked && c.i > p.j_begin) {
-    fwd_fill_rows<D>(c, p, reinterpret_cast<__nv_bfloat16*>(smem + Cfg::oFill));
+    if (c.ntiles > 0) fwd_softmax<D, kC, kOut>(c, p, (warp - 8) >> 2);
+  } else if ((warp == 2 || warp == 3) && !kCarryOnly && p.fill_masked) {
+    fwd_fill_rows<D, kC>(c, p, reinterpret_cast<__nv_bfloat16*>(smem + Cfg::oFill), fill_chunk, fill_lo, fill_hi);
   }
 
   tc_fence_before();
