@@ -79,28 +79,43 @@ BwdWorkspace bwd_layout(const ua::Shape& s, int rt) {
 }
 
 struct BwdWorkspaceTc {
-  size_t off_dk, off_dq, off_dt, off_dkr, off_carry, off_lse, off_gd, off_mt, off_ksum, off_nacc, acc_bytes, total;
+  size_t off_dk, off_dq, off_dt, off_dkr, off_dv, off_ds, off_carry, off_lse, off_gd, off_mt, off_ksum, off_nacc, off_seg, off_out, off_fwd;
+  size_t acc_bytes, acc_fp32_v_bytes, total;     // what is zeroed: without and with the fp32 dV / d static_src
 };
 
-// Scratch of the tensor-core backward: status | fp32 accumulators dK, dQ, d dest, row-side dK | decay-prefix table (two entries per
-// 128-row tile) | log-sum-exp (only written when the caller has none) | fp32 copy of g_denom (only written when the
-// caller's is bf16) | per-chunk data of the kernels for the rows before a chunk.
-BwdWorkspaceTc bwd_layout_tc(const ua::Shape& s) {
-  BwdWorkspaceTc w;
-  const size_t BH = (size_t)s.B * s.H, f = sizeof(float);
+// Scratch of the tensor-core backward.  s: the kernels' shape (chunks of 64 or 128 keys), m: kernel chunks per chunk of the
+// operator.  Status | fp32 accumulators dK, dQ, d dest, row-side dK, and dV, d src for sweeps that are cut into segments or share
+// them with the kernel of the rows before a chunk | decay-prefix table | log-sum-exp (only written when the caller has none) | fp32
+// g_denom or row term | per-chunk data of the kernels for the rows before a chunk / segment totals | for m > 1 the output and the
+// scratch of a forward run (only used for callers that kept neither).
+BwdWorkspaceTc bwd_layout_tc(const ua::Shape& s, int m, size_t fwd_bytes) {
+  BwdWorkspaceTc w{};
+  const size_t BH = (size_t)s.B * s.H, f = sizeof(float), rows = BH * (s.N / m) * (size_t)s.R * s.L;
+  const int seg = ua::sm100::bwd_split(s);
   size_t o = 256;   // [0, 256): status word
   w.off_dk = o; o = align_up(o + BH * s.L * s.D * f, 256);
   w.off_dq = o; o = align_up(o + BH * s.R * s.L * s.D * f, 256);
   w.off_dt = o; o = align_up(o + BH * s.L * f, 256);
   w.off_dkr = o; o = align_up(o + BH * s.L * s.D * f, 256);
   w.acc_bytes = o;
-  w.off_carry = o; o = align_up(o + BH * s.N * (size_t)s.N * 256 * f, 256);
-  w.off_lse = o; o = align_up(o + BH * s.N * (size_t)s.R * s.L * f, 256);
-  w.off_gd = o; o = align_up(o + BH * s.N * (size_t)s.R * s.L * f, 256);
-  // per-chunk constants and partial sums of the rows-before-the-chunk kernels: M^T images, ksum, N / w / u / vbar
-  w.off_mt = o; o = align_up(o + BH * s.N * (size_t)s.D * s.D * 2, 256);
+  if (seg || s.C == 64) {
+    w.off_dv = o; o = align_up(o + BH * s.L * s.D * f, 256);
+    w.off_ds = o; o = align_up(o + BH * s.L * f, 256);
+  }
+  w.acc_fp32_v_bytes = o;
+  w.off_carry = o; o = align_up(o + BH * s.N * (size_t)(s.L / 64) * 128 * f, 256);
+  w.off_lse = o; o = align_up(o + rows * f, 256);
+  w.off_gd = o; o = align_up(o + rows * f, 256);
+  // per-chunk constants and partial sums of the rows-before-the-chunk kernels: M^T images (read for the last time before the
+  // sweep starts, so the segment totals share their place), ksum, N / w / u / vbar
+  w.off_mt = w.off_seg = o;
+  o = align_up(o + std::max(BH * s.N * (size_t)s.D * s.D * 2, BH * s.N * (size_t)ua::sm100::bwd_max_segments(s, seg) * 128 * f), 256);
   w.off_ksum = o; o = align_up(o + BH * s.N * (size_t)s.D * 2, 256);
   w.off_nacc = o; o = align_up(o + BH * s.N * (size_t)(s.D + 3) * s.D * f, 256);
+  if (m > 1) {
+    w.off_out = o; o = align_up(o + rows * s.D * 2, 256);
+    w.off_fwd = o; o = align_up(o + fwd_bytes, 256);
+  }
   w.total = o;
   return w;
 }
@@ -121,6 +136,13 @@ int launch_simt_bwd(const ua::simt::BwdParams& p, cudaStream_t st) {
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return UA_ERR_CUDA;
   kern<<<p.s.B * p.s.H * p.s.N, ua::simt::kThreads, smem, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+
+int launch_simt_bwd_any(const ua::simt::BwdParams& p, int dtype, int gate_dtype, const SimtCfg& cfg, cudaStream_t st) {
+  if (dtype == UA_F32) return launch_simt_bwd<float, float, float>(p, st);
+  if (cfg.compact) return gate_dtype == UA_F32 ? launch_simt_bwd<bf16, float, bf16>(p, st) : launch_simt_bwd<bf16, bf16, bf16>(p, st);
+  if (gate_dtype == UA_F32) return launch_simt_bwd<bf16, float, float>(p, st);
+  return launch_simt_bwd<bf16, bf16, float>(p, st);
 }
 
 __global__ void widen_bf16_kernel(const bf16* __restrict__ src, float* __restrict__ dst, size_t n) {
@@ -153,8 +175,8 @@ int convert_any(int dtype, const float* src, void* dst, size_t n, cudaStream_t s
 // The softmax of the operator runs over the keys of one chunk (universal_attention_autograd.py:85-93); everything else --
 // affinity, decay prefix along the rows, mask -- is per key.  A chunk of m * 128 keys is therefore swept as m sub-chunks
 // of 128 keys by the kernels above, and the m (out, log-sum-exp) pairs of each chunk are merged with softmax weights
-// exp(lse_sub - lse_chunk): the same merge as SMVecMatMul's, over groups of m neighbouring sub-chunks.  The backward
-// runs the sub-chunk forward again (the merge backward needs its outputs), the merge backward, and the sub-chunk backward.
+// exp(lse_sub - lse_chunk): the same merge as SMVecMatMul's, over groups of m neighbouring sub-chunks.  The backward needs
+// nothing of the kind: with the chunk's own log-sum-exp and row term every sub-chunk is a block of the sweep by itself.
 int sub_chunks(const ua::Shape& s, int dtype, int flags) {
   if ((flags & UA_FLAG_FORCE_SIMT) || dtype != UA_BF16 || s.C <= 128 || s.C % 128 != 0 || s.C / 128 > 8) return 0;
   ua::Shape t = s;
@@ -173,41 +195,18 @@ UaDims group_dims(const UaDims* d, int m) {
   return t;
 }
 struct SubWorkspace {
-  size_t off_inner, off_out, off_gout, off_lse, off_glse, off_carry, off_status, total;
+  size_t off_out, off_lse, total;
 };
-SubWorkspace sub_layout(const ua::Shape& s, int m, bool backward, size_t inner_bytes) {
+SubWorkspace sub_layout(const ua::Shape& s, int m, size_t inner_bytes) {
   SubWorkspace w{};
   const size_t rows = (size_t)s.B * s.H * s.N * m * s.R * s.L;
   size_t o = align_up(inner_bytes < 256 ? 256 : inner_bytes, 256);     // the inner call's workspace comes first: its status word is the caller's
   w.off_out = o; o = align_up(o + rows * s.D * 2, 256);
   w.off_lse = o; o = align_up(o + rows * sizeof(float), 256);
-  if (backward) {
-    w.off_gout = o; o = align_up(o + rows * s.D * 2, 256);
-    w.off_glse = o; o = align_up(o + rows * sizeof(float), 256);
-    w.off_carry = o; o = align_up(o + (size_t)s.B * s.H * s.N * m * s.N * m * 256 * sizeof(float), 256);
-    w.off_status = o; o += 256;
-  }
   w.total = o;
   return w;
 }
 
-// g_lse_sub += g_denom_chunk * exp(lse_sub - lse_chunk): the chunk's denom is the log-sum-exp over its sub-chunks
-template <typename TD>
-__global__ void group_denom_grad_kernel(const float* __restrict__ lse_sub, const TD* __restrict__ g_denom, float* __restrict__ g_lse_sub,
-                                        size_t groups, size_t rl, int m) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < groups * rl; idx += stride) {
-    const size_t grp = idx / rl, x = idx - grp * rl;
-    const float* l = lse_sub + grp * m * rl + x;
-    float mx = l[0];
-    for (int q = 1; q < m; ++q) mx = fmaxf(mx, l[q * rl]);
-    float z = 0.f;
-    for (int q = 0; q < m; ++q) z += expf(l[q * rl] - mx);
-    const float g = ua::Num<TD>::ld(g_denom + idx) / z;
-    float* gl = g_lse_sub + grp * m * rl + x;
-    for (int q = 0; q < m; ++q) gl[q * rl] += g * expf(l[q * rl] - mx);
-  }
-}
 // One block, two waiters on an mbarrier that nothing completes: thread 0 with the single-thread wait, warp 1 with the
 // warp-collective one, both with a short wall-time limit.  Both give up, and the block reports it as the kernels do.
 __global__ void wait_selftest_kernel(int* status, unsigned long long limit_ns) {
@@ -349,7 +348,7 @@ size_t ua_fwd_workspace_bytes(const UaDims* dims, int dtype, int flags) {
     ua::Shape s = to_shape(dims);
     if (const int m = sub_chunks(s, dtype, flags)) {
       const UaDims sd = sub_dims(dims, m);
-      return sub_layout(s, m, false, ua_fwd_workspace_bytes(&sd, dtype, flags)).total;
+      return sub_layout(s, m, ua_fwd_workspace_bytes(&sd, dtype, flags)).total;
     }
     if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::fwd_supported(s, dtype) && ua::sm100::fwd_split(s))
       return 256 + ua::sm100::fwd_totals_bytes(s);      // status word, tile totals of the segmented sweep
@@ -362,9 +361,9 @@ size_t ua_bwd_workspace_bytes(const UaDims* dims, int dtype, int flags) {
   ua::Shape s = to_shape(dims);
   if (const int m = sub_chunks(s, dtype, flags)) {
     const UaDims sd = sub_dims(dims, m);
-    return sub_layout(s, m, true, bwd_layout_tc(to_shape(&sd)).total).total;
+    return bwd_layout_tc(to_shape(&sd), m, ua_fwd_workspace_bytes(dims, dtype, 0)).total;
   }
-  if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype)) return bwd_layout_tc(s).total;
+  if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype)) return bwd_layout_tc(s, 1, 0).total;
   const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
   if (!cfg.rt) return 0;
   return bwd_layout(s, cfg.rt).total;
@@ -375,7 +374,7 @@ size_t ua_carry_bytes(const UaDims* dims, int dtype, int flags) {
   ua::Shape s = to_shape(dims);
   if (const int m = sub_chunks(s, dtype, flags)) return (size_t)s.B * s.H * s.N * m * s.N * m * 256 * sizeof(float);
   if ((flags & UA_FLAG_FORCE_SIMT) || !ua::sm100::bwd2_supported(s, dtype)) return 0;
-  return (size_t)s.B * s.H * s.N * s.N * 256 * sizeof(float);
+  return (size_t)s.B * s.H * s.N * (s.L / 64) * 128 * sizeof(float);
 }
 
 int ua_fwd(const UaDims* dims, int dtype, int gate_dtype, const void* kc, const void* vc, const void* xq,
@@ -400,7 +399,7 @@ int ua_fwd_keep(const UaDims* dims, int dtype, int gate_dtype, const void* kc, c
     // sub-chunks of 128 keys, then the merge inside each chunk (see sub_chunks)
     const UaDims sd = sub_dims(dims, m), gd = group_dims(dims, m);
     const size_t inner = ua_fwd_workspace_bytes(&sd, dtype, flags);
-    const SubWorkspace w = sub_layout(s, m, false, inner);
+    const SubWorkspace w = sub_layout(s, m, inner);
     if (workspace_bytes < w.total) return UA_ERR_WORKSPACE;
     char* ws = static_cast<char*>(workspace);
     void* out_sub = ws + w.off_out;
@@ -507,7 +506,7 @@ int ua_decay_totals_rows(const UaDims* dims, int dtype, int gate_dtype, const Ua
 size_t ua_bwd_rows_workspace_bytes(const UaDims* dims, int dtype) {
   if (check_dims(dims) != UA_OK) return 0;
   ua::Shape s = to_shape(dims);
-  if (!ua::sm100::bwd2_supported(s, dtype)) return 0;
+  if (!ua::sm100::bwd2_supported(s, dtype) || !ua::sm100::chunk128(s)) return 0;
   // status | row-side dK scratch (as for ua_bwd_rows_suffix) | decay-prefix table | log-sum-exp of the range's rows | fp32
   // copy of a bf16 g_denom (both sized for Ls = L) | per-chunk data of the kernels for the rows before a chunk (M^T images,
   // ksum, N / w / u / vbar)
@@ -552,7 +551,7 @@ int ua_bwd_rows_kept(const UaDims* dims, int dtype, int gate_dtype, const UaRows
       !aligned16(dv_f32) || !aligned16(dxq_rows_f32))
     return UA_ERR_ALIGNMENT;
   ua::Shape s = to_shape(dims);
-  if ((e = check_rows(s, ua::sm100::bwd2_supported(s, dtype), rows))) return e;
+  if ((e = check_rows(s, ua::sm100::bwd2_supported(s, dtype) && ua::sm100::chunk128(s), rows))) return e;
   const bool skip_masked = (flags & UA_FLAG_SKIP_MASKED_GRADS) != 0;
   const size_t need = ua_bwd_rows_workspace_bytes(dims, dtype);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
@@ -599,7 +598,7 @@ int ua_bwd_rows_kept(const UaDims* dims, int dtype, int gate_dtype, const UaRows
     mp.nacc = reinterpret_cast<float*>(q);
     mp.acc_dk = dk_f32; mp.status = status;
     mp.j_begin = rows->tile_begin; mp.j_end = rows->tile_end; mp.Lr = rows->rows_total; mp.r0 = rows->row_offset;
-    mp.acc_dv = dv_f32;
+    mp.acc_dv = dv_f32; mp.m = 1;
     if ((e = ua::sm100::launch_masked(s, kc, vc, xq_rows, g_out_cm_rows, dxq_rows_f32, mp, st))) return e;
   }
   // (3) the rows that see their chunk: the keys-on-lanes kernel over the range
@@ -609,8 +608,8 @@ int ua_bwd_rows_kept(const UaDims* dims, int dtype, int gate_dtype, const UaRows
   qp.dvc = nullptr; qp.dss = nullptr; qp.status = status; qp.trace = nullptr;
   qp.j_begin = rows->tile_begin; qp.j_end = rows->tile_end; qp.Lr = rows->rows_total; qp.r0 = rows->row_offset;
   qp.heads = s.R; qp.suffix_in = suffix_in; qp.dctot_out = dctot_out; qp.acc_dv = dv_f32; qp.acc_ds = dsrc_f32;
-  qp.acc_dkr = acc_dkr;
-  return ua::sm100::launch_bwd2(s, gate_dtype, false, kc, vc, xq_rows, g_out_cm_rows, qp, st);
+  qp.acc_dkr = acc_dkr; qp.m = 1;
+  return ua::sm100::launch_bwd2(s, gate_dtype, 1, kc, vc, xq_rows, g_out_cm_rows, qp, st);
 }
 
 int ua_bwd_rows_suffix(const UaDims* dims, int dtype, int gate_dtype, const UaRows* rows, const void* kc, const void* vc,
@@ -622,7 +621,7 @@ int ua_bwd_rows_suffix(const UaDims* dims, int dtype, int gate_dtype, const UaRo
   if (!kc || !vc || !static_src || !static_dest_rows || !suffix || !dk_f32 || !dsrc_f32 || !ddest_rows_f32) return UA_ERR_NULL_POINTER;
   if (!aligned16(kc) || !aligned16(vc) || !aligned16(dk_f32)) return UA_ERR_ALIGNMENT;
   ua::Shape s = to_shape(dims);
-  if ((e = check_rows(s, ua::sm100::bwd2_supported(s, dtype), rows))) return e;
+  if ((e = check_rows(s, ua::sm100::bwd2_supported(s, dtype) && ua::sm100::chunk128(s), rows))) return e;
   const size_t need = ua_bwd_rows_suffix_workspace_bytes(dims, dtype);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
   if (!aligned16(static_dest_rows)) return UA_ERR_ALIGNMENT;
@@ -635,8 +634,8 @@ int ua_bwd_rows_suffix(const UaDims* dims, int dtype, int gate_dtype, const UaRo
   qp.dvc = nullptr; qp.dss = nullptr; qp.status = static_cast<int*>(workspace); qp.trace = nullptr;
   qp.j_begin = rows->tile_begin; qp.j_end = rows->tile_end; qp.Lr = rows->rows_total; qp.r0 = rows->row_offset;
   qp.acc_dkr = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
-  qp.heads = 0; qp.suffix_in = suffix; qp.dctot_out = nullptr; qp.acc_dv = nullptr; qp.acc_ds = dsrc_f32;
-  return ua::sm100::launch_bwd2(s, gate_dtype, false, kc, vc, nullptr, nullptr, qp, st);
+  qp.heads = 0; qp.suffix_in = suffix; qp.dctot_out = nullptr; qp.acc_dv = nullptr; qp.acc_ds = dsrc_f32; qp.m = 1;
+  return ua::sm100::launch_bwd2(s, gate_dtype, 1, kc, vc, nullptr, nullptr, qp, st);
 }
 
 int ua_bwd(const UaDims* dims, int dtype, int gate_dtype, const void* kc, const void* vc, const void* xq,
@@ -671,109 +670,110 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ua::Shape s = to_shape(dims);
 
-  if (const int m = sub_chunks(s, dtype, flags)) {
-    // chunks of m * 128 keys (see sub_chunks): sub-chunk forward again, merge backward inside each chunk, sub-chunk backward.
-    // (lse_cm, the chunks' log-sum-exp, is not what the sub-chunk kernels need; carry_in is already per sub-chunk.)
-    const UaDims sd = sub_dims(dims, m), gd = group_dims(dims, m);
-    const size_t inner = bwd_layout_tc(to_shape(&sd)).total;
-    const SubWorkspace w = sub_layout(s, m, true, inner);
-    if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
-    char* ws = static_cast<char*>(workspace);
-    void* out_sub = ws + w.off_out;
-    void* g_out_sub = ws + w.off_gout;
-    float* lse_sub = reinterpret_cast<float*>(ws + w.off_lse);
-    float* g_lse_sub = reinterpret_cast<float*>(ws + w.off_glse);
-    void* carry_sub = carry_in ? nullptr : static_cast<void*>(ws + w.off_carry);
-    if ((e = ua_fwd_keep(&sd, dtype, gate_dtype, kc, vc, xq, static_src, static_dest, out_sub, lse_sub, nullptr, carry_sub,
-                         ws + w.off_status, 256, flags & ~UA_FLAG_SKIP_MASKED_FILL, stream)))
-      return e;
-    if ((e = ua_merge_bwd(&gd, dtype, out_sub, lse_sub, g_out_cm, g_out_sub, g_lse_sub, 0, stream))) return e;
-    {
-      const size_t groups = (size_t)s.B * s.H * s.N, rl = (size_t)s.R * s.L;
-      if (g_denom_dtype == UA_F32)
-        group_denom_grad_kernel<float><<<148 * 8, 256, 0, st>>>(lse_sub, static_cast<const float*>(g_denom_cm), g_lse_sub, groups, rl, m);
-      else
-        group_denom_grad_kernel<bf16><<<148 * 8, 256, 0, st>>>(lse_sub, static_cast<const bf16*>(g_denom_cm), g_lse_sub, groups, rl, m);
-      if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
-    }
-    // (the sub-chunk output tiles were just recomputed: the inner call takes its row term from them)
-    if ((e = ua_bwd_saved(&sd, dtype, gate_dtype, kc, vc, xq, static_src, static_dest, g_out_sub, g_lse_sub, UA_F32,
-                          carry_in ? carry_in : carry_sub, lse_sub, out_sub, dkc, dvc, dxq, dstatic_src, dstatic_dest, workspace,
-                          inner, flags, stream)))
-      return e;
-    carry_status_kernel<<<1, 1, 0, st>>>(reinterpret_cast<const int*>(ws + w.off_status), reinterpret_cast<int*>(ws));
-    return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
-  }
-
-  if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype)) {
+  const int wide = sub_chunks(s, dtype, flags);
+  if (wide || (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype))) {
     if (!aligned16(dvc) || !aligned16(dkc) || !aligned16(dxq)) return UA_ERR_ALIGNMENT;
-    BwdWorkspaceTc w = bwd_layout_tc(s);
+    const int m = wide ? wide : 1;
+    const UaDims kd = wide ? sub_dims(dims, m) : *dims;
+    const ua::Shape ks = to_shape(&kd);                 // the kernels' shape
+    const size_t fwd_bytes = wide ? ua_fwd_workspace_bytes(dims, dtype, 0) : 0;
+    const BwdWorkspaceTc w = bwd_layout_tc(ks, m, fwd_bytes);
     if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
     char* ws = static_cast<char*>(workspace);
-    if (cudaMemsetAsync(ws, 0, w.acc_bytes, st) != cudaSuccess) return UA_ERR_CUDA;
-    float* carry_tab = carry_in ? const_cast<float*>(static_cast<const float*>(carry_in)) : reinterpret_cast<float*>(ws + w.off_carry);
-    float* acc_dk = reinterpret_cast<float*>(ws + w.off_dk);
-    float* acc_dq = reinterpret_cast<float*>(ws + w.off_dq);
-    float* acc_dt = reinterpret_cast<float*>(ws + w.off_dt);
-    const bool skip_masked = (flags & UA_FLAG_SKIP_MASKED_GRADS) != 0;
-    const size_t BHs = (size_t)s.B * s.H;
-    // What the keys-on-lanes kernel needs besides the inputs: the decay-prefix table and the forward's log-sum-exp.  A
-    // caller that has neither gets both from one statistics-only run of the forward kernel (no output tile is written).
+    auto at = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
+    const bool masked = !(flags & UA_FLAG_SKIP_MASKED_GRADS) && s.N > 1;
+    const int seg = ua::sm100::bwd_split(ks);
+    // dV and d static_src are added up in fp32 where several blocks share a key
+    const bool fp32_v = seg || (masked && ks.C == 64);
+    if (cudaMemsetAsync(ws, 0, fp32_v ? w.acc_fp32_v_bytes : w.acc_bytes, st) != cudaSuccess) return UA_ERR_CUDA;
+    const float* carry_tab = static_cast<const float*>(carry_in);
+    float *acc_dk = at(w.off_dk), *acc_dq = at(w.off_dq);
+    // What the keys-on-lanes kernel needs besides the inputs: the decay-prefix table and the forward's log-sum-exp (for wide
+    // chunks the output too).  A caller that has neither gets both from one statistics-only run of the forward kernel (no output
+    // tile is written).
     const float* lse = lse_cm;
-    if (!lse || !carry_in) {
+    const void* out = out_cm;
+    if (wide && (!lse || !carry_tab || !out)) {
+      if ((e = ua_fwd_keep(dims, dtype, gate_dtype, kc, vc, xq, static_src, static_dest, ws + w.off_out, at(w.off_lse), nullptr, at(w.off_carry),
+                           ws + w.off_fwd, fwd_bytes, UA_FLAG_SKIP_MASKED_FILL, stream)))
+        return e;
+      carry_status_kernel<<<1, 1, 0, st>>>(reinterpret_cast<const int*>(ws + w.off_fwd), reinterpret_cast<int*>(ws));
+      lse = at(w.off_lse); carry_tab = at(w.off_carry); out = ws + w.off_out;
+    } else if (!lse || !carry_tab) {
       ua::sm100::FwdParams fp{};
-      fp.s = s; fp.ssrc = static_src; fp.sdest = static_dest; fp.out = nullptr; fp.denom = nullptr;
-      fp.lse = lse ? nullptr : reinterpret_cast<float*>(ws + w.off_lse);
+      fp.s = ks; fp.ssrc = static_src; fp.sdest = static_dest; fp.out = nullptr; fp.denom = nullptr;
+      fp.lse = lse ? nullptr : at(w.off_lse);
       fp.status = reinterpret_cast<int*>(ws);
-      fp.carry = carry_in ? nullptr : carry_tab;
+      fp.carry = carry_tab ? nullptr : at(w.off_carry);
       ua::sm100::whole_sequence(fp);
-      if (lse) e = ua::sm100::launch_fwd_carry(s, gate_dtype, kc, fp, st);      // decay-only pass
-      else e = ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, false, nullptr, st);
+      if (lse) e = ua::sm100::launch_fwd_carry(ks, gate_dtype, kc, fp, st);      // decay-only pass
+      else e = ua::sm100::launch_fwd(ks, gate_dtype, kc, vc, xq, fp, false, nullptr, st);
       if (e) return e;
       if (!lse) lse = fp.lse;
+      if (!carry_tab) carry_tab = fp.carry;
     }
-    // the kernel's producer copies rows of lse / g_denom with 16-byte bulk copies: fp32, 16-byte aligned
+    // The kernels' producers copy rows of lse / g_denom with 16-byte bulk copies: 16-byte aligned, and fp32 but for the sweep that
+    // takes its row term from the output tiles, which widens a bf16 g_denom by itself.  For wide chunks the table holds the row term.
+    const bool out_tiles = !wide && s.D == 64 && out && aligned16(out);
     const float* gd32 = static_cast<const float*>(g_denom_cm);
-    if (g_denom_dtype != UA_F32) {
-      float* tmp = reinterpret_cast<float*>(ws + w.off_gd);
-      const size_t n_gd = BHs * s.N * (size_t)s.R * s.L;
-      widen_bf16_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const bf16*>(g_denom_cm), tmp, n_gd);
+    if (wide) {
+      if ((e = ua::sm100::launch_row_term(ks, m, out, g_out_cm, g_denom_cm, g_denom_dtype, at(w.off_gd), st))) return e;
+      gd32 = at(w.off_gd);
+    } else if (g_denom_dtype != UA_F32 && (!out_tiles || (masked && ks.C == 128) || !aligned16(g_denom_cm))) {
+      const size_t n_gd = (size_t)s.B * s.H * s.N * (size_t)s.R * s.L;
+      widen_bf16_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const bf16*>(g_denom_cm), at(w.off_gd), n_gd);
       if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
-      gd32 = tmp;
+      gd32 = at(w.off_gd);
+    } else if (g_denom_dtype != UA_F32) {
+      gd32 = nullptr;
     }
     if (!aligned16(gd32) || !aligned16(lse) || !aligned16(static_dest) || !aligned16(carry_tab)) return UA_ERR_ALIGNMENT;
-    // Rows before a chunk (uniform softmax): their gradient is added to the accumulators by a kernel of its own.
+    // Rows before a chunk (uniform softmax): their gradient is added to the accumulators by kernels of their own.
     const float* dv_chunk = nullptr;
-    if (!skip_masked && s.N > 1) {
+    if (masked && ks.C == 128) {
       ua::sm100::MaskedParams mp{};
-      mp.s = s; ua::sm100::whole_sequence(mp); mp.g_denom = gd32;
+      mp.s = ks; ua::sm100::whole_sequence(mp); mp.g_denom = gd32; mp.m = m;
       mp.mt = reinterpret_cast<uint8_t*>(ws + w.off_mt);
       mp.ksum = reinterpret_cast<__nv_bfloat16*>(ws + w.off_ksum);
-      mp.nacc = reinterpret_cast<float*>(ws + w.off_nacc);
+      mp.nacc = at(w.off_nacc);
       mp.acc_dk = acc_dk; mp.status = reinterpret_cast<int*>(ws);
       dv_chunk = mp.nacc + (size_t)(s.D + 1) * s.D;
-      e = ua::sm100::launch_masked(s, kc, vc, xq, g_out_cm, acc_dq, mp, st);
-      if (e) return e;
+      if ((e = ua::sm100::launch_masked(ks, kc, vc, xq, g_out_cm, acc_dq, mp, st))) return e;
+    } else if (masked) {
+      // chunks of 64 keys: the generic kernel, for those rows only
+      const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
+      if (!cfg.rt) return UA_ERR_UNSUPPORTED;
+      ua::simt::BwdParams sp{};
+      sp.s = s; sp.kc = kc; sp.vc = vc; sp.xq = xq; sp.ssrc = static_src; sp.sdest = static_dest;
+      sp.g_out = g_out_cm; sp.g_denom = g_denom_cm; sp.g_denom_is_f32 = (g_denom_dtype == UA_F32);
+      sp.acc_dk = acc_dk; sp.acc_dv = at(w.off_dv); sp.acc_dq = acc_dq; sp.acc_ds = at(w.off_ds); sp.acc_dt = at(w.off_dt);
+      sp.rt = cfg.rt; sp.masked_only = 1;
+      if ((e = launch_simt_bwd_any(sp, dtype, gate_dtype, cfg, st))) return e;
     }
     ua::sm100::Bwd2Params qp{};
-    qp.s = s; ua::sm100::whole_sequence(qp); qp.ssrc = static_src; qp.sdest = static_dest;
-    qp.g_denom = gd32;
-    qp.lse = lse; qp.row_lse = nullptr; qp.row_delta = nullptr; qp.carry = carry_tab;
-    qp.acc_dk = acc_dk; qp.acc_dq = acc_dq; qp.acc_dt = acc_dt;
-    qp.acc_dkr = reinterpret_cast<float*>(ws + w.off_dkr);
-    qp.dv_chunk = dv_chunk; qp.dv_chunk_stride = (s.D + 3) * s.D;
+    qp.s = ks; ua::sm100::whole_sequence(qp); qp.ssrc = static_src; qp.sdest = static_dest;
+    qp.g_denom = gd32; qp.g_denom16 = gd32 ? nullptr : static_cast<const bf16*>(g_denom_cm);
+    qp.lse = lse; qp.carry = carry_tab; qp.m = m;
+    qp.acc_dk = acc_dk; qp.acc_dq = acc_dq; qp.acc_dt = nullptr; qp.acc_dkr = at(w.off_dkr);
+    qp.dv_chunk = dv_chunk; qp.dv_chunk_stride = (s.D + 3) * s.D; qp.dv_scale = 1.0f / (float)s.C;
     qp.dvc = static_cast<bf16*>(dvc); qp.dss = dstatic_src; qp.status = reinterpret_cast<int*>(ws);
     qp.trace = nullptr;
-    qp.out_tiles = (out_cm && aligned16(out_cm)) ? out_cm : nullptr;
+    qp.out_tiles = out_tiles ? out : nullptr;
+    if (fp32_v) qp.acc_dv = at(w.off_dv);
+    if (seg) {
+      qp.acc_ds = at(w.off_ds);
+      qp.seg = seg; qp.max_seg = ua::sm100::bwd_max_segments(ks, seg); qp.seg_totals = at(w.off_seg);
+    }
 #ifdef UA_PROFILE_BWD2
     if (const char* tp = getenv("UA_TRACE_PTR")) qp.trace = reinterpret_cast<long long*>(strtoull(tp, nullptr, 0));
 #endif
-    e = ua::sm100::launch_bwd2(s, gate_dtype, false, kc, vc, xq, g_out_cm, qp, st);
-    if (e) return e;
-    if ((e = convert_any(dtype, acc_dk, dkc, BHs * s.L * s.D, st))) return e;
-    if ((e = convert_any(dtype, acc_dq, dxq, BHs * s.R * s.L * s.D, st))) return e;
-    if ((e = convert_any(gate_dtype, acc_dt, dstatic_dest, BHs * s.L, st))) return e;
-    return UA_OK;
+    if ((e = ua::sm100::launch_bwd2(ks, gate_dtype, wide ? 3 : 1, kc, vc, xq, g_out_cm, qp, st))) return e;
+    if (seg) {
+      ua::sm100::Bwd2Params cp = qp;      // what the rows after each segment induce in it
+      cp.heads = 0; cp.acc_dq = nullptr; cp.out_tiles = nullptr;
+      if ((e = ua::sm100::launch_bwd2(ks, gate_dtype, 1, kc, vc, nullptr, nullptr, cp, st))) return e;
+    }
+    return ua::sm100::launch_bwd_finish(ks, gate_dtype, kc, qp, dkc, dxq, dvc, dstatic_src, dstatic_dest, st);
   }
 
   const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
@@ -796,11 +796,7 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
   p.rt = rt;
   p.skip_masked = (flags & UA_FLAG_SKIP_MASKED_GRADS) ? 1 : 0;
   p.masked_only = 0;
-  if (dtype == UA_F32) e = launch_simt_bwd<float, float, float>(p, st);
-  else if (cfg.compact) e = gate_dtype == UA_F32 ? launch_simt_bwd<bf16, float, bf16>(p, st) : launch_simt_bwd<bf16, bf16, bf16>(p, st);
-  else if (gate_dtype == UA_F32) e = launch_simt_bwd<bf16, float, float>(p, st);
-  else e = launch_simt_bwd<bf16, bf16, float>(p, st);
-  if (e) return e;
+  if ((e = launch_simt_bwd_any(p, dtype, gate_dtype, cfg, st))) return e;
 
   const size_t BH = (size_t)s.B * s.H;
   if ((e = convert_any(dtype, p.acc_dk, dkc, BH * s.L * s.D, st))) return e;
@@ -1082,12 +1078,13 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
       !aligned16(dxq))
     return UA_ERR_ALIGNMENT;
   ua::Shape s = to_shape(dims);
-  if (!ua::sm100::bwd2_supported(s, dtype)) return UA_ERR_UNSUPPORTED;
+  if (!ua::sm100::bwd2_supported(s, dtype) || !ua::sm100::chunk128(s)) return UA_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BwdWorkspaceTc w = bwd_layout_tc(s);
+  BwdWorkspaceTc w = bwd_layout_tc(s, 1, 0);
   if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
   char* ws = static_cast<char*>(workspace);
-  if (cudaMemsetAsync(ws, 0, w.acc_bytes, st) != cudaSuccess) return UA_ERR_CUDA;
+  const int seg = ua::sm100::bwd_split(s);
+  if (cudaMemsetAsync(ws, 0, seg ? w.acc_fp32_v_bytes : w.acc_bytes, st) != cudaSuccess) return UA_ERR_CUDA;
   float* carry_tab = carry_in ? const_cast<float*>(static_cast<const float*>(carry_in)) : reinterpret_cast<float*>(ws + w.off_carry);
   if (!carry_in) {
     ua::sm100::FwdParams fp{};
@@ -1102,17 +1099,21 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
   qp.lse = nullptr; qp.row_lse = row_lse; qp.row_delta = row_delta; qp.carry = carry_tab;
   qp.acc_dk = reinterpret_cast<float*>(ws + w.off_dk);
   qp.acc_dq = reinterpret_cast<float*>(ws + w.off_dq);
-  qp.acc_dt = reinterpret_cast<float*>(ws + w.off_dt);
+  qp.acc_dt = nullptr;
   qp.acc_dkr = reinterpret_cast<float*>(ws + w.off_dkr);
   qp.dvc = static_cast<bf16*>(dvc); qp.dss = dstatic_src; qp.status = reinterpret_cast<int*>(ws);
   qp.trace = nullptr;
-  e = ua::sm100::launch_bwd2(s, gate_dtype, true, kc, vc, xq, g_merged, qp, st);
-  if (e) return e;
-  const size_t BHs = (size_t)s.B * s.H;
-  if ((e = convert_any(dtype, qp.acc_dk, dkc, BHs * s.L * s.D, st))) return e;
-  if ((e = convert_any(dtype, qp.acc_dq, dxq, BHs * s.R * s.L * s.D, st))) return e;
-  if ((e = convert_any(gate_dtype, qp.acc_dt, dstatic_dest, BHs * s.L, st))) return e;
-  return UA_OK;
+  if (seg) {
+    qp.acc_dv = reinterpret_cast<float*>(ws + w.off_dv); qp.acc_ds = reinterpret_cast<float*>(ws + w.off_ds);
+    qp.seg = seg; qp.max_seg = ua::sm100::bwd_max_segments(s, seg); qp.seg_totals = reinterpret_cast<float*>(ws + w.off_seg);
+  }
+  if ((e = ua::sm100::launch_bwd2(s, gate_dtype, 2, kc, vc, xq, g_merged, qp, st))) return e;
+  if (seg) {
+    ua::sm100::Bwd2Params cp = qp;
+    cp.heads = 0; cp.acc_dq = nullptr;
+    if ((e = ua::sm100::launch_bwd2(s, gate_dtype, 1, kc, vc, nullptr, nullptr, cp, st))) return e;
+  }
+  return ua::sm100::launch_bwd_finish(s, gate_dtype, kc, qp, dkc, dxq, dvc, dstatic_src, dstatic_dest, st);
 }
 
 int ua_merge_bwd(const UaDims* dims, int dtype, const void* out_cm, const float* lse_cm, const void* g_merged,

@@ -19,10 +19,8 @@ namespace {
 #endif
 template <int D> constexpr int bwd2_cols() { return D == 64 ? UA_BWD2_COLS_64 : UA_BWD2_COLS_128; }
 
-// Backward over the row tiles [p.j_begin, p.j_end) (the caller sets the range fields, e.g. with whole_sequence()).
-// With p.heads == 0 (correction pass) xq, g_out and p.acc_dq are not touched and may be null.
-template <int D, typename TG, int kMode>
-int launch_bwd2_t(const Shape& s, const void* kc, const void* vc, const void* xq, const void* g_out, const Bwd2Params& p,
+template <int D, int kC, typename TG>
+int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, const void* xq, const void* g_out, const Bwd2Params& p,
                   cudaStream_t st) {
   using Cfg = Bwd2Cfg<D>;
   CUtensorMap tmK, tmV, tmQ, tmG, tmDQ, tmDK;
@@ -33,41 +31,89 @@ int launch_bwd2_t(const Shape& s, const void* kc, const void* vc, const void* xq
   if (p.heads == 0) {
     tmQ = tmK; tmG = tmK; tmDQ = tmDK;       // never used
   } else if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D, 64) ||
-             !make_rows_map(&tmG, g_out, (kMode == 2 ? BH : BH * s.N) * s.R * p.Lr, D, 64) ||
+             !make_rows_map(&tmG, g_out, (mode == 2 ? BH : BH * (s.N / p.m)) * s.R * p.Lr, D, 64) ||
              !make_f32_rows_map(&tmDQ, p.acc_dq, BH * s.R * p.Lr, D, 64)) {
     return UA_ERR_CUDA;
   }
   constexpr int kCols = bwd2_cols<D>();
-  auto kern = p.heads > 0 ? bwd2_kernel<D, TG, kMode, kCols, true> : bwd2_kernel<D, TG, kMode, kCols, false>;
   const int threads = 32 * (8 + 4 * (64 / kCols));
-  // the forward's output tiles at hand (per-chunk form, head_dim 64): the row term comes from them
   CUtensorMap tmO = tmG;
-  if constexpr (kMode == 1 && Cfg::kOutTiles) {
-    if (p.heads > 0 && p.out_tiles != nullptr) {
-      if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
-      kern = bwd2_kernel<D, TG, 1, kCols, true, true>;
+  auto kern = bwd2_kernel<D, kC, TG, 1, kCols, false>;
+  if (p.heads > 0) {
+    kern = bwd2_kernel<D, kC, TG, 1, kCols, true>;
+    if constexpr (kC == 128) {
+      if (mode == 2) kern = bwd2_kernel<D, kC, TG, 2, kCols, true>;
+      if (mode == 3) kern = bwd2_kernel<D, kC, TG, 3, kCols, true>;
+    }
+    // the forward's output tiles at hand (per-chunk form, head_dim 64): the row term comes from them
+    if constexpr (Cfg::kOutTiles) {
+      if (mode == 1 && p.out_tiles != nullptr) {
+        if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
+        kern = bwd2_kernel<D, kC, TG, 1, kCols, true, true>;
+      }
     }
   }
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
-  kern<<<(unsigned)(BH * s.N), threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
-  // the row-side dK joins the accumulator; d static_dest of the range's rows comes out of it
-  const int row_begin = p.j_begin * 128, row_end = p.j_end * 128;
-  const long long warps = (long long)BH * (row_end - row_begin);
-  if (warps > 0)
-    row_side_finish_kernel<D, TG><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dt, (int)BH, s.L, p.Lr,
-        p.r0, row_begin, row_end);
+  unsigned per = (unsigned)s.N;
+  if (p.seg) {
+    per = 0;
+    for (int i = 0; i < s.N; ++i) per += ((s.L - i * kC) / 64 + p.seg - 1) / p.seg;
+  }
+  kern<<<(unsigned)BH * per, threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
+  if (p.acc_dt) {
+    // row ranges: the row-side dK joins the accumulator; d static_dest of the range's rows comes out of it
+    const int row_begin = p.j_begin * 128, row_end = p.j_end * 128;
+    const long long warps = (long long)BH * (row_end - row_begin);
+    if (warps > 0)
+      row_side_finish_kernel<D, TG><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(
+          static_cast<const __nv_bfloat16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dt, (int)BH, s.L, p.Lr,
+          p.r0, row_begin, row_end);
+  }
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+
+template <int D, typename TG>
+int launch_finish_t(const Shape& s, const void* kc, const Bwd2Params& p, void* dkc, void* dxq, void* dvc, void* dss, void* ddest, cudaStream_t st) {
+  const int rows = s.B * s.H * s.L, row_blocks = (rows + 8 * 128 / D - 1) / (8 * 128 / D);
+  const size_t dq_vec = (size_t)rows * s.R * D / 8;
+  using bf16 = __nv_bfloat16;
+  bwd_finish_kernel<D, TG><<<(unsigned)(row_blocks + (dq_vec + 255) / 256), 256, 0, st>>>(
+      static_cast<const bf16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dq, p.acc_dv, p.acc_ds, static_cast<bf16*>(dkc),
+      static_cast<bf16*>(dxq), static_cast<bf16*>(dvc), static_cast<TG*>(dss), static_cast<TG*>(ddest), rows, row_blocks, dq_vec);
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
 
 }  // namespace
 
-int launch_bwd2(const Shape& s, int gate_dtype, bool merged, const void* kc, const void* vc, const void* xq,
-                       const void* g_out, const Bwd2Params& p, cudaStream_t st) {
-#define UA_BWD2(D_, TG_) (merged ? launch_bwd2_t<D_, TG_, 2>(s, kc, vc, xq, g_out, p, st) : launch_bwd2_t<D_, TG_, 1>(s, kc, vc, xq, g_out, p, st))
-  if (s.D == 64) return gate_dtype == UA_F32 ? UA_BWD2(64, float) : UA_BWD2(64, __nv_bfloat16);
-  return gate_dtype == UA_F32 ? UA_BWD2(128, float) : UA_BWD2(128, __nv_bfloat16);
+int launch_bwd2(const Shape& s, int gate_dtype, int mode, const void* kc, const void* vc, const void* xq, const void* g_out,
+                const Bwd2Params& p, cudaStream_t st) {
+#define UA_BWD2(D_, C_) (gate_dtype == UA_F32 ? launch_bwd2_t<D_, C_, float>(s, mode, kc, vc, xq, g_out, p, st) \
+                                              : launch_bwd2_t<D_, C_, __nv_bfloat16>(s, mode, kc, vc, xq, g_out, p, st))
+  if (s.C == 64) return s.D == 64 ? UA_BWD2(64, 64) : UA_BWD2(128, 64);
+  return s.D == 64 ? UA_BWD2(64, 128) : UA_BWD2(128, 128);
 #undef UA_BWD2
+}
+
+int launch_bwd_finish(const Shape& s, int gate_dtype, const void* kc, const Bwd2Params& p, void* dkc, void* dxq, void* dvc, void* dss,
+                      void* ddest, cudaStream_t st) {
+#define UA_FINISH(D_) (gate_dtype == UA_F32 ? launch_finish_t<D_, float>(s, kc, p, dkc, dxq, dvc, dss, ddest, st) \
+                                            : launch_finish_t<D_, __nv_bfloat16>(s, kc, p, dkc, dxq, dvc, dss, ddest, st))
+  return s.D == 64 ? UA_FINISH(64) : UA_FINISH(128);
+#undef UA_FINISH
+}
+
+int launch_row_term(const Shape& s, int m, const void* out, const void* g_out, const void* g_denom, int g_denom_dtype, float* table, cudaStream_t st) {
+  const int n = s.N / m;
+  const long long rows = (long long)s.B * s.H * n * s.R * s.L;
+  const int per = 256 / (s.D / 8);
+  const unsigned blocks = (unsigned)((rows + per - 1) / per);
+  const auto* o = static_cast<const __nv_bfloat16*>(out);
+  const auto* g = static_cast<const __nv_bfloat16*>(g_out);
+#define UA_ROW_TERM(D_, TD_) row_term_kernel<D_, TD_><<<blocks, 256, 0, st>>>(o, g, static_cast<const TD_*>(g_denom), table, n, s.R, s.L, s.C * m, rows)
+  if (s.D == 64) { if (g_denom_dtype == UA_F32) UA_ROW_TERM(64, float); else UA_ROW_TERM(64, __nv_bfloat16); }
+  else { if (g_denom_dtype == UA_F32) UA_ROW_TERM(128, float); else UA_ROW_TERM(128, __nv_bfloat16); }
+#undef UA_ROW_TERM
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
 
 namespace {
@@ -79,15 +125,15 @@ int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* 
   using Cfg = MkCfg<D>;
   const uint64_t BH = (uint64_t)s.B * s.H;
   CUtensorMap tmQ, tmG, tmDQ;
-  if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D) || !make_rows_map(&tmG, g_out, BH * s.N * s.R * p.Lr, D) ||
+  if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D) || !make_rows_map(&tmG, g_out, BH * (s.N / p.m) * s.R * p.Lr, D) ||
       !make_f32_rows_map(&tmDQ, acc_dq, BH * s.R * p.Lr, D))
     return UA_ERR_CUDA;
   static const int jp_env = []() { const char* e = getenv("UA_MASKED_TILES"); return e ? atoi(e) : 0; }();
   p.jp = jp_env > 0 ? jp_env : 8;
   p.items_per_bh = 0;
-  const int jcap = (s.N - 1 < p.j_end) ? s.N - 1 : p.j_end;      // no row tile at or after the last chunk is before any chunk
+  const int last = (s.N - 1) / p.m * p.m, jcap = (last < p.j_end) ? last : p.j_end;      // no row tile at or after the last chunk is before any chunk
   for (int g = 0; g * Cfg::kG < s.N; ++g) {
-    int jmax = (((g + 1) * Cfg::kG < s.N) ? (g + 1) * Cfg::kG : s.N) - 1;
+    int jmax = ((((g + 1) * Cfg::kG < s.N) ? (g + 1) * Cfg::kG : s.N) - 1) / p.m * p.m;
     if (jmax > jcap) jmax = jcap;
     if (jmax > p.j_begin) p.items_per_bh += (jmax - p.j_begin + p.jp - 1) / p.jp;
   }

@@ -1,5 +1,5 @@
 // Tensor-core backward of the Universal Attention operator for sm_100a, keys-on-lanes form
-// (bf16, key chunk = 128, head_dim 64 or 128).  Needs the log-sum-exp of the forward.
+// (bf16, key chunk kC = 128 or 64, head_dim 64 or 128).  Needs the log-sum-exp of the forward.
 //
 // One thread block owns one key chunk (b, h, i) and sweeps the rows that see it DOWNWARDS in
 // half tiles of 64 rows, so that the reverse cumulative sum of the decay gradient is carried
@@ -30,6 +30,15 @@
 // dQ_rj / dK_j (64 rows, M = 128 MMAs whose upper 64 lanes compute on whatever the next buffer holds and are
 // never read) leave as TMA reduce-adds into fp32 accumulators.  Rows BEFORE the chunk are not handled here.
 //
+// kC = 64: the keys are TMEM lanes 0..63; lanes 64..127 compute on what lies behind the 64 rows in shared memory and are
+// never read, sums over the keys take 64 of them.
+// Segments (p.seg > 0): where one block per chunk leaves the chip idle, a sweep is cut into blocks of p.seg half tiles, each
+// with a zero reverse carry; every gradient is linear in that carry, so the correction pass (the same kernel without heads)
+// adds what the rows after a segment induce, from the totals that the segments leave (see bwd_split for when).
+// Wide chunks (p.m > 1): a chunk of m * 128 keys is m blocks of 128.  Only the row tables and the upstream gradient are the
+// chunk's: with the chunk's log-sum-exp P = exp(s - lse) needs nothing from the other blocks, and the row term arrives
+// in the table (mode 3).
+//
 // Every mbarrier wait is bounded; on a timeout the block raises a shared abort flag, every role
 // leaves, TMEM is freed and status[0] is set (status[1]: where the first block gave up).
 #pragma once
@@ -44,17 +53,18 @@ struct Bwd2Params {
   Shape s;
   const void* ssrc;
   const void* sdest;
-  const float* g_denom;      // (b,h,n,r,L) fp32                             [mode 1]
-  const float* lse;          // (b,h,n,r,L) fp32: the forward's log-sum-exp   [mode 1]
+  const float* g_denom;      // (b,h,n,r,L) fp32; in mode 3 the final row term g_denom - out . dO   [modes 1, 3]
+  const float* lse;          // (b,h,n,r,L) fp32: the forward's log-sum-exp   [modes 1, 3]
   const float* row_lse;      // (b,h,r,L) fp32: log-sum-exp over all keys     [mode 2]
   const float* row_delta;    // (b,h,r,L) fp32: g . merged                    [mode 2]
-  const float* carry;        // (b*h*n, n, 2, 128): decay prefix of key k at the start of each 64-row half tile
+  const float* carry;        // (b*h*n, L / 64, 128): decay prefix of key k at the start of each 64-row half tile
   float* acc_dk;             // (b*h, L, D) fp32, zeroed (or holding the masked-block part)
   float* acc_dq;             // (b*h, r, L, D) fp32, likewise
   float* acc_dt;             // (b*h, Lr) fp32: d static_dest is ADDED here (by row_side_finish_kernel, after the sweep)
   float* acc_dkr;            // (b*h, L, D) fp32 scratch, zeroed: the row-side dK_j = dG^T K_i of all chunks (see there)
-  const float* dv_chunk;     // optional: row dv_chunk[chunk * dv_chunk_stride + d] / 128 is added to every key's dV_i (the
+  const float* dv_chunk;     // optional: row dv_chunk[chunk * dv_chunk_stride + d] * dv_scale is added to every key's dV_i (the
   int dv_chunk_stride;       // masked-block part when it comes from the kernels of the rows before a chunk)
+  float dv_scale;            // 1 / keys of the operator's chunk
   __nv_bfloat16* dvc;
   void* dss;
   int* status;
@@ -72,6 +82,10 @@ struct Bwd2Params {
   // softmax-gradient row term sum_k P dP is the dot product of a row's output and its upstream gradient (P V = out), which
   // two otherwise idle warps form ahead of the workers; without them the workers sum P dP over the keys themselves.
   const void* out_tiles;
+  const __nv_bfloat16* g_denom16;   // output-tile builds: g_denom as bf16 instead of fp32 (the row-dot warps widen it)
+  int m;                     // kernel chunks per chunk of the operator (1, or chunk / 128)
+  int seg, max_seg;          // half tiles per block (0: whole sweeps), and the row stride of seg_totals
+  float* seg_totals;         // (b*h*n, max_seg, 128): sum of dC per key over each segment's rows, written by the pass with heads, read by the other
 };
 
 template <int D>
@@ -109,7 +123,8 @@ struct Bwd2Cfg {
   // scratch tiles would be, and sum the decay gradient's columns with shuffles
   static constexpr bool kOutTiles = kScratch;
   static constexpr int oOut = (oScr + 1023) / 1024 * 1024;
-  static_assert(!kOutTiles || oOut + kNS * kHalf <= oScr + 40960, "output tiles fit the scratch area");
+  static constexpr int oGd16 = oOut + kNS * kHalf;         // kNS x bf16[64]: g_denom rows of a head before they are widened
+  static_assert(!kOutTiles || oGd16 + kNS * 128 <= oScr + 40960, "output tiles fit the scratch area");
   // TMEM columns
   static constexpr uint32_t tDV = 0, tDK = D, tY = 2 * D;
   static constexpr uint32_t tS0 = (D == 64) ? 192 : 384, tP0 = tS0 + 64, tS1 = tS0 + 128, tP1 = tS0 + 192;
@@ -139,7 +154,8 @@ struct Bwd2Ctx {
   uint32_t tmem;
   volatile int* abort_flag;
   int i, bh, nht;
-  int jtop, jb, r0;          // the sweep starts at row tile jtop - 1; the slabs hold row tile jb at row r0
+  int htop, jb, r0;          // the sweep starts at half tile htop - 1 (64 rows each); the slabs hold row tile jb at row r0
+  int segment;               // number of this block's segment, counted from the end of the sequence
   __device__ __forceinline__ uint32_t bar(int idx) const { return bars + 8u * idx; }
   __device__ __forceinline__ void note_failure(int idx, uint32_t parity) const {
     atomicCAS(const_cast<int*>(abort_flag) + 1, 0, (idx + 1) | ((int)threadIdx.x << 8) | ((int)(parity & 0x7ff) << 20));
@@ -155,12 +171,9 @@ struct Bwd2Ctx {
     return ok;
   }
   __device__ __forceinline__ void arrive_w(int idx) const { mbar_arrive_warp(bar(idx)); }
-  // half tile ht of the sweep: row tile j (descending), upper half first
-  __device__ __forceinline__ int tile_j(int ht) const { return jtop - 1 - (ht >> 1); }
-  __device__ __forceinline__ int half_of(int ht) const { return 1 - (ht & 1); }
-  // first row of half tile ht: in the sequence (keys of the same positions, the diagonal), and inside the slabs
-  __device__ __forceinline__ int row0_of(int ht) const { return tile_j(ht) * 128 + 64 * half_of(ht); }
-  __device__ __forceinline__ int srow0_of(int ht) const { return r0 + (tile_j(ht) - jb) * 128 + 64 * half_of(ht); }
+  // first row of half tile ht (descending): in the sequence (keys of the same positions, the diagonal), and inside the slabs
+  __device__ __forceinline__ int row0_of(int ht) const { return (htop - 1 - ht) * 64; }
+  __device__ __forceinline__ int srow0_of(int ht) const { return r0 + row0_of(ht) - jb * 128; }
 };
 
 // Optional phase timing (compile with -DUA_PROFILE_BWD2): thread 0 of worker warp 4 of block UA_PROFILE_BLOCK accumulates
@@ -214,19 +227,19 @@ __device__ __forceinline__ void mma4_ts(uint32_t d, uint32_t a0, uint32_t a1, ui
 }
 
 // ------------------------------------------------------------- TMA producer --
-template <int D, typename TG, int kMode, bool kOutDelta>
+template <int D, int kC, typename TG, int kMode, bool kOutDelta>
 __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params& p, const CUtensorMap* tmK, const CUtensorMap* tmV,
                                               const CUtensorMap* tmQ, const CUtensorMap* tmG, const CUtensorMap* tmO) {
   using Cfg = Bwd2Cfg<D>;
   const int L = p.s.L, R = p.s.R, N = p.s.N;
   const uint32_t sb = smem_u32(c.smem);
-  const int krow = c.bh * L + c.i * 128;
-  const size_t chunk_id = (size_t)c.bh * N + c.i;
-  mbar_expect_tx(c.bar(qKvFull), 2 * Cfg::kFull);
+  const int krow = c.bh * L + c.i * kC;
+  const size_t chunk_id = (size_t)c.bh * N + c.i, out_chunk = p.m > 1 ? (size_t)c.bh * (N / p.m) + c.i / p.m : chunk_id;
+  mbar_expect_tx(c.bar(qKvFull), 2 * Cfg::kFull * kC / 128);
 #pragma unroll
   for (int b = 0; b < Cfg::kBoxes; ++b)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < kC / 64; ++h) {
       tma_load_2d(sb + Cfg::oKi + b * 16384 + h * 8192, tmK, b * 64, krow + h * 64, c.bar(qKvFull));
       tma_load_2d(sb + Cfg::oVi + b * 16384 + h * 8192, tmV, b * 64, krow + h * 64, c.bar(qKvFull));
     }
@@ -240,7 +253,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
     // (the correction pass has no heads and needs no decay prefix: only the gate values travel)
     mbar_expect_tx(c.bar(qTabFull + tb), (Rh > 0 ? 512u : 0u) + 64 * (uint32_t)sizeof(TG));
     if (Rh > 0)
-      bulk_load_1d(dst, p.carry + ((chunk_id * N + c.tile_j(ht)) * 2 + c.half_of(ht)) * 128, 512, c.bar(qTabFull + tb));
+      bulk_load_1d(dst, p.carry + (chunk_id * (L / 64) + c.row0_of(ht) / 64) * 128, 512, c.bar(qTabFull + tb));
     bulk_load_1d(dst + 512, sd + c.srow0_of(ht), 64 * (uint32_t)sizeof(TG), c.bar(qTabFull + tb));
     return true;
   };
@@ -263,9 +276,10 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
       const int sl = hc % Cfg::kNS, use = hc / Cfg::kNS;
       if (use >= 1 && !c.wait(qInFree + sl, use - 1)) return;
       const int qrow = (c.bh * R + r) * p.Lr + srow0;
-      const int grow = (kMode == 2) ? qrow : (int)((chunk_id * R + r) * p.Lr + srow0);
+      const int grow = (kMode == 2) ? qrow : (int)((out_chunk * R + r) * p.Lr + srow0);
       const uint32_t dst = sb + Cfg::oSlot + sl * Cfg::kSlot, tab = sb + Cfg::oHeadTab + sl * 512;
-      mbar_expect_tx(c.bar(qInFull + sl), (kOutDelta ? 3 : 2) * Cfg::kHalf + 512);
+      const bool gd16 = kOutDelta && p.g_denom16 != nullptr;
+      mbar_expect_tx(c.bar(qInFull + sl), (kOutDelta ? 3 : 2) * Cfg::kHalf + (gd16 ? 384 : 512));
       if (kOutDelta) tma_load_2d(sb + Cfg::oOut + sl * Cfg::kHalf, tmO, 0, grow, c.bar(qInFull + sl));
 #pragma unroll
       for (int b = 0; b < Cfg::kBoxes; ++b) {
@@ -277,7 +291,8 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
         bulk_load_1d(tab + 256, p.row_delta + qrow, 256, c.bar(qInFull + sl));
       } else {
         bulk_load_1d(tab, p.lse + grow, 256, c.bar(qInFull + sl));
-        bulk_load_1d(tab + 256, p.g_denom + grow, 256, c.bar(qInFull + sl));
+        if (gd16) bulk_load_1d(sb + Cfg::oGd16 + sl * 128, p.g_denom16 + grow, 128, c.bar(qInFull + sl));
+        else bulk_load_1d(tab + 256, p.g_denom + grow, 256, c.bar(qInFull + sl));
       }
     }
   }
@@ -355,7 +370,7 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
 // which = 0: the accumulators that live for the whole sweep (dV_i += P dO, dK_i += dS Q, dK_i += dG K_j);
 // which = 1: the row-side results that leave after every unit (Y = dQ_rj = dS^T K_i, Y = dK_j = dG^T K_i).
 // MMAs into one accumulator always come from the same thread, so their order is kept.
-template <int D, int CG>
+template <int D, int kC, int CG>
 __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p, const int which) {
   using Cfg = Bwd2Cfg<D>;
   const int R = p.heads;
@@ -371,7 +386,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   // after the tile and are never read
   auto mma_rows_out = [&](uint64_t t_mn) {
     mma4_ss(Y, t_mn, mKi, 128, 128, id_tn, 0);
-    mma4_ss(Y, t_mn + 512, mKi + 512, 128, 128, id_tn, 1);
+    if (kC == 128) mma4_ss(Y, t_mn + 512, mKi + 512, 128, 128, id_tn, 1);
   };
   if (!c.wait(qKvFull, 0)) return;
   UQ_DECL
@@ -604,7 +619,8 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
       dot_bf16x8(*reinterpret_cast<const uint4*>(oo + off), *reinterpret_cast<const uint4*>(go + off), lo, hi);
     }
     float* tabC = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512) + 64;
-    tabC[row] -= lo + hi;
+    const float gd = p.g_denom16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(c.smem + Cfg::oGd16 + sl * 128)[row]) : tabC[row];
+    tabC[row] = gd - (lo + hi);
     c.arrive_w(qDelta + sl);
   }
 }
@@ -613,12 +629,13 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
 // kHeads = false: the correction pass (p.heads == 0).  A compile-time switch: as a run-time condition around the decay
 // recomputation it cost the whole-sequence kernel 2 % (measured).
 // kOutDelta: the row term comes from the delta warps (see bwd2_delta).
-template <int D, typename TG, int kMode, int CG, bool kHeads, bool kOutDelta>
+template <int D, int kC, typename TG, int kMode, int CG, bool kHeads, bool kOutDelta>
 __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& p) {
   using Cfg = Bwd2Cfg<D>;
   constexpr int NG = 64 / CG;                    // column groups
   constexpr int H2 = CG / 2;                     // packed pairs per thread
-  constexpr int kWorkers = 128 * NG;
+  constexpr int kWorkers = kC * NG;
+  constexpr int kGateQuad = kC / 64;             // the quadrant whose warps fetch the gates of the next half tile
   const int L = p.s.L, R = kHeads ? p.heads : 0, N = p.s.N;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = (warp - 8) >> 2;                 // column group: columns [CG g, CG g + CG) of a half tile
@@ -630,7 +647,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   const float kLog2e = 1.4426950408889634f;
   const float2 kLog2e2 = make_float2(kLog2e, kLog2e), kNegLog2e2 = make_float2(-kLog2e, -kLog2e);
   const TG* ss = static_cast<const TG*>(p.ssrc) + (size_t)c.bh * L;
-  const float s3 = cbrtf(Num<TG>::ld(ss + c.i * 128 + key));
+  if (key >= kC) return;                         // (kC = 64: half of the worker warps hold no key)
+  const float s3 = cbrtf(Num<TG>::ld(ss + c.i * kC + key));
   const float2 s32 = make_float2(s3, s3);
   float* sT3 = reinterpret_cast<float*>(c.smem + Cfg::oT3);
   float* sXch = reinterpret_cast<float*>(c.smem + Cfg::oXch);
@@ -670,15 +688,17 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
 
   // ---- prologue: static_dest^(1/3) of the first half tile ----
   if (!c.wait_w(qTabFull, 0)) return;
-  if (helper && quad == 2) sT3[col0 + lane] = t3_from_table(0);
+  if (helper && quad == kGateQuad) sT3[col0 + lane] = t3_from_table(0);
   float suffix = p.suffix_in ? p.suffix_in[((size_t)c.bh * N + c.i) * 128 + key] : 0.f, ds_acc = 0.f;
+  if (!kHeads && p.seg)                          // what the segments of later rows leave
+    for (int q = 0; q < c.segment; ++q) suffix += p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + q) * 128 + key];
   named_bar_sync(kBarAll, kWorkers);
 
   int u = 0, hc = 0;
   for (int ht = 0; ht < c.nht; ++ht) {
-    const int j = p.j_end - 1 - (ht >> 1), half = c.half_of(ht);
-    const bool diag = (j == c.i);
-    const int qbase = 64 * half + col0;            // row of this thread's first column inside the 128-row tile
+    const int rel = c.row0_of(ht) - c.i * kC;
+    const bool diag = rel < kC;                    // rows at positions of the chunk's own keys
+    const int qbase = rel + col0;                  // this thread's first row, counted from the chunk's first key
     const float* t3v = sT3 + (ht & 1) * 64 + col0;
 
     // ================= decay recomputation: c2 = log2(e) * decay prefix of (key, CG rows) =================
@@ -823,7 +843,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       if (kOutDelta) {
         if (!c.wait_w(qDelta + sl, hc / Cfg::kNS)) return;
       } else if (kColSums) {
-        named_bar_sync(kBarGroup + g, 128);           // the group's column sums are complete
+        named_bar_sync(kBarGroup + g, kC);           // the group's column sums are complete
       }
       UQ(4)
       {
@@ -858,7 +878,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         dc[x].x = run;
       }
       sXch[(NG + g) * 128 + key] = run;
-      if (more && quad == 2) {                   // static_dest^(1/3) of the next half tile's rows
+      if (more && quad == kGateQuad) {                   // static_dest^(1/3) of the next half tile's rows
         if (!c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
         if (helper) sT3[((ht + 1) & 1) * 64 + col0 + lane] = t3_from_table(ht + 1);
       }
@@ -943,7 +963,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   // ---- end of the sweep: dV_i, dK_i, d static_src (thread = key, D / NG columns each) ----
   if (!c.wait_w(qFinal, 0)) return;
   tc_fence_after();
-  const size_t krow = (size_t)c.bh * L + c.i * 128 + key;
+  const size_t krow = (size_t)c.bh * L + c.i * kC + key;
+  if (kHeads && g == 0 && p.seg) p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + c.segment) * 128 + key] = suffix;
   if (g == 0 && p.dctot_out) {                     // the range's own dC: what left minus what came in from the rows after it
     const size_t key_id = ((size_t)c.bh * N + c.i) * 128 + key;
     p.dctot_out[key_id] = suffix - (p.suffix_in ? p.suffix_in[key_id] : 0.f);
@@ -956,15 +977,15 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     if (kHeads) {                                  // (the correction pass has no heads: no dV)
     tmem_ld16(c.tmem + Cfg::tDV + lane_base + d0, o);
     tc_wait_ld();
-    if (p.dv_chunk) {
+    if (p.dv_chunk && c.segment == 0) {
       const float4* extra = reinterpret_cast<const float4*>(p.dv_chunk + ((size_t)c.bh * p.s.N + c.i) * p.dv_chunk_stride + d0);
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         const float4 ev = extra[x];
-        o[4 * x] = __float_as_uint(fmaf(ev.x, 1.0f / 128.0f, __uint_as_float(o[4 * x])));
-        o[4 * x + 1] = __float_as_uint(fmaf(ev.y, 1.0f / 128.0f, __uint_as_float(o[4 * x + 1])));
-        o[4 * x + 2] = __float_as_uint(fmaf(ev.z, 1.0f / 128.0f, __uint_as_float(o[4 * x + 2])));
-        o[4 * x + 3] = __float_as_uint(fmaf(ev.w, 1.0f / 128.0f, __uint_as_float(o[4 * x + 3])));
+        o[4 * x] = __float_as_uint(fmaf(ev.x, p.dv_scale, __uint_as_float(o[4 * x])));
+        o[4 * x + 1] = __float_as_uint(fmaf(ev.y, p.dv_scale, __uint_as_float(o[4 * x + 1])));
+        o[4 * x + 2] = __float_as_uint(fmaf(ev.z, p.dv_scale, __uint_as_float(o[4 * x + 2])));
+        o[4 * x + 3] = __float_as_uint(fmaf(ev.w, p.dv_scale, __uint_as_float(o[4 * x + 3])));
       }
     }
     if (p.acc_dv) {                                // several row ranges add to the same keys
@@ -1004,7 +1025,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   }
 }
 
-template <int D, typename TG, int kMode, int CG, bool kHeads, bool kOutDelta = false>
+template <int D, int kC, typename TG, int kMode, int CG, bool kHeads, bool kOutDelta = false>
 __global__ void __launch_bounds__(32 * (8 + 4 * (64 / CG)), 1)
 bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
             const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
@@ -1023,10 +1044,28 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   c.smem = smem;
   c.bars = smem_u32(smem + Cfg::oBar);
   c.abort_flag = reinterpret_cast<volatile int*>(misc + 1);
-  c.i = blockIdx.x / BH;                       // heavy chunks (small i: most rows) first
-  c.bh = blockIdx.x - c.i * BH;
-  c.jtop = p.j_end; c.jb = p.j_begin; c.r0 = p.r0;
-  c.nht = 2 * (p.j_end - (c.i > p.j_begin ? c.i : p.j_begin));
+  // heavy chunks (small i: most rows) first
+  int x = blockIdx.x / BH;
+  c.bh = blockIdx.x - x * BH;
+  c.jb = p.j_begin; c.r0 = p.r0;
+  c.segment = 0;
+  if (p.seg == 0) {
+    c.i = x;
+    c.htop = kC == 128 ? 2 * p.j_end : p.s.L / 64;
+    c.nht = c.htop - (kC == 128 ? 2 * (c.i > p.j_begin ? c.i : p.j_begin) : c.i);
+  } else {
+    int nht;
+    for (c.i = 0;; ++c.i) {
+      nht = (p.s.L - c.i * kC) / 64;
+      const int ns = (nht + p.seg - 1) / p.seg;
+      if (x < ns) break;
+      x -= ns;
+    }
+    c.segment = x;
+    c.htop = p.s.L / 64 - x * p.seg;
+    c.nht = nht - x * p.seg < p.seg ? nht - x * p.seg : p.seg;
+    if (!kHeads && x == 0) return;             // no rows after the last segment
+  }
   if (c.nht <= 0) {
     // no row of the range sees this chunk (sequence sharding only): nothing to add anywhere
     if (p.dctot_out && threadIdx.x < 128) p.dctot_out[((size_t)c.bh * p.s.N + c.i) * 128 + threadIdx.x] = 0.f;
@@ -1038,7 +1077,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     misc[2] = 0;
     for (int b = 0; b < qNumBars; ++b) {
       uint32_t count = 1;
-      if (b == qLdDone || b == qLdDone + 1 || b == qDsReady || b == qDsReady + 1 || b == qDgReady) count = 4 * NG;   // one arrival per worker warp
+      if (b == qLdDone || b == qLdDone + 1 || b == qDsReady || b == qDsReady + 1 || b == qDgReady) count = kC / 32 * NG;   // one arrival per worker warp
       if (b == qYFree || (b >= qDelta && b < qDelta + 4)) count = 2;                                                                                  // the two draining warps
       if (b == qDsFree || b == qDsFree + 1 || b == qDgFree || b == qFinal) count = 2;                               // both back issuers
       mbar_init(c.bar(b), count);
@@ -1075,9 +1114,9 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
     if (lane == 0) {
       if (warp == 0) bwd2_front<D>(c, p);
-      else if (warp == 1) bwd2_back<D, CG>(c, p, 0);
-      else if (warp == 2) bwd2_producer<D, TG, kMode, kOutDelta>(c, p, &tmK, &tmV, &tmQ, &tmG, &tmO);
-      else bwd2_back<D, CG>(c, p, 1);
+      else if (warp == 1) bwd2_back<D, kC, CG>(c, p, 0);
+      else if (warp == 2) bwd2_producer<D, kC, TG, kMode, kOutDelta>(c, p, &tmK, &tmV, &tmQ, &tmG, &tmO);
+      else bwd2_back<D, kC, CG>(c, p, 1);
     }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
@@ -1085,7 +1124,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     else if (kOutDelta) bwd2_rowdots<D>(c, p);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
-    bwd2_worker<D, TG, kMode, CG, kHeads, kOutDelta>(c, p);
+    bwd2_worker<D, kC, TG, kMode, CG, kHeads, kOutDelta>(c, p);
   }
 
   tc_fence_before();
@@ -1141,6 +1180,72 @@ row_side_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restric
     const size_t grow = (size_t)bh * Lr + r0 + rr;
     acc_dt[grow] += 0.5f * dot / Num<TG>::ld(sdest + grow);
   }
+}
+
+// ... and, for a whole sequence, everything that is left to do in one launch: blocks [0, row_blocks): one warp per row of K as
+// above, with dK (accumulator + row side), d static_dest and, where the sweep added them up in fp32, dV and d static_src leaving
+// in their own types; the other blocks: dQ, eight elements per thread.
+template <int D, typename TG>
+__global__ void __launch_bounds__(256)
+bwd_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restrict__ sdest, const float* __restrict__ dkr,
+                  const float* __restrict__ acc_dk, const float* __restrict__ acc_dq, const float* __restrict__ acc_dv,
+                  const float* __restrict__ acc_ds, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dq,
+                  __nv_bfloat16* __restrict__ dv, TG* __restrict__ ds, TG* __restrict__ dt, int rows, int row_blocks, size_t dq_vec) {
+  auto pack2 = [](float a, float b) -> uint32_t {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  if ((int)blockIdx.x >= row_blocks) {
+    const size_t at = (size_t)(blockIdx.x - row_blocks) * 256 + threadIdx.x;
+    if (at >= dq_vec) return;
+    const float4 a = reinterpret_cast<const float4*>(acc_dq)[2 * at], b = reinterpret_cast<const float4*>(acc_dq)[2 * at + 1];
+    reinterpret_cast<uint4*>(dq)[at] = make_uint4(pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w));
+    return;
+  }
+  // D / 4 lanes per row: 16-byte reads of the accumulators
+  constexpr int kLanes = D / 4, kRows = 32 / kLanes;
+  const int lane = threadIdx.x & 31, sub = lane % kLanes;
+  const int row = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kRows + lane / kLanes;
+  const bool live = row < rows;
+  const size_t at = (size_t)(live ? row : rows - 1) * D + sub * 4;
+  const float4 r = *reinterpret_cast<const float4*>(dkr + at), acc = *reinterpret_cast<const float4*>(acc_dk + at);
+  const uint2 kk = *reinterpret_cast<const uint2*>(kc + at);
+  float dot = fmaf(r.x, __uint_as_float(kk.x << 16), fmaf(r.y, __uint_as_float(kk.x & 0xffff0000u),
+              fmaf(r.z, __uint_as_float(kk.y << 16), r.w * __uint_as_float(kk.y & 0xffff0000u))));
+#pragma unroll
+  for (int o = kLanes / 2; o >= 1; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if (!live) return;
+  *reinterpret_cast<uint2*>(dk + at) = make_uint2(pack2(acc.x + r.x, acc.y + r.y), pack2(acc.z + r.z, acc.w + r.w));
+  if (acc_dv) {
+    const float4 v = *reinterpret_cast<const float4*>(acc_dv + at);
+    *reinterpret_cast<uint2*>(dv + at) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+  }
+  if (sub == 0) {
+    Num<TG>::st(dt + row, dot != 0.f ? 0.5f * dot / Num<TG>::ld(sdest + row) : 0.f);
+    if (acc_ds) Num<TG>::st(ds + row, acc_ds[row]);
+  }
+}
+
+// The row term of the softmax gradient as a table, for chunks whose keys are spread over several blocks (mode 3):
+//   table[chunk][head][row] = g_denom - out . dO      for the rows that see the chunk, g_denom for those before it.
+// Reads the output and its gradient once where they matter; 16 bytes of a row per thread.
+template <int D, typename TD>
+__global__ void __launch_bounds__(256)
+row_term_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ g_out, const TD* __restrict__ g_denom,
+                float* __restrict__ table, int N, int R, int L, int chunk, long long rows) {
+  constexpr int kLanes = D / 8, kRows = 256 / kLanes;
+  const long long first = (long long)blockIdx.x * kRows + threadIdx.x / kLanes, at = first < rows ? first : rows - 1;
+  const int sub = threadIdx.x % kLanes;
+  const int row = (int)(at % L), i = (int)(at / ((long long)L * R) % N);
+  float dot = 0.f;
+  if (row >= i * chunk) {
+    float hi = 0.f;
+    dot_bf16x8(__ldcs(reinterpret_cast<const uint4*>(out + at * D + sub * 8)), *reinterpret_cast<const uint4*>(g_out + at * D + sub * 8), dot, hi);
+    dot += hi;
+  }
+#pragma unroll
+  for (int o = kLanes / 2; o >= 1; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if (first < rows && sub == 0) table[at] = Num<TD>::ld(g_denom + at) - dot;
 }
 
 }  // namespace sm100

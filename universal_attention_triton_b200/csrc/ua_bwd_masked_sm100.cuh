@@ -18,6 +18,8 @@
 // w_c += gd_c^T Q_rj from the Q tile in shared memory, and the drain warps add gd_c (x) ksum_c / 128 to Y on its way out.
 // head_dim 128 runs as two blocks per work item, one per 64-wide half of the output columns of Y / lanes of Nt.
 // A work item is (batch*head, group of G chunks, range of row tiles); partial N / w / u leave as fp32 global adds.
+// Chunks of m * 128 keys come as m neighbouring "chunks" of 128 here (p.m): vbar and the weight 1 / (128 m) are the whole
+// chunk's, and all m read the same gradient rows, those before the whole chunk.
 #pragma once
 #include "ua_fwd_sm100.cuh"
 
@@ -37,6 +39,7 @@ struct MaskedParams {
   // Range of row tiles [j_begin, j_end) (sequence-chunk sharding; whole sequence: 0, N, L, 0): xq, g_out, g_denom and
   // the dQ accumulator are slabs of Lr rows that hold the range at row r0.
   int j_begin, j_end, Lr, r0;
+  int m;                         // kernel chunks per chunk of the operator
   float* acc_dv;                 // row ranges only: (b*h, L, D) fp32, dV_i = 1 (x) u_i / 128 is ADDED here by the finish kernel
 };
 
@@ -93,7 +96,10 @@ struct MkCtx {
   }
   __device__ __forceinline__ void arrive_w(int idx) const { mbar_arrive_warp(bar(idx)); }
   // first chunk of the group that has row tile j before it
-  __device__ __forceinline__ int clo(int j) const { return max(0, j + 1 - i0); }
+  __device__ __forceinline__ int clo(int j) const { return max(0, m * (j / m + 1) - i0); }
+  int m;
+  // the operator's chunk that chunk c of the group belongs to, in the gradient tensors
+  __device__ __forceinline__ size_t out_chunk(int N, int cc) const { return m == 1 ? (size_t)bh * N + i0 + cc : (size_t)bh * (N / m) + (i0 + cc) / m; }
   int jb, r0;                          // the slabs hold row tile jb at row r0
   __device__ __forceinline__ int srow(int j) const { return r0 + (j - jb) * 128; }
 };
@@ -118,7 +124,7 @@ template <int D> struct MkDense {
 
 // ------------------------------------------------------------------ prep kernel --
 // One block per chunk: ksum / 128 (bf16), M^T / 128 (bf16, in the swizzled layout the sweep kernel's MMAs read), and the
-// chunk's N / w / u accumulators set to zero.  M = K^T V - ksum (x) vsum / 128 from exact bf16 products with fp32 sums.
+// chunk's N / w / u accumulators set to zero.  M = K^T V - ksum (x) vbar from exact bf16 products with fp32 sums.
 template <int D>
 __global__ void __launch_bounds__(256) masked_prep_kernel(const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                                                           MaskedParams p) {
@@ -129,6 +135,7 @@ __global__ void __launch_bounds__(256) masked_prep_kernel(const __nv_bfloat16* _
   float* sSum = reinterpret_cast<float*>(sV + 128 * Dn::kStride);
   const size_t chunk = blockIdx.x;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const float scale = 1.0f / (float)(128 * p.m);
   float* nacc = p.nacc + chunk * (size_t)kNaccRows<D>() * D;
   const uint4* gk = reinterpret_cast<const uint4*>(kc + chunk * 128 * D);
   const uint4* gv = reinterpret_cast<const uint4*>(vc + chunk * 128 * D);
@@ -145,9 +152,16 @@ __global__ void __launch_bounds__(256) masked_prep_kernel(const __nv_bfloat16* _
     float acc = 0.f;
 #pragma unroll 16
     for (int k = 0; k < 128; ++k) acc += __bfloat162float(src[k * Dn::kStride]);
+    if (t >= D && p.m > 1) {             // the values of the whole chunk
+      const __nv_bfloat16* v0 = vc + chunk / p.m * p.m * 128 * D + (t - D);
+      acc = 0.f;
+#pragma unroll 16
+      for (int k = 0; k < p.m * 128; ++k) acc += __bfloat162float(v0[(size_t)k * D]);
+    }
+    if (t >= D) acc *= scale;            // vbar
     sSum[t] = acc;
-    if (t < D) p.ksum[chunk * D + t] = __float2bfloat16_rn(acc * (1.0f / 128.0f));
-    else nacc[(size_t)(D + 2) * D + (t - D)] = acc * (1.0f / 128.0f);
+    if (t < D) p.ksum[chunk * D + t] = __float2bfloat16_rn(acc * scale);
+    else nacc[(size_t)(D + 2) * D + (t - D)] = acc;
   }
   // M^T: warp = 16 rows d' x kCols columns d
   constexpr int kMT = D / 16, kSplit = 8 / kMT, kCols = D / kSplit;
@@ -174,12 +188,12 @@ __global__ void __launch_bounds__(256) masked_prep_kernel(const __nv_bfloat16* _
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int dp = m0 + (lane >> 2) + 8 * h, half = dp >> 6, row = dp & 63;
-    const float ks = sSum[dp] * (1.0f / 128.0f);
+    const float ks = sSum[dp];
 #pragma unroll
     for (int n = 0; n < kCols / 8; ++n) {
       const int d = n0 + 8 * n + (lane & 3) * 2, box = d >> 6, piece = (d & 63) >> 3;
-      const __nv_bfloat162 v = __floats2bfloat162_rn((acc[n][2 * h] - ks * sSum[D + d]) * (1.0f / 128.0f),
-                                                     (acc[n][2 * h + 1] - ks * sSum[D + d + 1]) * (1.0f / 128.0f));
+      const __nv_bfloat162 v = __floats2bfloat162_rn((acc[n][2 * h] - ks * sSum[D + d]) * scale,
+                                                     (acc[n][2 * h + 1] - ks * sSum[D + d + 1]) * scale);
       *reinterpret_cast<__nv_bfloat162*>(img + ((size_t)(half * (D / 64) + box) * 64 + row) * 128 + (((piece ^ row) & 7) << 4) +
                                          (d & 7) * 2) = v;
     }
@@ -199,7 +213,8 @@ __global__ void __launch_bounds__(256) masked_finish_kernel(const __nv_bfloat16*
   float* sVbar = reinterpret_cast<float*>(fin_smem + Dn::kTile);
   const int N = p.s.N;
   const size_t chunk = blockIdx.x;
-  if (chunk % N == 0) return;           // no rows before the first chunk
+  if (chunk % N < p.m) return;          // no rows before the first chunk
+  const float scale = 1.0f / (float)(128 * p.m);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const float* nacc = p.nacc + chunk * (size_t)kNaccRows<D>() * D;
   const uint4* gv = reinterpret_cast<const uint4*>(vc + chunk * 128 * D);
@@ -214,8 +229,8 @@ __global__ void __launch_bounds__(256) masked_finish_kernel(const __nv_bfloat16*
     for (int x = t; x < 128 * D / 4; x += 256) {
       const float4 add = u[x % (D / 4)];
       float4 cur = dv[x];
-      cur.x += add.x * (1.0f / 128.0f); cur.y += add.y * (1.0f / 128.0f);
-      cur.z += add.z * (1.0f / 128.0f); cur.w += add.w * (1.0f / 128.0f);
+      cur.x += add.x * scale; cur.y += add.y * scale;
+      cur.z += add.z * scale; cur.w += add.w * scale;
       dv[x] = cur;
     }
   }
@@ -271,8 +286,8 @@ __global__ void __launch_bounds__(256) masked_finish_kernel(const __nv_bfloat16*
       for (int h = 0; h < 2; ++h) {
         float2* at = reinterpret_cast<float2*>(dk + (size_t)(m * 16 + 8 * h) * D);
         float2 cur = *at;
-        cur.x += (acc[n][m][2 * h] + c0) * (1.0f / 128.0f);
-        cur.y += (acc[n][m][2 * h + 1] + c1) * (1.0f / 128.0f);
+        cur.x += (acc[n][m][2 * h] + c0) * scale;
+        cur.y += (acc[n][m][2 * h + 1] + c1) * scale;
         *at = cur;
       }
   }
@@ -322,7 +337,7 @@ __device__ __forceinline__ void mk_producer(const MkCtx& c, const MaskedParams& 
     if (pj >= c.jhi) return;
 #pragma unroll
     for (int b = 0; b < Cfg::kKB; ++b)
-      tma_prefetch_2d(tmG, 64 * b, (int)((((size_t)c.bh * N + c.i0 + pc) * R + pr) * L + (size_t)c.srow(pj)));
+      tma_prefetch_2d(tmG, 64 * b, (int)(((c.out_chunk(N, pc)) * R + pr) * L + (size_t)c.srow(pj)));
     if (++pc >= c.chi) {
       if (++pr >= R) { pr = 0; ++pj; }
       pc = c.clo(pj);
@@ -342,7 +357,7 @@ __device__ __forceinline__ void mk_producer(const MkCtx& c, const MaskedParams& 
       tma_load_2d(sb + Cfg::oQ + qs * 16384, tmQ, 64 * c.h, (c.bh * R + r) * L + c.srow(j), c.bar(mQFull + qs));
       for (int cc = c0; cc < c.chi; ++cc)
         bulk_load_1d(sb + Cfg::oGd + (qs * Cfg::kG + cc) * 512,
-                     p.g_denom + (((size_t)c.bh * N + c.i0 + cc) * R + r) * L + (size_t)c.srow(j), 512, c.bar(mQFull + qs));
+                     p.g_denom + (c.out_chunk(N, cc) * R + r) * L + (size_t)c.srow(j), 512, c.bar(mQFull + qs));
       for (int u = 0; u < Cfg::kUnits; ++u) {
         const MkUnit<D> un(u, c0, c.chi);
         if (!un.active()) continue;
@@ -356,7 +371,7 @@ __device__ __forceinline__ void mk_producer(const MkCtx& c, const MaskedParams& 
 #pragma unroll
           for (int b = 0; b < Cfg::kKB; ++b)
             tma_load_2d(sb + Cfg::oSlot + sl * 32768 + (cc - u * Cfg::kPer) * Cfg::kDoBytes + b * 16384, tmG, 64 * b,
-                        (int)((((size_t)c.bh * N + c.i0 + cc) * R + r) * L + (size_t)c.srow(j)), c.bar(mSlotFull + sl));
+                        (int)((c.out_chunk(N, cc) * R + r) * L + (size_t)c.srow(j)), c.bar(mSlotFull + sl));
           prefetch_next();
         }
       }
@@ -624,10 +639,10 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     c.h = blockIdx.x % Cfg::kKB;
     int g = 0;
     bool found = false;
-    c.jb = p.j_begin; c.r0 = p.r0;
+    c.jb = p.j_begin; c.r0 = p.r0; c.m = p.m;
     // row tiles of the range that lie before the last chunk of group gg: [j_begin, min(j_end, last chunk of gg))
-    auto jmax_of = [&](int gg) { return min(min((gg + 1) * Cfg::kG, N) - 1, p.j_end); };
-    for (int piece = 0; p.j_begin + piece * p.jp < min(N - 1, p.j_end); ++piece) {
+    auto jmax_of = [&](int gg) { return min((min((gg + 1) * Cfg::kG, N) - 1) / p.m * p.m, p.j_end); };
+    for (int piece = 0; p.j_begin + piece * p.jp < min((N - 1) / p.m * p.m, p.j_end); ++piece) {
       const int jlo = p.j_begin + piece * p.jp;
       int cnt = 0;                                                       // groups that have row tiles of this piece before a chunk
       for (int gg = 0; gg < groups; ++gg) cnt += (jmax_of(gg) > jlo) ? 1 : 0;

@@ -104,23 +104,55 @@ int launch_fwd_carry(const Shape& s, int gate_dtype, const void* kc, const FwdPa
 int launch_fwd_merge(const Shape& s, int gate_dtype, const void* kc, const void* vc, const void* xq, const FwdParams& p, cudaStream_t st);
 
 // Shapes of the keys-on-lanes backward kernel.
-inline bool bwd2_supported(const Shape& s, int dtype) { return dtype == UA_BF16 && s.C == 128 && (s.D == 64 || s.D == 128); }
+inline bool bwd2_supported(const Shape& s, int dtype) { return fwd_supported(s, dtype); }
+
+// Half tiles (64 rows) per block of the backward, 0 = one block per chunk: the same reckoning as fwd_split, in units of a half tile
+// with heads.  What a cut costs here is the correction pass, a launch of its own that repeats the decay gradient of every half tile
+// but those of the last segments: 5.5 of the 7.9 + 2.7 R thousand cycles a half tile takes, beside a start-up of about 5 thousand
+// per block in each pass.
+inline int bwd_split(const Shape& s) {
+  constexpr double kSms = 148.0;
+  const double unit = 7.9 + 2.7 * s.R, start = 5.0 / unit, corr = 5.5 / unit, BH = (double)s.B * s.H;
+  const int top = s.L / 64, per = s.C / 64;
+  double halves = 0;
+  for (int i = 0; i < s.N; ++i) halves += top - i * per;
+  double best = (BH * halves / kSms > top ? BH * halves / kSms : top) + start;
+  int seg = 0;
+  for (int t = 2; t < top; t *= 2) {
+    double blocks = 0;
+    for (int i = 0; i < s.N; ++i) blocks += (top - i * per + t - 1) / t;
+    auto pass = [&](double cost, double n) {
+      const double one = cost * t + start;
+      return BH * n <= kSms ? one : BH * (cost * halves + start * n) / kSms + 0.5 * one;
+    };
+    const double est = pass(1.0, blocks) + pass(corr, blocks - s.N > 1 ? blocks - s.N : 1) + 0.4;
+    if (est < 0.9 * best) { best = est; seg = t; }
+  }
+  return seg;
+}
+inline int bwd_max_segments(const Shape& s, int seg) { return seg ? (s.L / 64 + seg - 1) / seg : 0; }
 
 // Fills the row-range fields of Bwd2Params for a call over the whole sequence.
 inline void whole_sequence(Bwd2Params& p) {
   p.j_begin = 0; p.j_end = p.s.N; p.Lr = p.s.L; p.r0 = 0; p.heads = p.s.R;
-  p.suffix_in = nullptr; p.dctot_out = nullptr; p.acc_dv = nullptr; p.acc_ds = nullptr;
+  p.suffix_in = nullptr; p.dctot_out = nullptr; p.acc_dv = nullptr; p.acc_ds = nullptr; p.m = 1;
 }
 
 // Fills the row-range fields of MaskedParams for a call over the whole sequence.
 inline void whole_sequence(MaskedParams& p) {
-  p.j_begin = 0; p.j_end = p.s.N; p.Lr = p.s.L; p.r0 = 0; p.acc_dv = nullptr;
+  p.j_begin = 0; p.j_end = p.s.N; p.Lr = p.s.L; p.r0 = 0; p.acc_dv = nullptr; p.m = 1;
 }
 
 // Backward over the row tiles [p.j_begin, p.j_end) (ua_bwd.cu; the caller sets the range fields, e.g. with whole_sequence()).
-// With p.heads == 0 (correction pass) xq, g_out and p.acc_dq are not touched and may be null.
-int launch_bwd2(const Shape& s, int gate_dtype, bool merged, const void* kc, const void* vc, const void* xq, const void* g_out,
+// With p.heads == 0 (correction pass) xq, g_out and p.acc_dq are not touched and may be null.  mode: 1 per-chunk outputs, 2 merged,
+// 3 per-chunk outputs with the row term in the table.  Where p.acc_dt is set the row-side dK and d static_dest are finished too.
+int launch_bwd2(const Shape& s, int gate_dtype, int mode, const void* kc, const void* vc, const void* xq, const void* g_out,
                 const Bwd2Params& p, cudaStream_t st);
+// Everything that a whole-sequence backward leaves to do after its sweep (see bwd_finish_kernel).
+int launch_bwd_finish(const Shape& s, int gate_dtype, const void* kc, const Bwd2Params& p, void* dkc, void* dxq, void* dvc, void* dss,
+                      void* ddest, cudaStream_t st);
+// table = g_denom - out . dO (see row_term_kernel) for chunks of m * 128 keys
+int launch_row_term(const Shape& s, int m, const void* out, const void* g_out, const void* g_denom, int g_denom_dtype, float* table, cudaStream_t st);
 // Rows before a chunk over the row tiles [p.j_begin, p.j_end): prep (per-chunk constants), sweep (one pass over the upstream
 // gradient), finish (dK_i, and dV_i for a row range).  The caller has zeroed (or shares) acc_dq / acc_dk / acc_dv.
 int launch_masked(const Shape& s, const void* kc, const void* vc, const void* xq, const void* g_out, float* acc_dq,
