@@ -17,7 +17,7 @@ from concurrent.futures import ThreadPoolExecutor
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libua_b200.so")
-SOURCES = ["ua_bwd.cu", "ua_fwd.cu", "ua_api.cu"]      # compiled side by side
+SOURCES = ["ua_bwd.cu", "ua_fwd.cu", "ua_tiled.cu", "ua_api.cu"]      # compiled side by side
 # the tensor plumbing above the library: an extension module, host code only
 TORCH_SOURCE = "ua_torch.cpp"
 TORCH_PATH = os.path.join(PKG_DIR, "_ua_torch.so")

@@ -14,6 +14,7 @@
 #include "ua_decode.cuh"
 #include "ua_simt.cuh"
 #include "ua_sm100_host.cuh"
+#include "ua_tiled_host.h"
 
 namespace {
 
@@ -77,6 +78,31 @@ BwdWorkspace bwd_layout(const ua::Shape& s, int rt) {
   w.total = o;
   return w;
 }
+
+// Scratch of the tiled fp32 backward: status | accumulators | dC and its tile totals | log-retention totals.
+struct BwdWorkspaceTiled {
+  size_t off_dk, off_dv, off_dq, off_ds, off_dt, off_dc, off_dct, off_totals, zero_bytes, total;
+};
+BwdWorkspaceTiled bwd_layout_tiled(const ua::Shape& s) {
+  BwdWorkspaceTiled w;
+  const size_t BH = (size_t)s.B * s.H, f = sizeof(float);
+  size_t o = 256;   // [0, 256): status word
+  w.off_dk = o; o = align_up(o + BH * s.L * s.D * f, 256);
+  w.off_dv = o; o = align_up(o + BH * s.L * s.D * f, 256);
+  w.off_dq = o; o = align_up(o + BH * s.R * s.L * s.D * f, 256);
+  w.off_ds = o; o = align_up(o + BH * s.L * f, 256);
+  w.off_dt = o; o = align_up(o + BH * s.L * f, 256);
+  w.off_dc = o;
+  if (s.R == 1) w.zero_bytes = o;                      // one head: dC is written, not added to
+  o = align_up(o + BH * (size_t)s.L * s.L * f, 256);
+  if (s.R > 1) w.zero_bytes = o;
+  w.off_dct = o; o = align_up(o + ua::tiled::table_bytes(s), 256);
+  w.off_totals = o; o = align_up(o + ua::tiled::table_bytes(s), 256);
+  w.total = o;
+  return w;
+}
+// what the tensor-core kernels leave to the CUDA cores, but for the cross-check of the sweeping kernels
+bool runs_tiled(const ua::Shape& s, int flags) { return !(flags & UA_FLAG_FORCE_SIMT) && ua::tiled::fits(s); }
 
 struct BwdWorkspaceTc {
   size_t off_dk, off_dq, off_dt, off_dkr, off_dv, off_ds, off_carry, off_lse, off_gd, off_mt, off_ksum, off_nacc, off_seg, off_out, off_fwd;
@@ -352,6 +378,7 @@ size_t ua_fwd_workspace_bytes(const UaDims* dims, int dtype, int flags) {
     }
     if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::fwd_supported(s, dtype) && ua::sm100::fwd_split(s))
       return 256 + ua::sm100::fwd_totals_bytes(s);      // status word, tile totals of the segmented sweep
+    if (!ua::sm100::fwd_supported(s, dtype) && runs_tiled(s, flags)) return 256 + ua::tiled::table_bytes(s);
   }
   return 256;   // status word
 }
@@ -364,6 +391,7 @@ size_t ua_bwd_workspace_bytes(const UaDims* dims, int dtype, int flags) {
     return bwd_layout_tc(to_shape(&sd), m, ua_fwd_workspace_bytes(dims, dtype, 0)).total;
   }
   if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype)) return bwd_layout_tc(s, 1, 0).total;
+  if (runs_tiled(s, flags)) return bwd_layout_tiled(s).total;
   const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
   if (!cfg.rt) return 0;
   return bwd_layout(s, cfg.rt).total;
@@ -426,6 +454,15 @@ int ua_fwd_keep(const UaDims* dims, int dtype, int gate_dtype, const void* kc, c
     return ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, !(flags & UA_FLAG_SKIP_MASKED_FILL), totals, st);
   }
 
+  const size_t want = ua_fwd_workspace_bytes(dims, dtype, flags);
+  if (runs_tiled(s, flags) && workspace_bytes >= want) {
+    ua::tiled::Params tp{};
+    tp.s = s; tp.kc = kc; tp.vc = vc; tp.xq = xq; tp.ssrc = static_src; tp.sdest = static_dest;
+    tp.out = out_cm; tp.lse = lse_cm; tp.denom = denom_cm;
+    tp.fill_masked = (flags & UA_FLAG_SKIP_MASKED_FILL) ? 0 : 1;
+    tp.totals = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
+    return ua::tiled::forward(tp, dtype == UA_F32, gate_dtype == UA_F32, st) && cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  }
   ua::simt::FwdParams p;
   p.s = s; p.kc = kc; p.vc = vc; p.xq = xq; p.ssrc = static_src; p.sdest = static_dest;
   p.out = out_cm; p.lse = lse_cm; p.denom = denom_cm;
@@ -740,15 +777,12 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
       dv_chunk = mp.nacc + (size_t)(s.D + 1) * s.D;
       if ((e = ua::sm100::launch_masked(ks, kc, vc, xq, g_out_cm, acc_dq, mp, st))) return e;
     } else if (masked) {
-      // chunks of 64 keys: the generic kernel, for those rows only
-      const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
-      if (!cfg.rt) return UA_ERR_UNSUPPORTED;
-      ua::simt::BwdParams sp{};
-      sp.s = s; sp.kc = kc; sp.vc = vc; sp.xq = xq; sp.ssrc = static_src; sp.sdest = static_dest;
-      sp.g_out = g_out_cm; sp.g_denom = g_denom_cm; sp.g_denom_is_f32 = (g_denom_dtype == UA_F32);
-      sp.acc_dk = acc_dk; sp.acc_dv = at(w.off_dv); sp.acc_dq = acc_dq; sp.acc_ds = at(w.off_ds); sp.acc_dt = at(w.off_dt);
-      sp.rt = cfg.rt; sp.masked_only = 1;
-      if ((e = launch_simt_bwd_any(sp, dtype, gate_dtype, cfg, st))) return e;
+      // chunks of 64 keys: the tiled kernel, for those rows only
+      ua::tiled::Params tp{};
+      tp.s = s; tp.kc = kc; tp.vc = vc; tp.xq = xq; tp.ssrc = static_src; tp.sdest = static_dest;
+      tp.g_out = g_out_cm; tp.g_denom = g_denom_cm; tp.g_denom_is_f32 = (g_denom_dtype == UA_F32);
+      tp.acc_dk = acc_dk; tp.acc_dv = at(w.off_dv); tp.acc_dq = acc_dq; tp.only_masked = 1;
+      if (!ua::tiled::backward(tp, false, gate_dtype == UA_F32, st) || cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
     }
     ua::sm100::Bwd2Params qp{};
     qp.s = ks; ua::sm100::whole_sequence(qp); qp.ssrc = static_src; qp.sdest = static_dest;
@@ -776,6 +810,35 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     return ua::sm100::launch_bwd_finish(ks, gate_dtype, kc, qp, dkc, dxq, dvc, dstatic_src, dstatic_dest, st);
   }
 
+  if (runs_tiled(s, flags)) {
+    const BwdWorkspaceTiled w = bwd_layout_tiled(s);
+    if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
+    char* ws = static_cast<char*>(workspace);
+    auto at = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
+    if (cudaMemsetAsync(ws, 0, w.zero_bytes, st) != cudaSuccess) return UA_ERR_CUDA;
+    ua::tiled::Params tp{};
+    tp.s = s; tp.kc = kc; tp.vc = vc; tp.xq = xq; tp.ssrc = static_src; tp.sdest = static_dest;
+    tp.g_out = g_out_cm; tp.g_denom = g_denom_cm; tp.g_denom_is_f32 = (g_denom_dtype == UA_F32);
+    tp.skip_masked = (flags & UA_FLAG_SKIP_MASKED_GRADS) ? 1 : 0;
+    tp.acc_dk = at(w.off_dk); tp.acc_dv = at(w.off_dv); tp.acc_dq = at(w.off_dq); tp.acc_ds = at(w.off_ds); tp.acc_dt = at(w.off_dt);
+    tp.dc = at(w.off_dc); tp.dc_total = at(w.off_dct); tp.totals = at(w.off_totals);
+    if (!ua::tiled::backward(tp, dtype == UA_F32, gate_dtype == UA_F32, st)) return UA_ERR_CUDA;
+    const size_t BH = (size_t)s.B * s.H;
+    const ua::tiled::Leave v = {{tp.acc_dk, tp.acc_dv, tp.acc_dq, tp.acc_ds, tp.acc_dt},
+                                {dkc, dvc, dxq, dstatic_src, dstatic_dest},
+                                {BH * s.L * s.D, BH * s.L * s.D, BH * s.R * s.L * s.D, BH * s.L, BH * s.L},
+                                {0, 0, 0, 1, 1}};
+    bool vectors = true;
+    for (const void* o : v.dst) vectors = vectors && aligned16(o);
+    if (!vectors) {
+      for (int t = 0; t < 5; ++t)
+        if ((e = convert_any(v.gate[t] ? gate_dtype : dtype, v.src[t], v.dst[t], v.n[t], st))) return e;
+      return UA_OK;
+    }
+    ua::tiled::leave(v, dtype == UA_F32, gate_dtype == UA_F32, st);
+    return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  }
+
   const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
   const int rt = cfg.rt;
   if (!rt) return UA_ERR_UNSUPPORTED;
@@ -795,7 +858,6 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
   p.carry = reinterpret_cast<float*>(ws + w.off_carry);
   p.rt = rt;
   p.skip_masked = (flags & UA_FLAG_SKIP_MASKED_GRADS) ? 1 : 0;
-  p.masked_only = 0;
   if ((e = launch_simt_bwd_any(p, dtype, gate_dtype, cfg, st))) return e;
 
   const size_t BH = (size_t)s.B * s.H;
