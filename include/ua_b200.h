@@ -371,6 +371,12 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype,
 int ua_merge_bwd(const UaDims* dims, int dtype, const void* out_cm, const float* lse_cm,
                  const void* g_merged, void* g_out_cm, float* g_lse_cm, int flags, void* stream);
 
+/* ua_merge_fwd_stats and ua_merge_bwd for log-sum-exps (and their gradient) in lse_dtype: UA_F32, or dtype. */
+int ua_merge_fwd_typed(const UaDims* dims, int dtype, int lse_dtype, const void* out_cm, const void* lse_cm, void* merged,
+                       float* row_lse, void* stream);
+int ua_merge_bwd_typed(const UaDims* dims, int dtype, int lse_dtype, const void* out_cm, const void* lse_cm,
+                       const void* g_merged, void* g_out_cm, void* g_lse_cm, int flags, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -63,6 +63,8 @@ SIGNATURES = {
     "ua_merge_fwd": (_i, [_dp, _i, _vp, _vp, _vp, _vp]),
     "ua_merge_bwd": (_i, [_dp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "ua_merge_fwd_stats": (_i, [_dp, _i, _vp, _vp, _vp, _vp, _vp]),
+    "ua_merge_fwd_typed": (_i, [_dp, _i, _i, _vp, _vp, _vp, _vp, _vp]),
+    "ua_merge_bwd_typed": (_i, [_dp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "ua_row_dot": (_i, [ctypes.c_longlong, _i, _i, _vp, _vp, _vp, _vp]),
     "ua_fwd_merged_workspace_bytes": (_sz, [_dp, _i]),
     "ua_fwd_merged": (_i, [_dp, _i, _i] + [_vp] * 9 + [_sz, _vp]),

@@ -307,31 +307,38 @@ int static_scratch_for_current_device(void** out) {
 }  // namespace
 
 namespace {
+// Either direction of the input prologue.
+struct PrepCall {
+  const void *q, *k, *v, *g, *g2, *kc, *src, *dest;      // backward: gradients of xq, kc, vc, static_src (g), static_dest (g2); forward's kc and gates
+  const float* norm_in;
+  void *oq, *ok, *ov, *og, *og2;                         // forward: xq, kc, vc, static_src, static_dest; backward: the four projections' gradients
+  float* norm_out;
+  bool backward;
+};
 template <typename T, int TPR>
-int launch_prepare(const ua::aux::PrepDims& pd, int backward, const void* a0, const void* a1, const void* a2, const void* a3,
-                   const float* key_norm_in, void* o0, void* o1, void* o2, float* key_norm_out, cudaStream_t st) {
-  const long long rows = (long long)pd.b * pd.s * (pd.n + 2 * pd.n_kv);
-  const unsigned blocks = (unsigned)((rows * TPR + ua::aux::kMergeThreads - 1) / ua::aux::kMergeThreads);
-  if (!backward)
-    ua::aux::prepare_fwd_kernel<T, TPR><<<blocks, ua::aux::kMergeThreads, 0, st>>>(
-        pd, static_cast<const T*>(a0), static_cast<const T*>(a1), static_cast<const T*>(a2), static_cast<T*>(o0), static_cast<T*>(o1),
-        static_cast<T*>(o2), key_norm_out);
+int launch_prepare(ua::aux::PrepDims pd, const PrepCall& c, cudaStream_t st) {
+  const long long gates = (long long)pd.b * pd.s * 2 * pd.n_kv;
+  pd.row_blocks = (unsigned)(((long long)pd.rows * TPR + ua::aux::kMergeThreads - 1) / ua::aux::kMergeThreads);
+  const unsigned blocks = pd.row_blocks + (unsigned)std::min<long long>((gates + ua::aux::kMergeThreads - 1) / ua::aux::kMergeThreads, 1024);
+  auto in = [](const void* x) { return static_cast<const T*>(x); };
+  auto out = [](void* x) { return static_cast<T*>(x); };
+  if (!c.backward)
+    ua::aux::prepare_fwd_kernel<T, TPR><<<blocks, ua::aux::kMergeThreads, 0, st>>>(pd, in(c.q), in(c.k), in(c.v), in(c.g), out(c.oq), out(c.ok),
+                                                                                  out(c.ov), out(c.og), out(c.og2), c.norm_out);
   else
-    ua::aux::prepare_bwd_kernel<T, TPR><<<blocks, ua::aux::kMergeThreads, 0, st>>>(
-        pd, static_cast<const T*>(a0), static_cast<const T*>(a1), static_cast<const T*>(a2), static_cast<const T*>(a3), key_norm_in,
-        static_cast<T*>(o0), static_cast<T*>(o1), static_cast<T*>(o2));
+    ua::aux::prepare_bwd_kernel<T, TPR><<<blocks, ua::aux::kMergeThreads, 0, st>>>(pd, in(c.q), in(c.k), in(c.v), in(c.g), in(c.g2), in(c.kc), c.norm_in,
+                                                                                  in(c.src), in(c.dest), out(c.oq), out(c.ok), out(c.ov), out(c.og));
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
 template <typename T>
-int dispatch_prepare(int tpr, const ua::aux::PrepDims& pd, int backward, const void* a0, const void* a1, const void* a2,
-                     const void* a3, const float* kn_in, void* o0, void* o1, void* o2, float* kn_out, cudaStream_t st) {
+int dispatch_prepare(int tpr, const ua::aux::PrepDims& pd, const PrepCall& c, cudaStream_t st) {
   switch (tpr) {
-    case 1: return launch_prepare<T, 1>(pd, backward, a0, a1, a2, a3, kn_in, o0, o1, o2, kn_out, st);
-    case 2: return launch_prepare<T, 2>(pd, backward, a0, a1, a2, a3, kn_in, o0, o1, o2, kn_out, st);
-    case 4: return launch_prepare<T, 4>(pd, backward, a0, a1, a2, a3, kn_in, o0, o1, o2, kn_out, st);
-    case 8: return launch_prepare<T, 8>(pd, backward, a0, a1, a2, a3, kn_in, o0, o1, o2, kn_out, st);
-    case 16: return launch_prepare<T, 16>(pd, backward, a0, a1, a2, a3, kn_in, o0, o1, o2, kn_out, st);
-    case 32: return launch_prepare<T, 32>(pd, backward, a0, a1, a2, a3, kn_in, o0, o1, o2, kn_out, st);
+    case 1: return launch_prepare<T, 1>(pd, c, st);
+    case 2: return launch_prepare<T, 2>(pd, c, st);
+    case 4: return launch_prepare<T, 4>(pd, c, st);
+    case 8: return launch_prepare<T, 8>(pd, c, st);
+    case 16: return launch_prepare<T, 16>(pd, c, st);
+    case 32: return launch_prepare<T, 32>(pd, c, st);
     default: return UA_ERR_UNSUPPORTED;
   }
 }
@@ -344,7 +351,75 @@ int prepare_common(int b, int s, int n_heads, int n_kv, int head_dim, int dtype,
   pd->b = b; pd->s = s; pd->n = n_heads; pd->n_kv = n_kv;
   pd->normalize_keys = (flags & UA_PREP_NORMALIZE_KEYS) ? 1 : 0;
   pd->sigmoid_gates = (flags & UA_PREP_SIGMOID_GATES) ? 1 : 0;
+  const long long rows = (long long)b * s * (n_heads + 2 * n_kv);
+  if (rows > 0x7fffffff) return UA_ERR_UNSUPPORTED;
+  pd->rows = (unsigned)rows;
   return UA_OK;
+}
+}  // namespace
+
+namespace {
+// Merge over key chunks, either direction.
+struct MergeCall {
+  const void *out, *lse, *g;
+  void *merged, *g_out, *g_lse;
+  float* row_lse;
+  bool backward;
+  int skip;
+};
+template <typename T, typename TL, int TPR>
+int launch_merge(const ua::Shape& s, const MergeCall& c, cudaStream_t st) {
+  constexpr int kRows = ua::aux::kMergeThreads / TPR;
+  if (!c.backward && s.N >= 2 && s.N <= 4) {
+    const long long rows = (long long)s.B * s.H * s.R * s.L;
+    auto few = s.N == 2 ? ua::aux::merge_few_kernel<T, TL, TPR, 2> : s.N == 3 ? ua::aux::merge_few_kernel<T, TL, TPR, 3> : ua::aux::merge_few_kernel<T, TL, TPR, 4>;
+    few<<<(unsigned)((rows + kRows - 1) / kRows), ua::aux::kMergeThreads, 0, st>>>(static_cast<const T*>(c.out), static_cast<const TL*>(c.lse),
+                                                                                  static_cast<T*>(c.merged), c.row_lse, rows, s.R, s.L);
+    return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  }
+  const size_t smem = ua::aux::merge_smem<TPR>(s.N, c.backward);
+  if (smem > kMaxDynSmem) {
+    const long long rows = (long long)s.B * s.H * s.R * s.L;
+    ua::aux::merge_many_kernel<T, TL, TPR><<<(unsigned)((rows + kRows - 1) / kRows), ua::aux::kMergeThreads, 0, st>>>(
+        static_cast<const T*>(c.out), static_cast<const TL*>(c.lse), static_cast<T*>(c.merged), c.row_lse, static_cast<const T*>(c.g),
+        static_cast<T*>(c.g_out), static_cast<TL*>(c.g_lse), rows, s.N, s.R, s.L, c.skip);
+    return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  }
+  const unsigned blocks = (unsigned)((long long)s.B * s.H * s.R * ((s.L + kRows - 1) / kRows));
+  if (c.backward) {
+    auto kern = ua::aux::merge_bwd_kernel<T, TL, TPR>;
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return UA_ERR_CUDA;
+    kern<<<blocks, ua::aux::kMergeThreads, smem, st>>>(static_cast<const T*>(c.out), static_cast<const TL*>(c.lse), static_cast<const T*>(c.g),
+                                                       static_cast<T*>(c.g_out), static_cast<TL*>(c.g_lse), s.N, s.R, s.L, c.skip);
+  } else {
+    auto kern = ua::aux::merge_fwd_kernel<T, TL, TPR>;
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return UA_ERR_CUDA;
+    kern<<<blocks, ua::aux::kMergeThreads, smem, st>>>(static_cast<const T*>(c.out), static_cast<const TL*>(c.lse), static_cast<T*>(c.merged),
+                                                       c.row_lse, s.N, s.R, s.L);
+  }
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+template <typename T, typename TL>
+int launch_merge_d(const ua::Shape& s, const MergeCall& c, cudaStream_t st) {
+  switch (s.D * (int)sizeof(T)) {      // bytes per row, 16 per thread
+    case 16: return launch_merge<T, TL, 1>(s, c, st);
+    case 32: return launch_merge<T, TL, 2>(s, c, st);
+    case 64: return launch_merge<T, TL, 4>(s, c, st);
+    case 128: return launch_merge<T, TL, 8>(s, c, st);
+    case 256: return launch_merge<T, TL, 16>(s, c, st);
+    case 512: if (sizeof(T) == 4) return launch_merge<T, TL, 32>(s, c, st);
+  }
+  return UA_ERR_UNSUPPORTED;
+}
+int merge_call(const UaDims* dims, int dtype, int lse_dtype, const MergeCall& c, cudaStream_t st) {
+  int e = check_dims(dims);
+  if (e) return e;
+  if ((dtype != UA_F32 && dtype != UA_BF16) || (lse_dtype != UA_F32 && lse_dtype != dtype)) return UA_ERR_BAD_DTYPE;
+  if (!c.out || !c.lse || !(c.backward ? c.g && c.g_out && c.g_lse : c.merged != nullptr)) return UA_ERR_NULL_POINTER;
+  if (!aligned16(c.out) || !aligned16(c.merged) || !aligned16(c.g) || !aligned16(c.g_out)) return UA_ERR_ALIGNMENT;
+  const ua::Shape s = to_shape(dims);
+  if (dtype == UA_F32) return launch_merge_d<float, float>(s, c, st);
+  return lse_dtype == UA_F32 ? launch_merge_d<bf16, float>(s, c, st) : launch_merge_d<bf16, bf16>(s, c, st);
 }
 }  // namespace
 
@@ -947,18 +1022,10 @@ int ua_prepare_inputs(int batch, int seq, int n_heads, int n_kv_heads, int head_
   if (!aligned16(query_state) || !aligned16(key_state) || !aligned16(value_state) || !aligned16(xq) || !aligned16(kc) || !aligned16(vc))
     return UA_ERR_ALIGNMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  e = dtype == UA_F32 ? dispatch_prepare<float>(tpr, pd, 0, query_state, key_state, value_state, nullptr, nullptr, xq, kc, vc, key_norm, st)
-                      : dispatch_prepare<bf16>(tpr, pd, 0, query_state, key_state, value_state, nullptr, nullptr, xq, kc, vc, key_norm, st);
-  if (e) return e;
-  const long long total = (long long)batch * seq * 2 * n_kv_heads;
-  const unsigned gblocks = (unsigned)std::min<long long>((total + 255) / 256, 4096);
-  if (dtype == UA_F32)
-    ua::aux::prepare_gates_kernel<float><<<gblocks, 256, 0, st>>>(pd, static_cast<const float*>(gate_state), static_cast<float*>(static_src),
-                                                                 static_cast<float*>(static_dest), 0, nullptr, nullptr, nullptr);
-  else
-    ua::aux::prepare_gates_kernel<bf16><<<gblocks, 256, 0, st>>>(pd, static_cast<const bf16*>(gate_state), static_cast<bf16*>(static_src),
-                                                                static_cast<bf16*>(static_dest), 0, nullptr, nullptr, nullptr);
-  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  PrepCall c{};
+  c.q = query_state; c.k = key_state; c.v = value_state; c.g = gate_state;
+  c.oq = xq; c.ok = kc; c.ov = vc; c.og = static_src; c.og2 = static_dest; c.norm_out = key_norm;
+  return dtype == UA_F32 ? dispatch_prepare<float>(tpr, pd, c, st) : dispatch_prepare<bf16>(tpr, pd, c, st);
 }
 
 int ua_prepare_inputs_bwd(int batch, int seq, int n_heads, int n_kv_heads, int head_dim, int dtype, int flags,
@@ -977,20 +1044,11 @@ int ua_prepare_inputs_bwd(int batch, int seq, int n_heads, int n_kv_heads, int h
       !aligned16(d_value_state) || (kc && !aligned16(kc)))
     return UA_ERR_ALIGNMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  e = dtype == UA_F32 ? dispatch_prepare<float>(tpr, pd, 1, g_xq, g_kc, g_vc, kc, key_norm, d_query_state, d_key_state, d_value_state, nullptr, st)
-                      : dispatch_prepare<bf16>(tpr, pd, 1, g_xq, g_kc, g_vc, kc, key_norm, d_query_state, d_key_state, d_value_state, nullptr, st);
-  if (e) return e;
-  const long long total = (long long)batch * seq * 2 * n_kv_heads;
-  const unsigned gblocks = (unsigned)std::min<long long>((total + 255) / 256, 4096);
-  if (dtype == UA_F32)
-    ua::aux::prepare_gates_kernel<float><<<gblocks, 256, 0, st>>>(
-        pd, nullptr, const_cast<float*>(static_cast<const float*>(static_src)), const_cast<float*>(static_cast<const float*>(static_dest)), 1,
-        static_cast<const float*>(g_static_src), static_cast<const float*>(g_static_dest), static_cast<float*>(d_gate_state));
-  else
-    ua::aux::prepare_gates_kernel<bf16><<<gblocks, 256, 0, st>>>(
-        pd, nullptr, const_cast<bf16*>(static_cast<const bf16*>(static_src)), const_cast<bf16*>(static_cast<const bf16*>(static_dest)), 1,
-        static_cast<const bf16*>(g_static_src), static_cast<const bf16*>(g_static_dest), static_cast<bf16*>(d_gate_state));
-  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  PrepCall c{};
+  c.backward = true;
+  c.q = g_xq; c.k = g_kc; c.v = g_vc; c.g = g_static_src; c.g2 = g_static_dest; c.kc = kc; c.src = static_src; c.dest = static_dest; c.norm_in = key_norm;
+  c.oq = d_query_state; c.ok = d_key_state; c.ov = d_value_state; c.og = d_gate_state;
+  return dtype == UA_F32 ? dispatch_prepare<float>(tpr, pd, c, st) : dispatch_prepare<bf16>(tpr, pd, c, st);
 }
 
 int ua_decode_step(const UaDims* dims, int dtype, int gate_dtype, int t, const void* k_cache, const void* v_cache,
@@ -1032,33 +1090,14 @@ int ua_merge_fwd(const UaDims* dims, int dtype, const void* out_cm, const float*
 
 int ua_merge_fwd_stats(const UaDims* dims, int dtype, const void* out_cm, const float* lse_cm, void* merged, float* row_lse,
                        void* stream) {
-  int e = check_dims(dims);
-  if (e) return e;
-  if (dtype != UA_F32 && dtype != UA_BF16) return UA_ERR_BAD_DTYPE;
-  if (!out_cm || !lse_cm || !merged) return UA_ERR_NULL_POINTER;
-  if (!aligned16(out_cm) || !aligned16(merged)) return UA_ERR_ALIGNMENT;
-  ua::Shape s = to_shape(dims);
-  const long long rows = (long long)s.B * s.H * s.R * s.L;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int tpr = s.D * (dtype == UA_F32 ? 4 : 2) / 16;
-  const unsigned blocks = (unsigned)((rows * tpr + ua::aux::kMergeThreads - 1) / ua::aux::kMergeThreads);
-#define UA_MERGE_FWD(T, TPR)                                                                                         \
-  ua::aux::merge_fwd_kernel<T, TPR><<<blocks, ua::aux::kMergeThreads, 0, st>>>(static_cast<const T*>(out_cm), lse_cm, \
-                                                                                static_cast<T*>(merged), row_lse, rows, s.N, s.R, s.L)
-  if (dtype == UA_BF16 && s.D == 64) UA_MERGE_FWD(bf16, 8);
-  else if (dtype == UA_BF16 && s.D == 128) UA_MERGE_FWD(bf16, 16);
-  else if (dtype == UA_BF16 && s.D == 32) UA_MERGE_FWD(bf16, 4);
-  else if (dtype == UA_BF16 && s.D == 16) UA_MERGE_FWD(bf16, 2);
-  else if (dtype == UA_BF16 && s.D == 8) UA_MERGE_FWD(bf16, 1);
-  else if (dtype == UA_F32 && s.D == 128) UA_MERGE_FWD(float, 32);
-  else if (dtype == UA_F32 && s.D == 64) UA_MERGE_FWD(float, 16);
-  else if (dtype == UA_F32 && s.D == 32) UA_MERGE_FWD(float, 8);
-  else if (dtype == UA_F32 && s.D == 16) UA_MERGE_FWD(float, 4);
-  else if (dtype == UA_F32 && s.D == 8) UA_MERGE_FWD(float, 2);
-  else if (dtype == UA_F32 && s.D == 4) UA_MERGE_FWD(float, 1);
-  else return UA_ERR_UNSUPPORTED;
-#undef UA_MERGE_FWD
-  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  return ua_merge_fwd_typed(dims, dtype, UA_F32, out_cm, lse_cm, merged, row_lse, stream);
+}
+
+int ua_merge_fwd_typed(const UaDims* dims, int dtype, int lse_dtype, const void* out_cm, const void* lse_cm, void* merged, float* row_lse,
+                       void* stream) {
+  MergeCall c{};
+  c.out = out_cm; c.lse = lse_cm; c.merged = merged; c.row_lse = row_lse;
+  return merge_call(dims, dtype, lse_dtype, c, static_cast<cudaStream_t>(stream));
 }
 
 size_t ua_fwd_merged_workspace_bytes(const UaDims* dims, int dtype) {
@@ -1180,35 +1219,15 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
 
 int ua_merge_bwd(const UaDims* dims, int dtype, const void* out_cm, const float* lse_cm, const void* g_merged,
                  void* g_out_cm, float* g_lse_cm, int flags, void* stream) {
-  int e = check_dims(dims);
-  if (e) return e;
-  if (dtype != UA_F32 && dtype != UA_BF16) return UA_ERR_BAD_DTYPE;
-  if (!out_cm || !lse_cm || !g_merged || !g_out_cm || !g_lse_cm) return UA_ERR_NULL_POINTER;
-  if (!aligned16(out_cm) || !aligned16(g_merged) || !aligned16(g_out_cm)) return UA_ERR_ALIGNMENT;
-  ua::Shape s = to_shape(dims);
-  const long long rows = (long long)s.B * s.H * s.R * s.L;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int tpr = s.D * (dtype == UA_F32 ? 4 : 2) / 16;
-  const unsigned blocks = (unsigned)((rows * tpr + ua::aux::kMergeThreads - 1) / ua::aux::kMergeThreads);
-  const int skip = (flags & UA_FLAG_SKIP_MASKED_FILL) ? 1 : 0;
-#define UA_MERGE_BWD(T, TPR)                                                                                          \
-  ua::aux::merge_bwd_kernel<T, TPR><<<blocks, ua::aux::kMergeThreads, 0, st>>>(                                       \
-      static_cast<const T*>(out_cm), lse_cm, static_cast<const T*>(g_merged), static_cast<T*>(g_out_cm), g_lse_cm, rows, \
-      s.N, s.R, s.L, skip)
-  if (dtype == UA_BF16 && s.D == 64) UA_MERGE_BWD(bf16, 8);
-  else if (dtype == UA_BF16 && s.D == 128) UA_MERGE_BWD(bf16, 16);
-  else if (dtype == UA_BF16 && s.D == 32) UA_MERGE_BWD(bf16, 4);
-  else if (dtype == UA_BF16 && s.D == 16) UA_MERGE_BWD(bf16, 2);
-  else if (dtype == UA_BF16 && s.D == 8) UA_MERGE_BWD(bf16, 1);
-  else if (dtype == UA_F32 && s.D == 128) UA_MERGE_BWD(float, 32);
-  else if (dtype == UA_F32 && s.D == 64) UA_MERGE_BWD(float, 16);
-  else if (dtype == UA_F32 && s.D == 32) UA_MERGE_BWD(float, 8);
-  else if (dtype == UA_F32 && s.D == 16) UA_MERGE_BWD(float, 4);
-  else if (dtype == UA_F32 && s.D == 8) UA_MERGE_BWD(float, 2);
-  else if (dtype == UA_F32 && s.D == 4) UA_MERGE_BWD(float, 1);
-  else return UA_ERR_UNSUPPORTED;
-#undef UA_MERGE_BWD
-  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  return ua_merge_bwd_typed(dims, dtype, UA_F32, out_cm, lse_cm, g_merged, g_out_cm, g_lse_cm, flags, stream);
+}
+
+int ua_merge_bwd_typed(const UaDims* dims, int dtype, int lse_dtype, const void* out_cm, const void* lse_cm, const void* g_merged,
+                       void* g_out_cm, void* g_lse_cm, int flags, void* stream) {
+  MergeCall c{};
+  c.out = out_cm; c.lse = lse_cm; c.backward = true; c.g = g_merged; c.g_out = g_out_cm; c.g_lse = g_lse_cm;
+  c.skip = (flags & UA_FLAG_SKIP_MASKED_FILL) ? 1 : 0;
+  return merge_call(dims, dtype, lse_dtype, c, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -48,9 +48,9 @@ __global__ void __launch_bounds__(256) relayout_kernel(const E* __restrict__ src
 }
 
 // ---- merge over key chunks (SMVecMatMul) -----------------------------------------
-// One group of TPR = D * sizeof(T) / 16 threads per output row (b,h,r,l); every thread owns
-// one 16-byte slice of the row (8 bf16 or 4 floats), so a warp reads whole contiguous rows of
-// out_cm.  Chunks whose softmax weight is exactly zero (rows before a key chunk have
+// A block takes 256 / TPR neighbouring rows (b,h,r,l), TPR = D * sizeof(T) / 16 threads each; every thread
+// owns one 16-byte slice of the row (8 bf16 or 4 floats), so a block reads a contiguous piece of
+// every chunk of out_cm.  Chunks whose softmax weight is exactly zero (rows before a key chunk have
 // lse = -1e12) are never read; on B4 H8 L4096 that halves the traffic.
 constexpr int kMergeThreads = 256;
 
@@ -64,11 +64,17 @@ template <> struct Vec16<float> {
   static __device__ __forceinline__ void store(float* p, const float* v) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
   }
+  static __device__ __forceinline__ void unpack(const uint4& x, float* v) {
+    v[0] = __uint_as_float(x.x); v[1] = __uint_as_float(x.y); v[2] = __uint_as_float(x.z); v[3] = __uint_as_float(x.w);
+  }
+  static __device__ __forceinline__ uint4 pack(const float* v) {
+    return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+  }
 };
 template <> struct Vec16<__nv_bfloat16> {
   static constexpr int kN = 8;
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float* v) {
-    const uint4 x = *reinterpret_cast<const uint4*>(p);
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float* v) { unpack(*reinterpret_cast<const uint4*>(p), v); }
+  static __device__ __forceinline__ void unpack(const uint4& x, float* v) {
     const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -77,14 +83,15 @@ template <> struct Vec16<__nv_bfloat16> {
       v[2 * i + 1] = __bfloat162float(h.y);
     }
   }
-  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* v) {
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* v) { *reinterpret_cast<uint4*>(p) = pack(v); }
+  static __device__ __forceinline__ uint4 pack(const float* v) {
     uint32_t w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
       w[i] = *reinterpret_cast<uint32_t*>(&h);
     }
-    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+    return make_uint4(w[0], w[1], w[2], w[3]);
   }
 };
 
@@ -101,50 +108,233 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
-// row statistics of the softmax over chunks: max and 1 / sum exp
-template <int TPR>
-__device__ __forceinline__ void merge_row_stats(const float* lse_row, size_t nstride, int N, int sub, float& m, float& zinv) {
+// Weights of a block's kRows rows: W[n][row] = softmax over n of lse[n][row], in shared memory (pitch kRows + 1).  The log-sum-exps
+// are read once, coalesced along the rows; the TPR threads of a row share its statistics.  Returns the number of chunks up to the last
+// one with a weight that is not zero, for any row of the warp: behind it nothing needs to be read.
+template <typename TL, int TPR>
+__device__ __forceinline__ int merge_weights(const TL* lse, size_t nstride, int N, int rows_here, float* W, float& m, float& zinv) {
+  constexpr int kRows = kMergeThreads / TPR, kPitch = kRows + 1;
+  for (int e = threadIdx.x; e < N * kRows; e += kMergeThreads) {
+    const int n = e / kRows, q = e % kRows;
+    W[n * kPitch + q] = Num<TL>::ld(lse + (size_t)n * nstride + (q < rows_here ? q : rows_here - 1));
+  }
+  __syncthreads();
+  const int sub = threadIdx.x % TPR;
+  float* mine = W + threadIdx.x / TPR;
   float mm = -INFINITY;
-  for (int n = sub; n < N; n += TPR) mm = fmaxf(mm, lse_row[(size_t)n * nstride]);
+  for (int n = sub; n < N; n += TPR) mm = fmaxf(mm, mine[n * kPitch]);
   m = group_max<TPR>(mm);
   float z = 0.f;
-  for (int n = sub; n < N; n += TPR) z += expf(lse_row[(size_t)n * nstride] - m);
+  for (int n = sub; n < N; n += TPR) z += expf(mine[n * kPitch] - m);
   zinv = 1.0f / group_sum<TPR>(z);
+  int last = 0;
+  for (int n = sub; n < N; n += TPR) {
+    const float w = expf(mine[n * kPitch] - m) * zinv;
+    mine[n * kPitch] = w;
+    if (w != 0.f) last = n + 1;
+  }
+  __syncwarp();
+  return __reduce_max_sync(0xffffffffu, last);
 }
+constexpr int kMergeAhead = 8;      // chunks whose loads a thread has in flight
 
 // merged[row][d] = sum_n softmax_n(lse[n][row]) * out_cm[n][row][d]
-template <typename T, int TPR>
-__global__ void __launch_bounds__(kMergeThreads) merge_fwd_kernel(const T* __restrict__ out_cm, const float* __restrict__ lse_cm,
-                                                                  T* __restrict__ merged, float* __restrict__ row_lse,
-                                                                  long long rows, int N, int R, int L) {
-  constexpr int kN = Vec16<T>::kN;
-  constexpr int D = TPR * kN;
-  const long long row = (long long)blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
-  const int sub = threadIdx.x % TPR;
-  const bool live = row < rows;
-  const long long rr = live ? row : rows - 1;          // keep whole warps in the shuffles
-  const int l = (int)(rr % L);
-  const long long gr = rr / L;
-  const int r = (int)(gr % R);
-  const long long bh = gr / R;
-  const size_t nstride = (size_t)R * L;
-  const size_t base = ((size_t)bh * N * R + r) * L + l;
+// Bound by the read of the chunks that count; eight 16-byte loads in flight per thread.  B4 H8 R4 L4096 D64 (1.07 GB read):
+// 306 us with one load in flight behind its own exponential -> 223 us (4.8 TB/s).
+template <typename T, typename TL, int TPR>
+__global__ void __launch_bounds__(kMergeThreads) merge_fwd_kernel(const T* __restrict__ out_cm, const TL* __restrict__ lse_cm,
+                                                                  T* __restrict__ merged, float* __restrict__ row_lse, int N, int R, int L) {
+  constexpr int kN = Vec16<T>::kN, D = TPR * kN, kRows = kMergeThreads / TPR, kPitch = kRows + 1;
+  extern __shared__ float sW[];
+  const int tiles = (L + kRows - 1) / kRows, gr = blockIdx.x / tiles, l0 = (blockIdx.x - gr * tiles) * kRows;      // gr = bh * R + r
+  const int r = gr % R, row = threadIdx.x / TPR, sub = threadIdx.x % TPR;
+  const size_t nstride = (size_t)R * L, base = ((size_t)(gr / R) * N * R + r) * L + l0;
+  const int rows_here = L - l0 < kRows ? L - l0 : kRows;
+  const bool live = row < rows_here;
   float m, zinv;
-  merge_row_stats<TPR>(lse_cm + base, nstride, N, sub, m, zinv);
+  const int last = merge_weights<TL, TPR>(lse_cm + base, nstride, N, rows_here, sW, m, zinv);
   float acc[kN];
 #pragma unroll
   for (int i = 0; i < kN; ++i) acc[i] = 0.f;
-  for (int n = 0; n < N; ++n) {
-    const float w = expf(lse_cm[base + (size_t)n * nstride] - m) * zinv;
-    if (w != 0.f) {
-      float v[kN];
-      Vec16<T>::load(out_cm + (base + (size_t)n * nstride) * D + sub * kN, v);
+  const uint4* src = reinterpret_cast<const uint4*>(out_cm + (base + row) * D) + sub;
+  const size_t step = nstride * D * sizeof(T) / 16;
+  for (int n0 = 0; n0 < last; n0 += kMergeAhead) {
+    uint4 raw[kMergeAhead];
+    float w[kMergeAhead];
 #pragma unroll
-      for (int i = 0; i < kN; ++i) acc[i] = fmaf(w, v[i], acc[i]);
+    for (int u = 0; u < kMergeAhead; ++u) {
+      w[u] = (live && n0 + u < last) ? sW[(n0 + u) * kPitch + row] : 0.f;
+      raw[u] = w[u] != 0.f ? __ldcs(src + (n0 + u) * step) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < kMergeAhead; ++u) {
+      float v[kN];
+      Vec16<T>::unpack(raw[u], v);
+#pragma unroll
+      for (int i = 0; i < kN; ++i) acc[i] = fmaf(w[u], v[i], acc[i]);
     }
   }
-  if (live) Vec16<T>::store(merged + (size_t)row * D + sub * kN, acc);
-  if (live && sub == 0 && row_lse) row_lse[row] = m - logf(zinv);      // log-sum-exp of the row over all key chunks
+  if (!live) return;
+  const size_t orow = (size_t)gr * L + l0 + row;
+  Vec16<T>::store(merged + orow * D + sub * kN, acc);
+  if (sub == 0 && row_lse) row_lse[orow] = m - logf(zinv);      // log-sum-exp of the row over all key chunks
+}
+
+// ... of a few chunks (kFew = 2 .. 4, the sub-chunks of a wide chunk): no tables and no barrier, all of a thread's reads at once.  With
+// the kernel above, whose blocks then have next to nothing to do between their barriers, 2 sub-chunks of B1 H8 R4 L2048 D128
+// took 179 us.
+template <typename T, typename TL, int TPR, int kFew>
+__global__ void __launch_bounds__(kMergeThreads) merge_few_kernel(const T* __restrict__ out_cm, const TL* __restrict__ lse_cm,
+                                                                  T* __restrict__ merged, float* __restrict__ row_lse, long long rows, int R, int L) {
+  constexpr int kN = Vec16<T>::kN, D = TPR * kN;
+  const long long row = (long long)blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
+  if (row >= rows) return;
+  const int sub = threadIdx.x % TPR;
+  const size_t nstride = (size_t)R * L, base = (size_t)(row / (long long)nstride) * kFew * nstride + (size_t)(row % (long long)nstride);
+  uint4 raw[kFew];
+  float e[kFew], m = -INFINITY, z = 0.f, acc[kN];
+#pragma unroll
+  for (int n = 0; n < kFew; ++n) {
+    e[n] = Num<TL>::ld(lse_cm + base + n * nstride);
+    raw[n] = __ldcs(reinterpret_cast<const uint4*>(out_cm + (base + n * nstride) * D) + sub);
+  }
+#pragma unroll
+  for (int n = 0; n < kFew; ++n) m = fmaxf(m, e[n]);
+#pragma unroll
+  for (int n = 0; n < kFew; ++n) z += e[n] = expf(e[n] - m);
+  const float zinv = 1.0f / z;
+#pragma unroll
+  for (int i = 0; i < kN; ++i) acc[i] = 0.f;
+#pragma unroll
+  for (int n = 0; n < kFew; ++n) {
+    const float w = e[n] * zinv;
+    float v[kN];
+    Vec16<T>::unpack(raw[n], v);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) acc[i] = w != 0.f ? fmaf(w, v[i], acc[i]) : acc[i];
+  }
+  Vec16<T>::store(merged + (size_t)row * D + sub * kN, acc);
+  if (sub == 0 && row_lse) row_lse[row] = m - logf(zinv);
+}
+
+// Backward of the merge: g_out_cm[n][row][:] = g[row][:] w_n ; g_lse[n][row] = (s_n - sum_m s_m w_m) w_n,
+// s_n = g[row] . out_cm[n][row].  With skip_masked, the (row, chunk) blocks with row < n * chunk (rows before
+// the key chunk, whose weight is exactly zero) are not written: the caller promises not to read them.
+// Bound by HBM: the chunks that count are read, all are written.  Same shape as the forward; B4 H8 R4 L4096 D64: 952 -> 533 us (6.0 TB/s).
+template <typename T, typename TL, int TPR>
+__global__ void __launch_bounds__(kMergeThreads) merge_bwd_kernel(const T* __restrict__ out_cm, const TL* __restrict__ lse_cm,
+                                                                  const T* __restrict__ g_merged, T* __restrict__ g_out_cm,
+                                                                  TL* __restrict__ g_lse_cm, int N, int R, int L, int skip_masked) {
+  constexpr int kN = Vec16<T>::kN, D = TPR * kN, kRows = kMergeThreads / TPR, kPitch = kRows + 1;
+  extern __shared__ float sW[];
+  float *sS = sW + N * kPitch, *sT = sS + N * kPitch;
+  const int tiles = (L + kRows - 1) / kRows, gr = blockIdx.x / tiles, l0 = (blockIdx.x - gr * tiles) * kRows;
+  const int r = gr % R, row = threadIdx.x / TPR, sub = threadIdx.x % TPR, chunk = L / N;
+  const size_t nstride = (size_t)R * L, base = ((size_t)(gr / R) * N * R + r) * L + l0;
+  const int rows_here = L - l0 < kRows ? L - l0 : kRows;
+  const bool live = row < rows_here;
+  float g[kN];
+  Vec16<T>::load(g_merged + ((size_t)gr * L + l0 + (live ? row : 0)) * D + sub * kN, g);
+  float m, zinv;
+  const int last = merge_weights<TL, TPR>(lse_cm + base, nstride, N, rows_here, sW, m, zinv);
+  const size_t step = nstride * D * sizeof(T) / 16, first = (base + row) * D * sizeof(T) / 16 + sub;
+  const uint4* src = reinterpret_cast<const uint4*>(out_cm) + first;
+  uint4* dst = reinterpret_cast<uint4*>(g_out_cm) + first;
+  float t = 0.f;
+  for (int n0 = 0; n0 < last; n0 += kMergeAhead) {
+    uint4 raw[kMergeAhead];
+    float w[kMergeAhead];
+#pragma unroll
+    for (int u = 0; u < kMergeAhead; ++u) {
+      w[u] = (live && n0 + u < last) ? sW[(n0 + u) * kPitch + row] : 0.f;
+      raw[u] = w[u] != 0.f ? __ldcs(src + (n0 + u) * step) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < kMergeAhead; ++u) {
+      if (n0 + u >= last) break;
+      float v[kN], o[kN], s = 0.f;
+      Vec16<T>::unpack(raw[u], v);
+#pragma unroll
+      for (int i = 0; i < kN; ++i) {
+        s = fmaf(g[i], v[i], s);
+        o[i] = g[i] * w[u];
+      }
+      if (live && (w[u] != 0.f || !(skip_masked && l0 + row < (n0 + u) * chunk))) __stcs(dst + (n0 + u) * step, Vec16<T>::pack(o));
+      s = group_sum<TPR>(s);
+      t = fmaf(s, w[u], t);
+      if (sub == 0) sS[(n0 + u) * kPitch + row] = s;
+    }
+  }
+  for (int n = last; n < N; ++n) {
+    if (live && !(skip_masked && l0 + row < n * chunk)) __stcs(dst + n * step, make_uint4(0, 0, 0, 0));
+    if (sub == 0) sS[n * kPitch + row] = 0.f;
+  }
+  if (sub == 0) sT[row] = t;
+  __syncthreads();
+  for (int e = threadIdx.x; e < N * kRows; e += kMergeThreads) {
+    const int n = e / kRows, q = e % kRows;
+    if (q < rows_here && !(skip_masked && l0 + q < n * chunk))
+      Num<TL>::st(g_lse_cm + base + (size_t)n * nstride + q, (sS[n * kPitch + q] - sT[q]) * sW[n * kPitch + q]);
+  }
+}
+// ... for so many chunks that the tables do not fit shared memory (N above about 860 at head_dim 64): weights from the log-sum-exps on
+// the fly, TPR threads per row, and in the backward a first pass over the outputs for sum_m s_m w_m alone.
+template <typename T, typename TL, int TPR>
+__global__ void __launch_bounds__(kMergeThreads) merge_many_kernel(const T* __restrict__ out_cm, const TL* __restrict__ lse_cm,
+                                                                   T* __restrict__ merged, float* __restrict__ row_lse,
+                                                                   const T* __restrict__ g_merged, T* __restrict__ g_out_cm, TL* __restrict__ g_lse_cm,
+                                                                   long long rows, int N, int R, int L, int skip_masked) {
+  constexpr int kN = Vec16<T>::kN, D = TPR * kN;
+  const long long first = (long long)blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR, row = first < rows ? first : rows - 1;
+  const bool live = first < rows;
+  const int sub = threadIdx.x % TPR, l = (int)(row % L), r = (int)(row / L % R), chunk = L / N;
+  const size_t nstride = (size_t)R * L, base = ((size_t)(row / L / R) * N * R + r) * L + l;
+  auto lse = [&](int n) { return Num<TL>::ld(lse_cm + base + (size_t)n * nstride); };
+  float m = -INFINITY, z = 0.f;
+  for (int n = sub; n < N; n += TPR) m = fmaxf(m, lse(n));
+  m = group_max<TPR>(m);
+  for (int n = sub; n < N; n += TPR) z += expf(lse(n) - m);
+  const float zinv = 1.0f / group_sum<TPR>(z);
+  auto weight = [&](int n) { return expf(lse(n) - m) * zinv; };
+  float g[kN], acc[kN], t = 0.f;
+#pragma unroll
+  for (int i = 0; i < kN; ++i) g[i] = acc[i] = 0.f;
+  if (g_merged) Vec16<T>::load(g_merged + (size_t)row * D + sub * kN, g);
+  auto product = [&](int n, float w) {      // s_n, and the weighted sum
+    float v[kN], s = 0.f;
+    if (w != 0.f) {
+      Vec16<T>::load(out_cm + (base + (size_t)n * nstride) * D + sub * kN, v);
+#pragma unroll
+      for (int i = 0; i < kN; ++i) {
+        s = fmaf(g[i], v[i], s);
+        acc[i] = fmaf(w, v[i], acc[i]);
+      }
+    }
+    return s;
+  };
+  for (int n = 0; n < N; ++n) {
+    const float w = weight(n), s = product(n, w);
+    if (g_merged) t = fmaf(group_sum<TPR>(s), w, t);
+  }
+  if (!g_merged) {
+    if (live) Vec16<T>::store(merged + (size_t)row * D + sub * kN, acc);
+    if (live && sub == 0 && row_lse) row_lse[row] = m - logf(zinv);
+    return;
+  }
+  for (int n = 0; n < N; ++n) {
+    const size_t at = base + (size_t)n * nstride;
+    const float w = weight(n), s = group_sum<TPR>(product(n, w));
+    if (!live || (skip_masked && w == 0.f && l < n * chunk)) continue;
+    float o[kN];
+#pragma unroll
+    for (int i = 0; i < kN; ++i) o[i] = g[i] * w;
+    Vec16<T>::store(g_out_cm + at * D + sub * kN, o);
+    if (sub == 0) Num<TL>::st(g_lse_cm + at, (s - t) * w);
+  }
+}
+template <int TPR> inline size_t merge_smem(int N, bool backward) {
+  constexpr int kRows = kMergeThreads / TPR;
+  return ((size_t)N * (kRows + 1) * (backward ? 2 : 1) + kRows) * sizeof(float);
 }
 
 // out[row] = a[row] . b[row] over D = TPR * kN elements (the delta = g . merged of the merged backward)
@@ -167,91 +357,52 @@ __global__ void __launch_bounds__(kMergeThreads) row_dot_kernel(const T* __restr
   if (live && sub == 0) out[row] = acc;
 }
 
-// Backward of the merge: g_out_cm[n][row][:] = g[row][:] w_n ; g_lse[n][row] = (s_n - sum_m s_m w_m) w_n,
-// s_n = g[row] . out_cm[n][row].  With skip_masked, the (row, chunk) blocks with row < n * chunk (rows before
-// the key chunk, whose weight is exactly zero) are not written: the caller promises not to read them.
-template <typename T, int TPR>
-__global__ void __launch_bounds__(kMergeThreads) merge_bwd_kernel(const T* __restrict__ out_cm, const float* __restrict__ lse_cm,
-                                                                  const T* __restrict__ g_merged, T* __restrict__ g_out_cm,
-                                                                  float* __restrict__ g_lse_cm, long long rows, int N, int R,
-                                                                  int L, int skip_masked) {
-  constexpr int kN = Vec16<T>::kN;
-  constexpr int D = TPR * kN;
-  const long long row = (long long)blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
-  const int sub = threadIdx.x % TPR;
-  const bool live = row < rows;
-  const long long rr = live ? row : rows - 1;
-  const int l = (int)(rr % L);
-  const long long gr = rr / L;
-  const int r = (int)(gr % R);
-  const long long bh = gr / R;
-  const size_t nstride = (size_t)R * L;
-  const size_t base = ((size_t)bh * N * R + r) * L + l;
-  const int chunk = L / N;
-  float m, zinv;
-  merge_row_stats<TPR>(lse_cm + base, nstride, N, sub, m, zinv);
-  float g[kN];
-  Vec16<T>::load(g_merged + (size_t)rr * D + sub * kN, g);
-  float t = 0.f;
-  for (int n = 0; n < N; ++n) {
-    const size_t idx = base + (size_t)n * nstride;
-    const float w = expf(lse_cm[idx] - m) * zinv;
-    float s = 0.f;
-    if (w != 0.f) {
-      float v[kN], o[kN];
-      Vec16<T>::load(out_cm + idx * D + sub * kN, v);
-#pragma unroll
-      for (int i = 0; i < kN; ++i) {
-        s = fmaf(g[i], v[i], s);
-        o[i] = g[i] * w;
-      }
-      if (live) Vec16<T>::store(g_out_cm + idx * D + sub * kN, o);
-    } else if (!(skip_masked && l < n * chunk) && live) {
-      float o[kN];
-#pragma unroll
-      for (int i = 0; i < kN; ++i) o[i] = 0.f;
-      Vec16<T>::store(g_out_cm + idx * D + sub * kN, o);
-    }
-    s = group_sum<TPR>(s);
-    t = fmaf(s, w, t);
-    if (live && sub == 0 && !(skip_masked && l < n * chunk)) g_lse_cm[idx] = s;     // parked; finished below by the same thread
-  }
-  if (live && sub == 0) {
-    for (int n = 0; n < N; ++n) {
-      const size_t idx = base + (size_t)n * nstride;
-      const float w = expf(lse_cm[idx] - m) * zinv;
-      if (!(skip_masked && l < n * chunk)) g_lse_cm[idx] = (g_lse_cm[idx] - t) * w;
-    }
-  }
-}
-
 // ---- input prologue -----------------------------------------------------------------
 // The model hands over projections in token-major order: query_state (b,s,n,d), key_state / value_state (b,s,n_kv,d)
 // and gate logits (b,s,2,n_kv).  The operator wants head-major tensors: xq (b,n_kv,rep,s,d) (query head kv*rep + r),
 // kc / vc (b,n_kv,s,d), static_src / static_dest (b,n_kv,s) (the reference's driver does this with transposes and
 // views, main.py:24-31).  One pass does the transposes and, on request, the two things a model applies on the way
 // (Universal_Attention/triton/_debug.py:470-475): keys divided by (|k| + 1e-6) and gates through a sigmoid.
-// One group of TPR threads per row of d elements; rows = b * s * (n + 2 n_kv).
+// One group of TPR threads per row of d elements; rows = b * s * (n + 2 n_kv); the blocks behind the rows' take the gates.
+// Bound by HBM in 128-byte pieces on the head-major side: B4 L4096, 32 + 8 heads of 64, 200 MB each way: 45 + 5 us forward and
+// 64 + 5 us backward with 64-bit index divisions and the gates in launches of their own -> 44 and 62 us.  (A thread that owns one
+// slice of a head for several tokens, or several rows, was slower: 46 - 48 us and 65 - 84 us, and twice as slow at 1024 tokens.)
 struct PrepDims {
   int b, s, n, n_kv, normalize_keys, sigmoid_gates;
+  unsigned rows, row_blocks;
 };
+
+// gates (b, s, 2, n_kv) <-> two (b, n_kv, s): f(token-major index, head-major index, which), consecutive threads along s
+template <typename F>
+__device__ __forceinline__ void prep_gates(const PrepDims& pd, F f) {
+  const unsigned total = (unsigned)pd.b * pd.s * 2 * pd.n_kv, stride = (gridDim.x - pd.row_blocks) * kMergeThreads;
+  for (unsigned e = (blockIdx.x - pd.row_blocks) * kMergeThreads + threadIdx.x; e < total; e += stride) {
+    const unsigned z = e / pd.s, ss = e - z * pd.s, bb = z / (2 * pd.n_kv), y = z - bb * 2 * pd.n_kv, which = y / pd.n_kv, kv = y - which * pd.n_kv;
+    f(((size_t)bb * pd.s + ss) * 2 * pd.n_kv + y, ((size_t)bb * pd.n_kv + kv) * pd.s + ss, (int)which);
+  }
+}
 
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kMergeThreads) prepare_fwd_kernel(PrepDims pd, const T* __restrict__ qs, const T* __restrict__ ks,
-                                                                    const T* __restrict__ vs, T* __restrict__ xq, T* __restrict__ kc,
-                                                                    T* __restrict__ vc, float* __restrict__ key_norm) {
+                                                                    const T* __restrict__ vs, const T* __restrict__ gs, T* __restrict__ xq,
+                                                                    T* __restrict__ kc, T* __restrict__ vc, T* __restrict__ ssrc,
+                                                                    T* __restrict__ sdest, float* __restrict__ key_norm) {
+  if (blockIdx.x >= pd.row_blocks) {
+    prep_gates(pd, [&](size_t tm, size_t hm, int which) {
+      float x = Num<T>::ld(gs + tm);
+      if (pd.sigmoid_gates) x = 1.0f / (1.0f + __expf(-x));
+      Num<T>::st((which ? sdest : ssrc) + hm, x);
+    });
+    return;
+  }
   constexpr int kN = Vec16<T>::kN;
   constexpr int D = TPR * kN;
-  const int heads = pd.n + 2 * pd.n_kv;
-  const long long rows = (long long)pd.b * pd.s * heads;
-  const long long row = (long long)blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
+  const unsigned heads = pd.n + 2 * pd.n_kv;
+  const unsigned row = blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
   const int sub = threadIdx.x % TPR;
-  const bool live = row < rows;
-  const long long rr = live ? row : rows - 1;
-  const int hh = (int)(rr % heads);
-  const long long tok = rr / heads;                 // bb * s + ss
-  const int ss = (int)(tok % pd.s);
-  const long long bb = tok / pd.s;
+  const bool live = row < pd.rows;
+  const unsigned rr = live ? row : pd.rows - 1, tok = rr / heads, bb = tok / pd.s;      // tok = bb * s + ss
+  const int hh = (int)(rr - tok * heads), ss = (int)(tok - bb * pd.s);
   const bool is_q = hh < pd.n, is_k = !is_q && hh < pd.n + pd.n_kv;
   const int kv = is_q ? 0 : (is_k ? hh - pd.n : hh - pd.n - pd.n_kv);
   const size_t hm = ((size_t)bb * pd.n_kv + kv) * pd.s + ss;          // head-major row of a key / value
@@ -277,51 +428,33 @@ __global__ void __launch_bounds__(kMergeThreads) prepare_fwd_kernel(PrepDims pd,
   }
 }
 
-// gates: one thread per (b, s, which, kv)
-template <typename T>
-__global__ void prepare_gates_kernel(PrepDims pd, const T* __restrict__ gs, T* __restrict__ ssrc, T* __restrict__ sdest, int backward,
-                                     const T* __restrict__ g_src, const T* __restrict__ g_dest, T* __restrict__ d_gs) {
-  const long long total = (long long)pd.b * pd.s * 2 * pd.n_kv;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int kv = (int)(e % pd.n_kv);
-    const int which = (int)((e / pd.n_kv) % 2);
-    const long long tok = e / (2 * pd.n_kv);
-    const int ss = (int)(tok % pd.s);
-    const long long bb = tok / pd.s;
-    const size_t dst = ((size_t)bb * pd.n_kv + kv) * pd.s + ss;
-    if (!backward) {
-      float x = Num<T>::ld(gs + e);
-      if (pd.sigmoid_gates) x = 1.0f / (1.0f + __expf(-x));
-      Num<T>::st((which ? sdest : ssrc) + dst, x);
-    } else {
-      // ssrc / sdest hold the forward's outputs (the gate values), g_* their gradients
-      const float gate = Num<T>::ld((which ? sdest : ssrc) + dst);
-      float g = Num<T>::ld((which ? g_dest : g_src) + dst);
-      if (pd.sigmoid_gates) g *= gate * (1.0f - gate);
-      Num<T>::st(d_gs + e, g);
-    }
-  }
-}
-
 // backward of prepare_fwd_kernel: gradients flow back along the same row mapping; key rows pass through the
 // derivative of k / (|k| + eps):  dk = g / (|k| + eps) - khat (g . khat) / |k|
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kMergeThreads) prepare_bwd_kernel(PrepDims pd, const T* __restrict__ g_xq, const T* __restrict__ g_kc,
-                                                                    const T* __restrict__ g_vc, const T* __restrict__ kc,
-                                                                    const float* __restrict__ key_norm, T* __restrict__ d_qs,
-                                                                    T* __restrict__ d_ks, T* __restrict__ d_vs) {
+                                                                    const T* __restrict__ g_vc, const T* __restrict__ g_src,
+                                                                    const T* __restrict__ g_dest, const T* __restrict__ kc,
+                                                                    const float* __restrict__ key_norm, const T* __restrict__ ssrc,
+                                                                    const T* __restrict__ sdest, T* __restrict__ d_qs, T* __restrict__ d_ks,
+                                                                    T* __restrict__ d_vs, T* __restrict__ d_gs) {
+  if (blockIdx.x >= pd.row_blocks) {
+    prep_gates(pd, [&](size_t tm, size_t hm, int which) {
+      // ssrc / sdest hold the forward's outputs (the gate values), g_* their gradients
+      const float gate = Num<T>::ld((which ? sdest : ssrc) + hm);
+      float g = Num<T>::ld((which ? g_dest : g_src) + hm);
+      if (pd.sigmoid_gates) g *= gate * (1.0f - gate);
+      Num<T>::st(d_gs + tm, g);
+    });
+    return;
+  }
   constexpr int kN = Vec16<T>::kN;
   constexpr int D = TPR * kN;
-  const int heads = pd.n + 2 * pd.n_kv;
-  const long long rows = (long long)pd.b * pd.s * heads;
-  const long long row = (long long)blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
+  const unsigned heads = pd.n + 2 * pd.n_kv;
+  const unsigned row = blockIdx.x * (kMergeThreads / TPR) + threadIdx.x / TPR;
   const int sub = threadIdx.x % TPR;
-  const bool live = row < rows;
-  const long long rr = live ? row : rows - 1;
-  const int hh = (int)(rr % heads);
-  const long long tok = rr / heads;
-  const int ss = (int)(tok % pd.s);
-  const long long bb = tok / pd.s;
+  const bool live = row < pd.rows;
+  const unsigned rr = live ? row : pd.rows - 1, tok = rr / heads, bb = tok / pd.s;      // tok = bb * s + ss
+  const int hh = (int)(rr - tok * heads), ss = (int)(tok - bb * pd.s);
   const bool is_q = hh < pd.n, is_k = !is_q && hh < pd.n + pd.n_kv;
   const int kv = is_q ? 0 : (is_k ? hh - pd.n : hh - pd.n - pd.n_kv);
   const size_t hm = ((size_t)bb * pd.n_kv + kv) * pd.s + ss;

@@ -171,10 +171,15 @@ UaDims merge_dims(const Tensor& out_cm) {
   const int64_t n = out_cm.size(2), L = out_cm.size(4);
   return UaDims{(int)out_cm.size(0), (int)out_cm.size(1), (int)out_cm.size(3), (int)n, (int)(L / n), (int)out_cm.size(5)};
 }
+// the merge takes log-sum-exps in fp32 or in the outputs' type
+Tensor merge_lse(const Tensor& out, const Tensor& lse_) {
+  const Tensor lse = plain(lse_);
+  return (lse.scalar_type() == at::kFloat || lse.scalar_type() == out.scalar_type() ? lse : lse.to(at::kFloat)).contiguous();
+}
 // merged (b,h,r,L,d) and, on request, the rows' log-sum-exp over all chunks
 std::tuple<Tensor, OptTensor> merge_fwd_cm(const Tensor& out_, const Tensor& lse_, bool stats) {
   require_cuda(out_, lse_);
-  const Tensor out = plain(out_).contiguous(), lse = plain(lse_).to(at::kFloat).contiguous();
+  const Tensor out = plain(out_).contiguous(), lse = merge_lse(out, lse_);
   const UaDims dims = merge_dims(out);
   const c10::cuda::CUDAGuard guard(out.device());
   TORCH_CHECK(lse.numel() * out.size(5) == out.numel(), "log-sum-exp does not fit the outputs");
@@ -182,20 +187,20 @@ std::tuple<Tensor, OptTensor> merge_fwd_cm(const Tensor& out_, const Tensor& lse
   Tensor merged = at::empty({out.size(0), out.size(1), out.size(3), out.size(4), out.size(5)}, opt);
   OptTensor row_lse;
   if (stats) row_lse = at::empty({out.size(0), out.size(1), out.size(3), out.size(4)}, opt.dtype(at::kFloat));
-  check(ua_merge_fwd_stats(&dims, code_of(out.scalar_type()), ptr(out), static_cast<float*>(ptr(lse)), ptr(merged),
+  check(ua_merge_fwd_typed(&dims, code_of(out.scalar_type()), code_of(lse.scalar_type()), ptr(out), ptr(lse), ptr(merged),
                            row_lse ? static_cast<float*>(ptr(*row_lse)) : nullptr, stream_of(out)), stats ? "ua_merge_fwd_stats" : "ua_merge_fwd");
   return {merged, row_lse};
 }
 std::tuple<Tensor, Tensor> merge_bwd_cm(const Tensor& out_, const Tensor& lse_, const Tensor& g_, bool skip_zero_weight_blocks) {
   require_cuda(out_, lse_, g_);
-  const Tensor out = plain(out_).contiguous(), lse = plain(lse_).to(at::kFloat).contiguous();
+  const Tensor out = plain(out_).contiguous(), lse = merge_lse(out, lse_);
   const Tensor g = plain(g_).to(out.scalar_type()).contiguous();
   const UaDims dims = merge_dims(out);
   const c10::cuda::CUDAGuard guard(out.device());
   TORCH_CHECK(lse.numel() * out.size(5) == out.numel() && g.numel() * out.size(2) == out.numel(), "gradient or log-sum-exp does not fit the outputs");
   const auto opt = out.options().requires_grad(false);
-  Tensor g_out = at::empty(out.sizes(), opt), g_lse = at::empty(lse.sizes(), opt.dtype(at::kFloat));
-  check(ua_merge_bwd(&dims, code_of(out.scalar_type()), ptr(out), static_cast<float*>(ptr(lse)), ptr(g), ptr(g_out), static_cast<float*>(ptr(g_lse)),
+  Tensor g_out = at::empty(out.sizes(), opt), g_lse = at::empty(lse.sizes(), opt.dtype(lse.scalar_type()));
+  check(ua_merge_bwd_typed(&dims, code_of(out.scalar_type()), code_of(lse.scalar_type()), ptr(out), ptr(lse), ptr(g), ptr(g_out), ptr(g_lse),
                      skip_zero_weight_blocks ? UA_FLAG_SKIP_MASKED_FILL : 0, stream_of(out)), "ua_merge_bwd");
   return {g_out, g_lse};
 }

@@ -227,7 +227,7 @@ def backward_merged(kc, vc, xq, static_src, static_dest, g_merged, merged, row_l
 
 
 def merge_bwd_cm(out_cm, lse_cm, g_merged, skip_zero_weight_blocks: bool = False):
-    """SMVecMatMul backward on chunk-major storage -> (g_out_cm, g_lse_cm fp32).
+    """SMVecMatMul backward on chunk-major storage -> (g_out_cm, g_lse_cm in the type of ``lse_cm``).
     ``skip_zero_weight_blocks``: leave the blocks whose merge weight is exactly zero unwritten
     (only valid when the consumer never reads them: backward with masked-block gradients skipped)."""
     return _lib.native().merge_bwd_cm(out_cm, lse_cm, g_merged, skip_zero_weight_blocks)
