@@ -137,10 +137,17 @@ __device__ __forceinline__ int merge_weights(const TL* lse, size_t nstride, int 
   return __reduce_max_sync(0xffffffffu, last);
 }
 constexpr int kMergeAhead = 8;      // chunks whose loads a thread has in flight
+// (in an order the compiler keeps: it would otherwise issue each read beside its use, a few at a time)
+__device__ __forceinline__ uint4 load_if(const uint4* p, bool on) {
+  uint4 x = make_uint4(0, 0, 0, 0);
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "+r"(x.x), "+r"(x.y), "+r"(x.z), "+r"(x.w) : "l"(p), "r"((int)on));
+  return x;
+}
 
 // merged[row][d] = sum_n softmax_n(lse[n][row]) * out_cm[n][row][d]
 // Bound by the read of the chunks that count; eight 16-byte loads in flight per thread.  B4 H8 R4 L4096 D64 (1.07 GB read):
-// 306 us with one load in flight behind its own exponential -> 223 us (4.8 TB/s).
+// 306 us with one load in flight behind its own exponential -> 205 us (5.2 TB/s).
 template <typename T, typename TL, int TPR>
 __global__ void __launch_bounds__(kMergeThreads) merge_fwd_kernel(const T* __restrict__ out_cm, const TL* __restrict__ lse_cm,
                                                                   T* __restrict__ merged, float* __restrict__ row_lse, int N, int R, int L) {
@@ -164,7 +171,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_fwd_kernel(const T* __res
 #pragma unroll
     for (int u = 0; u < kMergeAhead; ++u) {
       w[u] = (live && n0 + u < last) ? sW[(n0 + u) * kPitch + row] : 0.f;
-      raw[u] = w[u] != 0.f ? __ldcs(src + (n0 + u) * step) : make_uint4(0, 0, 0, 0);
+      raw[u] = load_if(src + (n0 + u) * step, w[u] != 0.f);
     }
 #pragma unroll
     for (int u = 0; u < kMergeAhead; ++u) {
@@ -247,7 +254,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_bwd_kernel(const T* __res
 #pragma unroll
     for (int u = 0; u < kMergeAhead; ++u) {
       w[u] = (live && n0 + u < last) ? sW[(n0 + u) * kPitch + row] : 0.f;
-      raw[u] = w[u] != 0.f ? __ldcs(src + (n0 + u) * step) : make_uint4(0, 0, 0, 0);
+      raw[u] = load_if(src + (n0 + u) * step, w[u] != 0.f);
     }
 #pragma unroll
     for (int u = 0; u < kMergeAhead; ++u) {
