@@ -371,6 +371,17 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype,
 int ua_merge_bwd(const UaDims* dims, int dtype, const void* out_cm, const float* lse_cm,
                  const void* g_merged, void* g_out_cm, float* g_lse_cm, int flags, void* stream);
 
+/* Copies (batch, heads, rows) rows of src_bytes into rows of dst_bytes with the heads in another order: destination head hd takes
+ * source head (hd % a) * (heads / a) + hd / a.  Missing bytes are zero, surplus bytes are dropped (the head order and the zero
+ * padding of universal_attention_kernel_opt.py:142, :445-453).  Row widths are multiples of 16; 1 to 3 copies per call. */
+typedef struct UaHeadCopy {
+  const void* src;
+  void* dst;
+  int32_t batch, heads, rows, a;
+  int32_t src_bytes, dst_bytes;
+} UaHeadCopy;
+int ua_copy_heads(const UaHeadCopy* copies, int count, void* stream);
+
 /* ua_merge_fwd_stats and ua_merge_bwd for log-sum-exps (and their gradient) in lse_dtype: UA_F32, or dtype. */
 int ua_merge_fwd_typed(const UaDims* dims, int dtype, int lse_dtype, const void* out_cm, const void* lse_cm, void* merged,
                        float* row_lse, void* stream);

@@ -17,7 +17,8 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from ..universal_attention_autograd import UniversalAttentionMerged
+from .. import _lib
+from .. import universal_attention_autograd as _ua
 
 CHUNK = 128
 
@@ -31,15 +32,19 @@ def attention(q, k, v, causal=True, sm_scale=None, static_src=None, static_dest=
     assert k.shape == (b, n_kv, s, d) and v.shape == (b, n_kv, s, d) and n_heads % n_kv == 0
     assert static_src.shape == (b, n_kv, s) and static_dest.shape == (b, n_kv, s)
     rep = n_heads // n_kv
+    dp = 64 if d <= 64 else (128 if d <= 128 else d)
+    # the whole call as one graph node in native code; functorch's transforms, the other modes of the merged output and rows
+    # that are not whole 16-byte pieces take the composition below
+    if not _ua._transforms_active() and _ua._default_merge_modes() and (d * q.element_size()) % 16 == 0:
+        return _lib.native().attention_apply(q, k, v, static_src, static_dest, dp, CHUNK)
     # head dims the tensor-core kernels do not take are zero-padded: zero columns change neither k.k, q.k nor the
     # leading d columns of the output
-    dp = 64 if d <= 64 else (128 if d <= 128 else d)
     if dp != d:
         q, k, v = (F.pad(t, (0, dp - d)) for t in (q, k, v))
     n = s // CHUNK
     xq = q.view(b, rep, n_kv, s, dp).transpose(1, 2)          # query head r * n_kv + kv reads kv head kv
     kc = k.reshape(b, n_kv, n, CHUNK, dp)
     vc = v.reshape(b, n_kv, n, CHUNK, dp)
-    merged = UniversalAttentionMerged.apply(kc, vc, xq.contiguous(), static_src.reshape(b, n_kv, n, CHUNK), static_dest)
+    merged = _ua.UniversalAttentionMerged.apply(kc, vc, xq.contiguous(), static_src.reshape(b, n_kv, n, CHUNK), static_dest)
     o = merged.view(b, n_kv, rep, s, dp).transpose(1, 2).reshape(b, n_heads, s, dp)
     return o[..., :d]

@@ -63,6 +63,7 @@ SIGNATURES = {
     "ua_merge_fwd": (_i, [_dp, _i, _vp, _vp, _vp, _vp]),
     "ua_merge_bwd": (_i, [_dp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "ua_merge_fwd_stats": (_i, [_dp, _i, _vp, _vp, _vp, _vp, _vp]),
+    "ua_copy_heads": (_i, [_vp, _i, _vp]),
     "ua_merge_fwd_typed": (_i, [_dp, _i, _i, _vp, _vp, _vp, _vp, _vp]),
     "ua_merge_bwd_typed": (_i, [_dp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "ua_row_dot": (_i, [ctypes.c_longlong, _i, _i, _vp, _vp, _vp, _vp]),

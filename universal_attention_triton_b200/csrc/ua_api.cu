@@ -105,16 +105,16 @@ BwdWorkspaceTiled bwd_layout_tiled(const ua::Shape& s) {
 bool runs_tiled(const ua::Shape& s, int flags) { return !(flags & UA_FLAG_FORCE_SIMT) && ua::tiled::fits(s); }
 
 struct BwdWorkspaceTc {
-  size_t off_dk, off_dq, off_dt, off_dkr, off_dv, off_ds, off_carry, off_lse, off_gd, off_mt, off_ksum, off_nacc, off_seg, off_out, off_fwd;
+  size_t off_dk, off_dq, off_dt, off_dkr, off_dv, off_ds, off_carry, off_lse, off_gd, off_mt, off_ksum, off_nacc, off_seg, off_lse_sub;
   size_t acc_bytes, acc_fp32_v_bytes, total;     // what is zeroed: without and with the fp32 dV / d static_src
 };
 
 // Scratch of the tensor-core backward.  s: the kernels' shape (chunks of 64 or 128 keys), m: kernel chunks per chunk of the
 // operator.  Status | fp32 accumulators dK, dQ, d dest, row-side dK, and dV, d src for sweeps that are cut into segments or share
 // them with the kernel of the rows before a chunk | decay-prefix table | log-sum-exp (only written when the caller has none) | fp32
-// g_denom or row term | per-chunk data of the kernels for the rows before a chunk / segment totals | for m > 1 the output and the
-// scratch of a forward run (only used for callers that kept neither).
-BwdWorkspaceTc bwd_layout_tc(const ua::Shape& s, int m, size_t fwd_bytes) {
+// g_denom or row term | per-chunk data of the kernels for the rows before a chunk / segment totals | for m > 1 the sub-chunks'
+// log-sum-exps (only written for callers that kept none).
+BwdWorkspaceTc bwd_layout_tc(const ua::Shape& s, int m) {
   BwdWorkspaceTc w{};
   const size_t BH = (size_t)s.B * s.H, f = sizeof(float), rows = BH * (s.N / m) * (size_t)s.R * s.L;
   const int seg = ua::sm100::bwd_split(s);
@@ -139,8 +139,8 @@ BwdWorkspaceTc bwd_layout_tc(const ua::Shape& s, int m, size_t fwd_bytes) {
   w.off_ksum = o; o = align_up(o + BH * s.N * (size_t)s.D * 2, 256);
   w.off_nacc = o; o = align_up(o + BH * s.N * (size_t)(s.D + 3) * s.D * f, 256);
   if (m > 1) {
-    w.off_out = o; o = align_up(o + rows * s.D * 2, 256);
-    w.off_fwd = o; o = align_up(o + fwd_bytes, 256);
+    w.off_lse_sub = o; o = align_up(o + m * rows * f, 256);
+    o = std::max(o, align_up(2 * m * rows * s.D * 2, 256));      // (never less than the two sub-chunk tensors that callers have planned for)
   }
   w.total = o;
   return w;
@@ -275,9 +275,21 @@ __global__ void row_lse_kernel(const float* __restrict__ lse_cm, float* __restri
   }
 }
 
-// a status word raised by an inner call on its own buffer is carried over to the caller's
-__global__ void carry_status_kernel(const int* __restrict__ from, int* __restrict__ to) {
-  if (from[0] != 0 && atomicCAS(to, 0, from[0]) == 0) to[1] = from[1];
+// log-sum-exp over the m sub-chunks of a wide chunk, for the rows that see the chunk (a sub-chunk's entries before its own first row
+// need not have been written: nothing of it is seen there)
+__global__ void group_lse_kernel(const float* __restrict__ sub, float* __restrict__ lse, size_t groups, size_t rl, int L, int N, int C, int m) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < groups * rl; idx += stride) {
+    const size_t grp = idx / rl, x = idx - grp * rl;
+    const int past = (int)(x % L) - (int)(grp % N) * C;      // rows past the chunk's first key
+    if (past < 0) continue;
+    const int seen = min(m, past / 128 + 1);
+    const float* l = sub + grp * m * rl + x;
+    float mx = l[0], z = 0.f;
+    for (int q = 1; q < seen; ++q) mx = fmaxf(mx, l[q * rl]);
+    for (int q = 0; q < seen; ++q) z += expf(l[q * rl] - mx);
+    lse[idx] = mx + logf(z);
+  }
 }
 
 bool dtype_ok(int dtype, int gate_dtype) {
@@ -463,9 +475,9 @@ size_t ua_bwd_workspace_bytes(const UaDims* dims, int dtype, int flags) {
   ua::Shape s = to_shape(dims);
   if (const int m = sub_chunks(s, dtype, flags)) {
     const UaDims sd = sub_dims(dims, m);
-    return bwd_layout_tc(to_shape(&sd), m, ua_fwd_workspace_bytes(dims, dtype, 0)).total;
+    return bwd_layout_tc(to_shape(&sd), m).total;
   }
-  if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype)) return bwd_layout_tc(s, 1, 0).total;
+  if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::bwd2_supported(s, dtype)) return bwd_layout_tc(s, 1).total;
   if (runs_tiled(s, flags)) return bwd_layout_tiled(s).total;
   const SimtCfg cfg = simt_cfg(s.C, s.D, dtype, true);
   if (!cfg.rt) return 0;
@@ -788,8 +800,7 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     const int m = wide ? wide : 1;
     const UaDims kd = wide ? sub_dims(dims, m) : *dims;
     const ua::Shape ks = to_shape(&kd);                 // the kernels' shape
-    const size_t fwd_bytes = wide ? ua_fwd_workspace_bytes(dims, dtype, 0) : 0;
-    const BwdWorkspaceTc w = bwd_layout_tc(ks, m, fwd_bytes);
+    const BwdWorkspaceTc w = bwd_layout_tc(ks, m);
     if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
     char* ws = static_cast<char*>(workspace);
     auto at = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
@@ -800,44 +811,43 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     if (cudaMemsetAsync(ws, 0, fp32_v ? w.acc_fp32_v_bytes : w.acc_bytes, st) != cudaSuccess) return UA_ERR_CUDA;
     const float* carry_tab = static_cast<const float*>(carry_in);
     float *acc_dk = at(w.off_dk), *acc_dq = at(w.off_dq);
-    // What the keys-on-lanes kernel needs besides the inputs: the decay-prefix table and the forward's log-sum-exp (for wide
-    // chunks the output too).  A caller that has neither gets both from one statistics-only run of the forward kernel (no output
-    // tile is written).
+    // What the keys-on-lanes kernel needs besides the inputs: the decay-prefix table and the forward's log-sum-exp.  A
+    // caller that has neither gets both from one statistics-only run of the forward kernel (no output tile is written).
     const float* lse = lse_cm;
-    const void* out = out_cm;
-    if (wide && (!lse || !carry_tab || !out)) {
-      if ((e = ua_fwd_keep(dims, dtype, gate_dtype, kc, vc, xq, static_src, static_dest, ws + w.off_out, at(w.off_lse), nullptr, at(w.off_carry),
-                           ws + w.off_fwd, fwd_bytes, UA_FLAG_SKIP_MASKED_FILL, stream)))
-        return e;
-      carry_status_kernel<<<1, 1, 0, st>>>(reinterpret_cast<const int*>(ws + w.off_fwd), reinterpret_cast<int*>(ws));
-      lse = at(w.off_lse); carry_tab = at(w.off_carry); out = ws + w.off_out;
-    } else if (!lse || !carry_tab) {
+    const size_t rows = (size_t)s.B * s.H * s.N * (size_t)s.R * s.L;
+    if (!lse || !carry_tab) {
       ua::sm100::FwdParams fp{};
       fp.s = ks; fp.ssrc = static_src; fp.sdest = static_dest; fp.out = nullptr; fp.denom = nullptr;
-      fp.lse = lse ? nullptr : at(w.off_lse);
+      fp.lse = lse ? nullptr : at(wide ? w.off_lse_sub : w.off_lse);
       fp.status = reinterpret_cast<int*>(ws);
       fp.carry = carry_tab ? nullptr : at(w.off_carry);
       ua::sm100::whole_sequence(fp);
       if (lse) e = ua::sm100::launch_fwd_carry(ks, gate_dtype, kc, fp, st);      // decay-only pass
       else e = ua::sm100::launch_fwd(ks, gate_dtype, kc, vc, xq, fp, false, nullptr, st);
       if (e) return e;
-      if (!lse) lse = fp.lse;
       if (!carry_tab) carry_tab = fp.carry;
+      if (!lse) {
+        lse = at(w.off_lse);
+        if (wide) {
+          group_lse_kernel<<<148 * 8, 256, 0, st>>>(fp.lse, at(w.off_lse), (size_t)s.B * s.H * s.N, (size_t)s.R * s.L, s.L, s.N, s.C, m);
+          if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
+        }
+      }
     }
     // The kernels' producers copy rows of lse / g_denom with 16-byte bulk copies: 16-byte aligned, and fp32 but for the sweep that
-    // takes its row term from the output tiles, which widens a bf16 g_denom by itself.  For wide chunks the table holds the row term.
-    const bool out_tiles = !wide && s.D == 64 && out && aligned16(out);
+    // takes its row term from the output tiles, which widens a bf16 g_denom by itself.  For wide chunks the table is a copy in which
+    // the row term is formed.
+    const bool out_tiles = !wide && s.D == 64 && out_cm && aligned16(out_cm);
     const float* gd32 = static_cast<const float*>(g_denom_cm);
-    if (wide) {
-      if ((e = ua::sm100::launch_row_term(ks, m, out, g_out_cm, g_denom_cm, g_denom_dtype, at(w.off_gd), st))) return e;
-      gd32 = at(w.off_gd);
-    } else if (g_denom_dtype != UA_F32 && (!out_tiles || (masked && ks.C == 128) || !aligned16(g_denom_cm))) {
-      const size_t n_gd = (size_t)s.B * s.H * s.N * (size_t)s.R * s.L;
-      widen_bf16_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const bf16*>(g_denom_cm), at(w.off_gd), n_gd);
+    if (g_denom_dtype != UA_F32 && (!out_tiles || (masked && ks.C == 128) || !aligned16(g_denom_cm))) {
+      widen_bf16_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const bf16*>(g_denom_cm), at(w.off_gd), rows);
       if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
       gd32 = at(w.off_gd);
     } else if (g_denom_dtype != UA_F32) {
       gd32 = nullptr;
+    } else if (wide) {
+      if (cudaMemcpyAsync(at(w.off_gd), g_denom_cm, rows * sizeof(float), cudaMemcpyDeviceToDevice, st) != cudaSuccess) return UA_ERR_CUDA;
+      gd32 = at(w.off_gd);
     }
     if (!aligned16(gd32) || !aligned16(lse) || !aligned16(static_dest) || !aligned16(carry_tab)) return UA_ERR_ALIGNMENT;
     // Rows before a chunk (uniform softmax): their gradient is added to the accumulators by kernels of their own.
@@ -867,7 +877,7 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     qp.dv_chunk = dv_chunk; qp.dv_chunk_stride = (s.D + 3) * s.D; qp.dv_scale = 1.0f / (float)s.C;
     qp.dvc = static_cast<bf16*>(dvc); qp.dss = dstatic_src; qp.status = reinterpret_cast<int*>(ws);
     qp.trace = nullptr;
-    qp.out_tiles = out_tiles ? out : nullptr;
+    qp.out_tiles = out_tiles ? out_cm : nullptr;
     if (fp32_v) qp.acc_dv = at(w.off_dv);
     if (seg) {
       qp.acc_ds = at(w.off_ds);
@@ -876,6 +886,10 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
 #ifdef UA_PROFILE_BWD2
     if (const char* tp = getenv("UA_TRACE_PTR")) qp.trace = reinterpret_cast<long long*>(strtoull(tp, nullptr, 0));
 #endif
+    if (wide) {
+      qp.row_term = at(w.off_gd);
+      if ((e = ua::sm100::launch_bwd2(ks, gate_dtype, 4, kc, vc, xq, g_out_cm, qp, st))) return e;
+    }
     if ((e = ua::sm100::launch_bwd2(ks, gate_dtype, wide ? 3 : 1, kc, vc, xq, g_out_cm, qp, st))) return e;
     if (seg) {
       ua::sm100::Bwd2Params cp = qp;      // what the rows after each segment induce in it
@@ -1051,6 +1065,27 @@ int ua_prepare_inputs_bwd(int batch, int seq, int n_heads, int n_kv_heads, int h
   return dtype == UA_F32 ? dispatch_prepare<float>(tpr, pd, c, st) : dispatch_prepare<bf16>(tpr, pd, c, st);
 }
 
+int ua_copy_heads(const UaHeadCopy* copies, int count, void* stream) {
+  if (!copies) return UA_ERR_NULL_POINTER;
+  if (count < 1 || count > 3) return UA_ERR_BAD_DIMS;
+  ua::aux::HeadCopies all{};
+  unsigned most = 0;
+  for (int i = 0; i < count; ++i) {
+    const UaHeadCopy& c = copies[i];
+    if (!c.src || !c.dst) return UA_ERR_NULL_POINTER;
+    if (c.batch <= 0 || c.heads <= 0 || c.rows <= 0 || c.a <= 0 || c.heads % c.a || c.src_bytes <= 0 || c.dst_bytes <= 0) return UA_ERR_BAD_DIMS;
+    if (c.src_bytes % 16 || c.dst_bytes % 16) return UA_ERR_UNSUPPORTED;
+    if (!aligned16(c.src) || !aligned16(c.dst)) return UA_ERR_ALIGNMENT;
+    const long long pieces = (long long)c.batch * c.heads * c.rows * (c.dst_bytes / 16);
+    if (pieces > 0x7fffffff) return UA_ERR_UNSUPPORTED;
+    all.t[i] = {static_cast<const uint4*>(c.src), static_cast<uint4*>(c.dst), (unsigned)pieces, c.heads, c.rows, c.a, c.heads / c.a, c.src_bytes / 16, c.dst_bytes / 16};
+    most = std::max(most, (unsigned)pieces);
+  }
+  const dim3 grid((most + ua::aux::kMergeThreads - 1) / ua::aux::kMergeThreads, (unsigned)count);
+  ua::aux::copy_heads_kernel<<<grid, ua::aux::kMergeThreads, 0, static_cast<cudaStream_t>(stream)>>>(all);
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+
 int ua_decode_step(const UaDims* dims, int dtype, int gate_dtype, int t, const void* k_cache, const void* v_cache,
                    const void* src_cache, const void* q_t, const void* dest_t, float* decay_state, void* out_t, float* lse_t,
                    void* stream) {
@@ -1181,7 +1216,7 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
   ua::Shape s = to_shape(dims);
   if (!ua::sm100::bwd2_supported(s, dtype) || !ua::sm100::chunk128(s)) return UA_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  BwdWorkspaceTc w = bwd_layout_tc(s, 1, 0);
+  BwdWorkspaceTc w = bwd_layout_tc(s, 1);
   if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 255u)) return UA_ERR_WORKSPACE;
   char* ws = static_cast<char*>(workspace);
   const int seg = ua::sm100::bwd_split(s);

@@ -364,6 +364,28 @@ __global__ void __launch_bounds__(kMergeThreads) row_dot_kernel(const T* __restr
   if (live && sub == 0) out[row] = acc;
 }
 
+// ---- rows between layouts of heads ----------------------------------------------------------
+// Copies (batch, heads, rows) of one width into the rows of another, with the heads in another order: destination head hd takes source
+// head (hd % a) * b + hd / a; columns that the source does not have are zero, columns that the destination does not have are
+// dropped.  One thread per 16-byte piece of the destination, up to three tensors per launch.
+struct HeadCopy {
+  const uint4* src;
+  uint4* dst;
+  unsigned pieces;          // of the destination
+  int heads, rows, a, b, src_width, dst_width;      // widths in 16-byte pieces
+};
+struct HeadCopies {
+  HeadCopy t[3];
+};
+__global__ void __launch_bounds__(kMergeThreads) copy_heads_kernel(HeadCopies all) {
+  const HeadCopy& t = all.t[blockIdx.y];
+  const unsigned e = blockIdx.x * kMergeThreads + threadIdx.x;
+  if (e >= t.pieces) return;
+  const unsigned row = e / t.dst_width, c = e - row * t.dst_width, bh = row / t.rows, bb = bh / t.heads, hd = bh - bb * t.heads;
+  const size_t from = ((size_t)bb * t.heads + (hd % t.a) * t.b + hd / t.a) * t.rows + (row - bh * t.rows);
+  t.dst[e] = (int)c < t.src_width ? __ldg(t.src + from * t.src_width + c) : make_uint4(0, 0, 0, 0);
+}
+
 // ---- input prologue -----------------------------------------------------------------
 // The model hands over projections in token-major order: query_state (b,s,n,d), key_state / value_state (b,s,n_kv,d)
 // and gate logits (b,s,2,n_kv).  The operator wants head-major tensors: xq (b,n_kv,rep,s,d) (query head kv*rep + r),

@@ -44,6 +44,7 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
     if constexpr (kC == 128) {
       if (mode == 2) kern = bwd2_kernel<D, kC, TG, 2, kCols, true>;
       if (mode == 3) kern = bwd2_kernel<D, kC, TG, 3, kCols, true>;
+      if (mode == 4) kern = bwd2_kernel<D, kC, TG, 4, kCols, true>;
     }
     // the forward's output tiles at hand (per-chunk form, head_dim 64): the row term comes from them
     if constexpr (Cfg::kOutTiles) {
@@ -60,7 +61,7 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
     for (int i = 0; i < s.N; ++i) per += ((s.L - i * kC) / 64 + p.seg - 1) / p.seg;
   }
   kern<<<(unsigned)BH * per, threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
-  if (p.acc_dt) {
+  if (p.acc_dt && mode != 4) {
     // row ranges: the row-side dK joins the accumulator; d static_dest of the range's rows comes out of it
     const int row_begin = p.j_begin * 128, row_end = p.j_end * 128;
     const long long warps = (long long)BH * (row_end - row_begin);
@@ -100,20 +101,6 @@ int launch_bwd_finish(const Shape& s, int gate_dtype, const void* kc, const Bwd2
                                             : launch_finish_t<D_, __nv_bfloat16>(s, kc, p, dkc, dxq, dvc, dss, ddest, st))
   return s.D == 64 ? UA_FINISH(64) : UA_FINISH(128);
 #undef UA_FINISH
-}
-
-int launch_row_term(const Shape& s, int m, const void* out, const void* g_out, const void* g_denom, int g_denom_dtype, float* table, cudaStream_t st) {
-  const int n = s.N / m;
-  const long long rows = (long long)s.B * s.H * n * s.R * s.L;
-  const int per = 256 / (s.D / 8);
-  const unsigned blocks = (unsigned)((rows + per - 1) / per);
-  const auto* o = static_cast<const __nv_bfloat16*>(out);
-  const auto* g = static_cast<const __nv_bfloat16*>(g_out);
-#define UA_ROW_TERM(D_, TD_) row_term_kernel<D_, TD_><<<blocks, 256, 0, st>>>(o, g, static_cast<const TD_*>(g_denom), table, n, s.R, s.L, s.C * m, rows)
-  if (s.D == 64) { if (g_denom_dtype == UA_F32) UA_ROW_TERM(64, float); else UA_ROW_TERM(64, __nv_bfloat16); }
-  else { if (g_denom_dtype == UA_F32) UA_ROW_TERM(128, float); else UA_ROW_TERM(128, __nv_bfloat16); }
-#undef UA_ROW_TERM
-  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
 
 namespace {

@@ -36,8 +36,10 @@
 // with a zero reverse carry; every gradient is linear in that carry, so the correction pass (the same kernel without heads)
 // adds what the rows after a segment induce, from the totals that the segments leave (see bwd_split for when).
 // Wide chunks (p.m > 1): a chunk of m * 128 keys is m blocks of 128.  Only the row tables and the upstream gradient are the
-// chunk's: with the chunk's log-sum-exp P = exp(s - lse) needs nothing from the other blocks, and the row term arrives
-// in the table (mode 3).
+// chunk's: with the chunk's log-sum-exp P = exp(s - lse) needs nothing from the other blocks.  The row term is a sum over the keys
+// of all m blocks: a pass of its own (mode 4: scores, dP and nothing else) adds it into the table, which the sweep then
+// reads (mode 3).  (Taken from the bf16 output rows instead, as out . dO, it would cost less, but the rounding of the outputs
+// runs through the cumulative sum: 7e-3 instead of 3e-3 in dQ, per cents in dK when a merge follows.)
 //
 // Every mbarrier wait is bounded; on a timeout the block raises a shared abort flag, every role
 // leaves, TMEM is freed and status[0] is set (status[1]: where the first block gave up).
@@ -53,7 +55,8 @@ struct Bwd2Params {
   Shape s;
   const void* ssrc;
   const void* sdest;
-  const float* g_denom;      // (b,h,n,r,L) fp32; in mode 3 the final row term g_denom - out . dO   [modes 1, 3]
+  const float* g_denom;      // (b,h,n,r,L) fp32; in mode 3 the final row term g_denom - sum_k P dP   [modes 1, 3]
+  float* row_term;           // (b,h,n,r,L) fp32, holds g_denom: sum_k P dP is subtracted here          [mode 4]
   const float* lse;          // (b,h,n,r,L) fp32: the forward's log-sum-exp   [modes 1, 3]
   const float* row_lse;      // (b,h,r,L) fp32: log-sum-exp over all keys     [mode 2]
   const float* row_delta;    // (b,h,r,L) fp32: g . merged                    [mode 2]
@@ -279,7 +282,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
       const int grow = (kMode == 2) ? qrow : (int)((out_chunk * R + r) * p.Lr + srow0);
       const uint32_t dst = sb + Cfg::oSlot + sl * Cfg::kSlot, tab = sb + Cfg::oHeadTab + sl * 512;
       const bool gd16 = kOutDelta && p.g_denom16 != nullptr;
-      mbar_expect_tx(c.bar(qInFull + sl), (kOutDelta ? 3 : 2) * Cfg::kHalf + (gd16 ? 384 : 512));
+      mbar_expect_tx(c.bar(qInFull + sl), (kOutDelta ? 3 : 2) * Cfg::kHalf + (kMode == 4 ? 256 : gd16 ? 384 : 512));
       if (kOutDelta) tma_load_2d(sb + Cfg::oOut + sl * Cfg::kHalf, tmO, 0, grow, c.bar(qInFull + sl));
 #pragma unroll
       for (int b = 0; b < Cfg::kBoxes; ++b) {
@@ -291,6 +294,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
         bulk_load_1d(tab + 256, p.row_delta + qrow, 256, c.bar(qInFull + sl));
       } else {
         bulk_load_1d(tab, p.lse + grow, 256, c.bar(qInFull + sl));
+        if (kMode == 4) continue;
         if (gd16) bulk_load_1d(sb + Cfg::oGd16 + sl * 128, p.g_denom16 + grow, 128, c.bar(qInFull + sl));
         else bulk_load_1d(tab + 256, p.g_denom + grow, 256, c.bar(qInFull + sl));
       }
@@ -300,7 +304,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
 
 // ----------------------------------------------------------- front MMA issuer --
 // G, S^T and dP^T: everything that only needs loaded tiles and a free (S, dP) buffer.
-template <int D>
+template <int D, int kMode>
 __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p) {
   using Cfg = Bwd2Cfg<D>;
   const int R = p.heads;
@@ -320,7 +324,7 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
   auto acquire = [&](int b) -> bool {
     const int uses = u / Cfg::kNB;                                // units before u that used buffer b = u % kNB
     if (uses == 0) return true;
-    if (!Cfg::kPtSeparate && last_was_head[b]) return c.wait(qPtFree + b, head_uses[b] - 1);
+    if (kMode != 4 && !Cfg::kPtSeparate && last_was_head[b]) return c.wait(qPtFree + b, head_uses[b] - 1);
     return c.wait(qLdDone + b, uses - 1);
   };
   auto unit_g = [&](int ht) -> bool {
@@ -341,6 +345,7 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
   for (int ht = 0; ht < c.nht; ++ht) {
     if (!c.wait(qKjFull + ht % Cfg::kKj, ht / Cfg::kKj)) return;
     if (R > 0 && !unit_g(ht)) return;                               // G for the decay recomputation (none without heads)
+    if (kMode == 4) tc_commit(c.bar(qKjFree + ht % Cfg::kKj));      // (no back issuers: the tiles are free once these products are done)
     UQ(0)
     for (int r = 0; r < R; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, b = u % Cfg::kNB;
@@ -360,7 +365,7 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
       ++u;
       UQ(3)
     }
-    if (!unit_g(ht)) return;                                        // G again for the decay gradient
+    if (kMode != 4 && !unit_g(ht)) return;                          // G again for the decay gradient
     UQ(0)
   }
   UQ_STORE_AT(16)
@@ -793,7 +798,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       c.arrive_w(qDsReady + db);
       return true;
     };
-    for (int r = 0; r < R; ++r, ++hc) {
+    for (int r = 0; r < R; ++r, hc += (kMode == 4 ? 0 : 1)) {
       const int b = u % Cfg::kNB, sl = hc % Cfg::kNS;
       float* tabL = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512);      // lse[64] of the head's rows (raw)
       float* tabC = tabL + 64;                                                         // g_denom[64] (or delta[64])
@@ -814,6 +819,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         tc_wait_ld();
         tc_fence_before();
         c.arrive_w(qLdDone + b);
+        // (mode 4: the products that read the slot are done, and this was the last look at its table)
+        if (kMode == 4) c.arrive_w(qInFree + sl);
         ++u;
         UQ(15)
 #pragma unroll
@@ -824,7 +831,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           dp[x] = make_float2(__uint_as_float(dr[2 * x]), __uint_as_float(dr[2 * x + 1]));
         }
       }
-      if (kColSums) {
+      if (kColSums || kMode == 4) {
         float e[CG];
 #pragma unroll
         for (int x = 0; x < H2; ++x) {
@@ -837,6 +844,12 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
 #else
         const float part = warp_colsum<CG>(e, scr, lane);            // this warp's 32 keys, column col0 + lane % CG
 #endif
+        if (kMode == 4) {
+          const size_t out_chunk = (size_t)c.bh * (N / p.m) + c.i / p.m;
+          if (helper) atomicAdd(p.row_term + (out_chunk * p.s.R + r) * p.Lr + c.srow0_of(ht) + col0 + lane, -part);
+          ++hc;
+          continue;
+        }
         if (helper) atomicAdd(tabC + col0 + lane, -part);           // g_denom - sum_k P dP, in place
       }
       UQ(2)
@@ -866,6 +879,16 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     if (!kDeferTail && !flush_tail()) return;
 
     // ================= decay gradient =================
+    if (kMode == 4) {
+      // (every worker has read this half tile's rows and its tables; static_dest of the next one)
+      if (ht + 1 < c.nht && quad == kGateQuad) {
+        if (!c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
+        if (helper) sT3[((ht + 1) & 1) * 64 + col0 + lane] = t3_from_table(ht + 1);
+      }
+      c.arrive_w(qDgReady);
+      named_bar_sync(kBarAll, kWorkers);
+      continue;
+    }
     {
       if (kDeferTail && !flush_tail()) return;     // the last head's tail
       const bool more = ht + 1 < c.nht;
@@ -960,6 +983,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   }
   UQ_STORE
 
+  if (kMode == 4) return;
   // ---- end of the sweep: dV_i, dK_i, d static_src (thread = key, D / NG columns each) ----
   if (!c.wait_w(qFinal, 0)) return;
   tc_fence_after();
@@ -1078,6 +1102,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     for (int b = 0; b < qNumBars; ++b) {
       uint32_t count = 1;
       if (b == qLdDone || b == qLdDone + 1 || b == qDsReady || b == qDsReady + 1 || b == qDgReady) count = kC / 32 * NG;   // one arrival per worker warp
+      if (kMode == 4 && b >= qInFree && b < qInFree + 4) count = kC / 32 * NG;
       if (b == qYFree || (b >= qDelta && b < qDelta + 4)) count = 2;                                                                                  // the two draining warps
       if (b == qDsFree || b == qDsFree + 1 || b == qDgFree || b == qFinal) count = 2;                               // both back issuers
       mbar_init(c.bar(b), count);
@@ -1113,14 +1138,16 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
     if (lane == 0) {
-      if (warp == 0) bwd2_front<D>(c, p);
+      if (warp == 0) bwd2_front<D, kMode>(c, p);
+      else if (kMode == 4 && warp != 2) {}      // (the row-term pass has nothing for the back issuers and the drain warps)
       else if (warp == 1) bwd2_back<D, kC, CG>(c, p, 0);
       else if (warp == 2) bwd2_producer<D, kC, TG, kMode, kOutDelta>(c, p, &tmK, &tmV, &tmQ, &tmG, &tmO);
       else bwd2_back<D, kC, CG>(c, p, 1);
     }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
-    if (warp < 6) bwd2_drain<D>(c, p, &tmDQ, &tmDK);
+    if (kMode == 4) {}
+    else if (warp < 6) bwd2_drain<D>(c, p, &tmDQ, &tmDK);
     else if (kOutDelta) bwd2_rowdots<D>(c, p);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
@@ -1224,28 +1251,6 @@ bwd_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restrict__ s
     Num<TG>::st(dt + row, dot != 0.f ? 0.5f * dot / Num<TG>::ld(sdest + row) : 0.f);
     if (acc_ds) Num<TG>::st(ds + row, acc_ds[row]);
   }
-}
-
-// The row term of the softmax gradient as a table, for chunks whose keys are spread over several blocks (mode 3):
-//   table[chunk][head][row] = g_denom - out . dO      for the rows that see the chunk, g_denom for those before it.
-// Reads the output and its gradient once where they matter; 16 bytes of a row per thread.
-template <int D, typename TD>
-__global__ void __launch_bounds__(256)
-row_term_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ g_out, const TD* __restrict__ g_denom,
-                float* __restrict__ table, int N, int R, int L, int chunk, long long rows) {
-  constexpr int kLanes = D / 8, kRows = 256 / kLanes;
-  const long long first = (long long)blockIdx.x * kRows + threadIdx.x / kLanes, at = first < rows ? first : rows - 1;
-  const int sub = threadIdx.x % kLanes;
-  const int row = (int)(at % L), i = (int)(at / ((long long)L * R) % N);
-  float dot = 0.f;
-  if (row >= i * chunk) {
-    float hi = 0.f;
-    dot_bf16x8(__ldcs(reinterpret_cast<const uint4*>(out + at * D + sub * 8)), *reinterpret_cast<const uint4*>(g_out + at * D + sub * 8), dot, hi);
-    dot += hi;
-  }
-#pragma unroll
-  for (int o = kLanes / 2; o >= 1; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-  if (first < rows && sub == 0) table[at] = Num<TD>::ld(g_denom + at) - dot;
 }
 
 }  // namespace sm100

@@ -145,14 +145,12 @@ inline void whole_sequence(MaskedParams& p) {
 
 // Backward over the row tiles [p.j_begin, p.j_end) (ua_bwd.cu; the caller sets the range fields, e.g. with whole_sequence()).
 // With p.heads == 0 (correction pass) xq, g_out and p.acc_dq are not touched and may be null.  mode: 1 per-chunk outputs, 2 merged,
-// 3 per-chunk outputs with the row term in the table.  Where p.acc_dt is set the row-side dK and d static_dest are finished too.
+// 3 per-chunk outputs with the row term in the table, 4 that table's pass.  Where p.acc_dt is set the row-side dK and d static_dest are finished too.
 int launch_bwd2(const Shape& s, int gate_dtype, int mode, const void* kc, const void* vc, const void* xq, const void* g_out,
                 const Bwd2Params& p, cudaStream_t st);
 // Everything that a whole-sequence backward leaves to do after its sweep (see bwd_finish_kernel).
 int launch_bwd_finish(const Shape& s, int gate_dtype, const void* kc, const Bwd2Params& p, void* dkc, void* dxq, void* dvc, void* dss,
                       void* ddest, cudaStream_t st);
-// table = g_denom - out . dO (see row_term_kernel) for chunks of m * 128 keys
-int launch_row_term(const Shape& s, int m, const void* out, const void* g_out, const void* g_denom, int g_denom_dtype, float* table, cudaStream_t st);
 // Rows before a chunk over the row tiles [p.j_begin, p.j_end): prep (per-chunk constants), sweep (one pass over the upstream
 // gradient), finish (dK_i, and dV_i for a row range).  The caller has zeroed (or shares) acc_dq / acc_dk / acc_dv.
 int launch_masked(const Shape& s, const void* kc, const void* vc, const void* xq, const void* g_out, float* acc_dq,

@@ -96,8 +96,8 @@ Inputs inputs(const Problem& p, const Tensor& kc, const Tensor& vc, const Tensor
 }
 
 // (out_cm, lse_cm, denom_cm, carry or None)
-std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_cm(const Tensor& kc_, const Tensor& vc_, const Tensor& xq_, const Tensor& ss_,
-                                                         const Tensor& sd_, int flags, bool keep_carry) {
+std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_with(const Tensor& kc_, const Tensor& vc_, const Tensor& xq_, const Tensor& ss_,
+                                                           const Tensor& sd_, int flags, bool keep_carry, bool want_denom) {
   require_cuda(kc_, vc_, xq_, ss_, sd_);
   const Tensor kc = plain(kc_), xq = plain(xq_);
   const Problem p = problem(kc, xq);
@@ -106,7 +106,7 @@ std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_cm(const Tensor& kc_, cons
   const auto opt = kc.options().requires_grad(false);
   Tensor out = at::empty({p.b, p.h, p.n, p.r, p.L, p.d}, opt.dtype(p.dt));
   Tensor lse = at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(at::kFloat));
-  Tensor denom = p.code == UA_F32 ? lse : at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(p.dt));
+  Tensor denom = p.code == UA_F32 || !want_denom ? lse : at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(p.dt));
   const size_t ws_bytes = std::max<size_t>(ua_fwd_workspace_bytes(&p.dims, p.code, flags), 256);
   Tensor ws = at::empty({(int64_t)ws_bytes}, opt.dtype(at::kByte));
   OptTensor carry;
@@ -115,10 +115,15 @@ std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_cm(const Tensor& kc_, cons
   }
   void* st = stream_of(kc);
   check(ua_fwd_keep(&p.dims, p.code, code_of(in.g.src.scalar_type()), ptr(in.kc), ptr(in.vc), ptr(in.q), ptr(in.g.src), ptr(in.g.dest),
-                    ptr(out), static_cast<float*>(ptr(lse)), p.code == UA_F32 ? nullptr : ptr(denom), carry ? ptr(*carry) : nullptr,
+                    ptr(out), static_cast<float*>(ptr(lse)), denom.is_same(lse) ? nullptr : ptr(denom), carry ? ptr(*carry) : nullptr,
                     ptr(ws), ws_bytes, flags, st), "ua_fwd");
   check_status(ws, st, "ua_fwd");
   return {out, lse, denom, carry};
+}
+
+std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_cm(const Tensor& kc, const Tensor& vc, const Tensor& xq, const Tensor& ss, const Tensor& sd,
+                                                         int flags, bool keep_carry) {
+  return forward_with(kc, vc, xq, ss, sd, flags, keep_carry, true);
 }
 
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> backward_cm(const Tensor& kc_, const Tensor& vc_, const Tensor& xq_, const Tensor& ss_,
@@ -444,6 +449,172 @@ Tensor merge_apply(const Tensor& mat, const Tensor& vec) {
   return merged;
 }
 
+// The composition of the operator and the merge, for callers of the merged output alone (UniversalAttentionMerged in its default
+// modes): merge weights from the fp32 log-sum-exp, backward through the merge's and the operator's.
+struct Composed {
+  SavedVariable kc, vc, xq, ss, sd, out, lse, carry;
+  bool has_carry = false;
+  void save(const Tensor& kc_, const Tensor& vc_, const Tensor& xq_, const Tensor& ss_, const Tensor& sd_, const Tensor& out_, const Tensor& lse_,
+            const OptTensor& carry_) {
+    kc = SavedVariable(kc_, false); vc = SavedVariable(vc_, false); xq = SavedVariable(xq_, false);
+    ss = SavedVariable(ss_, false); sd = SavedVariable(sd_, false); out = SavedVariable(out_, false); lse = SavedVariable(lse_, false);
+    if ((has_carry = carry_.has_value())) carry = SavedVariable(*carry_, false);
+  }
+  void release() {
+    for (SavedVariable* v : {&kc, &vc, &xq, &ss, &sd, &out, &lse, &carry}) v->reset_data();
+  }
+  // g: gradient of the merged output, (b,h,r,L,d) in any view of these elements
+  std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> backward(const Tensor& g) {
+    const Tensor o = out.unpack(), l = lse.unpack();
+    auto [g_out, g_lse] = merge_bwd_cm(o, l, g, true);
+    OptTensor c;
+    if (has_carry) c = carry.unpack();
+    // (without the output tiles: the row term from the bf16 outputs moves dK by per cents here, sums over the keys do not)
+    return backward_cm(kc.unpack(), vc.unpack(), xq.unpack(), ss.unpack(), sd.unpack(), g_out, g_lse, UA_FLAG_SKIP_MASKED_GRADS, c, l, {});
+  }
+};
+struct MergedNode : torch::autograd::Node {
+  Composed c;
+  std::string name() const override { return "UniversalAttentionMergedBackward"; }
+  void release_variables() override { c.release(); }
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return variable_list(5);
+    return with_python([&] {
+      const at::AutoDispatchBelowADInplaceOrView below;
+      auto [a, b, d, e, f] = c.backward(g[0]);
+      return variable_list{a, b, d, e, f};
+    });
+  }
+};
+Tensor merged_apply(const Tensor& kc, const Tensor& vc, const Tensor& xq, const Tensor& ss, const Tensor& sd) {
+  const bool grad = wants_grad(kc, vc, xq, ss, sd);
+  Tensor out, lse, merged;
+  OptTensor carry;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    Tensor denom;
+    std::tie(out, lse, denom, carry) = forward_with(kc, vc, xq, ss, sd, 0, grad, false);
+    merged = std::get<0>(merge_fwd_cm(out, lse, false)).view(xq.sizes());
+  }
+  if (grad) {
+    auto n = make_node<MergedNode>(kc, vc, xq, ss, sd);
+    n->c.save(kc, vc, xq, ss, sd, out, lse, carry);
+    torch::autograd::set_history(merged, n);
+  }
+  return merged;
+}
+
+// ---- attention(q, k, v, ...) -------------------------------------------------------------------------------------------
+// The flash-style call on the composition above: queries from (b, heads, s, d), head r * kv + g reading kv head g, to (b, kv, r, s, D) and
+// back, rows zero-padded to a head_dim D of the kernels on the way.  One copy launch per side and direction.
+struct HeadMap {
+  Tensor src, dst;
+  int64_t heads, a;      // see ua_copy_heads
+};
+void copy_heads(std::initializer_list<HeadMap> maps) {
+  UaHeadCopy c[3];
+  int n = 0;
+  for (const HeadMap& m : maps) {
+    if (!m.src.defined()) continue;
+    const int64_t es = m.src.element_size(), rows = m.src.size(-2), total = m.src.numel() / m.src.size(-1);
+    c[n++] = UaHeadCopy{ptr(m.src), ptr(m.dst), (int32_t)(total / (m.heads * rows)), (int32_t)m.heads, (int32_t)rows, (int32_t)m.a,
+                        (int32_t)(m.src.size(-1) * es), (int32_t)(m.dst.size(-1) * es)};
+  }
+  if (n) check(ua_copy_heads(c, n, stream_of(maps.begin()->dst)), "ua_copy_heads");
+}
+struct AttentionNode : torch::autograd::Node {
+  Composed c;
+  int64_t heads = 0, kv = 0, d = 0;
+  at::DimVector gate_sizes;
+  SavedVariable in[5];      // the inputs as they were given: some of what `c` holds shares their memory, and these notice an in-place change
+  std::string name() const override { return "AttentionBackward"; }
+  void release_variables() override {
+    c.release();
+    for (SavedVariable& v : in) v.reset_data();
+  }
+  variable_list apply(variable_list&& g_) override {
+    if (!g_[0].defined()) return variable_list(5);
+    return with_python([&] {
+      const at::AutoDispatchBelowADInplaceOrView below;
+      for (const SavedVariable& v : in) v.unpack();
+      const Tensor xq = c.xq.unpack();
+      const int64_t b = xq.size(0), s = xq.size(3), D = xq.size(4), rep = heads / kv;
+      const c10::cuda::CUDAGuard guard(xq.device());
+      const auto opt = xq.options().requires_grad(false);
+      Tensor g = g_[0].to(xq.scalar_type()).contiguous();
+      if (rep > 1 || D != d) {
+        Tensor packed = at::empty({b, kv, rep, s, D}, opt);
+        copy_heads({{g, packed, heads, rep}});
+        g = packed;
+      }
+      auto [dk, dv, dq, ds, dt] = c.backward(g);
+      if (rep > 1 || D != d) {
+        Tensor q = at::empty({b, heads, s, d}, opt);
+        HeadMap mk{}, mv{};
+        if (D != d) {
+          mk = HeadMap{dk.view({b, kv, s, D}), at::empty({b, kv, s, d}, opt), kv, kv};
+          mv = HeadMap{dv.view({b, kv, s, D}), at::empty({b, kv, s, d}, opt), kv, kv};
+        }
+        copy_heads({{dq, q, heads, kv}, mk, mv});
+        dq = q;
+        if (D != d) { dk = mk.dst; dv = mv.dst; }
+      }
+      return variable_list{dq.view({b, heads, s, d}), dk.view({b, kv, s, d}), dv.view({b, kv, s, d}), ds.view(gate_sizes), dt.view(gate_sizes)};
+    });
+  }
+};
+// D: the kernels' head_dim (>= d), chunk: keys per chunk
+Tensor attention_apply(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& src, const Tensor& dest, int64_t D, int64_t chunk) {
+  require_cuda(q, k, v, src, dest);
+  const bool grad = wants_grad(q, k, v, src, dest);
+  const int64_t b = q.size(0), heads = q.size(1), s = q.size(2), d = q.size(3), kv = k.size(1), rep = heads / kv, n = s / chunk;
+  TORCH_CHECK(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(), "queries, keys and values share one dtype");
+  Tensor kc, vc, xq, ss, sd, out, lse, o;
+  OptTensor carry;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(q.device());
+    const auto opt = q.options().requires_grad(false);
+    Tensor qs = q.contiguous(), ks = k.contiguous(), vs = v.contiguous();
+    if (rep > 1 || D != d) {
+      Tensor packed = at::empty({b, kv, rep, s, D}, opt);
+      HeadMap mk{}, mv{};
+      if (D != d) {
+        mk = HeadMap{ks, at::empty({b, kv, s, D}, opt), kv, kv};
+        mv = HeadMap{vs, at::empty({b, kv, s, D}, opt), kv, kv};
+      }
+      copy_heads({{qs, packed, heads, rep}, mk, mv});
+      qs = packed;
+      if (D != d) { ks = mk.dst; vs = mv.dst; }
+    }
+    xq = qs.view({b, kv, rep, s, D});
+    kc = ks.view({b, kv, n, chunk, D});
+    vc = vs.view({b, kv, n, chunk, D});
+    ss = src.reshape({b, kv, n, chunk});
+    sd = dest.reshape({b, kv, s});
+    Tensor denom;
+    std::tie(out, lse, denom, carry) = forward_with(kc, vc, xq, ss, sd, 0, grad, false);
+    o = std::get<0>(merge_fwd_cm(out, lse, false));
+    if (rep > 1 || D != d) {
+      Tensor unpacked = at::empty({b, heads, s, d}, opt);
+      copy_heads({{o, unpacked, heads, kv}});
+      o = unpacked;
+    } else {
+      o = o.view({b, heads, s, d});
+    }
+  }
+  if (grad) {
+    auto node = make_node<AttentionNode>(q, k, v, src, dest);
+    const Tensor* in[5] = {&q, &k, &v, &src, &dest};
+    for (int i = 0; i < 5; ++i) node->in[i] = SavedVariable(*in[i], false);
+    node->c.save(kc, vc, xq, ss, sd, out, lse, carry);
+    node->heads = heads; node->kv = kv; node->d = d;
+    node->gate_sizes = src.sizes();
+    torch::autograd::set_history(o, node);
+  }
+  return o;
+}
+
 struct PrepareNode : torch::autograd::Node {
   SavedVariable kc, src, dest, norm;
   bool has_norm = false;
@@ -507,6 +678,8 @@ PYBIND11_MODULE(_ua_torch, m) {
   m.def("set_strict_masked_grads", [](bool on) { g_strict_masked_grads = on; });
   m.def("ua_apply", &ua_apply);
   m.def("merge_apply", &merge_apply);
+  m.def("merged_apply", outside_functorch(&merged_apply));
+  m.def("attention_apply", outside_functorch(&attention_apply));
   m.def("prepare_apply", &prepare_apply);
   m.def("forward_cm", outside_functorch(&forward_cm));
   m.def("backward_cm", outside_functorch(&backward_cm));

@@ -140,6 +140,10 @@ def _masked_zero(t) -> bool:
     return v is not None and v == t._version
 
 
+def _default_merge_modes() -> bool:
+    return _MERGED_BACKWARD == "composed" and _MERGED_FORWARD == "materialise"
+
+
 _transforms_active = torch._C._are_functorch_transforms_active
 
 
@@ -285,11 +289,22 @@ class UniversalAttentionMerged(Function):
     the 2-D form."""
 
     @staticmethod
-    def forward(kc, vc, xq, static_src, static_dest):
+    def _check(kc, vc, xq, static_src, static_dest):
         b, h, n, c, d = kc.shape
         assert vc.shape == kc.shape and static_src.shape == (b, h, n, c)
-        assert xq.shape[:2] == (b, h) and xq.shape[-1] == d and xq[0, 0, 0].numel() == n * c * d
+        assert xq.shape[:2] == (b, h) and xq.shape[-1] == d and xq.numel() == b * h * xq.shape[2] * n * c * d
         assert static_dest.numel() == b * h * n * c
+
+    @classmethod
+    def apply(cls, kc, vc, xq, static_src, static_dest):
+        if _transforms_active() or not _default_merge_modes():
+            return super().apply(kc, vc, xq, static_src, static_dest)
+        cls._check(kc, vc, xq, static_src, static_dest)
+        return _lib.native().merged_apply(kc, vc, xq, static_src, static_dest)
+
+    @staticmethod
+    def forward(kc, vc, xq, static_src, static_dest):
+        UniversalAttentionMerged._check(kc, vc, xq, static_src, static_dest)
         if _MERGED_FORWARD == "low_memory" and ops.merged_backward_supported(kc, xq):
             res = ops.forward_merged_lowmem(kc, vc, xq, static_src, static_dest)
             if res is not None:
