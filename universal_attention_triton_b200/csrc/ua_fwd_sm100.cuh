@@ -127,23 +127,26 @@ struct FwdCfg {
   static constexpr int kTileBytes = 128 * D * 2;   // one [128][D] bf16 tile
   static constexpr int kBoxBytes = 128 * 128;      // one TMA box: 128 rows x 64 elements
   static constexpr int kBoxes = D / 64;
-  static constexpr int kKjStages = (D == 64) ? 2 : 1;
-  static constexpr int kQStages = 2;
+  static constexpr bool kOneSlot = (D == 128);      // K_j and Q tiles share one slot
+  static constexpr int kKjStages = kOneSlot ? 0 : 2;
+  static constexpr int kQStages = kOneSlot ? 1 : 2;
   static constexpr int kOBufs = (D == 64) ? 2 : 1;
   static constexpr int oKi = 0;
   static constexpr int oVi = oKi + kTileBytes;
   static constexpr int oKj = oVi + kTileBytes;
   static constexpr int oQ = oKj + kKjStages * kTileBytes;
-  // The decay prefix crosses from keys-on-lanes to rows-on-lanes through a 64 KB fp32 tile C^T[row][key].  With two
-  // of them (head_dim 64: they fit) the decay group computes tile T+1 while the softmax groups consume tile T;
-  // with one, the two alternate (measured at head_dim 64: 18.7k cycles per tile = decay 9.8k + softmax 14k, minus overlap).
-  static constexpr int kCBufs = (D == 64) ? 2 : 1;
+  // The decay prefix crosses from keys-on-lanes to rows-on-lanes through 64 KB fp32 tiles C^T[row][key]; with two of them the decay
+  // group is a tile ahead of the softmax groups.  At head_dim 128 that leaves shared memory for ONE 32 KB slot, which K_j and Q
+  // tiles pass through in the order of their products (each is read for 0.3 us, and the next one is needed 2 us later); with two
+  // slots for Q, one for K_j and a single C^T tile the groups took turns: B1 H8 R4 L8192 D128 1523 -> @@PL us.
+  static constexpr int kCBufs = 2;
   static constexpr int oCs = oQ + kQStages * kTileBytes;
   static constexpr int oT3 = oCs + kCBufs * 65536;
   static constexpr int oBar = oT3 + 1024;
   static constexpr int oMisc = oBar + 256;
   static constexpr int oFill = oMisc + 64;                // bf16[D]: value of a fully masked output row
   static constexpr int kSmemBytes = oFill + 256 + 1024;  // + slack to align the base to 1024 B
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
   static constexpr uint32_t tG = 0, tS0 = 128, tS1 = 256, tO0 = 384, tO1 = 384 + D;
 };
 
@@ -182,8 +185,17 @@ __device__ __forceinline__ void fwd_producer(const FwdCtx<D>& c, const FwdParams
     tma_load_2d(sbase + Cfg::oKi + b * Cfg::kBoxBytes, tmK, b * 64, krow, c.bar(kKvFull));
     if (!kCarryOnly) tma_load_2d(sbase + Cfg::oVi + b * Cfg::kBoxBytes, tmV, b * 64, krow, c.bar(kKvFull));
   }
+  int use = 0;                          // of the one slot (head_dim 128)
+  auto load_slot = [&](const CUtensorMap* tm, int y) -> bool {
+    if (use >= 1 && !c.wait(kQEmpty, use - 1)) return false;
+    mbar_expect_tx(c.bar(kQFull), Cfg::kTileBytes);
+    for (int b = 0; b < Cfg::kBoxes; ++b) tma_load_2d(sbase + Cfg::oQ + b * Cfg::kBoxBytes, tm, b * 64, y, c.bar(kQFull));
+    ++use;
+    return true;
+  };
   auto load_kj = [&](int T) -> bool {
-    const int ks = T % Cfg::kKjStages, u = T / Cfg::kKjStages;
+    if constexpr (Cfg::kOneSlot) return load_slot(tmK, c.bh * L + c.row0 + T * 128);
+    const int ks = T & 1, u = T >> 1;
     if (u >= 1 && !c.wait(kKjEmpty + ks, u - 1)) return false;
     mbar_expect_tx(c.bar(kKjFull + ks), Cfg::kTileBytes);
     for (int b = 0; b < Cfg::kBoxes; ++b)
@@ -200,6 +212,11 @@ __device__ __forceinline__ void fwd_producer(const FwdCtx<D>& c, const FwdParams
   int t = 0;
   for (int T = 0; T < c.ntiles; ++T) {
     for (int r = 0; r < R; ++r, ++t) {
+      if constexpr (Cfg::kOneSlot) {
+        if (!load_slot(tmQ, (c.bh * R + r) * p.Lr + c.srow0 + T * 128)) return;
+        if (r == 0 && T + 1 < c.ntiles && !load_kj(T + 1)) return;
+        continue;
+      }
       const int qs = t & 1, u = t >> 1;
       if (u >= 1 && !c.wait(kQEmpty + qs, u - 1)) return;
       mbar_expect_tx(c.bar(kQFull + qs), Cfg::kTileBytes);
@@ -235,14 +252,15 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
   };
   const uint32_t kKi = desc_lo(sbase + Cfg::oKi, 16);
   const uint32_t mVi = desc_lo(sbase + Cfg::oVi, Cfg::kBoxBytes);
+  int use = 0;                          // of the one slot (head_dim 128)
   auto issue_g = [&](int T) -> bool {
-    const int ks = T % Cfg::kKjStages, u = T / Cfg::kKjStages;
-    if (!c.wait(kKjFull + ks, u)) return false;
+    const int ks = T & 1, u = T >> 1;
+    if (Cfg::kOneSlot ? !c.wait(kQFull, use++) : !c.wait(kKjFull + ks, u)) return false;
     if (T >= 1 && !c.wait(kGFree, T - 1)) return false;
     tc_fence_after();
-    issue_kmajor(c.tmem + Cfg::tG, kKi, desc_lo(sbase + Cfg::oKj + ks * Cfg::kTileBytes, 16), idesc_g);
+    issue_kmajor(c.tmem + Cfg::tG, kKi, desc_lo(sbase + (Cfg::kOneSlot ? Cfg::oQ : Cfg::oKj + ks * Cfg::kTileBytes), 16), idesc_g);
     tc_commit(c.bar(kGFull));
-    tc_commit(c.bar(kKjEmpty + ks));
+    tc_commit(c.bar(Cfg::kOneSlot ? kQEmpty : kKjEmpty + ks));
     return true;
   };
   auto issue_pv = [&](int tt) -> bool {
@@ -274,8 +292,8 @@ __device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) 
   int t = 0;
   for (int T = 0; T < c.ntiles; ++T) {
     for (int r = 0; r < R; ++r, ++t) {
-      const int qs = t & 1;
-      if (!c.wait(kQFull + qs, t >> 1)) return;
+      const int qs = Cfg::kOneSlot ? 0 : t & 1;
+      if (!c.wait(kQFull + qs, Cfg::kOneSlot ? use++ : t >> 1)) return;
       tc_fence_after();
       issue_kmajor(tS[t & 1], desc_lo(sbase + Cfg::oQ + qs * Cfg::kTileBytes, 16), kKi, idesc_s);
       tc_commit(c.bar(kSFull + (t & 1)));
