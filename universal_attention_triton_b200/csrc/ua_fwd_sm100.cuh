@@ -138,7 +138,7 @@ struct FwdCfg {
   // The decay prefix crosses from keys-on-lanes to rows-on-lanes through 64 KB fp32 tiles C^T[row][key]; with two of them the decay
   // group is a tile ahead of the softmax groups.  At head_dim 128 that leaves shared memory for ONE 32 KB slot, which K_j and Q
   // tiles pass through in the order of their products (each is read for 0.3 us, and the next one is needed 2 us later); with two
-  // slots for Q, one for K_j and a single C^T tile the groups took turns: B1 H8 R4 L8192 D128 1523 -> @@PL us.
+  // slots for Q, one for K_j and a single C^T tile the groups took turns: B1 H8 R4 L8192 D128 1523 -> 1312 us.
   static constexpr int kCBufs = 2;
   static constexpr int oCs = oQ + kQStages * kTileBytes;
   static constexpr int oT3 = oCs + kCBufs * 65536;
