@@ -425,11 +425,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
         if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
         UQ(2)
         tc_fence_after();
-        // (UA_EXP_NO_DQ_MMA / UA_EXP_NO_DRAIN / UA_EXP_NO_COLSUM: builds for timing experiments only -- each leaves one
-        // piece of the work out, with wrong results, to show what the kernel time does NOT depend on)
-#ifndef UA_EXP_NO_DQ_MMA
         mma_rows_out(desc_from_lo(desc_lo(dsb, 16384)));                                  // dQ_rj = dS^T K_i
-#endif
         ++yc;
         tc_commit(c.bar(qYFull));
         tc_commit(c.bar(qDsFree + db));
@@ -564,20 +560,14 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
           tc_fence_before();
           c.arrive_w(qYFree);
         }
-#ifndef UA_EXP_NO_DRAIN
         uint8_t* box = sStage + hb * 8192 + row * 128;
 #pragma unroll
         for (int x = 0; x < 8; ++x)
           *reinterpret_cast<uint4*>(box + ((((uint32_t)x ^ swz) & 7) << 4)) = make_uint4(o[4 * x], o[4 * x + 1], o[4 * x + 2], o[4 * x + 3]);
-#endif
       }
       fence_proxy_async();
       named_bar_sync(kBarDrain, 64);
-#ifdef UA_EXP_NO_DRAIN
-      if (false) {
-#else
       if (leader) {
-#endif
         const CUtensorMap* tm = (r < Rh) ? tmDQ : tmDK;
         const int y = (r < Rh) ? (c.bh * R + r) * p.Lr + c.srow0_of(ht) : c.bh * L + c.row0_of(ht);
 #pragma unroll
@@ -839,11 +829,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           e[2 * x] = ev.x;
           e[2 * x + 1] = ev.y;
         }
-#ifdef UA_EXP_NO_COLSUM
-        const float part = e[0] + e[1];
-#else
         const float part = warp_colsum<CG>(e, scr, lane);            // this warp's 32 keys, column col0 + lane % CG
-#endif
         if (kMode == 4) {
           const size_t out_chunk = (size_t)c.bh * (N / p.m) + c.i / p.m;
           if (helper) atomicAdd(p.row_term + (out_chunk * p.s.R + r) * p.Lr + c.srow0_of(ht) + col0 + lane, -part);

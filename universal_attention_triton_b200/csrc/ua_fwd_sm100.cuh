@@ -381,15 +381,14 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
           const float2 a = fmul2(fmul2(pw, s32), make_float2(t3r[x], t3r[x + 1]));
           const float2 om = ffma2(make_float2(fminf(a.x, clamp_hi()), fminf(a.y, clamp_hi())), mone2, one2);
           const float2 el = fmul2(make_float2(lg2(om.x), lg2(om.y)), ln2);
-#pragma unroll
-          for (int y = 0; y < 2; ++y) {
-            const int q = cb * 32 + x + y;
-            float ell = y ? el.y : el.x;
-            if (kDiag && q <= k) ell = 0.f;
-            local += ell;
-            cval = carry + (tprev + local);
-            v[x + y] = (kDiag && q < k) ? mask_value() : cval;
-          }
+          const int q = cb * 32 + x;
+          float2 run;
+          run.x = local + (kDiag && q <= k ? 0.f : el.x);
+          run.y = local = run.x + (kDiag && q + 1 <= k ? 0.f : el.y);
+          const float2 cv = fadd2(make_float2(carry, carry), fadd2(make_float2(tprev, tprev), run));
+          cval = cv.y;
+          v[x] = (kDiag && q < k) ? mask_value() : cv.x;
+          v[x + 1] = (kDiag && q + 1 < k) ? mask_value() : cv.y;
         }
       };
       if (diag) scan32(std::true_type{});
@@ -521,40 +520,82 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
       if (!c.wait_w(kOFull + sb, t >> 1)) return;
       UF(6)
       tc_fence_after();
-      __nv_bfloat16* orow_ptr = p.out + orow * D;
+      if (kMerge) {
 #pragma unroll 1
-      for (int cb = 0; cb < D / 32; ++cb) {
-        uint32_t o[32];
-        tmem_ld32(tO + cb * 32, o);
-        tc_wait_ld();
-        if (cb == D / 32 - 1) {
-          tc_fence_before();
-          c.arrive_w(kOFree + sb);
-        }
-        if (kMerge) {
+        for (int cb = 0; cb < D / 32; ++cb) {
+          uint32_t o[32];
+          tmem_ld32(tO + cb * 32, o);
+          tc_wait_ld();
+          if (cb == D / 32 - 1) {
+            tc_fence_before();
+            c.arrive_w(kOFree + sb);
+          }
           float* dst = p.merged_acc + mrow * D + cb * 32;
 #pragma unroll
           for (int u = 0; u < 8; ++u)
             red_add_v4(dst + 4 * u, __uint_as_float(o[4 * u]) * linv, __uint_as_float(o[4 * u + 1]) * linv,
                        __uint_as_float(o[4 * u + 2]) * linv, __uint_as_float(o[4 * u + 3]) * linv);
-          continue;
         }
-        if (!p.out || !in_range) continue;    // statistics-only run (the log-sum-exp for a backward that was not given one)
-#ifdef UA_EXPERIMENT_NO_OUT_STORE
-        if (cb >= 0) continue;
-#endif
-        uint32_t pk[16];
-        const float2 linv2 = make_float2(linv, linv);
+      } else if constexpr (D == 128) {
+        // head_dim 128: rows leave as whole 128-byte lines, eight rows per store instruction: O is loaded in the fragment order, in
+        // which a quad of threads holds a row, and regrouped to 32 contiguous bytes per thread.  Against the form below: B1 H16 R1 L4096
+        // 331 -> 314 us, 2 x (8 x 2) heads of L1536 87 -> 76 us, B1 H8 R4 L8192 1312 -> 1301 us (at head_dim 64, with half as
+        // much to store per score, the shuffles cost 1 % more than they give).
+        const int lane = threadIdx.x & 31;
+        __nv_bfloat16* out0 = p.out + (orow - lane) * D;      // the warp's first row
+#pragma unroll 1
+        for (int piece = 0; piece < 2 * D / 64; ++piece) {
+          const int hh = piece & 1, cb = piece >> 1;          // 16 of the warp's 32 rows, 64 of the columns
+          uint32_t o[32];
+          tmem_ld_16x64(tO + ((uint32_t)(hh * 16) << 16) + cb * 64, o);
+          const int ra = hh * 16 + (lane >> 2);
+          const float la = __shfl_sync(0xffffffffu, linv, ra), lb = __shfl_sync(0xffffffffu, linv, ra + 8);
+          tc_wait_ld();
+          if (piece == 2 * D / 64 - 1) {
+            tc_fence_before();
+            c.arrive_w(kOFree + sb);
+          }
+          if (!in_range) continue;
+          uint32_t wa[8], wb[8];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const float2 ov = fmul2(make_float2(__uint_as_float(o[2 * u]), __uint_as_float(o[2 * u + 1])), linv2);
-          __nv_bfloat162 h = __floats2bfloat162_rn(ov.x, ov.y);
-          pk[u] = *reinterpret_cast<uint32_t*>(&h);
+          for (int j = 0; j < 8; ++j) {
+            const float2 va = fmul2(make_float2(__uint_as_float(o[4 * j]), __uint_as_float(o[4 * j + 1])), make_float2(la, la));
+            const float2 vb = fmul2(make_float2(__uint_as_float(o[4 * j + 2]), __uint_as_float(o[4 * j + 3])), make_float2(lb, lb));
+            const __nv_bfloat162 ha = __floats2bfloat162_rn(va.x, va.y), hb = __floats2bfloat162_rn(vb.x, vb.y);
+            wa[j] = *reinterpret_cast<const uint32_t*>(&ha);
+            wb[j] = *reinterpret_cast<const uint32_t*>(&hb);
+          }
+          quad_gather(wa, lane);
+          quad_gather(wb, lane);
+          __nv_bfloat16* dst = out0 + (size_t)ra * D + cb * 64 + (lane & 3) * 16;
+          st_global_v8(dst, wa);
+          st_global_v8(dst + 8 * D, wb);
         }
-        // (32 bytes per thread: as 16-byte stores every one of a warp's 32 rows got half a sector at a time, and the way from L1 to L2
-        // was busy half of the time with them: B1 H8 R4 L8192 D128 1720 -> 1523 us, B4 H8 R4 L4096 D64 970 -> 935 us)
-        st_global_v8(orow_ptr + cb * 32, pk);
-        st_global_v8(orow_ptr + cb * 32 + 16, pk + 8);
+      } else {
+        // 32 bytes per thread and row: with 16-byte stores every one of a warp's 32 rows got half a sector at a time, and the way from
+        // L1 to L2 was busy half of the time with them (B4 H8 R4 L4096 970 -> 935 us)
+        __nv_bfloat16* orow_ptr = p.out + orow * D;
+#pragma unroll 1
+        for (int cb = 0; cb < D / 32; ++cb) {
+          uint32_t o[32];
+          tmem_ld32(tO + cb * 32, o);
+          tc_wait_ld();
+          if (cb == D / 32 - 1) {
+            tc_fence_before();
+            c.arrive_w(kOFree + sb);
+          }
+          if (!in_range) continue;
+          uint32_t pk[16];
+          const float2 linv2 = make_float2(linv, linv);
+#pragma unroll
+          for (int u = 0; u < 16; ++u) {
+            const float2 ov = fmul2(make_float2(__uint_as_float(o[2 * u]), __uint_as_float(o[2 * u + 1])), linv2);
+            __nv_bfloat162 h = __floats2bfloat162_rn(ov.x, ov.y);
+            pk[u] = *reinterpret_cast<uint32_t*>(&h);
+          }
+          st_global_v8(orow_ptr + cb * 32, pk);
+          st_global_v8(orow_ptr + cb * 32 + 16, pk + 8);
+        }
       }
       UF(7)
     }

@@ -215,6 +215,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
+// 16 lanes x 64 consecutive 32-bit columns in the fragment order of 16 x 8 tiles: r[4 j + {0, 1}] = columns 8 j + 2 (t % 4) + {0, 1} of
+// lane t / 4, r[4 j + {2, 3}] = the same columns of lane t / 4 + 8 (t = thread of the warp)
+__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
+        "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
+        "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -249,6 +262,28 @@ __device__ __forceinline__ void st_global_v8(void* addr, const uint32_t* r) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]),
                "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
+}
+
+// The four threads of a quad hold word j = 0..7 (two columns each) of the same row; afterwards thread q of the quad holds the row's
+// words of blocks 2 q and 2 q + 1 in column order, i.e. 32 contiguous bytes.  Eight shuffles.
+__device__ __forceinline__ void quad_gather(uint32_t (&w)[8], int lane) {
+  const bool b1 = lane & 2, b0 = lane & 1;
+  uint32_t lo[4], hi[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t keep = b1 ? w[4 + i] : w[i], got = __shfl_xor_sync(0xffffffffu, b1 ? w[i] : w[4 + i], 2);
+    lo[i] = b1 ? got : keep;
+    hi[i] = b1 ? keep : got;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t kl = b0 ? lo[2 + i] : lo[i], gl = __shfl_xor_sync(0xffffffffu, b0 ? lo[i] : lo[2 + i], 1);
+    const uint32_t kh = b0 ? hi[2 + i] : hi[i], gh = __shfl_xor_sync(0xffffffffu, b0 ? hi[i] : hi[2 + i], 1);
+    w[4 * i] = b0 ? gl : kl;
+    w[4 * i + 1] = b0 ? kl : gl;
+    w[4 * i + 2] = b0 ? gh : kh;
+    w[4 * i + 3] = b0 ? kh : gh;
+  }
 }
 
 // four floats added to global memory in one instruction (16-byte aligned address)
