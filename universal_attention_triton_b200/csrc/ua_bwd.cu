@@ -7,15 +7,15 @@ namespace ua {
 namespace sm100 {
 namespace {
 
-// Columns of a half tile per worker thread: 16 (sixteen worker warps, 96 registers each) at head_dim 64, 32 (eight worker
-// warps, ~200 registers each) at head_dim 128.  At head_dim 64 sixteen warps (four per scheduler hide the TMEM and
-// shared-memory latencies) that hand dS over at once are 5-6 % faster than eight that defer the tail of a head, in every
-// build; sixteen that defer are slower than either (measured).
+// Columns of a half tile per worker thread: 16 (sixteen worker warps, 96 registers each).  Four warps per scheduler hide the TMEM and
+// shared-memory latencies; at head_dim 64 sixteen that hand dS over at once are 5-6 % faster than eight that defer the tail of a
+// head, in every build (sixteen that defer are slower than either); at head_dim 128 they are 2 % faster with one query head and
+// level with four (measured).
 #ifndef UA_BWD2_COLS_64
 #define UA_BWD2_COLS_64 16
 #endif
 #ifndef UA_BWD2_COLS_128
-#define UA_BWD2_COLS_128 32
+#define UA_BWD2_COLS_128 16
 #endif
 template <int D> constexpr int bwd2_cols() { return D == 64 ? UA_BWD2_COLS_64 : UA_BWD2_COLS_128; }
 
@@ -131,7 +131,7 @@ int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* 
   auto prep = masked_prep_kernel<D>;
   if (cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem) != cudaSuccess) return UA_ERR_CUDA;
   prep<<<(unsigned)(BH * s.N), 256, prep_smem, st>>>(k16, v16, p);
-  auto sweep = masked_sweep_kernel<D>;
+  auto sweep = p.m > 1 ? masked_sweep_kernel<D, true> : masked_sweep_kernel<D, false>;
   if (cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
   sweep<<<(unsigned)(BH * p.items_per_bh * Cfg::kKB), 384, Cfg::kSmemBytes, st>>>(tmQ, tmG, tmDQ, p);
   masked_finish_kernel<D><<<(unsigned)(BH * s.N), 256, finish_smem, st>>>(v16, p);      // (at most 35 KB: no opt-in needed)

@@ -128,12 +128,13 @@ struct Bwd2Cfg {
   static constexpr int oOut = (oScr + 1023) / 1024 * 1024;
   static constexpr int oGd16 = oOut + kNS * kHalf;         // kNS x bf16[64]: g_denom rows of a head before they are widened
   static_assert(!kOutTiles || oGd16 + kNS * 128 <= oScr + 40960, "output tiles fit the scratch area");
-  // TMEM columns
+  // TMEM columns.  The row-side results Y are 64 columns wide and taken D / 64 times per unit: at head_dim 128 that leaves room for
+  // probabilities (bf16 pairs, 32 columns per head) in a buffer pair of their own.  Written over the S columns they kept the (S, dP)
+  // buffer until the dV product had read them, and every head waited for two rounds of products one after the other:
+  // B1 H16 R1 L4096 D128 849 -> 814 us, 2 x (8 x 2) heads of L1536 D128 250 -> 225 us.
   static constexpr uint32_t tDV = 0, tDK = D, tY = 2 * D;
   static constexpr uint32_t tS0 = (D == 64) ? 192 : 384, tP0 = tS0 + 64, tS1 = tS0 + 128, tP1 = tS0 + 192;
-  // probabilities (bf16 pairs, 32 columns per head): a buffer pair of their own where TMEM has room, else over S
-  static constexpr bool kPtSeparate = (D == 64);
-  static constexpr uint32_t tPT = 448;
+  static constexpr uint32_t tPT = (D == 64) ? 448 : 320;
   static_assert(D == 64 || D == 128, "head_dim 64 or 128");
   static_assert(D == 64 ? (tP1 + 64 <= 512) : (tP0 + 64 <= 512), "TMEM budget");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
@@ -317,14 +318,11 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
   };
   const uint32_t kKi = desc_lo(sb + Cfg::oKi, 16), kVi = desc_lo(sb + Cfg::oVi, 16);
 
-  // (S, dP) buffer b is free again when its previous unit has been consumed: once the workers have loaded it, or -- where
-  // the probabilities are written over S (head_dim 128) -- once the dV MMA of a head unit has read them.
-  int u = 0, head_uses[2] = {0, 0};
-  bool last_was_head[2] = {false, false};
+  // (S, dP) buffer b is free again once the workers have loaded its previous unit.
+  int u = 0;
   auto acquire = [&](int b) -> bool {
     const int uses = u / Cfg::kNB;                                // units before u that used buffer b = u % kNB
     if (uses == 0) return true;
-    if (kMode != 4 && !Cfg::kPtSeparate && last_was_head[b]) return c.wait(qPtFree + b, head_uses[b] - 1);
     return c.wait(qLdDone + b, uses - 1);
   };
   auto unit_g = [&](int ht) -> bool {
@@ -334,7 +332,6 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
     mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(sb + Cfg::oKj + (ht % Cfg::kKj) * Cfg::kHalf, 16));
     tc_commit(c.bar(qSFull + b));
     UQ_TRACE(u, 0)
-    last_was_head[b] = false;
     ++u;
     return true;
   };
@@ -360,8 +357,6 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
       mma_kk(c.tmem + (b ? Cfg::tP1 : Cfg::tP0), kVi, desc_lo(slot + Cfg::kHalf, 16));       // dP^T = V_i dO^T
       tc_commit(c.bar(qSFull + b));
       UQ_TRACE(u, 0)
-      last_was_head[b] = true;
-      ++head_uses[b];
       ++u;
       UQ(3)
     }
@@ -381,7 +376,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   const int R = p.heads;
   const uint32_t sb = smem_u32(c.smem);
   constexpr uint32_t id_kn = idesc_bf16(128, D, 0, 1);     // A K-major (or TMEM), B MN-major
-  constexpr uint32_t id_tn = idesc_bf16(128, D, 1, 1);     // A MN-major, B MN-major
+  constexpr uint32_t id_tn = idesc_bf16(128, 64, 1, 1);    // A MN-major, B MN-major
   const uint32_t DV = c.tmem + Cfg::tDV, DK = c.tmem + Cfg::tDK, Y = c.tmem + Cfg::tY;
   const uint64_t mKi = desc_from_lo(desc_lo(sb + Cfg::oKi, 16384));      // K_i as [K = keys][N = D] (MN-major, 64-wide groups 16 KB apart)
   const uint64_t kdG = desc_from_lo(desc_lo(sb + Cfg::oDg, 16)), mdG = desc_from_lo(desc_lo(sb + Cfg::oDg, 16384));
@@ -389,16 +384,16 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   int yc = 0, hc = 0;
   // Y[rows][D] = T^T K_i with T a [128 keys][64 rows] bf16 tile read MN-major; M = 128: lanes 64..127 come from the 16 KB
   // after the tile and are never read
-  auto mma_rows_out = [&](uint64_t t_mn) {
-    mma4_ss(Y, t_mn, mKi, 128, 128, id_tn, 0);
-    if (kC == 128) mma4_ss(Y, t_mn + 512, mKi + 512, 128, 128, id_tn, 1);
+  auto mma_rows_out = [&](uint64_t t_mn, int cb) {       // 64 columns of D: those of K_i's column group cb
+    const uint64_t k = mKi + cb * 1024;
+    mma4_ss(Y, t_mn, k, 128, 128, id_tn, 0);
+    if (kC == 128) mma4_ss(Y, t_mn + 512, k + 512, 128, 128, id_tn, 1);
   };
   if (!c.wait(qKvFull, 0)) return;
   UQ_DECL
   for (int ht = 0; ht < c.nht; ++ht) {
-    const int u0 = ht * (R + 2);
     for (int r = 0; r < R; ++r, ++hc) {
-      const int b = (u0 + 1 + r) % Cfg::kNB, sl = hc % Cfg::kNS, db = hc % Cfg::kDs;
+      const int sl = hc % Cfg::kNS, db = hc % Cfg::kDs;
       const uint32_t dsb = sb + Cfg::oDs + db * 16384;
       UQ(0)
       if (!c.wait(qDsReady + db, hc / Cfg::kDs)) return;
@@ -408,26 +403,26 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
         tc_fence_after();
         const uint32_t slot = sb + Cfg::oSlot + sl * Cfg::kSlot;
         const uint64_t mQ = desc_from_lo(desc_lo(slot, 8192)), mGo = desc_from_lo(desc_lo(slot + Cfg::kHalf, 8192));
-        // dV_i += P dO: P^T as bf16 pairs in TMEM (its own buffer, or over the S columns of each column group)
+        // dV_i += P dO: P^T as bf16 pairs in TMEM
         uint32_t pa[4];
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          pa[ks] = Cfg::kPtSeparate ? c.tmem + Cfg::tPT + 32 * (hc & 1) + 8 * ks
-                                    : c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + CG * ((16 * ks) / CG) + ((16 * ks) % CG) / 2;
+          pa[ks] = c.tmem + Cfg::tPT + 32 * (hc & 1) + 8 * ks;
         mma4_ts(DV, pa[0], pa[1], pa[2], pa[3], mGo, 128, id_kn, have_dv);
         have_dv = 1;
-        tc_commit(c.bar(qPtFree + (Cfg::kPtSeparate ? (hc & 1) : b)));
+        tc_commit(c.bar(qPtFree + (hc & 1)));
         mma4_ss(DK, desc_from_lo(desc_lo(dsb, 16)), mQ, 2, 128, id_kn, have_dk);          // dK_i += dS Q
         have_dk = 1;
         tc_commit(c.bar(qInFree + sl));
         tc_commit(c.bar(qDsFree + db));
       } else {
-        if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
-        UQ(2)
-        tc_fence_after();
-        mma_rows_out(desc_from_lo(desc_lo(dsb, 16384)));                                  // dQ_rj = dS^T K_i
-        ++yc;
-        tc_commit(c.bar(qYFull));
+        for (int cb = 0; cb < D / 64; ++cb, ++yc) {
+          if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
+          UQ(2)
+          tc_fence_after();
+          mma_rows_out(desc_from_lo(desc_lo(dsb, 16384)), cb);                            // dQ_rj = dS^T K_i
+          tc_commit(c.bar(qYFull));
+        }
         tc_commit(c.bar(qDsFree + db));
       }
     }
@@ -442,11 +437,12 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
       tc_commit(c.bar(qKjFree + ht % Cfg::kKj));
       tc_commit(c.bar(qDgFree));
     } else {
-      if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
-      tc_fence_after();
-      mma_rows_out(mdG);                                                                  // dK_j = dG^T K_i
-      ++yc;
-      tc_commit(c.bar(qYFull));
+      for (int cb = 0; cb < D / 64; ++cb, ++yc) {
+        if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
+        tc_fence_after();
+        mma_rows_out(mdG, cb);                                                            // dK_j = dG^T K_i
+        tc_commit(c.bar(qYFull));
+      }
       tc_commit(c.bar(qDgFree));
     }
   }
@@ -546,21 +542,27 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
   uint8_t* sStage = c.smem + Cfg::oStage;
   int yc = 0;
   for (int ht = 0; ht < c.nht; ++ht) {
-    for (int r = 0; r <= Rh; ++r, ++yc) {
+    for (int z = 0; z < (Rh + 1) * (D / 64); ++z, ++yc) {
+      const int r = z / (D / 64), cb = z % (D / 64);
       if (!c.wait_w(qYFull, yc)) return;
       tc_fence_after();
-      if (leader) bulk_wait_read_all();                 // the previous reduce-add has read the staging tile
+      // the reduce-add that used this staging tile last has read it (head_dim 128 has two tiles: the one before may still be reading)
+      if (leader) {
+        if (D == 64) bulk_wait_read_all();
+        else bulk_wait_read_but_last();
+      }
       named_bar_sync(kBarDrain, 64);
+      uint8_t* stage = sStage + cb * 16384;
 #pragma unroll 1
-      for (int hb = 0; hb < D / 32; ++hb) {
+      for (int hb = 0; hb < 2; ++hb) {
         uint32_t o[32];
         tmem_ld32(c.tmem + Cfg::tY + lane_base + 32 * hb, o);
         tc_wait_ld();
-        if (hb == D / 32 - 1) {
+        if (hb == 1) {
           tc_fence_before();
           c.arrive_w(qYFree);
         }
-        uint8_t* box = sStage + hb * 8192 + row * 128;
+        uint8_t* box = stage + hb * 8192 + row * 128;
 #pragma unroll
         for (int x = 0; x < 8; ++x)
           *reinterpret_cast<uint4*>(box + ((((uint32_t)x ^ swz) & 7) << 4)) = make_uint4(o[4 * x], o[4 * x + 1], o[4 * x + 2], o[4 * x + 3]);
@@ -571,7 +573,7 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
         const CUtensorMap* tm = (r < Rh) ? tmDQ : tmDK;
         const int y = (r < Rh) ? (c.bh * R + r) * p.Lr + c.srow0_of(ht) : c.bh * L + c.row0_of(ht);
 #pragma unroll
-        for (int bx = 0; bx < D / 32; ++bx) tma_reduce_add_2d(tm, 32 * bx, y, smem_u32(sStage) + bx * 8192);
+        for (int bx = 0; bx < 2; ++bx) tma_reduce_add_2d(tm, 64 * cb + 32 * bx, y, smem_u32(stage) + bx * 8192);
         bulk_commit_group();
       }
       __syncwarp();
@@ -759,27 +761,25 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     // ================= heads =================
     // Software pipelining inside the warp: the tail of a head (storing dS and the probabilities, the hand-over to the MMA
     // issuers) is deferred until the TMEM loads of the NEXT unit have been issued, so that their latency runs under it.
-    // (Only where the next unit's MMAs do not wait for that hand-over: with a single (S, dP) buffer whose S columns also
-    // hold the probabilities, at head_dim 128, the tail comes first.  And only with eight worker warps and the column sums:
+    // (Only with eight worker warps and the column sums:
     // sixteen warps do better handing dS over at once (5-6 % against eight that defer, more against sixteen that defer),
     // and so do eight without the group barrier in the middle of a head (4.6 %) -- all measured.)
     constexpr bool kColSums = (kMode == 1 && !kOutDelta);     // the workers sum P dP over the keys themselves
-    constexpr bool kDeferTail = Cfg::kPtSeparate && kColSums && (CG == 32);
+    constexpr bool kDeferTail = kColSums && (CG == 32) && (D == 64);
     float2 dc[H2];
 #pragma unroll
     for (int x = 0; x < H2; ++x) dc[x] = make_float2(0.f, 0.f);
     uint32_t pk[H2], dk[H2];                       // the pending tail: packed probabilities and dS of head tail_hc
-    int tail_hc = -1, tail_b = 0;
+    int tail_hc = -1;
     auto flush_tail = [&]() -> bool {
       if (tail_hc < 0) return true;
       const int thc = tail_hc, db = thc % Cfg::kDs;
       tail_hc = -1;
       if (thc >= Cfg::kDs && !c.wait_w(qDsFree + db, thc / Cfg::kDs - 1)) return false;
       store_row(c.smem + Cfg::oDs + db * 16384, dk);
-      // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column): in its own buffer, or over this group's own S columns
-      if (Cfg::kPtSeparate && thc >= 2 && !c.wait_w(qPtFree + (thc & 1), (thc >> 1) - 1)) return false;
-      const uint32_t pt = Cfg::kPtSeparate ? c.tmem + Cfg::tPT + 32 * (thc & 1) + col0 / 2
-                                           : c.tmem + (tail_b ? Cfg::tS1 : Cfg::tS0) + col0;
+      // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column)
+      if (thc >= 2 && !c.wait_w(qPtFree + (thc & 1), (thc >> 1) - 1)) return false;
+      const uint32_t pt = c.tmem + Cfg::tPT + 32 * (thc & 1) + col0 / 2;
       if (CG == 32) tmem_st16(pt + lane_base, pk);
       else tmem_st8(pt + lane_base, pk);
       tc_wait_st();
@@ -859,7 +859,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         }
       }
       tail_hc = hc;
-      tail_b = b;
       UQ(5)
     }
     if (!kDeferTail && !flush_tail()) return;

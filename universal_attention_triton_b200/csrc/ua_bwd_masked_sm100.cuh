@@ -75,6 +75,9 @@ enum MkBar {
   mMtFull = 0, mQFull = 1, mQFree = 3, mYFull = 5, mYFree = 7, mDone = 9, mSlotFull = 10, mSlotFree = 13, mNumBars = 16
 };
 
+// kWide: chunks of p.m * 128 keys.  A compile-time switch: the producer and the issuer, single threads both, ask for these indices
+// for every tile, and with the divisions of wide chunks in their way the sweep of narrow ones took 20 % longer.
+template <bool kWide>
 struct MkCtx {
   uint8_t* smem;
   uint32_t bars, tmem;
@@ -96,10 +99,10 @@ struct MkCtx {
   }
   __device__ __forceinline__ void arrive_w(int idx) const { mbar_arrive_warp(bar(idx)); }
   // first chunk of the group that has row tile j before it
-  __device__ __forceinline__ int clo(int j) const { return max(0, m * (j / m + 1) - i0); }
+  __device__ __forceinline__ int clo(int j) const { return max(0, (kWide ? m * (j / m + 1) : j + 1) - i0); }
   int m;
   // the operator's chunk that chunk c of the group belongs to, in the gradient tensors
-  __device__ __forceinline__ size_t out_chunk(int N, int cc) const { return m == 1 ? (size_t)bh * N + i0 + cc : (size_t)bh * (N / m) + (i0 + cc) / m; }
+  __device__ __forceinline__ size_t out_chunk(int N, int cc) const { return kWide ? (size_t)bh * (N / m) + (i0 + cc) / m : (size_t)bh * N + i0 + cc; }
   int jb, r0;                          // the slabs hold row tile jb at row r0
   __device__ __forceinline__ int srow(int j) const { return r0 + (j - jb) * 128; }
 };
@@ -317,8 +320,8 @@ struct MkUnit {
   __device__ __forceinline__ bool active() const { return lo < hi; }
 };
 
-template <int D>
-__device__ __forceinline__ void mk_producer(const MkCtx& c, const MaskedParams& p, const CUtensorMap* tmQ, const CUtensorMap* tmG) {
+template <int D, bool kWide>
+__device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedParams& p, const CUtensorMap* tmQ, const CUtensorMap* tmG) {
   using Cfg = MkCfg<D>;
   const int L = p.Lr, R = p.s.R, N = p.s.N;      // (L: rows per slab of the row-indexed tensors)
   const uint32_t sb = smem_u32(c.smem);
@@ -380,8 +383,8 @@ __device__ __forceinline__ void mk_producer(const MkCtx& c, const MaskedParams& 
   MQ_STORE(8)
 }
 
-template <int D>
-__device__ __forceinline__ void mk_issuer(const MkCtx& c, const MaskedParams& p) {
+template <int D, bool kWide>
+__device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedParams& p) {
   using Cfg = MkCfg<D>;
   const int R = p.s.R;
   const uint32_t sb = smem_u32(c.smem);
@@ -444,8 +447,8 @@ __device__ __forceinline__ void mk_issuer(const MkCtx& c, const MaskedParams& p)
 // memory.  Warp = 16 of the 64 columns, lane = row (four passes of 32 rows): every shared-memory access is conflict free
 // and nothing is broadcast, so the warps take little of the bandwidth that the MMA operands need.  The sums stay in
 // registers over the whole work item and are added up over the lanes once, at its end.
-template <int D>
-__device__ __forceinline__ void mk_gate_sums(const MkCtx& c, const MaskedParams& p) {
+template <int D, bool kWide>
+__device__ __forceinline__ void mk_gate_sums(const MkCtx<kWide>& c, const MaskedParams& p) {
   using Cfg = MkCfg<D>;
   const int R = p.s.R, N = p.s.N;
   const int t = threadIdx.x & 127, lane = t & 31, w = t >> 5;
@@ -503,8 +506,8 @@ __device__ __forceinline__ void mk_gate_sums(const MkCtx& c, const MaskedParams&
 
 // Four warps (TMEM lane quadrant = warp % 4): Y of each step, plus sum_c gd_c (x) ksum_c / 128 -> staging tile -> TMA
 // reduce-add into the dQ accumulator; after the last step the group's N^T / u partial sums -> global adds.
-template <int D>
-__device__ __forceinline__ void mk_drain(const MkCtx& c, const MaskedParams& p, const CUtensorMap* tmDQ) {
+template <int D, bool kWide>
+__device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedParams& p, const CUtensorMap* tmDQ) {
   using Cfg = MkCfg<D>;
   const int L = p.Lr, R = p.s.R, N = p.s.N;      // (L: rows per slab of the row-indexed tensors)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -614,7 +617,7 @@ __device__ __forceinline__ void mk_drain(const MkCtx& c, const MaskedParams& p, 
   if (leader) bulk_wait_all();
 }
 
-template <int D>
+template <int D, bool kWide>
 __global__ void __launch_bounds__(384, 1)
 masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                     const __grid_constant__ CUtensorMap tmDQ, MaskedParams p) {
@@ -625,7 +628,7 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int N = p.s.N;
 
-  MkCtx c;
+  MkCtx<kWide> c;
   c.smem = smem;
   c.bars = smem_u32(smem + Cfg::oBar);
   c.abort_flag = reinterpret_cast<volatile int*>(misc + 1);
@@ -700,13 +703,13 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const long long mk_t0 = clock64();
 #endif
   if (warp == 0) {
-    if (lane == 0) mk_producer<D>(c, p, &tmQ, &tmG);
+    if (lane == 0) mk_producer<D, kWide>(c, p, &tmQ, &tmG);
   } else if (warp == 1) {
-    if (lane == 0) mk_issuer<D>(c, p);
+    if (lane == 0) mk_issuer<D, kWide>(c, p);
   } else if (warp >= 4 && warp < 8) {
-    mk_drain<D>(c, p, &tmDQ);
+    mk_drain<D, kWide>(c, p, &tmDQ);
   } else if (warp >= 8) {
-    mk_gate_sums<D>(c, p);
+    mk_gate_sums<D, kWide>(c, p);
   }
 
   tc_fence_before();
