@@ -133,7 +133,9 @@ __global__ void step_kernel(Params p) {
 // ---- bf16, head_dim 64 / 128, chunks of 64 / 128 / 256 keys ----------------------------------------------------------
 // Bound by the one read of the caches; what it needs is bytes in flight.  One block of 2 C threads per (b, h, chunk): every
 // thread issues its 16-byte pieces of K AND of V (128 bytes of each at head_dim 128) before anything else, so that a
-// resident block keeps its whole chunk (64 KB at C = 128, D = 128) on the way.
+// resident block keeps its whole chunk (64 KB at C = 128, D = 128) on the way.  K goes to registers, V through cp.async to the
+// thread's own places in shared memory (only the thread that fetched a piece reads it: no barrier), so that four such blocks fit
+// an SM; with V in registers as well two did (97 -> 86 us below).
 //   scores  mma.sync m16n8k16: the rows are 16 keys of a warp, the columns are the new row's key and its queries (1 + R <= 9:
 //           one or two column tiles, the rest zero).  The contraction index is permuted so that a thread's A pieces are 16
 //           contiguous bytes of a key row; no shuffles, exact bf16 products, fp32 sums.  (Eight columns are too few for tcgen05:
@@ -141,7 +143,7 @@ __global__ void step_kernel(Params p) {
 //   state   thread = key.   softmax  warp = query head: shuffles only.
 //   P V     thread = (8 columns of V, every 2C*8/D-th key), partial sums over the keys through shuffles and shared memory.
 // Against the kernel above (one thread per key row, V one 2-byte element at a time): B16 H8 R4 D128 at t = 6150 (418 MB of
-// caches) 332 -> 97 us = 4.3 TB/s; B1 H8 R4 D64 at t = 300 13.8 -> 3.6 us.
+// caches) 332 -> 86 us = 4.9 TB/s; B1 H8 R4 D64 at t = 300 13.8 -> 3.7 us.
 template <int D, int C, int RT>
 struct StepCfg {
   static constexpr int kThreads = 2 * C, kWarps = kThreads / 32;
@@ -152,7 +154,10 @@ struct StepCfg {
   static constexpr int kNT = RT == 8 ? 2 : 1;            // column tiles of the score product
   static constexpr int kSW = 8 * kNT + 1;                // row stride of the score tile (odd: thread = key reads a column)
   static constexpr int oS = 0, oC = oS + C * kSW, oP = (oC + C + 3) / 4 * 4, oAcc = oP + C * RT;
-  static constexpr int kSmemFloats = oAcc + kWarps * RT * D;
+  // a thread's pieces of V, 16 bytes each and kThreads apart; the partial sums take their place once all have been read (so that
+  // chunks of up to 128 keys stay within the 48 KB that need no opt-in)
+  static constexpr int oV = oAcc, kAcc = kWarps * RT * D, kV = C * D / 2;
+  static constexpr int kSmemFloats = oAcc + (kAcc > kV ? kAcc : kV);
 };
 
 template <int D, int C, int RT, typename TG>
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
 
   // all reads of the caches first
   const int kr0 = warp * 16 + (lane >> 2), kr1 = kr0 + 8, c8 = (lane & 3) * 8;
-  uint4 a0[Cfg::kKLoads], a1[Cfg::kKLoads], bq[Cfg::kNT][Cfg::kKLoads], v[Cfg::kVLoads];
+  uint4 a0[Cfg::kKLoads], a1[Cfg::kKLoads], bq[Cfg::kNT][Cfg::kKLoads];
   const __nv_bfloat16* krow = kc + (size_t)i * C * D + c8;
 #pragma unroll
   for (int x = 0; x < Cfg::kKLoads; ++x) {
@@ -183,12 +188,17 @@ __global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
 #pragma unroll
     for (int x = 0; x < Cfg::kKLoads; ++x) bq[n][x] = col <= R ? __ldg(reinterpret_cast<const uint4*>(row + c8 + x * 32)) : zero;
   }
+  const uint32_t my_v = (uint32_t)__cvta_generic_to_shared(sm + Cfg::oV) + tid * 16;
   const int vg = tid / Cfg::kTPR, vc8 = (tid % Cfg::kTPR) * 8;
 #pragma unroll
   for (int x = 0; x < Cfg::kVLoads; ++x) {
     const int k = vg + x * Cfg::kGroups;
-    v[x] = k < nkeys ? __ldg(reinterpret_cast<const uint4*>(vrow + (size_t)k * D + vc8)) : zero;
+    // (a piece beyond the live keys is filled with zeros and not read)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(my_v + x * Cfg::kThreads * 16),
+                 "l"(vrow + (size_t)(k < nkeys ? k : 0) * D + vc8), "r"(k < nkeys ? 16 : 0)
+                 : "memory");
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
   // (per-key values of the state update; a thread beyond the live keys reads nothing)
   const size_t key_at = (size_t)bh * p.Lcap + (size_t)i * C + tid;
   const bool updates = tid < nkeys && i * C + tid < p.t;
@@ -259,10 +269,12 @@ __global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
   for (int r = 0; r < RT; ++r)
 #pragma unroll
     for (int u = 0; u < 8; ++u) acc[r][u] = 0.f;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
   for (int x = 0; x < Cfg::kVLoads; ++x) {
     const float* pk = s_p + (vg + x * Cfg::kGroups) * RT;
-    const uint32_t w[4] = {v[x].x, v[x].y, v[x].z, v[x].w};
+    const uint4 v = reinterpret_cast<const uint4*>(sm + Cfg::oV)[x * Cfg::kThreads + tid];
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     float pr[RT];
 #pragma unroll
     for (int r = 0; r < RT; ++r) pr[r] = pk[r];
@@ -276,6 +288,7 @@ __global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
       }
     }
   }
+  __syncthreads();      // (every thread has read its pieces of V)
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
 #pragma unroll
