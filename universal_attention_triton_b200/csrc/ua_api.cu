@@ -171,10 +171,22 @@ int launch_simt_bwd_any(const ua::simt::BwdParams& p, int dtype, int gate_dtype,
   return launch_simt_bwd<bf16, bf16, float>(p, st);
 }
 
-__global__ void widen_bf16_kernel(const bf16* __restrict__ src, float* __restrict__ dst, size_t n) {
-  size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (; idx < n; idx += stride) dst[idx] = __bfloat162float(src[idx]);
+// eight elements per thread and step where the pointers allow (n8 of them), the rest one by one
+__global__ void __launch_bounds__(256) widen_bf16_kernel(const bf16* __restrict__ src, float* __restrict__ dst, size_t n8, size_t n) {
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t idx = first; idx < n8; idx += stride) {
+    const uint4 x = reinterpret_cast<const uint4*>(src)[idx];
+    float4* d = reinterpret_cast<float4*>(dst) + 2 * idx;
+    d[0] = make_float4(__uint_as_float(x.x << 16), __uint_as_float(x.x & 0xffff0000u), __uint_as_float(x.y << 16), __uint_as_float(x.y & 0xffff0000u));
+    d[1] = make_float4(__uint_as_float(x.z << 16), __uint_as_float(x.z & 0xffff0000u), __uint_as_float(x.w << 16), __uint_as_float(x.w & 0xffff0000u));
+  }
+  for (size_t idx = 8 * n8 + first; idx < n; idx += stride) dst[idx] = __bfloat162float(src[idx]);
+}
+int launch_widen(const void* src, float* dst, size_t n, cudaStream_t st) {
+  const size_t n8 = aligned16(src) && aligned16(dst) ? n / 8 : 0, work = n8 ? n8 : n;
+  const unsigned blocks = (unsigned)std::min<size_t>((work + 255) / 256, 148 * 16);
+  widen_bf16_kernel<<<blocks, 256, 0, st>>>(static_cast<const bf16*>(src), dst, n8, n);
+  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
 
 template <typename T>
@@ -706,8 +718,7 @@ int ua_bwd_rows_kept(const UaDims* dims, int dtype, int gate_dtype, const UaRows
   }
   const float* gd32 = static_cast<const float*>(g_denom_cm_rows);
   if (g_denom_dtype != UA_F32) {
-    widen_bf16_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const bf16*>(g_denom_cm_rows), gd_tmp, row_elems);
-    if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
+    if ((e = launch_widen(g_denom_cm_rows, gd_tmp, row_elems, st))) return e;
     gd32 = gd_tmp;
   }
   if (!aligned16(gd32) || !aligned16(static_dest_rows) || !aligned16(carry_tab) || !aligned16(lse_rows)) return UA_ERR_ALIGNMENT;
@@ -840,8 +851,7 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     const bool out_tiles = !wide && s.D == 64 && out_cm && aligned16(out_cm);
     const float* gd32 = static_cast<const float*>(g_denom_cm);
     if (g_denom_dtype != UA_F32 && (!out_tiles || (masked && ks.C == 128) || !aligned16(g_denom_cm))) {
-      widen_bf16_kernel<<<148 * 8, 256, 0, st>>>(static_cast<const bf16*>(g_denom_cm), at(w.off_gd), rows);
-      if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
+      if ((e = launch_widen(g_denom_cm, at(w.off_gd), rows, st))) return e;
       gd32 = at(w.off_gd);
     } else if (g_denom_dtype != UA_F32) {
       gd32 = nullptr;

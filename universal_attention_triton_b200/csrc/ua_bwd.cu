@@ -1,6 +1,4 @@
 // Launchers of the tensor-core backward.
-#include <cstdlib>
-
 #include "ua_sm100_host.cuh"
 
 namespace ua {
@@ -115,14 +113,18 @@ int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* 
   if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D) || !make_rows_map(&tmG, g_out, BH * (s.N / p.m) * s.R * p.Lr, D) ||
       !make_f32_rows_map(&tmDQ, acc_dq, BH * s.R * p.Lr, D))
     return UA_ERR_CUDA;
-  static const int jp_env = []() { const char* e = getenv("UA_MASKED_TILES"); return e ? atoi(e) : 0; }();
-  p.jp = jp_env > 0 ? jp_env : 8;
-  p.items_per_bh = 0;
+  // Row tiles per work item.  An item pays for its start-up once and adds to dQ where the groups at work share L2, so it should be
+  // neither short nor long: about 32 (tile, head) steps, but 16 tiles at most (B4 H8 R4 L4096 D64, 4 / 8 / 16 / 32 tiles: 466 / 438 / 471 /
+  // 564 us; B1 H16 R1 L4096 D128: 320 / 242 / 215 / 217 us), and fewer where that would leave SMs without one.
   const int last = (s.N - 1) / p.m * p.m, jcap = (last < p.j_end) ? last : p.j_end;      // no row tile at or after the last chunk is before any chunk
-  for (int g = 0; g * Cfg::kG < s.N; ++g) {
-    int jmax = ((((g + 1) * Cfg::kG < s.N) ? (g + 1) * Cfg::kG : s.N) - 1) / p.m * p.m;
-    if (jmax > jcap) jmax = jcap;
-    if (jmax > p.j_begin) p.items_per_bh += (jmax - p.j_begin + p.jp - 1) / p.jp;
+  for (p.jp = s.R >= 4 ? 8 : 16;; p.jp /= 2) {
+    p.items_per_bh = 0;
+    for (int g = 0; g * Cfg::kG < s.N; ++g) {
+      int jmax = ((((g + 1) * Cfg::kG < s.N) ? (g + 1) * Cfg::kG : s.N) - 1) / p.m * p.m;
+      if (jmax > jcap) jmax = jcap;
+      if (jmax > p.j_begin) p.items_per_bh += (jmax - p.j_begin + p.jp - 1) / p.jp;
+    }
+    if (p.jp <= 2 || BH * p.items_per_bh * Cfg::kKB >= 148) break;
   }
   if (p.items_per_bh == 0) return UA_OK;
   const auto* k16 = static_cast<const __nv_bfloat16*>(kc);
