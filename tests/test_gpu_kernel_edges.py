@@ -1,0 +1,135 @@
+"""The kernels at the edges of their ranges: chunks of 64 keys and half-filled tiles, sweeps cut into segments of every length, wide
+chunks, the tiled generic kernels, the decode step on every tile width, merges of few and of very many chunks."""
+import pytest
+import torch
+
+from oracle import ua_oracle as O
+from tests._util import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+GRADS = ["dkc", "dvc", "dxq", "dsrc", "ddest"]
+
+
+def _inputs(B, H, R, n, c, D, gate_fp32=False, dtype=torch.bfloat16, seed=17):
+    """Unit keys, as the drivers make them: decays that neither vanish nor saturate."""
+    kc, vc, xq, ss, sd = O.make_inputs(B, H, R, n * c, c, D, seed=seed)
+    kc = kc / kc.norm(dim=-1, keepdim=True)
+    gt = torch.float32 if gate_fp32 else dtype
+    return [kc.to(dtype), vc.to(dtype), xq.to(dtype), ss.to(gt), sd.to(gt)]
+
+
+@pytest.mark.parametrize("shape,gate_fp32", [
+    ((1, 2, 4, 1, 64, 64), False),        # B, H, R, chunks, chunk, D.  One chunk of 64: half of the only tile
+    ((2, 1, 3, 3, 64, 64), True),         # odd number of 64-key chunks
+    ((1, 2, 1, 2, 64, 128), False),
+    ((1, 1, 2, 13, 64, 128), True),       # ... cut
+    ((1, 2, 4, 5, 128, 64), False),       # cut into single tiles
+    ((1, 1, 2, 17, 128, 64), True),       # cut, the last segments shorter than the others
+    ((1, 1, 1, 24, 128, 128), False),     # segments of several tiles
+    ((2, 1, 2, 11, 128, 128), False),
+    ((8, 16, 2, 3, 128, 64), False),      # enough blocks to stay whole
+    ((1, 1, 2, 1, 256, 64), False),       # wide chunks
+    ((2, 1, 1, 3, 256, 128), True),
+    ((1, 2, 2, 2, 384, 64), False)])
+def test_tensor_core_sweeps_match_the_generic_kernels(shape, gate_fp32):
+    from universal_attention_triton_b200 import _lib, ops
+    B, H, R, n, c, D = shape
+    L = n * c
+    cu = [t.cuda() for t in _inputs(*shape, gate_fp32=gate_fp32)]
+    out, lse, _, carry = ops.forward_cm(*cu, keep_carry=True)
+    out_sm, lse_sm, _ = ops.forward_cm(*cu, flags=_lib.FLAG_FORCE_SIMT)
+    valid = (torch.arange(L).view(1, L) >= torch.arange(n).view(n, 1) * c).cuda().view(1, 1, n, 1, L).expand_as(lse)
+    assert ((out.float() - out_sm.float()).abs() <= 2e-2 + 2.0 ** -7 * out_sm.float().abs()).all()
+    assert (((lse - lse_sm).abs() - 1e-5 * lse_sm.abs()) * valid).max() <= 2e-2
+    assert torch.equal(lse[~valid], lse_sm[~valid])
+    gen = torch.Generator(device="cuda").manual_seed(78)
+    g_out = torch.randn(B, H, n, R, L, D, generator=gen, device="cuda", dtype=torch.bfloat16)
+    g_lse = torch.randn(B, H, n, R, L, generator=gen, device="cuda")
+    for flags in (0, _lib.FLAG_SKIP_MASKED_GRADS):
+        ref = ops.backward_cm(*cu, g_out, g_lse, flags=flags | _lib.FLAG_FORCE_SIMT)
+        for kept in ({}, {"lse": lse}, {"lse": lse, "carry": carry}, {"lse": lse, "carry": carry, "out_cm": out}):
+            got = ops.backward_cm(*cu, g_out, g_lse, flags=flags, **kept)
+            for a, b, key in zip(got, ref, GRADS):
+                assert a.dtype == b.dtype and torch.isfinite(a.float()).all(), key
+                assert rel_fro(a.float().cpu(), b.float().cpu()) <= 2e-2, (key, flags, sorted(kept), rel_fro(a.float().cpu(), b.float().cpu()))
+
+
+@pytest.mark.parametrize("dtype,shape", [
+    (torch.float32, (1, 1, 1, 1, 32, 4)), (torch.float32, (2, 1, 3, 5, 32, 64)), (torch.float32, (1, 2, 2, 3, 64, 20)),
+    (torch.float32, (1, 1, 5, 2, 128, 64)), (torch.float32, (1, 1, 2, 3, 128, 128)), (torch.float32, (1, 1, 1, 3, 64, 12)),
+    (torch.bfloat16, (1, 2, 2, 3, 64, 32)), (torch.bfloat16, (2, 1, 1, 5, 32, 64)), (torch.bfloat16, (1, 1, 3, 2, 128, 96))])
+def test_tiled_kernels_against_oracle(dtype, shape):
+    """fp32 1e-4; bf16 2e-2 forward, 5e-2 gradients, against the fp32 oracle on the same values."""
+    from universal_attention_triton_b200 import _lib, ops
+    B, H, R, n, c, D = shape
+    L = n * c
+    f32 = dtype == torch.float32
+    ins = _inputs(*shape, dtype=dtype)
+    ins32 = [t.float() for t in ins]
+    gen = torch.Generator().manual_seed(3)
+    g_out = torch.randn(B, H, R, L, D, n, generator=gen).to(dtype)
+    g_den = torch.randn(B, H, R, L, n, generator=gen)
+    cu = [t.cuda() for t in ins]
+    out, lse, _ = ops.forward_cm(*cu)
+    ref_out, _, ref_lse = O.ua_forward(*ins32)
+    e = (ops.as_reference_out(out).float().cpu() - ref_out).abs() - (0 if f32 else 2.0 ** -8) * ref_out.abs()
+    assert e.max() <= (1e-4 if f32 else 2e-2)
+    valid = (torch.arange(L).view(L, 1) >= torch.arange(n).view(1, n) * c)
+    assert (((ops.as_reference_denom(lse).cpu() - ref_lse).abs() - 1e-5 * ref_lse.abs()) * valid).max() <= (1e-4 if f32 else 2e-2)
+    for skip in (False, True):
+        go, gd = (g_out * valid.view(L, 1, n), g_den * valid) if skip else (g_out, g_den)
+        ref = O.ua_backward(*ins32, go.float(), gd)
+        flags = _lib.FLAG_SKIP_MASKED_GRADS if skip else 0
+        got = ops.backward_cm(*cu, ops.out_to_chunk_major(go.cuda()), ops.denom_to_chunk_major(gd.cuda()), flags=flags)
+        for a, b, key in zip(got, ref, GRADS):
+            assert rel_fro(a.float().cpu(), b) <= (1e-4 if f32 else 5e-2), (key, skip, rel_fro(a.float().cpu(), b))
+
+
+@pytest.mark.parametrize("H,R,chunk,D,gate_fp32", [(2, 1, 64, 64, False), (1, 2, 64, 128, True), (2, 4, 128, 64, True), (1, 3, 128, 128, False),
+                                                   (1, 8, 256, 64, False), (2, 5, 256, 128, True)])
+def test_decode_tensor_core_step_at_tile_edges(H, R, chunk, D, gate_fp32):
+    """Rows around the first key, quarter tiles and chunk boundaries, against the rows of the generic forward; the decay state
+    is carried through every step; the cache is longer than what is filled."""
+    from universal_attention_triton_b200 import _lib, ops
+    n = 3 if chunk < 256 else 2
+    L = n * chunk
+    kc, vc, xq, ss, sd = [t.cuda() for t in _inputs(1, H, R, n, chunk, D, gate_fp32=gate_fp32)]
+    out, lse, _ = ops.forward_cm(kc, vc, xq, ss, sd, flags=_lib.FLAG_FORCE_SIMT)        # (b,h,n,r,L,d), (b,h,n,r,L)
+    cap = L + chunk
+
+    def cache(t):
+        return torch.cat([t.reshape(1, H, L, *t.shape[4:]), t.new_zeros(1, H, cap - L, *t.shape[4:])], 2).contiguous()
+    k, v, src = cache(kc), cache(vc), cache(ss)
+    state = torch.zeros(1, H, cap, device="cuda")
+    edges = {0, 1, 7, 15, 16, 31, 32, 63, 64, chunk - 1, chunk, chunk + 1, chunk + 33, 2 * chunk - 1, L - 1}
+    for t in range(L):
+        o, l = ops.decode_step(t, k, v, src, xq[:, :, :, t].contiguous(), sd[:, :, t].contiguous(), state, chunk)
+        if t not in edges:
+            continue
+        nt = t // chunk + 1
+        ro, rl = out[:, :, :nt, :, t].permute(0, 1, 3, 4, 2).float(), lse[:, :, :nt, :, t].permute(0, 1, 3, 2)
+        assert ((o.float() - ro).abs() <= 2e-2 + 2.0 ** -7 * ro.abs()).all(), t
+        assert ((l - rl).abs() <= 2e-2 + 1e-5 * rl.abs()).all(), t
+        assert (state[:, :, t + 1:] == 0).all(), t
+
+
+@pytest.mark.parametrize("dtype,vec_dtype,N,D", [(torch.bfloat16, torch.bfloat16, 2, 64), (torch.bfloat16, torch.float32, 3, 128),
+                                                 (torch.float32, torch.float32, 4, 16), (torch.bfloat16, torch.bfloat16, 5, 128),
+                                                 (torch.bfloat16, torch.bfloat16, 1, 64), (torch.bfloat16, torch.float32, 150, 8)])
+def test_merge_of_few_and_of_many_chunks(dtype, vec_dtype, N, D):
+    from universal_attention_triton_b200 import ops
+    gen = torch.Generator().manual_seed(N)
+    rows = 16 * N
+    mat = torch.randn(1, 2, 2, rows, D, N, generator=gen).to(dtype)
+    vec = (torch.randn(1, 2, 2, rows, N, generator=gen) * 3).to(vec_dtype)
+    g = torch.randn(1, 2, 2, rows, D, generator=gen).to(dtype)
+    out_cm, lse_cm = ops.out_to_chunk_major(mat.cuda()), ops.denom_to_chunk_major(vec.cuda())
+    tol = 1e-5 if dtype == torch.float32 else 2e-2
+    ref = O.merge_forward(mat.float(), vec.float())
+    assert ((ops.merge_fwd_cm(out_cm, lse_cm).float().cpu() - ref).abs() <= tol * (1 + ref.abs())).all()
+    d_mat, d_vec = O.merge_backward(mat.float(), vec.float(), g.float())
+    g_out, g_lse = ops.merge_bwd_cm(out_cm, lse_cm, g.cuda())
+    assert rel_fro(ops.as_reference_out(g_out).float().cpu(), d_mat) <= tol
+    if N > 1:
+        assert rel_fro(ops.as_reference_denom(g_lse).float().cpu(), d_vec) <= tol

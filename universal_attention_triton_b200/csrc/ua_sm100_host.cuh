@@ -8,6 +8,7 @@
 #include "ua_bwd2_sm100.cuh"
 #include "ua_bwd_masked_sm100.cuh"
 #include "ua_fwd_sm100.cuh"
+#include "ua_split.h"
 
 namespace ua {
 namespace sm100 {
@@ -62,33 +63,6 @@ inline bool fwd_supported(const Shape& s, int dtype) {
 // The entry points over row ranges, and those of the merged output, are built for chunks of 128 keys.
 inline bool chunk128(const Shape& s) { return s.C == 128; }
 
-// 128-row tiles in the sweep of chunk i (chunks of 64 keys start a tile at their own first row)
-inline int sweep_tiles(const Shape& s, int i) { return (s.L - i * s.C + 127) / 128; }
-
-// Row tiles per block of the forward, 0 = one block per chunk.  A block takes about as long as it has tiles (a tile of B1 H8 R4
-// D64: 8.5 us); one block per chunk therefore lasts max(longest sweep, tiles / SMs) tile times.  That is the longest sweep, n
-// tiles, whenever there are few (batch, head) units, while most SMs idle.  Cut into segments of s tiles the same work lasts about
-// tiles / SMs plus half a segment, plus the fixed cost of more blocks (a quarter of a tile each) and of the totals kernel in
-// front (about half a tile, and a twelfth of a tile per tile).  The smallest of these estimates decides.
-inline int fwd_split(const Shape& s) {
-  constexpr double kSms = 148.0;
-  const double BH = (double)s.B * s.H;
-  double tiles = 0;
-  for (int i = 0; i < s.N; ++i) tiles += sweep_tiles(s, i);
-  const int longest = sweep_tiles(s, 0);
-  double best = (BH * tiles / kSms > longest ? BH * tiles / kSms : longest) + 0.25;
-  int seg = 0;
-  for (int t = 1; t < longest; t *= 2) {
-    double blocks = 0;
-    for (int i = 0; i < s.N; ++i) blocks += (sweep_tiles(s, i) + t - 1) / t;
-    const double work = BH * (tiles + 0.25 * blocks) / kSms, one = t + 0.25;
-    const double est = (BH * blocks <= kSms ? one : work + 0.5 * one) + 0.5 + BH * tiles / kSms / 12;
-    if (est < 0.9 * best) { best = est; seg = t; }
-  }
-  return seg;
-}
-inline size_t fwd_totals_bytes(const Shape& s) { return (size_t)s.B * s.H * s.N * sweep_tiles(s, 0) * 128 * sizeof(float); }
-
 // Fills the row-range fields of FwdParams for a call over the whole sequence.
 inline void whole_sequence(FwdParams& p) {
   p.j_begin = 0; p.j_end = p.s.N; p.Lr = p.s.L; p.r0 = 0; p.carry_in = nullptr; p.total_out = nullptr;
@@ -105,32 +79,6 @@ int launch_fwd_merge(const Shape& s, int gate_dtype, const void* kc, const void*
 
 // Shapes of the keys-on-lanes backward kernel.
 inline bool bwd2_supported(const Shape& s, int dtype) { return fwd_supported(s, dtype); }
-
-// Half tiles (64 rows) per block of the backward, 0 = one block per chunk: the same reckoning as fwd_split, in units of a half tile
-// with heads.  What a cut costs here is the correction pass, a launch of its own that repeats the decay gradient of every half tile
-// but those of the last segments: 5.5 of the 7.9 + 2.7 R thousand cycles a half tile takes, beside a start-up of about 5 thousand
-// per block in each pass.
-inline int bwd_split(const Shape& s) {
-  constexpr double kSms = 148.0;
-  const double unit = 7.9 + 2.7 * s.R, start = 5.0 / unit, corr = 5.5 / unit, BH = (double)s.B * s.H;
-  const int top = s.L / 64, per = s.C / 64;
-  double halves = 0;
-  for (int i = 0; i < s.N; ++i) halves += top - i * per;
-  double best = (BH * halves / kSms > top ? BH * halves / kSms : top) + start;
-  int seg = 0;
-  for (int t = 2; t < top; t *= 2) {
-    double blocks = 0;
-    for (int i = 0; i < s.N; ++i) blocks += (top - i * per + t - 1) / t;
-    auto pass = [&](double cost, double n) {
-      const double one = cost * t + start;
-      return BH * n <= kSms ? one : BH * (cost * halves + start * n) / kSms + 0.5 * one;
-    };
-    const double est = pass(1.0, blocks) + pass(corr, blocks - s.N > 1 ? blocks - s.N : 1) + 0.4;
-    if (est < 0.9 * best) { best = est; seg = t; }
-  }
-  return seg;
-}
-inline int bwd_max_segments(const Shape& s, int seg) { return seg ? (s.L / 64 + seg - 1) / seg : 0; }
 
 // Fills the row-range fields of Bwd2Params for a call over the whole sequence.
 inline void whole_sequence(Bwd2Params& p) {
