@@ -5,18 +5,6 @@ namespace ua {
 namespace sm100 {
 namespace {
 
-// Columns of a half tile per worker thread: 16 (sixteen worker warps, 96 registers each).  Four warps per scheduler hide the TMEM and
-// shared-memory latencies; at head_dim 64 sixteen that hand dS over at once are 5-6 % faster than eight that defer the tail of a
-// head, in every build (sixteen that defer are slower than either); at head_dim 128 they are 2 % faster with one query head and
-// level with four (measured).
-#ifndef UA_BWD2_COLS_64
-#define UA_BWD2_COLS_64 16
-#endif
-#ifndef UA_BWD2_COLS_128
-#define UA_BWD2_COLS_128 16
-#endif
-template <int D> constexpr int bwd2_cols() { return D == 64 ? UA_BWD2_COLS_64 : UA_BWD2_COLS_128; }
-
 template <int D, int kC, typename TG>
 int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, const void* xq, const void* g_out, const Bwd2Params& p,
                   cudaStream_t st) {
@@ -33,22 +21,21 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
              !make_f32_rows_map(&tmDQ, p.acc_dq, BH * s.R * p.Lr, D, 64)) {
     return UA_ERR_CUDA;
   }
-  constexpr int kCols = bwd2_cols<D>();
-  const int threads = 32 * (8 + 4 * (64 / kCols));
+  const int threads = 32 * (8 + 4 * NG);
   CUtensorMap tmO = tmG;
-  auto kern = bwd2_kernel<D, kC, TG, 1, kCols, false>;
+  auto kern = bwd2_kernel<D, kC, TG, 1, false>;
   if (p.heads > 0) {
-    kern = bwd2_kernel<D, kC, TG, 1, kCols, true>;
+    kern = bwd2_kernel<D, kC, TG, 1, true>;
     if constexpr (kC == 128) {
-      if (mode == 2) kern = bwd2_kernel<D, kC, TG, 2, kCols, true>;
-      if (mode == 3) kern = bwd2_kernel<D, kC, TG, 3, kCols, true>;
-      if (mode == 4) kern = bwd2_kernel<D, kC, TG, 4, kCols, true>;
+      if (mode == 2) kern = bwd2_kernel<D, kC, TG, 2, true>;
+      if (mode == 3) kern = bwd2_kernel<D, kC, TG, 3, true>;
+      if (mode == 4) kern = bwd2_kernel<D, kC, TG, 4, true>;
     }
     // the forward's output tiles at hand (per-chunk form, head_dim 64): the row term comes from them
     if constexpr (Cfg::kOutTiles) {
       if (mode == 1 && p.out_tiles != nullptr) {
         if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
-        kern = bwd2_kernel<D, kC, TG, 1, kCols, true, true>;
+        kern = bwd2_kernel<D, kC, TG, 1, true, true>;
       }
     }
   }

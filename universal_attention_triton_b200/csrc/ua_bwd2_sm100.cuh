@@ -26,7 +26,7 @@
 //
 // Warps: 0 = "front" MMA issuer (G, S, dP: everything that only needs loaded tiles), 1 and 3 = "back" MMA issuers
 // (1: dV, dK_i; 3: dQ, dK_j: everything that needs a tile the workers wrote), 2 = TMA producer, 4.. = workers:
-// 64 / CG column groups of 128 threads (thread = key, CG of the 64 columns each, held in registers; CG = 16 or 32).
+// four column groups of 128 threads (thread = key, CG = 16 of the 64 columns each, held in registers).
 // dQ_rj / dK_j (64 rows, M = 128 MMAs whose upper 64 lanes compute on whatever the next buffer holds and are
 // never read) leave as TMA reduce-adds into fp32 accumulators.  Rows BEFORE the chunk are not handled here.
 //
@@ -91,6 +91,11 @@ struct Bwd2Params {
   float* seg_totals;         // (b*h*n, max_seg, 128): sum of dC per key over each segment's rows, written by the pass with heads, read by the other
 };
 
+// Columns of a half tile per worker thread: four column groups, sixteen worker warps of 96 registers.  Four warps per scheduler hide the
+// TMEM and shared-memory latencies; at head_dim 64 sixteen that hand dS over at once are 5-6 % faster than eight (32 columns) that defer the
+// tail of a head, at head_dim 128 they are 2 % faster with one query head and level with four (measured).
+constexpr int CG = 16, NG = 64 / CG;
+
 template <int D>
 struct Bwd2Cfg {
   static constexpr int kNB = (D == 64) ? 2 : 1;            // (S, dP) buffers in TMEM
@@ -117,17 +122,11 @@ struct Bwd2Cfg {
   static constexpr int oXch = oHtTab + kTab * kHtTab;      // float [8][128] totals crossing the column groups
   static constexpr int oBar = oXch + 4096;
   static constexpr int oMisc = oBar + 320;      // (35 barriers of 8 bytes)
-  // per-warp scratch tiles for the column sums over the keys ([32 lanes][CG + 4] floats each, at most 40 KB in all);
-  // head_dim 128 has no room for them and transposes with shuffles
-  static constexpr bool kScratch = (D == 64);
-  static constexpr int oScr = oMisc + 256;
-  static constexpr int kSmemBytes = oScr + (kScratch ? 40960 : 0) + 1024;     // + slack to align the base to 1024 B
-  // builds that take the row term from the forward's output tiles (head_dim 64) keep kNS output half tiles where the
-  // scratch tiles would be, and sum the decay gradient's columns with shuffles
-  static constexpr bool kOutTiles = kScratch;
-  static constexpr int oOut = (oScr + 1023) / 1024 * 1024;
+  // builds that take the row term from the forward's output tiles (head_dim 64; 128 has no room for them): kNS output half tiles
+  static constexpr bool kOutTiles = (D == 64);
+  static constexpr int oOut = (oMisc + 256 + 1023) / 1024 * 1024;
   static constexpr int oGd16 = oOut + kNS * kHalf;         // kNS x bf16[64]: g_denom rows of a head before they are widened
-  static_assert(!kOutTiles || oGd16 + kNS * 128 <= oScr + 40960, "output tiles fit the scratch area");
+  static constexpr int kSmemBytes = (kOutTiles ? oGd16 + kNS * 128 : oMisc + 256) + 1024;     // + slack to align the base to 1024 B
   // TMEM columns.  The row-side results Y are 64 columns wide and taken D / 64 times per unit: at head_dim 128 that leaves room for
   // probabilities (bf16 pairs, 32 columns per head) in a buffer pair of their own.  Written over the S columns they kept the (S, dP)
   // buffer until the dV product had read them, and every head waited for two rounds of products one after the other:
@@ -370,7 +369,7 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
 // which = 0: the accumulators that live for the whole sweep (dV_i += P dO, dK_i += dS Q, dK_i += dG K_j);
 // which = 1: the row-side results that leave after every unit (Y = dQ_rj = dS^T K_i, Y = dK_j = dG^T K_i).
 // MMAs into one accumulator always come from the same thread, so their order is kept.
-template <int D, int kC, int CG>
+template <int D, int kC>
 __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p, const int which) {
   using Cfg = Bwd2Cfg<D>;
   const int R = p.heads;
@@ -463,65 +462,21 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
                "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
-template <int N>
-__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t* r) {
-  if (N == 32) tmem_ld32(taddr, r);
-  else tmem_ld16(taddr, r);
-}
-
-// Sum over the 32 lanes of a warp of v[0..CG): afterwards every lane holds the sum of column (lane % CG).
-// With a per-warp shared-memory scratch tile this costs CG/4 vector stores + 32 loads and adds per lane; without one it is
-// a shuffle transpose (about 4 instructions per element).
-template <int CG>
-__device__ __forceinline__ float warp_colsum(float* v, float* scr, int lane) {
-  if (scr == nullptr) {
-    if (CG == 32) return warp_transpose_reduce(v, lane);
-    // 16 columns: halve 8, 4, 2, 1 (the lane keeps the half its bit selects), then the two half warps add up
+// Sum over the 32 lanes of a warp of v[0..CG): afterwards every lane holds the sum of column (lane % CG).  A shuffle transpose, about 4
+// instructions per element: halve 8, 4, 2, 1 (the lane keeps the half its bit selects), then the two half warps add up.  (Through a
+// shared-memory tile per warp it is 2.5 % slower with sixteen worker warps, measured: shared memory is the busier resource.)
+__device__ __forceinline__ float warp_colsum(float* v, int lane) {
 #pragma unroll
-    for (int s = 8; s >= 1; s >>= 1) {
-      const bool upper = (lane & s) != 0;
+  for (int s = CG / 2; s >= 1; s >>= 1) {
+    const bool upper = (lane & s) != 0;
 #pragma unroll
-      for (int x = 0; x < s; ++x) {
-        const float send = upper ? v[x] : v[x + s];
-        const float keep = upper ? v[x + s] : v[x];
-        v[x] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-      }
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
-  }
-  // scratch rows of CG + 4 floats: the 16-byte row writes and the column reads are both conflict free without any
-  // address swizzling, so every access is one instruction with an immediate offset
-  constexpr int PITCH = CG + 4;
-  float4* row = reinterpret_cast<float4*>(scr + lane * PITCH);
-#pragma unroll
-  for (int cidx = 0; cidx < CG / 4; ++cidx) row[cidx] = make_float4(v[4 * cidx], v[4 * cidx + 1], v[4 * cidx + 2], v[4 * cidx + 3]);
-  __syncwarp();
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-  if (CG == 32) {
-    const float* col = scr + lane;
-#pragma unroll
-    for (int t = 0; t < 32; t += 4) {
-      a0 += col[(t + 0) * PITCH];
-      a1 += col[(t + 1) * PITCH];
-      a2 += col[(t + 2) * PITCH];
-      a3 += col[(t + 3) * PITCH];
-    }
-  } else {
-    // lanes 0..15 read rows 0..15, lanes 16..31 rows 16..31 starting four rows further on (opposite bank halves)
-    const int hi = lane >> 4;
-    const float* col = scr + (lane & 15) + hi * (16 + 4) * PITCH;
-#pragma unroll
-    for (int t = 0; t < 16; t += 4) {
-      a0 += col[(((t + 0) < 12 || !hi) ? (t + 0) : (t + 0) - 16) * PITCH];
-      a1 += col[(((t + 1) < 12 || !hi) ? (t + 1) : (t + 1) - 16) * PITCH];
-      a2 += col[(((t + 2) < 12 || !hi) ? (t + 2) : (t + 2) - 16) * PITCH];
-      a3 += col[(((t + 3) < 12 || !hi) ? (t + 3) : (t + 3) - 16) * PITCH];
+    for (int x = 0; x < s; ++x) {
+      const float send = upper ? v[x] : v[x + s];
+      const float keep = upper ? v[x + s] : v[x];
+      v[x] = keep + __shfl_xor_sync(0xffffffffu, send, s);
     }
   }
-  float acc = (a0 + a1) + (a2 + a3);
-  if (CG == 16) acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-  __syncwarp();
-  return acc;
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
 // ----------------------------------------------------------------- drain warps --
@@ -622,14 +577,12 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
   }
 }
 
-// CG: columns of a half tile per thread (32: two column groups, 8 worker warps; 16: four groups, 16 worker warps)
 // kHeads = false: the correction pass (p.heads == 0).  A compile-time switch: as a run-time condition around the decay
 // recomputation it cost the whole-sequence kernel 2 % (measured).
 // kOutDelta: the row term comes from the delta warps (see bwd2_delta).
-template <int D, int kC, typename TG, int kMode, int CG, bool kHeads, bool kOutDelta>
+template <int D, int kC, typename TG, int kMode, bool kHeads, bool kOutDelta>
 __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& p) {
   using Cfg = Bwd2Cfg<D>;
-  constexpr int NG = 64 / CG;                    // column groups
   constexpr int H2 = CG / 2;                     // packed pairs per thread
   constexpr int kWorkers = kC * NG;
   constexpr int kGateQuad = kC / 64;             // the quadrant whose warps fetch the gates of the next half tile
@@ -649,9 +602,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   const float2 s32 = make_float2(s3, s3);
   float* sT3 = reinterpret_cast<float*>(c.smem + Cfg::oT3);
   float* sXch = reinterpret_cast<float*>(c.smem + Cfg::oXch);
-  // (per-warp scratch tiles for the column sums: only with eight worker warps -- with sixteen the shuffle form is 2.5 %
-  // faster, measured, as shared memory is the busier resource then)
-  float* scr = (Cfg::kScratch && !kOutDelta && CG == 32) ? reinterpret_cast<float*>(c.smem + Cfg::oScr) + (warp - 8) * (32 * (CG + 4)) : nullptr;
   const uint32_t swz = (uint32_t)(key & 7);
   UQ_DECL
 
@@ -707,7 +657,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
       tc_fence_after();
       uint32_t gr[CG];
-      tmem_ld_n<CG>(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
+      tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
       float2 t3p[H2];
       load_pairs(t3v, t3p);
       tc_wait_ld();
@@ -759,13 +709,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     UQ(0)
 
     // ================= heads =================
-    // Software pipelining inside the warp: the tail of a head (storing dS and the probabilities, the hand-over to the MMA
-    // issuers) is deferred until the TMEM loads of the NEXT unit have been issued, so that their latency runs under it.
-    // (Only with eight worker warps and the column sums:
-    // sixteen warps do better handing dS over at once (5-6 % against eight that defer, more against sixteen that defer),
-    // and so do eight without the group barrier in the middle of a head (4.6 %) -- all measured.)
     constexpr bool kColSums = (kMode == 1 && !kOutDelta);     // the workers sum P dP over the keys themselves
-    constexpr bool kDeferTail = kColSums && (CG == 32) && (D == 64);
     float2 dc[H2];
 #pragma unroll
     for (int x = 0; x < H2; ++x) dc[x] = make_float2(0.f, 0.f);
@@ -780,8 +724,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column)
       if (thc >= 2 && !c.wait_w(qPtFree + (thc & 1), (thc >> 1) - 1)) return false;
       const uint32_t pt = c.tmem + Cfg::tPT + 32 * (thc & 1) + col0 / 2;
-      if (CG == 32) tmem_st16(pt + lane_base, pk);
-      else tmem_st8(pt + lane_base, pk);
+      tmem_st8(pt + lane_base, pk);
       tc_wait_st();
       fence_proxy_async();
       tc_fence_before();
@@ -792,7 +735,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       const int b = u % Cfg::kNB, sl = hc % Cfg::kNS;
       float* tabL = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512);      // lse[64] of the head's rows (raw)
       float* tabC = tabL + 64;                                                         // g_denom[64] (or delta[64])
-      if (!kDeferTail && !flush_tail()) return;
+      if (!flush_tail()) return;
       if (!c.wait_w(qInFull + sl, hc / Cfg::kNS)) return;                              // (the tables landed with the tiles)
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
       UQ(1)
@@ -800,9 +743,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       float2 pv[H2], dp[H2];
       {
         uint32_t sr[CG], dr[CG];
-        tmem_ld_n<CG>(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, sr);
-        tmem_ld_n<CG>(c.tmem + (b ? Cfg::tP1 : Cfg::tP0) + lane_base + col0, dr);
-        if (kDeferTail && !flush_tail()) return;                     // the previous head's tail, under the loads
+        tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, sr);
+        tmem_ld16(c.tmem + (b ? Cfg::tP1 : Cfg::tP0) + lane_base + col0, dr);
         UQ(6)
         float2 nl[H2];
         load_pairs(tabL + col0, nl);                                 // lse of the rows
@@ -829,7 +771,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           e[2 * x] = ev.x;
           e[2 * x + 1] = ev.y;
         }
-        const float part = warp_colsum<CG>(e, scr, lane);            // this warp's 32 keys, column col0 + lane % CG
+        const float part = warp_colsum(e, lane);            // this warp's 32 keys, column col0 + lane % CG
         if (kMode == 4) {
           const size_t out_chunk = (size_t)c.bh * (N / p.m) + c.i / p.m;
           if (helper) atomicAdd(p.row_term + (out_chunk * p.s.R + r) * p.Lr + c.srow0_of(ht) + col0 + lane, -part);
@@ -861,7 +803,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       tail_hc = hc;
       UQ(5)
     }
-    if (!kDeferTail && !flush_tail()) return;
+    if (!flush_tail()) return;
 
     // ================= decay gradient =================
     if (kMode == 4) {
@@ -875,7 +817,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       continue;
     }
     {
-      if (kDeferTail && !flush_tail()) return;     // the last head's tail
       const bool more = ht + 1 < c.nht;
       float run = 0.f;
 #pragma unroll
@@ -910,7 +851,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       UQ(9)
       tc_fence_after();
       uint32_t gr[CG];
-      tmem_ld_n<CG>(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
+      tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
       float2 t3p[H2];
       load_pairs(t3v, t3p);
       tc_wait_ld();
@@ -1034,7 +975,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   }
 }
 
-template <int D, int kC, typename TG, int kMode, int CG, bool kHeads, bool kOutDelta = false>
+template <int D, int kC, typename TG, int kMode, bool kHeads, bool kOutDelta = false>
 __global__ void __launch_bounds__(32 * (8 + 4 * (64 / CG)), 1)
 bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
             const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
@@ -1042,7 +983,6 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
             const __grid_constant__ CUtensorMap tmO, Bwd2Params p) {
   static_assert(!kOutDelta || (Bwd2Cfg<D>::kOutTiles && kMode == 1 && kHeads), "output-tile builds: head_dim 64, per-chunk form");
   using Cfg = Bwd2Cfg<D>;
-  constexpr int NG = 64 / CG;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);      // [0] TMEM base, [1] abort flag, [2] failure note
@@ -1114,7 +1054,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   constexpr int kThreads = 32 * (8 + 4 * NG);
   constexpr int kLaunchRegs = (65536 / kThreads) / 8 * 8;
   // (sixteen worker warps: 80 registers at launch; the tighter split leaves them 96 instead of 88, measured 2.5 % faster)
-  constexpr int kRoleRegs = (CG == 16) ? 40 : 48, kDrainRegs = (CG == 16) ? 56 : 64;
+  constexpr int kRoleRegs = 40, kDrainRegs = 56;
   constexpr int kWorkerRegs = kLaunchRegs + ((2 * kLaunchRegs - kRoleRegs - kDrainRegs) * 128 / (128 * NG)) / 8 * 8;
   static_assert(kRoleRegs <= kLaunchRegs && kDrainRegs <= kLaunchRegs, "setmaxnreg.dec must not ask for more");
   static_assert(128 * (kRoleRegs + kDrainRegs) + 128 * NG * kWorkerRegs <= kThreads * kLaunchRegs, "register pool");
@@ -1125,9 +1065,9 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     if (lane == 0) {
       if (warp == 0) bwd2_front<D, kMode>(c, p);
       else if (kMode == 4 && warp != 2) {}      // (the row-term pass has nothing for the back issuers and the drain warps)
-      else if (warp == 1) bwd2_back<D, kC, CG>(c, p, 0);
+      else if (warp == 1) bwd2_back<D, kC>(c, p, 0);
       else if (warp == 2) bwd2_producer<D, kC, TG, kMode, kOutDelta>(c, p, &tmK, &tmV, &tmQ, &tmG, &tmO);
-      else bwd2_back<D, kC, CG>(c, p, 1);
+      else bwd2_back<D, kC>(c, p, 1);
     }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
@@ -1136,7 +1076,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     else if (kOutDelta) bwd2_rowdots<D>(c, p);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
-    bwd2_worker<D, kC, TG, kMode, CG, kHeads, kOutDelta>(c, p);
+    bwd2_worker<D, kC, TG, kMode, kHeads, kOutDelta>(c, p);
   }
 
   tc_fence_before();
