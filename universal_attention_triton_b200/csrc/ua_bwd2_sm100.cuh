@@ -100,8 +100,10 @@ template <int D>
 struct Bwd2Cfg {
   static constexpr int kNB = (D == 64) ? 2 : 1;            // (S, dP) buffers in TMEM
   static constexpr int kNS = (D == 64) ? 4 : 2;            // (Q, dO) slots
-  static constexpr int kKj = (D == 64) ? 2 : 1;            // K_j slots
-  static constexpr int kDs = (D == 64) ? 2 : 1;            // dS buffers
+  // K_j slots.  Two at head_dim 128 as well, at the price of one staging tile instead of two: with one slot every half tile began with the
+  // wait for K_j, 3200 of 11600 cycles with one query head (B1 H16 R1 L4096 775 -> 668 us, B1 H8 R4 L4096 828 -> 734).
+  static constexpr int kKj = 2;
+  static constexpr int kRing = (D == 64) ? 3 : 2;          // buffers that dS of the heads and dG of the half tiles take in turn
   static constexpr int kHalf = 64 * D * 2;                 // [64][D] bf16
   static constexpr int kFull = 128 * D * 2;                // [128][D] bf16
   static constexpr int kBoxes = D / 64;
@@ -110,10 +112,9 @@ struct Bwd2Cfg {
   static constexpr int oKj = 2 * kFull;
   static constexpr int oSlot = oKj + kKj * kHalf;          // slot: Q half tile, then dO half tile
   static constexpr int kSlot = 2 * kHalf;
-  static constexpr int oDs = oSlot + kNS * kSlot;          // kDs x 16 KB [128 keys][64 rows] bf16, then dG, then the staging tile
-  static constexpr int oDg = oDs + kDs * 16384;
-  static constexpr int oStage = oDg + 16384;               // [64][D] fp32 as D/32 boxes of [64][32], 128-byte swizzle
-  static constexpr int oT3 = oStage + 256 * D;             // float [2][64]: static_dest^(1/3) of a half tile's rows
+  static constexpr int oDs = oSlot + kNS * kSlot;          // kRing x 16 KB [128 keys][64 rows] bf16, then the staging tile
+  static constexpr int oStage = oDs + kRing * 16384;               // [64][64] fp32 as two boxes of [64][32], 128-byte swizzle
+  static constexpr int oT3 = oStage + 16384;             // float [2][64]: static_dest^(1/3) of a half tile's rows
   // per-row tables that the producer copies next to the tiles (no global load is ever issued by a worker):
   static constexpr int oHeadTab = oT3 + 512;               // kNS x { float lse[64]; float cc[64] }: log-sum-exp and g_denom (or delta) of a head's rows
   static constexpr int kTab = 3;                           // half-tile tables in flight
@@ -121,7 +122,7 @@ struct Bwd2Cfg {
   static constexpr int oHtTab = oHeadTab + kNS * 512;
   static constexpr int oXch = oHtTab + kTab * kHtTab;      // float [8][128] totals crossing the column groups
   static constexpr int oBar = oXch + 4096;
-  static constexpr int oMisc = oBar + 320;      // (35 barriers of 8 bytes)
+  static constexpr int oMisc = oBar + 320;      // (36 barriers of 8 bytes)
   // builds that take the row term from the forward's output tiles (head_dim 64; 128 has no room for them): kNS output half tiles
   static constexpr bool kOutTiles = (D == 64);
   static constexpr int oOut = (oMisc + 256 + 1023) / 1024 * 1024;
@@ -144,11 +145,11 @@ enum Bwd2Bar {
   qKjFull = 1, qKjFree = 3,        // [2]
   qInFull = 5, qInFree = 9,        // [4]
   qSFull = 13, qLdDone = 15, qPtFree = 17,   // [2] per (S, dP) buffer / per probability buffer
-  qDsReady = 19, qDsFree = 21,     // [2] per dS buffer
-  qYFull = 23, qYFree = 24, qDgReady = 25, qDgFree = 26, qFinal = 27,
-  qTabFull = 28,                   // [3] per half-tile table buffer
-  qDelta = 31,                     // [4] per (Q, dO) slot: the row term of the head's table is final (output-tile builds)
-  qNumBars = 35
+  qDsReady = 19, qDsFree = 22,     // [3] per ring buffer
+  qYFull = 25, qYFree = 26, qTabDone = 27, qFinal = 28,      // (qTabDone: mode 4, where no product says that a half tile is over)
+  qTabFull = 29,                   // [3] per half-tile table buffer
+  qDelta = 32,                     // [4] per (Q, dO) slot: the row term of the head's table is final (output-tile builds)
+  qNumBars = 36
 };
 
 struct Bwd2Ctx {
@@ -251,7 +252,8 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
   const int Rh = p.heads;
   auto load_tables = [&](int ht) -> bool {
     const int tb = ht % Cfg::kTab, use = ht / Cfg::kTab;
-    if (use >= 1 && !c.wait(qDgReady, ht - Cfg::kTab)) return false;      // the half tile that used the buffer is done with it
+    // the half tile that used the buffer is done with it (but in mode 4: K_j's free slot, waited for before, says so already)
+    if (kMode == 4 && use >= 1 && !c.wait(qTabDone, ht - Cfg::kTab)) return false;
     const uint32_t dst = sb + Cfg::oHtTab + tb * Cfg::kHtTab;
     // (the correction pass has no heads and needs no decay prefix: only the gate values travel)
     mbar_expect_tx(c.bar(qTabFull + tb), (Rh > 0 ? 512u : 0u) + 64 * (uint32_t)sizeof(TG));
@@ -266,7 +268,6 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
   int hc = 0;
   for (int ht = 0; ht < c.nht; ++ht) {
     const int row0 = c.row0_of(ht), srow0 = c.srow0_of(ht);
-    if (ht + 1 < c.nht && !load_tables(ht + 1)) return;
     {
       const int sl = ht % Cfg::kKj, use = ht / Cfg::kKj;
       if (use >= 1 && !c.wait(qKjFree + sl, use - 1)) return;
@@ -275,6 +276,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
       for (int b = 0; b < Cfg::kBoxes; ++b)
         tma_load_2d(sb + Cfg::oKj + sl * Cfg::kHalf + b * 8192, tmK, b * 64, c.bh * L + row0, c.bar(qKjFull + sl));
     }
+    if (ht + 1 < c.nht && !load_tables(ht + 1)) return;
     for (int r = 0; r < Rh; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, use = hc / Cfg::kNS;
       if (use >= 1 && !c.wait(qInFree + sl, use - 1)) return;
@@ -304,7 +306,13 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
 
 // ----------------------------------------------------------- front MMA issuer --
 // G, S^T and dP^T: everything that only needs loaded tiles and a free (S, dP) buffer.
-template <int D, int kMode>
+// A wait costs each of the sixteen worker warps about a hundred cycles of its chain even where nothing is left to wait for, so all that a
+// worker needs for a unit (the tables of its rows, a free dS / dG buffer, a free probability buffer) is waited for here, by one thread,
+// and the workers wait for qSFull alone: the issuer arrives on it beside the commit, which hands on what it has seen.  (All but the
+// probability buffer at head_dim 64: waiting for that one here holds up the scores, and costs more than the workers' wait.)
+// B4 H8 R4 L4096 D64: 2015 -> 1745 us, B1 H16 R1 L4096 D128 806 -> 782; with the factors of the decay gradient formed ahead of the barrier
+// 1675 and 775.
+template <int D, int kMode, bool kOutDelta>
 __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p) {
   using Cfg = Bwd2Cfg<D>;
   const int R = p.heads;
@@ -324,12 +332,19 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
     if (uses == 0) return true;
     return c.wait(qLdDone + b, uses - 1);
   };
+  // (a head's or a half tile's gradient goes to ring buffer w % kRing, its last user's products are done)
+  int w = 0;
+  auto ring_free = [&]() -> bool {
+    const int at = w++;
+    return kMode == 4 || at < Cfg::kRing || c.wait(qDsFree + at % Cfg::kRing, at / Cfg::kRing - 1);
+  };
   auto unit_g = [&](int ht) -> bool {
     const int b = u % Cfg::kNB;
     if (!acquire(b)) return false;
     tc_fence_after();
     mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(sb + Cfg::oKj + (ht % Cfg::kKj) * Cfg::kHalf, 16));
     tc_commit(c.bar(qSFull + b));
+    mbar_arrive(c.bar(qSFull + b));
     UQ_TRACE(u, 0)
     ++u;
     return true;
@@ -340,14 +355,18 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
   UQ_DECL
   for (int ht = 0; ht < c.nht; ++ht) {
     if (!c.wait(qKjFull + ht % Cfg::kKj, ht / Cfg::kKj)) return;
+    // (the workers read the tables of the next half tile before this one is over)
+    if (kMode != 4 && R > 0 && ht + 1 < c.nht && !c.wait(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
     if (R > 0 && !unit_g(ht)) return;                               // G for the decay recomputation (none without heads)
     if (kMode == 4) tc_commit(c.bar(qKjFree + ht % Cfg::kKj));      // (no back issuers: the tiles are free once these products are done)
     UQ(0)
     for (int r = 0; r < R; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, b = u % Cfg::kNB;
       if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
+      if (kOutDelta && !c.wait(qDelta + sl, hc / Cfg::kNS)) return;
       UQ(1)
       if (!acquire(b)) return;
+      if (!ring_free()) return;
       UQ(2)
       UQ_TRACE(u, 4)
       tc_fence_after();
@@ -355,11 +374,12 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
       mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(slot, 16));                    // S^T  = K_i Q^T
       mma_kk(c.tmem + (b ? Cfg::tP1 : Cfg::tP0), kVi, desc_lo(slot + Cfg::kHalf, 16));       // dP^T = V_i dO^T
       tc_commit(c.bar(qSFull + b));
+      mbar_arrive(c.bar(qSFull + b));
       UQ_TRACE(u, 0)
       ++u;
       UQ(3)
     }
-    if (kMode != 4 && !unit_g(ht)) return;                          // G again for the decay gradient
+    if (kMode != 4 && !(ring_free() && unit_g(ht))) return;         // G again for the decay gradient
     UQ(0)
   }
   UQ_STORE_AT(16)
@@ -378,9 +398,8 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   constexpr uint32_t id_tn = idesc_bf16(128, 64, 1, 1);    // A MN-major, B MN-major
   const uint32_t DV = c.tmem + Cfg::tDV, DK = c.tmem + Cfg::tDK, Y = c.tmem + Cfg::tY;
   const uint64_t mKi = desc_from_lo(desc_lo(sb + Cfg::oKi, 16384));      // K_i as [K = keys][N = D] (MN-major, 64-wide groups 16 KB apart)
-  const uint64_t kdG = desc_from_lo(desc_lo(sb + Cfg::oDg, 16)), mdG = desc_from_lo(desc_lo(sb + Cfg::oDg, 16384));
   uint32_t have_dv = 0, have_dk = 0;
-  int yc = 0, hc = 0;
+  int yc = 0, hc = 0, w = 0;
   // Y[rows][D] = T^T K_i with T a [128 keys][64 rows] bf16 tile read MN-major; M = 128: lanes 64..127 come from the 16 KB
   // after the tile and are never read
   auto mma_rows_out = [&](uint64_t t_mn, int cb) {       // 64 columns of D: those of K_i's column group cb
@@ -391,11 +410,11 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   if (!c.wait(qKvFull, 0)) return;
   UQ_DECL
   for (int ht = 0; ht < c.nht; ++ht) {
-    for (int r = 0; r < R; ++r, ++hc) {
-      const int sl = hc % Cfg::kNS, db = hc % Cfg::kDs;
+    for (int r = 0; r < R; ++r, ++hc, ++w) {
+      const int sl = hc % Cfg::kNS, db = w % Cfg::kRing;
       const uint32_t dsb = sb + Cfg::oDs + db * 16384;
       UQ(0)
-      if (!c.wait(qDsReady + db, hc / Cfg::kDs)) return;
+      if (!c.wait(qDsReady + db, w / Cfg::kRing)) return;
       UQ(1)
       if (which == 0) {
         if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
@@ -426,7 +445,10 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
       }
     }
     UQ(0)
-    if (!c.wait(qDgReady, ht)) return;
+    const int gb = w % Cfg::kRing;
+    if (!c.wait(qDsReady + gb, w / Cfg::kRing)) return;
+    const uint64_t kdG = desc_from_lo(desc_lo(sb + Cfg::oDs + gb * 16384, 16)), mdG = desc_from_lo(desc_lo(sb + Cfg::oDs + gb * 16384, 16384));
+    ++w;
     UQ(3)
     if (which == 0) {
       tc_fence_after();
@@ -434,7 +456,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
       mma4_ss(DK, kdG, mKj, 2, 128, id_kn, have_dk);                                      // dK_i += dG K_j
       have_dk = 1;
       tc_commit(c.bar(qKjFree + ht % Cfg::kKj));
-      tc_commit(c.bar(qDgFree));
+      tc_commit(c.bar(qDsFree + gb));
     } else {
       for (int cb = 0; cb < D / 64; ++cb, ++yc) {
         if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
@@ -442,7 +464,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
         mma_rows_out(mdG, cb);                                                            // dK_j = dG^T K_i
         tc_commit(c.bar(qYFull));
       }
-      tc_commit(c.bar(qDgFree));
+      tc_commit(c.bar(qDsFree + gb));
     }
   }
   tc_commit(c.bar(qFinal));
@@ -481,7 +503,7 @@ __device__ __forceinline__ float warp_colsum(float* v, int lane) {
 
 // ----------------------------------------------------------------- drain warps --
 // Two warps (TMEM lanes 0..63 = the 64 result rows) take every row-side result out of Y, in sweep order: dQ_rj of each
-// head, then dK_j of the half tile.  The 64 x D fp32 tile is staged in shared memory as boxes of [64][32] floats and
+// head, then dK_j of the half tile.  The 64 x 64 fp32 tile is staged in shared memory as boxes of [64][32] floats and
 // leaves as TMA reduce-adds into the fp32 accumulators (other key chunks add to the same rows), which run behind the
 // next unit; the workers never touch it.
 //
@@ -501,13 +523,9 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
       const int r = z / (D / 64), cb = z % (D / 64);
       if (!c.wait_w(qYFull, yc)) return;
       tc_fence_after();
-      // the reduce-add that used this staging tile last has read it (head_dim 128 has two tiles: the one before may still be reading)
-      if (leader) {
-        if (D == 64) bulk_wait_read_all();
-        else bulk_wait_read_but_last();
-      }
+      if (leader) bulk_wait_read_all();                 // the reduce-add before has read the staging tile
       named_bar_sync(kBarDrain, 64);
-      uint8_t* stage = sStage + cb * 16384;
+      uint8_t* stage = sStage;
 #pragma unroll 1
       for (int hb = 0; hb < 2; ++hb) {
         uint32_t o[32];
@@ -641,7 +659,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     for (int q = 0; q < c.segment; ++q) suffix += p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + q) * 128 + key];
   named_bar_sync(kBarAll, kWorkers);
 
-  int u = 0, hc = 0;
+  int u = 0, hc = 0, w = 0;                       // units, heads, gradients handed over so far
   for (int ht = 0; ht < c.nht; ++ht) {
     const int rel = c.row0_of(ht) - c.i * kC;
     const bool diag = rel < kC;                    // rows at positions of the chunk's own keys
@@ -651,7 +669,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     // ================= decay recomputation: c2 = log2(e) * decay prefix of (key, CG rows) =================
     float2 c2[H2];
     if (kHeads) {                                  // (the correction pass has no heads: no prefix, no first G unit)
-      if (!c.wait_w(qTabFull + ht % Cfg::kTab, ht / Cfg::kTab)) return;
       const float carry = reinterpret_cast<const float*>(ht_table(ht))[key];
       const int b = u % Cfg::kNB;
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
@@ -675,7 +692,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           const float2 e23 = fmul2(lg, k23);
           const float2 pw = make_float2(ex2(e23.x), ex2(e23.y));
           const float2 a = fmul2(fmul2(pw, s32), t3p[x]);
-          const float2 om = fadd2(one2, make_float2(-fminf(a.x, clamp_hi()), -fminf(a.y, clamp_hi())));
+          const float2 om = ffma2(make_float2(fminf(a.x, clamp_hi()), fminf(a.y, clamp_hi())), make_float2(-1.0f, -1.0f), one2);
           float e0 = lg2(om.x), e1 = lg2(om.y);
           if (kDiag) {
             if (qbase + 2 * x <= key) e0 = 0.f;
@@ -713,30 +730,10 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     float2 dc[H2];
 #pragma unroll
     for (int x = 0; x < H2; ++x) dc[x] = make_float2(0.f, 0.f);
-    uint32_t pk[H2], dk[H2];                       // the pending tail: packed probabilities and dS of head tail_hc
-    int tail_hc = -1;
-    auto flush_tail = [&]() -> bool {
-      if (tail_hc < 0) return true;
-      const int thc = tail_hc, db = thc % Cfg::kDs;
-      tail_hc = -1;
-      if (thc >= Cfg::kDs && !c.wait_w(qDsFree + db, thc / Cfg::kDs - 1)) return false;
-      store_row(c.smem + Cfg::oDs + db * 16384, dk);
-      // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column)
-      if (thc >= 2 && !c.wait_w(qPtFree + (thc & 1), (thc >> 1) - 1)) return false;
-      const uint32_t pt = c.tmem + Cfg::tPT + 32 * (thc & 1) + col0 / 2;
-      tmem_st8(pt + lane_base, pk);
-      tc_wait_st();
-      fence_proxy_async();
-      tc_fence_before();
-      c.arrive_w(qDsReady + db);
-      return true;
-    };
     for (int r = 0; r < R; ++r, hc += (kMode == 4 ? 0 : 1)) {
       const int b = u % Cfg::kNB, sl = hc % Cfg::kNS;
       float* tabL = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512);      // lse[64] of the head's rows (raw)
       float* tabC = tabL + 64;                                                         // g_denom[64] (or delta[64])
-      if (!flush_tail()) return;
-      if (!c.wait_w(qInFull + sl, hc / Cfg::kNS)) return;                              // (the tables landed with the tiles)
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
       UQ(1)
       tc_fence_after();
@@ -781,14 +778,13 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         if (helper) atomicAdd(tabC + col0 + lane, -part);           // g_denom - sum_k P dP, in place
       }
       UQ(2)
-      if (kOutDelta) {
-        if (!c.wait_w(qDelta + sl, hc / Cfg::kNS)) return;
-      } else if (kColSums) {
+      if (kColSums) {
         named_bar_sync(kBarGroup + g, kC);           // the group's column sums are complete
       }
       UQ(4)
       {
         float2 cc[H2];
+        uint32_t pk[H2], dk[H2];
         load_pairs(tabC + col0, cc);
 #pragma unroll
         for (int x = 0; x < H2; ++x) {
@@ -799,11 +795,19 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           pk[x] = *reinterpret_cast<uint32_t*>(&hp);
           dk[x] = *reinterpret_cast<uint32_t*>(&hd);
         }
+        UQ(5)
+        store_row(c.smem + Cfg::oDs + w % Cfg::kRing * 16384, dk);
+        // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column).  With a ring of two, its free buffer says that the product with the
+        // probabilities of two heads ago is done as well; with three it does not.
+        if (Cfg::kRing > 2 && hc >= 2 && !c.wait_w(qPtFree + (hc & 1), (hc >> 1) - 1)) return;
+        tmem_st8(c.tmem + Cfg::tPT + 32 * (hc & 1) + col0 / 2 + lane_base, pk);
+        ++w;
+        tc_wait_st();
+        fence_proxy_async();
+        tc_fence_before();
+        c.arrive_w(qDsReady + (w - 1) % Cfg::kRing);
       }
-      tail_hc = hc;
-      UQ(5)
     }
-    if (!flush_tail()) return;
 
     // ================= decay gradient =================
     if (kMode == 4) {
@@ -812,7 +816,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         if (!c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
         if (helper) sT3[((ht + 1) & 1) * 64 + col0 + lane] = t3_from_table(ht + 1);
       }
-      c.arrive_w(qDgReady);
+      c.arrive_w(qTabDone);
       named_bar_sync(kBarAll, kWorkers);
       continue;
     }
@@ -828,24 +832,10 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       }
       sXch[(NG + g) * 128 + key] = run;
       if (more && quad == kGateQuad) {                   // static_dest^(1/3) of the next half tile's rows
-        if (!c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
+        if (!kHeads && !c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
         if (helper) sT3[((ht + 1) & 1) * 64 + col0 + lane] = t3_from_table(ht + 1);
       }
       UQ(7)
-      named_bar_sync(kBarAll, kWorkers);
-      UQ(8)
-      float later = 0.f, others = 0.f;             // totals of the groups to the right / of all other groups
-#pragma unroll
-      for (int q = 0; q < NG; ++q) {
-        if (q == g) continue;
-        const float v = sXch[(NG + q) * 128 + key];
-        others += v;
-        if (q > g) later += v;
-      }
-      const float add = suffix + later;            // rows after this thread's block
-      suffix = suffix + run + others;              // ... after this half tile (the next one lies below it)
-      const float2 add2 = make_float2(add, add);
-
       const int b = u % Cfg::kNB;
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
       UQ(9)
@@ -858,12 +848,45 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       tc_fence_before();
       c.arrive_w(qLdDone + b);
       ++u;
+      // The decay gradient is linear in dell = (sum of dC over the later rows): what does not depend on it is formed first, while
+      // the other groups' totals are on their way.
+      //   f1 = t^(1/3) g^(2/3) / (clamp(a) - 1)        d static_src += dell f1
+      //   f2 = t^(1/3) g^(-1/3) / (clamp(a) - 1)       dG = dell s^(1/3) (2/3) f2
+      // both zero above the clamp (it passes no gradient there) and for g <= 0; one exponential serves both powers, g^(2/3) = g g^(-1/3)
+      float2 f1[H2], f2[H2];
+      {
+        const float2 km13 = make_float2(-1.0f / 3.0f, -1.0f / 3.0f), mone2 = make_float2(-1.0f, -1.0f);
+#pragma unroll
+        for (int x = 0; x < H2; ++x) {
+          const float g0 = __uint_as_float(gr[2 * x]), g1 = __uint_as_float(gr[2 * x + 1]);
+          const float2 e13 = fmul2(make_float2(lg2(g0), lg2(g1)), km13);
+          const float2 r13 = make_float2(g0 > 0.f ? ex2(e13.x) : 0.f, g1 > 0.f ? ex2(e13.y) : 0.f);
+          const float2 pw = fmul2(make_float2(g0, g1), r13);
+          const float2 a = fmul2(fmul2(pw, s32), t3p[x]);
+          const float2 am = fadd2(make_float2(fmaxf(a.x, clamp_lo_bwd()), fmaxf(a.y, clamp_lo_bwd())), mone2);
+          const float2 iv = make_float2(a.x <= clamp_hi() ? rcp_approx(am.x) : 0.f, a.y <= clamp_hi() ? rcp_approx(am.y) : 0.f);
+          const float2 ivt = fmul2(iv, t3p[x]);
+          f1[x] = fmul2(ivt, pw);
+          f2[x] = fmul2(ivt, r13);
+        }
+      }
+      named_bar_sync(kBarAll, kWorkers);
+      UQ(8)
+      float later = 0.f, others = 0.f;             // totals of the groups to the right / of all other groups
+#pragma unroll
+      for (int q = 0; q < NG; ++q) {
+        if (q == g) continue;
+        const float v = sXch[(NG + q) * 128 + key];
+        others += v;
+        if (q > g) later += v;
+      }
+      const float add = suffix + later;            // rows after this thread's block
+      suffix = suffix + run + others;              // ... after this half tile (the next one lies below it)
+      const float2 add2 = make_float2(add, add), s32k = fmul2(s32, make_float2(2.0f / 3.0f, 2.0f / 3.0f));
       uint32_t pk[H2];
       float2 dsa = make_float2(0.f, 0.f);
       auto decay_grad = [&](auto on_diag) {
         constexpr bool kDiag = decltype(on_diag)::value;
-        const float2 k23 = make_float2(2.0f / 3.0f, 2.0f / 3.0f), km13 = make_float2(-1.0f / 3.0f, -1.0f / 3.0f);
-        const float2 mone2 = make_float2(-1.0f, -1.0f), s32k = fmul2(s32, k23);
 #pragma unroll
         for (int x = 0; x < H2; ++x) {
           float2 dl = fadd2(dc[x], add2);
@@ -871,27 +894,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
             if (qbase + 2 * x <= key) dl.x = 0.f;
             if (qbase + 2 * x + 1 <= key) dl.y = 0.f;
           }
-          const float g0 = __uint_as_float(gr[2 * x]), g1 = __uint_as_float(gr[2 * x + 1]);
-          const float2 lg = make_float2(lg2(fmaxf(g0, 0.f)), lg2(fmaxf(g1, 0.f)));      // -inf for g <= 0: pw = 0
-          // g^(2/3) = g * g^(-1/3): one exponential serves both powers (relu: zero for g <= 0, where lg = -inf)
-          const float2 e13 = fmul2(lg, km13);
-          const float2 r13 = make_float2(ex2(e13.x), ex2(e13.y));
-          float2 pw = fmul2(make_float2(g0, g1), r13);
-          if (!(g0 > 0.f)) pw.x = 0.f;
-          if (!(g1 > 0.f)) pw.y = 0.f;
-          const float2 st = fmul2(pw, s32);
-          const float2 a = fmul2(st, t3p[x]);
-          const float2 am = fadd2(make_float2(fminf(fmaxf(a.x, clamp_lo_bwd()), clamp_hi()), fminf(fmaxf(a.y, clamp_lo_bwd()), clamp_hi())), mone2);
-          // d affinity = d ell / (clamp(a) - 1), zero above the clamp (the clamp passes no gradient there)
-          float2 da = fmul2(dl, make_float2(rcp_approx(am.x), rcp_approx(am.y)));
-          if (!(a.x <= clamp_hi())) da.x = 0.f;
-          if (!(a.y <= clamp_hi())) da.y = 0.f;
-          const float2 dstat = fmul2(da, pw);
-          dsa = ffma2(dstat, t3p[x], dsa);
-          // dG = dA s^(1/3) t^(1/3) (2/3) g^(-1/3) for g > 0
-          float2 dg = fmul2(fmul2(da, t3p[x]), fmul2(s32k, r13));
-          if (!(g0 > 0.f)) dg.x = 0.f;
-          if (!(g1 > 0.f)) dg.y = 0.f;
+          dsa = ffma2(dl, f1[x], dsa);
+          const float2 dg = fmul2(fmul2(dl, s32k), f2[x]);
           __nv_bfloat162 h = __floats2bfloat162_rn(dg.x, dg.y);
           pk[x] = *reinterpret_cast<uint32_t*>(&h);
         }
@@ -899,11 +903,11 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       if (diag) decay_grad(std::true_type{});
       else decay_grad(std::false_type{});
       ds_acc += dsa.x + dsa.y;
-      if (ht >= 1 && !c.wait_w(qDgFree, ht - 1)) return;
-      store_row(c.smem + Cfg::oDg, pk);
+      const int db = w++ % Cfg::kRing;
+      store_row(c.smem + Cfg::oDs + db * 16384, pk);
       // (d static_dest needs no sum over the keys here: it is taken from dK_j afterwards, see row_side_finish_kernel)
       fence_proxy_async();
-      c.arrive_w(qDgReady);
+      c.arrive_w(qDsReady + db);
       UQ(10)
     }
   }
@@ -1026,10 +1030,10 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     misc[2] = 0;
     for (int b = 0; b < qNumBars; ++b) {
       uint32_t count = 1;
-      if (b == qLdDone || b == qLdDone + 1 || b == qDsReady || b == qDsReady + 1 || b == qDgReady) count = kC / 32 * NG;   // one arrival per worker warp
+      if (b == qLdDone || b == qLdDone + 1 || (b >= qDsReady && b < qDsReady + 3) || b == qTabDone) count = kC / 32 * NG;   // one arrival per worker warp
       if (kMode == 4 && b >= qInFree && b < qInFree + 4) count = kC / 32 * NG;
       if (b == qYFree || (b >= qDelta && b < qDelta + 4)) count = 2;                                                                                  // the two draining warps
-      if (b == qDsFree || b == qDsFree + 1 || b == qDgFree || b == qFinal) count = 2;                               // both back issuers
+      if ((b >= qDsFree && b < qDsFree + 3) || b == qFinal || b == qSFull || b == qSFull + 1) count = 2;      // both back issuers; commit and front issuer
       mbar_init(c.bar(b), count);
     }
     mbar_init_fence();
@@ -1063,7 +1067,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
     if (lane == 0) {
-      if (warp == 0) bwd2_front<D, kMode>(c, p);
+      if (warp == 0) bwd2_front<D, kMode, kOutDelta>(c, p);
       else if (kMode == 4 && warp != 2) {}      // (the row-term pass has nothing for the back issuers and the drain warps)
       else if (warp == 1) bwd2_back<D, kC>(c, p, 0);
       else if (warp == 2) bwd2_producer<D, kC, TG, kMode, kOutDelta>(c, p, &tmK, &tmV, &tmQ, &tmG, &tmO);

@@ -66,7 +66,7 @@ inline SplitPlan make_split_plan(const Shape& s) {
     }
   }
   {
-    const double start = 12.0, cost = narrow * (s.D == 64 ? 3.4 + 1.1 * R : 4.2 + 2.2 * R), corr_start = 6.0, corr = narrow * (s.D == 64 ? 2.2 : 2.6);
+    const double start = 12.0, cost = narrow * (s.D == 64 ? 3.3 + 0.9 * R : 3.4 + 1.9 * R), corr_start = 6.0, corr = narrow * (s.D == 64 ? 2.2 : 2.6);
     auto len = [&](int i) { return sweep_halves(s, i); };
     double best = 0.95 * play(s, len, 0, 0, start, cost);
     for (int t = 2; t < len(0); t *= 2) {
