@@ -88,11 +88,26 @@ def test_scratch_plan_routes_wide_chunks_to_the_tensor_core_kernels(lib):
         assert lib.ua_carry_bytes(ctypes.byref(dims), 1, 0) == b * h * (n * m) ** 2 * 256 * 4
         sub_out = b * h * n * m * r * L * d * 2
         assert lib.ua_fwd_workspace_bytes(ctypes.byref(dims), 1, 0) >= 256 + sub_out
-        assert lib.ua_bwd_workspace_bytes(ctypes.byref(dims), 1, 0) >= 2 * sub_out
+        assert lib.ua_bwd_workspace_bytes(ctypes.byref(dims), 1, 0) > 256      # (what it holds: the next test)
         # fp32, forced generic kernels, other head dims: no sub-chunk plan
         assert lib.ua_carry_bytes(ctypes.byref(dims), 0, 0) == 0
         assert lib.ua_carry_bytes(ctypes.byref(dims), 1, 4) == 0 and lib.ua_fwd_workspace_bytes(ctypes.byref(dims), 1, 4) == 256
     assert lib.ua_fwd_workspace_bytes(ctypes.byref(UaDims(b, h, r, n, 256, 32)), 1, 0) == 256
+
+
+@pytest.mark.parametrize("n,c,d", [(8, 256, 128), (32, 256, 128), (64, 256, 128), (16, 384, 64)])
+def test_backward_scratch_of_wide_chunks_holds_what_the_kernels_use(lib, n, c, d):
+    """The backward of chunks of m * 128 keys keeps no sub-chunk outputs (its row term is a table), so its scratch is accumulators,
+    tables and per-chunk constants: a fraction of the two (b,h,n*m,r,L,d) tensors, which at long sequences would decide what fits."""
+    b, h, r, m = 1, 8, 4, c // 128
+    L, units, blocks = n * c, b * h, b * h * n * m
+    rows = b * h * n * r * L
+    most = (units * L * d * (3 + r) + 2 * units * L) * 4                    # dK, row-side dK, dV, dQ and the gates, fp32
+    most += blocks * (L // 64) * 128 * 4 + (2 + m) * rows * 4               # decay prefixes, log-sum-exps (whole and per block), row term
+    # per-chunk constants, or the totals of a cut sweep's segments (two half tiles at the least), and the parts' rounding to 256 bytes
+    most += blocks * (d + 3) * d * 4 + blocks * (max(d * d * 2, L // 128 * 128 * 4) + d * 2) + 16 * 256
+    have = lib.ua_bwd_workspace_bytes(ctypes.byref(UaDims(b, h, r, n, c, d)), 1, 0)
+    assert most / 2 < have <= most, (have, most)
 
 
 def test_cpu_tensors_are_rejected():

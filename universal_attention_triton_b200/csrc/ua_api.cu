@@ -138,10 +138,7 @@ BwdWorkspaceTc bwd_layout_tc(const ua::Shape& s, int m) {
   o = align_up(o + std::max(BH * s.N * (size_t)s.D * s.D * 2, BH * s.N * (size_t)ua::sm100::bwd_max_segments(s, seg) * 128 * f), 256);
   w.off_ksum = o; o = align_up(o + BH * s.N * (size_t)s.D * 2, 256);
   w.off_nacc = o; o = align_up(o + BH * s.N * (size_t)(s.D + 3) * s.D * f, 256);
-  if (m > 1) {
-    w.off_lse_sub = o; o = align_up(o + m * rows * f, 256);
-    o = std::max(o, align_up(2 * m * rows * s.D * 2, 256));      // (never less than the two sub-chunk tensors that callers have planned for)
-  }
+  if (m > 1) { w.off_lse_sub = o; o = align_up(o + m * rows * f, 256); }
   w.total = o;
   return w;
 }
