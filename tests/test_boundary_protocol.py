@@ -210,3 +210,18 @@ def test_own_output_is_saved_for_backward_unless_switched_off():
         ua.set_save_output(True)
     for a, b_, name in zip(results[True], results[False], ("dkc", "dvc", "dxq", "dsrc", "ddest")):
         assert torch.isfinite(a).all() and rel_fro(a, b_) <= 2e-2, (name, rel_fro(a, b_))
+
+
+@pytest.mark.gpu
+def test_error_of_a_backward_reaches_the_caller_with_its_type():
+    """A call that the library refuses on the host (here: an upstream gradient off its 16-byte boundary) raises UaLibraryError from
+    the engine's thread too, with the library's message."""
+    from oracle import ua_oracle as O
+    from universal_attention_triton_b200 import ops
+    from universal_attention_triton_b200._lib import UaLibraryError
+    ua1 = _classes()[0]
+    xs = [t.cuda().requires_grad_() for t in O.make_inputs(1, 1, 1, 256, 128, 64, dtype=torch.bfloat16, seed=3)]
+    out, denom = ua1.apply(*xs)
+    shifted = torch.zeros(out.numel() + 1, dtype=out.dtype, device="cuda")[1:].view(1, 1, 2, 1, 256, 64)
+    with pytest.raises(UaLibraryError, match="ua_bwd failed"):
+        torch.autograd.grad([out, denom], xs, [ops.as_reference_out(shifted), torch.zeros_like(denom)])

@@ -4,6 +4,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -350,13 +351,17 @@ template <typename N, typename... Ts> std::shared_ptr<N> make_node(const Ts&... 
   n->set_next_edges(torch::autograd::collect_next_edges(ts...));
   return n;
 }
-// errors of the calls above are Python exceptions: the engine's threads hold no interpreter lock when they run a node
+// Errors of the calls above are Python exceptions, and the engine's threads hold no interpreter lock when they run a node: they go
+// on as the engine's own exception type, which keeps the Python error whole (type, message, traceback) on its way to the caller.
 template <typename F> auto with_python(F f) {
   try {
     return f();
   } catch (py::error_already_set& e) {
     const py::gil_scoped_acquire gil;
-    throw std::runtime_error(e.what());
+    e.restore();
+    python_error err;
+    err.persist();
+    throw err;
   }
 }
 
