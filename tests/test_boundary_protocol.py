@@ -95,6 +95,57 @@ def test_cpu_tensors_are_refused_not_computed():
         ua1.apply(*args)
 
 
+def _cpu_args():
+    b, h, r, n, c, d = 1, 1, 1, 2, 16, 8
+    return (torch.randn(b, h, n, c, d), torch.randn(b, h, n, c, d), torch.randn(b, h, r, n * c, d),
+            torch.rand(b, h, n, c), torch.rand(b, h, n * c))
+
+
+def test_a_subclass_runs_its_own_forward_and_backward():
+    """``apply`` of a subclass takes the Function protocol, with whatever the subclass overrides (host logic, no GPU)."""
+    for base in _classes()[:3]:
+        class Mine(base):
+            @staticmethod
+            def forward(kc, vc, xq, static_src, static_dest):
+                return kc.sum() + 0, vc * 3
+
+            @staticmethod
+            def setup_context(ctx, inputs, outputs):
+                ctx.save_for_backward(*inputs)
+
+            @staticmethod
+            def backward(ctx, g_out, g_denom):
+                kc = ctx.saved_tensors[0]
+                return g_out * torch.ones_like(kc), g_denom * 3, None, None, None
+
+        args = _cpu_args()
+        kc, vc = args[0].requires_grad_(), args[1].requires_grad_()
+        out, denom = Mine.apply(*args)
+        assert torch.equal(denom, vc * 3) and out.shape == ()
+        gk, gv = torch.autograd.grad([out, denom], [kc, vc], [torch.tensor(2.0), torch.ones_like(vc)])
+        assert torch.equal(gk, torch.full_like(kc, 2.0)) and torch.equal(gv, torch.full_like(vc, 3.0))
+
+    class Last(_classes()[3]):
+        @staticmethod
+        def forward(mat, vec):
+            return mat[..., -1] * 1.0
+    assert Last.apply(torch.randn(1, 1, 1, 4, 2, 3), torch.randn(1, 1, 1, 4, 3)).shape == (1, 1, 1, 4, 2)
+
+
+def test_forward_mode_is_refused_not_dropped(monkeypatch):
+    """The Functions have no forward-mode formula: a dual input raises in eager mode too (a native node would return results
+    without a tangent); a forward-mode level without dual inputs changes nothing."""
+    import torch.autograd.forward_ad as fwad
+    from universal_attention_triton_b200 import universal_attention_autograd as M
+    monkeypatch.setattr(M, "_forward", lambda kc, vc, xq, ss, sd: (kc * 1.0, vc * 1.0))
+    ua1 = _classes()[0]
+    args = _cpu_args()
+    with fwad.dual_level():
+        assert torch.equal(ua1.apply(*args)[0], args[0])
+        with pytest.raises(RuntimeError, match="forward AD|jvp"):
+            ua1.apply(fwad.make_dual(args[0], torch.ones_like(args[0])), *args[1:])
+
+
 def test_shape_asserts_fire_like_the_reference():
     ua1, ua2, kua, _ = _classes()
     b, h, r, n, c, d = 1, 1, 1, 2, 16, 8

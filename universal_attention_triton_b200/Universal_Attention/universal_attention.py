@@ -24,7 +24,7 @@ class UniversalAttention(Function):
 
     @classmethod
     def apply(cls, kc, vc, xq, static_src, static_dest):
-        if _ua._transforms_active():
+        if not _ua._native_route(cls, UniversalAttention):
             return super().apply(kc, vc, xq, static_src, static_dest)
         cls._check(kc, vc, xq, static_src, static_dest)
         return _ua._apply(kc, vc, xq, static_src, static_dest)

@@ -5,10 +5,10 @@ keys and passes the gates through a sigmoid (``Universal_Attention/triton/_debug
 all of it in ``ua_prepare_inputs`` and is differentiable (``ua_prepare_inputs_bwd``)."""
 from __future__ import annotations
 
-import torch
 from torch.autograd import Function
 
 from . import _lib
+from .universal_attention_autograd import _transforms_active
 
 
 class _PrepareInputs(Function):
@@ -36,5 +36,5 @@ def prepare_inputs(query_state, key_state, value_state, gate_state, chunk=128, n
     ``static_dest (b,n_kv,s)``.  ``normalize_keys``: keys divided by ``|k| + 1e-6``; ``sigmoid_gates``: gates =
     sigmoid(gate_state).  Differentiable with respect to the four projections."""
     flags = (_lib.PREP_NORMALIZE_KEYS if normalize_keys else 0) | (_lib.PREP_SIGMOID_GATES if sigmoid_gates else 0)
-    apply = _PrepareInputs.apply if torch._C._are_functorch_transforms_active() else _lib.native().prepare_apply
+    apply = _PrepareInputs.apply if _transforms_active() else _lib.native().prepare_apply
     return apply(query_state, key_state, value_state, gate_state, chunk, flags)

@@ -24,7 +24,7 @@ tensors: there is no CPU or PyTorch fallback.
 from __future__ import annotations
 
 import torch
-from torch.autograd import Function
+from torch.autograd import Function, forward_ad
 
 from . import _lib, ops
 
@@ -144,12 +144,21 @@ def _default_merge_modes() -> bool:
     return _MERGED_BACKWARD == "composed" and _MERGED_FORWARD == "materialise"
 
 
-_transforms_active = torch._C._are_functorch_transforms_active
+def _transforms_active() -> bool:
+    """Whether a functorch transform or a forward-mode level is active: both see the Python Functions (which refuse what they do
+    not support, forward-mode for instance), never the native nodes, which would pass their tensors by."""
+    return torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+
+
+def _native_route(cls, own) -> bool:
+    """Whether ``cls.apply`` may run as a native node: a subclass may bring its own ``forward``, ``setup_context`` or ``backward``
+    and takes the Python protocol, as do functorch's transforms."""
+    return cls is own and not _transforms_active()
 
 
 def _apply(kc, vc, xq, static_src, static_dest):
-    """``apply`` of the operator's Functions in eager mode: the same forward, saved tensors and backward as a graph node in
-    native code (``csrc/ua_torch.cpp``); functorch's transforms take the Python protocol."""
+    """``apply`` of the operator's Functions in eager mode (``_native_route``): the same forward, saved tensors and backward as a graph node in
+    native code (``csrc/ua_torch.cpp``); everything else takes the Python protocol."""
     return _lib.native().ua_apply(kc, vc, xq, static_src, static_dest, _OUTPUT_LAYOUT == "reference", _SAVE_OUTPUT)
 
 
@@ -191,7 +200,7 @@ class UniversalAttention(Function):
 
     @classmethod
     def apply(cls, kc, vc, xq, static_src, static_dest):
-        if _transforms_active():
+        if not _native_route(cls, UniversalAttention):
             return super().apply(kc, vc, xq, static_src, static_dest)
         cls._check(kc, vc, xq, static_src, static_dest)
         return _apply(kc, vc, xq, static_src, static_dest)
@@ -226,7 +235,7 @@ class UniversalAttention2(Function):
 
     @classmethod
     def apply(cls, kc, vc, xq, static_src, static_dest):
-        if _transforms_active():
+        if not _native_route(cls, UniversalAttention2):
             return super().apply(kc, vc, xq, static_src, static_dest)
         cls._check(kc, vc, xq, static_src, static_dest)
         return _apply(kc, vc, xq, static_src, static_dest)
@@ -255,7 +264,7 @@ class SMVecMatMul(Function):
 
     @classmethod
     def apply(cls, mat, vec):
-        if _transforms_active():
+        if not _native_route(cls, SMVecMatMul):
             return super().apply(mat, vec)
         cls._check(mat, vec)
         return _lib.native().merge_apply(mat, vec)
@@ -297,7 +306,7 @@ class UniversalAttentionMerged(Function):
 
     @classmethod
     def apply(cls, kc, vc, xq, static_src, static_dest):
-        if _transforms_active() or not _default_merge_modes():
+        if not _native_route(cls, UniversalAttentionMerged) or not _default_merge_modes():
             return super().apply(kc, vc, xq, static_src, static_dest)
         cls._check(kc, vc, xq, static_src, static_dest)
         return _lib.native().merged_apply(kc, vc, xq, static_src, static_dest)
