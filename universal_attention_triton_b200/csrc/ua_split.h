@@ -3,13 +3,18 @@
 // One block per chunk lasts as long as the longest sweep, whatever the chip has idle; many short blocks pay their start-up each.
 // Both are reckoned here: the launch is played through on 148 SMs with a block time of start + cost * tiles, for whole sweeps and
 // for segments of 1, 2, 4 .. tiles, and the shortest wins (whole sweeps unless another is at least 5 % shorter).  The constants are
-// microseconds, fitted to forwards and backwards of 1 to 4 query heads at head_dim 64 and 128 on one to 64 (batch, head) units; of the
-// shapes measured, with every segment length tried, the choice is the best one or within 5 % of it.  A plan depends on the shape
-// alone and the last ones are kept per thread: a call asks for it several times.
+// microseconds, fitted to forwards and backwards of 1 to 4 query heads at head_dim 64 and 128 on one to 64 (batch, head) units (more heads:
+// the same straight line, not measured); of the shapes measured, with every segment length tried, the choice is the best one or
+// within 5 % of it.
+//
+// A program whose lengths change from call to call pays for a plan in each of them, so a plan has to cost a small part of a launch:
+// only the direction asked for is reckoned, the blocks of a chunk's units are alike and are dealt out to SMs that come free at the same time
+// in one step, and a segment length is not played where the longest block or the work per SM already rules it out.  The
+// slowest of forty lengths from L640 to L5632 (H8 R4 D128), both ways, on one host core: 5 us, where playing block by block took
+// 930.  A plan depends on the shape alone; the last ones are kept per thread, as a call asks for its own several times.
 #pragma once
 #include <algorithm>
-#include <functional>
-#include <vector>
+#include <limits>
 
 #include "ua_common.cuh"
 
@@ -23,72 +28,117 @@ inline int sweep_tiles(const Shape& s, int i) { return (s.L - i * s.C + 127) / 1
 // ... and 64-row half tiles, the backward's unit
 inline int sweep_halves(const Shape& s, int i) { return (s.L - i * s.C) / 64; }
 
-// End of the last block when every chunk i of every (batch, head) unit takes len(i) units in blocks of seg (0: all of them), launched
-// chunk by chunk; skip: blocks at the start of each chunk's list that have nothing to do.
-template <typename Len>
-double play(const Shape& s, Len len, int seg, int skip, double start, double cost) {
-  static thread_local std::vector<double> free_at;
-  free_at.assign(kSms, 0.0);                          // a heap, earliest first
-  double end = 0;
-  for (int i = 0; i < s.N; ++i) {
-    const int n = len(i), step = seg ? seg : n;
-    for (int t = skip * step; t < n; t += step) {
-      const double d = start + cost * std::min(step, n - t);
-      for (int bh = 0; bh < s.B * s.H; ++bh) {
-        std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
-        free_at.back() += d;
-        end = std::max(end, free_at.back());
-        std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
+// The SMs of the chip by the time at which they come free, earliest first; those that do so together are one entry.
+class FreeSms {
+ public:
+  // n blocks of length d, each to the SM that is free first; returns when the last of them ends
+  double run(long long n, double d) {
+    double end = 0;
+    while (n > 0) {
+      const double t = at_[0].time + d;
+      if (at_[0].sms <= n) {
+        n -= at_[0].sms;
+        put(t, take_first());
+      } else {
+        at_[0].sms -= (int)n;
+        put(t, (int)n);
+        n = 0;
       }
+      end = t;
     }
+    return end;
+  }
+
+ private:
+  struct Entry { double time; int sms; };
+  Entry at_[kSms + 1] = {{0.0, kSms}};      // (one entry more while a part of the first moves on)
+  int count_ = 1;
+  int take_first() {
+    const int sms = at_[0].sms;
+    std::copy(at_ + 1, at_ + count_--, at_);
+    return sms;
+  }
+  void put(double time, int sms) {
+    int x = count_;
+    while (x > 0 && at_[x - 1].time > time) --x;
+    if (x > 0 && at_[x - 1].time == time) {
+      at_[x - 1].sms += sms;
+      return;
+    }
+    std::copy_backward(at_ + x, at_ + count_, at_ + count_ + 1);
+    at_[x] = Entry{time, sms};
+    ++count_;
+  }
+};
+
+// End of the last block when every chunk i of every (batch, head) unit takes len(i) units in blocks of seg (0: all of them), launched
+// chunk by chunk; skip: blocks at the start of each chunk's list that have nothing to do.  Gives up, with a later time, once
+// the end is past `limit`.
+template <typename Len>
+double play(const Shape& s, Len len, int seg, int skip, double start, double cost, double limit) {
+  const long long BH = (long long)s.B * s.H;
+  double longest = 0, work = 0;
+  for (int i = 0; i < s.N; ++i) {
+    const int n = len(i), step = seg ? seg : n, left = n - std::min(n, skip * step);
+    if (left <= 0) continue;
+    longest = std::max(longest, start + cost * std::min(step, left));
+    work += (double)BH * (start * ((left + step - 1) / step) + cost * left);
+  }
+  const double least = std::max(longest, work / kSms);
+  if (least > limit) return least;
+  FreeSms sms;
+  double end = 0;
+  for (int i = 0; i < s.N && end <= limit; ++i) {
+    const int n = len(i), step = seg ? seg : n, left = n - std::min(n, skip * step);
+    if (left >= step) end = std::max(end, sms.run(BH * (left / step), start + cost * step));
+    if (left % step) end = std::max(end, sms.run(BH, start + cost * (left % step)));
   }
   return end;
 }
 
-struct SplitPlan {
-  Shape s;
-  int fwd, bwd;
-};
-inline SplitPlan make_split_plan(const Shape& s) {
-  SplitPlan p{s, 0, 0};
+// Row tiles per block of the forward (kBackward: half tiles per block of the backward); 0: a block sweeps its whole chunk.
+template <bool kBackward>
+int make_split(const Shape& s) {
   const double BH = (double)s.B * s.H, R = s.R, narrow = s.C == 64 ? 0.7 : 1.0;
   double tiles = 0;
   for (int i = 0; i < s.N; ++i) tiles += sweep_tiles(s, i);
   // enough work for every SM behind the longest sweep: nothing to gain, and nothing to play through
-  if (BH * tiles > 1.3 * kSms * sweep_tiles(s, 0) || BH * tiles > 8192) return p;
-  {
+  if (BH * tiles > 1.3 * kSms * sweep_tiles(s, 0) || BH * tiles > 8192) return 0;
+  int split = 0;
+  if (!kBackward) {
     const double start = 9.0, cost = narrow * (s.D == 64 ? 3.8 + 0.8 * R : 3.2 + 1.35 * R), totals = 3.0 + BH * tiles * (s.D == 64 ? 0.01 : 0.018);
     auto len = [&](int i) { return sweep_tiles(s, i); };
-    double best = 0.95 * play(s, len, 0, 0, start, cost);
+    double best = 0.95 * play(s, len, 0, 0, start, cost, std::numeric_limits<double>::infinity());
     for (int t = 1; t < len(0); t *= 2) {
-      const double est = totals + play(s, len, t, 0, start, cost);
-      if (est < best) { best = est; p.fwd = t; }
+      const double est = totals + play(s, len, t, 0, start, cost, best - totals);
+      if (est < best) { best = est; split = t; }
     }
-  }
-  {
+  } else {
     const double start = 12.0, cost = narrow * (s.D == 64 ? 3.3 + 0.9 * R : 3.4 + 1.9 * R), corr_start = 6.0, corr = narrow * (s.D == 64 ? 2.2 : 2.6);
     auto len = [&](int i) { return sweep_halves(s, i); };
-    double best = 0.95 * play(s, len, 0, 0, start, cost);
+    double best = 0.95 * play(s, len, 0, 0, start, cost, std::numeric_limits<double>::infinity());
     for (int t = 2; t < len(0); t *= 2) {
-      const double est = 2.0 + play(s, len, t, 0, start, cost) + play(s, len, t, 1, corr_start, corr);
-      if (est < best) { best = est; p.bwd = t; }
+      double est = 2.0 + play(s, len, t, 0, start, cost, best);
+      if (est < best) est += play(s, len, t, 1, corr_start, corr, best - est);
+      if (est < best) { best = est; split = t; }
     }
   }
-  return p;
+  return split;
 }
-inline const SplitPlan& split_plan(const Shape& s) {
-  static thread_local SplitPlan kept[16] = {};
+template <bool kBackward>
+int split_of(const Shape& s) {
+  struct Kept { Shape s; int split; };
+  static thread_local Kept kept[16] = {};
   static thread_local int next = 0;
-  for (const SplitPlan& p : kept)
-    if (p.s.B == s.B && p.s.H == s.H && p.s.R == s.R && p.s.N == s.N && p.s.C == s.C && p.s.D == s.D) return p;
-  kept[next] = make_split_plan(s);
-  const SplitPlan& p = kept[next];
+  for (const Kept& k : kept)
+    if (k.s.B == s.B && k.s.H == s.H && k.s.R == s.R && k.s.N == s.N && k.s.C == s.C && k.s.D == s.D) return k.split;
+  const int split = make_split<kBackward>(s);
+  kept[next] = Kept{s, split};
   next = (next + 1) % 16;
-  return p;
+  return split;
 }
-// row tiles per block of the forward, half tiles per block of the backward; 0: a block sweeps its whole chunk
-inline int fwd_split(const Shape& s) { return split_plan(s).fwd; }
-inline int bwd_split(const Shape& s) { return split_plan(s).bwd; }
+inline int fwd_split(const Shape& s) { return split_of<false>(s); }
+inline int bwd_split(const Shape& s) { return split_of<true>(s); }
 
 inline size_t fwd_totals_bytes(const Shape& s) { return (size_t)s.B * s.H * s.N * sweep_tiles(s, 0) * 128 * sizeof(float); }
 inline int bwd_max_segments(const Shape& s, int seg) { return seg ? (s.L / 64 + seg - 1) / seg : 0; }
