@@ -21,9 +21,6 @@ SOURCES = ["ua_bwd.cu", "ua_fwd.cu", "ua_tiled.cu", "ua_api.cu"]      # compiled
 # the tensor plumbing above the library: an extension module, host code only
 TORCH_SOURCE = "ua_torch.cpp"
 TORCH_PATH = os.path.join(PKG_DIR, "_ua_torch.so")
-# developer micro-benchmark (stand-alone executable, not loaded by the package): `--tools` builds it next to the library
-TOOL_SOURCE = "mma_timing.cu"
-TOOL_PATH = os.path.join(PKG_DIR, "mma_timing.bin")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
@@ -85,15 +82,5 @@ def _build_torch_module() -> None:
     _run(cmd)
 
 
-def build_tools() -> str:
-    """Compile the stand-alone MMA timing micro-benchmark (run it on a B200: ``./mma_timing.bin 256``)."""
-    cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--expt-relaxed-constexpr",
-           os.path.join(CSRC, TOOL_SOURCE), "-o", TOOL_PATH, "-lcuda"]
-    _run(cmd)
-    return TOOL_PATH
-
-
 if __name__ == "__main__":
     print(build(force=True, verbose="--verbose" in sys.argv))
-    if "--tools" in sys.argv:
-        print(build_tools())

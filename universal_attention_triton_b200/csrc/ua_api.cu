@@ -5,7 +5,6 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
-#include <cstdlib>
 #include <mutex>
 
 #include <algorithm>
@@ -737,7 +736,7 @@ int ua_bwd_rows_kept(const UaDims* dims, int dtype, int gate_dtype, const UaRows
   ua::sm100::Bwd2Params qp{};
   qp.s = s; qp.ssrc = static_src; qp.sdest = static_dest_rows; qp.g_denom = gd32; qp.lse = lse_rows; qp.carry = carry_tab;
   qp.acc_dk = dk_f32; qp.acc_dq = dxq_rows_f32; qp.acc_dt = ddest_rows_f32; qp.dv_chunk = nullptr;
-  qp.dvc = nullptr; qp.dss = nullptr; qp.status = status; qp.trace = nullptr;
+  qp.dvc = nullptr; qp.dss = nullptr; qp.status = status;
   qp.j_begin = rows->tile_begin; qp.j_end = rows->tile_end; qp.Lr = rows->rows_total; qp.r0 = rows->row_offset;
   qp.heads = s.R; qp.suffix_in = suffix_in; qp.dctot_out = dctot_out; qp.acc_dv = dv_f32; qp.acc_ds = dsrc_f32;
   qp.acc_dkr = acc_dkr; qp.m = 1;
@@ -763,7 +762,7 @@ int ua_bwd_rows_suffix(const UaDims* dims, int dtype, int gate_dtype, const UaRo
   ua::sm100::Bwd2Params qp{};
   qp.s = s; qp.ssrc = static_src; qp.sdest = static_dest_rows; qp.g_denom = nullptr; qp.lse = nullptr; qp.carry = nullptr;
   qp.acc_dk = dk_f32; qp.acc_dq = nullptr; qp.acc_dt = ddest_rows_f32; qp.dv_chunk = nullptr;
-  qp.dvc = nullptr; qp.dss = nullptr; qp.status = static_cast<int*>(workspace); qp.trace = nullptr;
+  qp.dvc = nullptr; qp.dss = nullptr; qp.status = static_cast<int*>(workspace);
   qp.j_begin = rows->tile_begin; qp.j_end = rows->tile_end; qp.Lr = rows->rows_total; qp.r0 = rows->row_offset;
   qp.acc_dkr = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
   qp.heads = 0; qp.suffix_in = suffix; qp.dctot_out = nullptr; qp.acc_dv = nullptr; qp.acc_ds = dsrc_f32; qp.m = 1;
@@ -883,16 +882,12 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     qp.acc_dk = acc_dk; qp.acc_dq = acc_dq; qp.acc_dt = nullptr; qp.acc_dkr = at(w.off_dkr);
     qp.dv_chunk = dv_chunk; qp.dv_chunk_stride = (s.D + 3) * s.D; qp.dv_scale = 1.0f / (float)s.C;
     qp.dvc = static_cast<bf16*>(dvc); qp.dss = dstatic_src; qp.status = reinterpret_cast<int*>(ws);
-    qp.trace = nullptr;
     qp.out_tiles = out_tiles ? out_cm : nullptr;
     if (fp32_v) qp.acc_dv = at(w.off_dv);
     if (seg) {
       qp.acc_ds = at(w.off_ds);
       qp.seg = seg; qp.max_seg = ua::sm100::bwd_max_segments(ks, seg); qp.seg_totals = at(w.off_seg);
     }
-#ifdef UA_PROFILE_BWD2
-    if (const char* tp = getenv("UA_TRACE_PTR")) qp.trace = reinterpret_cast<long long*>(strtoull(tp, nullptr, 0));
-#endif
     if (wide) {
       qp.row_term = at(w.off_gd);
       if ((e = ua::sm100::launch_bwd2(ks, gate_dtype, 4, kc, vc, xq, g_out_cm, qp, st))) return e;
@@ -1245,7 +1240,6 @@ int ua_bwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
   qp.acc_dt = nullptr;
   qp.acc_dkr = reinterpret_cast<float*>(ws + w.off_dkr);
   qp.dvc = static_cast<bf16*>(dvc); qp.dss = dstatic_src; qp.status = reinterpret_cast<int*>(ws);
-  qp.trace = nullptr;
   if (seg) {
     qp.acc_dv = reinterpret_cast<float*>(ws + w.off_dv); qp.acc_ds = reinterpret_cast<float*>(ws + w.off_ds);
     qp.seg = seg; qp.max_seg = ua::sm100::bwd_max_segments(s, seg); qp.seg_totals = reinterpret_cast<float*>(ws + w.off_seg);

@@ -71,7 +71,6 @@ struct Bwd2Params {
   __nv_bfloat16* dvc;
   void* dss;
   int* status;
-  long long* trace;          // profile builds only: per-unit time stamps of block UA_PROFILE_BLOCK (else null)
   // Range of row tiles [j_begin, j_end) (sequence-chunk sharding; whole sequence: 0, N, L, 0).  The row-indexed tensors
   // (xq, g_out, g_denom, lse, static_dest, acc_dq, acc_dt) are slabs of Lr rows that hold the range at row r0; keys,
   // values, static_src and the key-side accumulators always span the whole sequence.
@@ -179,25 +178,6 @@ struct Bwd2Ctx {
   __device__ __forceinline__ int row0_of(int ht) const { return (htop - 1 - ht) * 64; }
   __device__ __forceinline__ int srow0_of(int ht) const { return r0 + row0_of(ht) - jb * 128; }
 };
-
-// Optional phase timing (compile with -DUA_PROFILE_BWD2): thread 0 of worker warp 4 of block UA_PROFILE_BLOCK accumulates
-// clock64() deltas per phase and stores them after the status words.
-#ifdef UA_PROFILE_BWD2
-#ifndef UA_PROFILE_BLOCK
-#define UA_PROFILE_BLOCK 0
-#endif
-#define UQ_DECL long long uq_t = clock64(), uq_acc[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-#define UQ(idx) { long long now_ = clock64(); uq_acc[idx] += now_ - uq_t; uq_t = now_; }
-#define UQ_STORE if (blockIdx.x == UA_PROFILE_BLOCK && warp == 8 && lane == 0) { for (int z = 0; z < 16; ++z) reinterpret_cast<long long*>(p.status)[2 + z] = uq_acc[z]; }
-#define UQ_STORE_AT(base) if (blockIdx.x == UA_PROFILE_BLOCK) { for (int z = 0; z < 4; ++z) reinterpret_cast<long long*>(p.status)[2 + (base) + z] = uq_acc[z]; }
-#define UQ_TRACE(unit, slot) if (p.trace && blockIdx.x == UA_PROFILE_BLOCK && (unit) < 96) p.trace[(unit) * 8 + (slot)] = clock64();
-#else
-#define UQ_DECL
-#define UQ(idx)
-#define UQ_STORE
-#define UQ_STORE_AT(base)
-#define UQ_TRACE(unit, slot)
-#endif
 
 // Four tcgen05.mma of one accumulation chain from ONE asm statement: what limits a single issuing thread is the
 // instruction count per MMA (descriptor arithmetic, predicate set-up), so the chain shares one predicate set-up and
@@ -345,44 +325,34 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
     mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(sb + Cfg::oKj + (ht % Cfg::kKj) * Cfg::kHalf, 16));
     tc_commit(c.bar(qSFull + b));
     mbar_arrive(c.bar(qSFull + b));
-    UQ_TRACE(u, 0)
     ++u;
     return true;
   };
 
   if (!c.wait(qKvFull, 0)) return;
   int hc = 0;
-  UQ_DECL
   for (int ht = 0; ht < c.nht; ++ht) {
     if (!c.wait(qKjFull + ht % Cfg::kKj, ht / Cfg::kKj)) return;
     // (the workers read the tables of the next half tile before this one is over)
     if (kMode != 4 && R > 0 && ht + 1 < c.nht && !c.wait(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
     if (R > 0 && !unit_g(ht)) return;                               // G for the decay recomputation (none without heads)
     if (kMode == 4) tc_commit(c.bar(qKjFree + ht % Cfg::kKj));      // (no back issuers: the tiles are free once these products are done)
-    UQ(0)
     for (int r = 0; r < R; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, b = u % Cfg::kNB;
       if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
       if (kOutDelta && !c.wait(qDelta + sl, hc / Cfg::kNS)) return;
-      UQ(1)
       if (!acquire(b)) return;
       if (!ring_free()) return;
-      UQ(2)
-      UQ_TRACE(u, 4)
       tc_fence_after();
       const uint32_t slot = sb + Cfg::oSlot + sl * Cfg::kSlot;
       mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(slot, 16));                    // S^T  = K_i Q^T
       mma_kk(c.tmem + (b ? Cfg::tP1 : Cfg::tP0), kVi, desc_lo(slot + Cfg::kHalf, 16));       // dP^T = V_i dO^T
       tc_commit(c.bar(qSFull + b));
       mbar_arrive(c.bar(qSFull + b));
-      UQ_TRACE(u, 0)
       ++u;
-      UQ(3)
     }
     if (kMode != 4 && !(ring_free() && unit_g(ht))) return;         // G again for the decay gradient
-    UQ(0)
   }
-  UQ_STORE_AT(16)
 }
 
 // ------------------------------------------------------------ back MMA issuers --
@@ -408,14 +378,11 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
     if (kC == 128) mma4_ss(Y, t_mn + 512, k + 512, 128, 128, id_tn, 1);
   };
   if (!c.wait(qKvFull, 0)) return;
-  UQ_DECL
   for (int ht = 0; ht < c.nht; ++ht) {
     for (int r = 0; r < R; ++r, ++hc, ++w) {
       const int sl = hc % Cfg::kNS, db = w % Cfg::kRing;
       const uint32_t dsb = sb + Cfg::oDs + db * 16384;
-      UQ(0)
       if (!c.wait(qDsReady + db, w / Cfg::kRing)) return;
-      UQ(1)
       if (which == 0) {
         if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
         tc_fence_after();
@@ -436,7 +403,6 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
       } else {
         for (int cb = 0; cb < D / 64; ++cb, ++yc) {
           if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
-          UQ(2)
           tc_fence_after();
           mma_rows_out(desc_from_lo(desc_lo(dsb, 16384)), cb);                            // dQ_rj = dS^T K_i
           tc_commit(c.bar(qYFull));
@@ -444,12 +410,10 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
         tc_commit(c.bar(qDsFree + db));
       }
     }
-    UQ(0)
     const int gb = w % Cfg::kRing;
     if (!c.wait(qDsReady + gb, w / Cfg::kRing)) return;
     const uint64_t kdG = desc_from_lo(desc_lo(sb + Cfg::oDs + gb * 16384, 16)), mdG = desc_from_lo(desc_lo(sb + Cfg::oDs + gb * 16384, 16384));
     ++w;
-    UQ(3)
     if (which == 0) {
       tc_fence_after();
       const uint64_t mKj = desc_from_lo(desc_lo(sb + Cfg::oKj + (ht % Cfg::kKj) * Cfg::kHalf, 8192));
@@ -468,7 +432,6 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
     }
   }
   tc_commit(c.bar(qFinal));
-  UQ_STORE_AT(20 + 4 * which)
 }
 
 // --------------------------------------------------------------------- workers --
@@ -621,7 +584,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   float* sT3 = reinterpret_cast<float*>(c.smem + Cfg::oT3);
   float* sXch = reinterpret_cast<float*>(c.smem + Cfg::oXch);
   const uint32_t swz = (uint32_t)(key & 7);
-  UQ_DECL
 
   // Per-row tables arrive in shared memory with the tiles (the TMA producer copies them): the workers issue no global
   // load inside the sweep.  (One coalesced load per head cost every warp ~1000 cycles here: it queues behind the
@@ -723,7 +685,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         }
       }
     }
-    UQ(0)
 
     // ================= heads =================
     constexpr bool kColSums = (kMode == 1 && !kOutDelta);     // the workers sum P dP over the keys themselves
@@ -735,14 +696,12 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       float* tabL = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512);      // lse[64] of the head's rows (raw)
       float* tabC = tabL + 64;                                                         // g_denom[64] (or delta[64])
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
-      UQ(1)
       tc_fence_after();
       float2 pv[H2], dp[H2];
       {
         uint32_t sr[CG], dr[CG];
         tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, sr);
         tmem_ld16(c.tmem + (b ? Cfg::tP1 : Cfg::tP0) + lane_base + col0, dr);
-        UQ(6)
         float2 nl[H2];
         load_pairs(tabL + col0, nl);                                 // lse of the rows
         tc_wait_ld();
@@ -751,7 +710,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         // (mode 4: the products that read the slot are done, and this was the last look at its table)
         if (kMode == 4) c.arrive_w(qInFree + sl);
         ++u;
-        UQ(15)
 #pragma unroll
         for (int x = 0; x < H2; ++x) {
           const float2 sv = make_float2(__uint_as_float(sr[2 * x]), __uint_as_float(sr[2 * x + 1]));
@@ -777,11 +735,9 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         }
         if (helper) atomicAdd(tabC + col0 + lane, -part);           // g_denom - sum_k P dP, in place
       }
-      UQ(2)
       if (kColSums) {
         named_bar_sync(kBarGroup + g, kC);           // the group's column sums are complete
       }
-      UQ(4)
       {
         float2 cc[H2];
         uint32_t pk[H2], dk[H2];
@@ -795,7 +751,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           pk[x] = *reinterpret_cast<uint32_t*>(&hp);
           dk[x] = *reinterpret_cast<uint32_t*>(&hd);
         }
-        UQ(5)
         store_row(c.smem + Cfg::oDs + w % Cfg::kRing * 16384, dk);
         // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column).  With a ring of two, its free buffer says that the product with the
         // probabilities of two heads ago is done as well; with three it does not.
@@ -835,10 +790,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         if (!kHeads && !c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
         if (helper) sT3[((ht + 1) & 1) * 64 + col0 + lane] = t3_from_table(ht + 1);
       }
-      UQ(7)
       const int b = u % Cfg::kNB;
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
-      UQ(9)
       tc_fence_after();
       uint32_t gr[CG];
       tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
@@ -871,7 +824,6 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         }
       }
       named_bar_sync(kBarAll, kWorkers);
-      UQ(8)
       float later = 0.f, others = 0.f;             // totals of the groups to the right / of all other groups
 #pragma unroll
       for (int q = 0; q < NG; ++q) {
@@ -908,10 +860,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       // (d static_dest needs no sum over the keys here: it is taken from dK_j afterwards, see row_side_finish_kernel)
       fence_proxy_async();
       c.arrive_w(qDsReady + db);
-      UQ(10)
     }
   }
-  UQ_STORE
 
   if (kMode == 4) return;
   // ---- end of the sweep: dV_i, dK_i, d static_src (thread = key, D / NG columns each) ----

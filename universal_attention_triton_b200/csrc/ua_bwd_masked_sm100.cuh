@@ -297,18 +297,6 @@ __global__ void __launch_bounds__(256) masked_finish_kernel(const __nv_bfloat16*
 }
 
 // ----------------------------------------------------------------- sweep kernel --
-// Optional phase timing (compile with -DUA_PROFILE_MK=<block>): each role of that block accumulates clock64() deltas per
-// phase and stores them after the status words.
-#ifdef UA_PROFILE_MK
-#define MQ_DECL long long mq_t = clock64(), mq_acc[4] = {0, 0, 0, 0};
-#define MQ(idx) { long long now_ = clock64(); mq_acc[idx] += now_ - mq_t; mq_t = now_; }
-#define MQ_STORE(base) if (blockIdx.x == UA_PROFILE_MK) { for (int z = 0; z < 4; ++z) reinterpret_cast<long long*>(p.status)[2 + (base) + z] = mq_acc[z]; }
-#else
-#define MQ_DECL
-#define MQ(idx)
-#define MQ_STORE(base)
-#endif
-
 // Slot unit u of a step: the chunks [u kPer, (u + 1) kPer) of the group that have the step's row tile before them.
 template <int D>
 struct MkUnit {
@@ -348,14 +336,11 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
   };
   for (int x = 0; x < Cfg::kAhead; ++x) prefetch_next();
   int s = 0, uc = 0;
-  MQ_DECL
   for (int j = c.jlo; j < c.jhi; ++j) {
     const int c0 = c.clo(j);
     for (int r = 0; r < R; ++r, ++s) {
       const int qs = s & 1;
-      MQ(0)
       if (s >= 2 && !c.wait(mQFree + qs, s / 2 - 1)) return;
-      MQ(1)
       mbar_expect_tx(c.bar(mQFull + qs), 16384u + (uint32_t)(c.chi - c0) * 512u);
       tma_load_2d(sb + Cfg::oQ + qs * 16384, tmQ, 64 * c.h, (c.bh * R + r) * L + c.srow(j), c.bar(mQFull + qs));
       for (int cc = c0; cc < c.chi; ++cc)
@@ -365,9 +350,7 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
         const MkUnit<D> un(u, c0, c.chi);
         if (!un.active()) continue;
         const int sl = uc % Cfg::kSlots;
-        MQ(0)
         if (uc >= Cfg::kSlots && !c.wait(mSlotFree + sl, uc / Cfg::kSlots - 1)) return;
-        MQ(2)
         ++uc;
         mbar_expect_tx(c.bar(mSlotFull + sl), (uint32_t)(un.hi - un.lo) * Cfg::kDoBytes);
         for (int cc = un.lo; cc < un.hi; ++cc) {
@@ -380,7 +363,6 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
       }
     }
   }
-  MQ_STORE(8)
 }
 
 template <int D, bool kWide>
@@ -391,17 +373,13 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
   constexpr uint32_t id_y = idesc_bf16(128, 64, 0, 0);       // rows x 64: A K-major, B K-major
   if (!c.wait(mMtFull, 0)) return;
   int s = 0, uc = 0;
-  MQ_DECL
   for (int j = c.jlo; j < c.jhi; ++j) {
     const int c0 = c.clo(j);
     for (int r = 0; r < R; ++r, ++s) {
       const int qs = s & 1;
       const uint32_t q_addr = sb + Cfg::oQ + qs * 16384;
-      MQ(3)
       if (!c.wait(mQFull + qs, s / 2)) return;
-      MQ(0)
       if (s >= 2 && !c.wait(mYFree + qs, s / 2 - 1)) return;
-      MQ(1)
       tc_fence_after();
       const uint32_t Y = c.tmem + (qs ? Cfg::tY1 : Cfg::tY0);
       // [K = rows][M = the 64 columns of Q, then the 64 columns of the ones tile]
@@ -411,9 +389,7 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
         const MkUnit<D> un(u, c0, c.chi);
         if (!un.active()) continue;
         const int sl = uc % Cfg::kSlots;
-        MQ(3)
         if (!c.wait(mSlotFull + sl, uc / Cfg::kSlots)) return;
-        MQ(2)
         ++uc;
         tc_fence_after();
         const uint32_t slot = sb + Cfg::oSlot + sl * 32768;
@@ -439,8 +415,6 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
     }
   }
   tc_commit(c.bar(mDone));
-  MQ(3)
-  MQ_STORE(0)
 }
 
 // Four warps on the CUDA cores: w_c[d'] += sum_rows gd_c[row] Q[row][d'] for the group's chunks, from the Q tile in shared
@@ -456,14 +430,11 @@ __device__ __forceinline__ void mk_gate_sums(const MkCtx<kWide>& c, const Masked
 #pragma unroll
   for (int x = 0; x < Cfg::kG * 16; ++x) acc[x] = 0.f;
   int s = 0;
-  MQ_DECL
   for (int j = c.jlo; j < c.jhi; ++j) {
     const int c0 = c.clo(j);
     for (int r = 0; r < R; ++r, ++s) {
       const int qs = s & 1;
-      MQ(1)
       if (!c.wait_w(mQFull + qs, s / 2)) return;
-      MQ(0)
       const uint8_t* q = c.smem + Cfg::oQ + qs * 16384;
       const float* gd = reinterpret_cast<const float*>(c.smem + Cfg::oGd + qs * Cfg::kG * 512);
 #pragma unroll 1
@@ -491,9 +462,6 @@ __device__ __forceinline__ void mk_gate_sums(const MkCtx<kWide>& c, const Masked
       c.arrive_w(mQFree + qs);
     }
   }
-#ifdef UA_PROFILE_MK
-  if (t == 0) { MQ(1) MQ_STORE(12) }
-#endif
   const int c0 = c.clo(c.jlo);
 #pragma unroll
   for (int grp = 0; grp < Cfg::kG / 2; ++grp) {
@@ -518,14 +486,11 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
   uint8_t* stage = c.smem + Cfg::oStage;
   const float* ks = reinterpret_cast<const float*>(c.smem + Cfg::oKs);
   int s = 0;
-  MQ_DECL
   for (int j = c.jlo; j < c.jhi; ++j) {
     const int c0 = c.clo(j);
     for (int r = 0; r < R; ++r, ++s) {
       const int qs = s & 1;
-      MQ(3)
       if (!c.wait_w(mYFull + qs, s / 2)) return;
-      MQ(0)
       tc_fence_after();
       float gd[Cfg::kG];
 #pragma unroll
@@ -534,7 +499,6 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
       c.arrive_w(mQFree + qs);                     // the step's g_denom rows have been read
       if (leader) bulk_wait_read_all();            // the previous reduce-add has read the staging tile
       named_bar_sync(2, 128);
-      MQ(1)
 #pragma unroll 1
       for (int hb = 0; hb < 2; ++hb) {
         uint32_t o[32];
@@ -562,7 +526,6 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
           *reinterpret_cast<float4*>(box + ((((uint32_t)x ^ swz) & 7) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
         }
       }
-      MQ(2)
       fence_proxy_async();
       named_bar_sync(2, 128);
       if (leader) {
@@ -573,9 +536,6 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
       }
     }
   }
-#ifdef UA_PROFILE_MK
-  if (leader) { MQ(3) MQ_STORE(4) }
-#endif
   if (!c.wait_w(mDone, 0)) {
     if (leader) bulk_wait_all();
     return;
@@ -699,9 +659,6 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   c.tmem = misc[0];
 
-#ifdef UA_PROFILE_MK
-  const long long mk_t0 = clock64();
-#endif
   if (warp == 0) {
     if (lane == 0) mk_producer<D, kWide>(c, p, &tmQ, &tmG);
   } else if (warp == 1) {
@@ -714,9 +671,6 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   tc_fence_before();
   __syncthreads();
-#ifdef UA_PROFILE_MK
-  if (blockIdx.x == UA_PROFILE_MK && threadIdx.x == 0) reinterpret_cast<long long*>(p.status)[2 + 16] = clock64() - mk_t0;
-#endif
   if (*c.abort_flag) {
     if (threadIdx.x == 0) {
       if (atomicExch(p.status, 3) == 0) p.status[1] = (int)misc[2];

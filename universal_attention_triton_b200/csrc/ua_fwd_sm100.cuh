@@ -43,16 +43,6 @@ namespace sm100 {
 
 using namespace ua::ptx;
 
-#ifdef UA_PROFILE_FWD
-#define UF_DECL long long uf_t = clock64(), uf_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#define UF(idx) { long long now_ = clock64(); uf_acc[idx] += now_ - uf_t; uf_t = now_; }
-#define UF_STORE(cond, base) if (blockIdx.x == 0 && (cond)) { for (int z = 0; z < 8; ++z) reinterpret_cast<long long*>(p.status)[2 + (base) + z] = uf_acc[z]; }
-#else
-#define UF_DECL
-#define UF(idx)
-#define UF_STORE(cond, base)
-#endif
-
 struct FwdParams {
   Shape s;
   const void* ssrc;
@@ -333,7 +323,6 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
   };
   if (live)
     for (int T = 0; T < c.t0; ++T) add_to_carry(carry_lo + p.tile_totals[(chunk_id * p.tiles + T) * 128 + k]);
-  UF_DECL
   for (int T = 0; T < c.ntiles; ++T) {
     float* t3buf = sT3 + (T & 1) * 128;
     t3buf[k] = cbrtf(raw_next);
@@ -341,9 +330,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     c.arrive_w(kT3Ready);
     if (!c.wait_w(kT3Ready, T)) return;
     if (!live) continue;
-    UF(0)
     if (!c.wait_w(kGFull, T)) return;
-    UF(1)
     tc_fence_after();
     const bool diag = (c.row0 + T * 128 == c.i * kC);
     float* carry_row = p.carry ? p.carry + (chunk_id * (L / 64) + (c.row0 + T * 128) / 64) * 128 + k : nullptr;
@@ -395,9 +382,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
       else scan32(std::false_type{});
       tprev += local;
       if (!kCarryOnly) {
-        UF(2)
         if (cb == 0 && T >= Cfg::kCBufs && !c.wait_w(kCFree + T % Cfg::kCBufs, T / Cfg::kCBufs - 1)) return;
-        UF(3)
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
           const int q = cb * 32 + x;
@@ -407,9 +392,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     }
     add_to_carry(tprev);      // (tprev = carry_lo + the tile's total)
     if (!kCarryOnly) c.arrive_w(kCReady + T % Cfg::kCBufs);
-    UF(2)
   }
-  UF_STORE(k == 0, 0)
   if (p.total_out) p.total_out[key_id] = carry;
 }
 
@@ -425,16 +408,13 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
   const size_t chunk_id = (size_t)c.bh * N + c.i;
   const float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
   int t = 0;
-  UF_DECL
   for (int T = 0; T < c.ntiles; ++T) {
     // Every softmax thread observes every phase of c_ready and arrives on c_free exactly
     // once per tile (after its last read of C in that tile), whether or not its group has
     // a head to process in this tile; parity waits stay within one phase of the barrier.
-    UF(0)
     const int cbuf = T % Cfg::kCBufs;
     const uint8_t* sCrow = sCrow0 + cbuf * 65536;
     if (!c.wait_w(kCReady + cbuf, T / Cfg::kCBufs)) return;
-    UF(1)
     int last_r = -1;
     for (int r = R - 1; r >= 0; --r)
       if (((T * R + r) & 1) == me) { last_r = r; break; }
@@ -444,9 +424,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
       const int sb = t & 1, ob = t % Cfg::kOBufs;
       const uint32_t tS = c.tmem + (sb ? Cfg::tS1 : Cfg::tS0) + lane_base;
       const uint32_t tO = c.tmem + ((Cfg::kOBufs == 2 && ob) ? Cfg::tO1 : Cfg::tO0) + lane_base;
-      UF(0)
       if (!c.wait_w(kSFull + sb, t >> 1)) return;
-      UF(2)
       tc_fence_after();
       // pass 1: s = S + C (written back to TMEM), row max.  64 columns per round trip: the two loads are in flight together.
       float m = -INFINITY;
@@ -470,7 +448,6 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
         tmem_st32(tS + cb * 64 + 32, s + 32);
       }
       tc_wait_st();
-      UF(3)
       if (r == last_r) c.arrive_w(kCFree + cbuf);
       // pass 2: P = exp(s - m) as bf16 into the first 64 columns of the S buffer
       const float mb = m * kLog2e;
@@ -498,7 +475,6 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
       if (kOut != kOutStats) tc_wait_st();
       tc_fence_before();
       c.arrive_w(kPReady + sb);
-      UF(4)
       const int qg = c.srow0 + T * 128 + row;                       // row index inside the slab
       const bool in_range = kC == 128 || qg < p.Lr;                 // (kC = 64: the last tile may be half a tile)
       const float l = l2.x + l2.y;
@@ -515,10 +491,8 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
         if (p.denom && in_range) p.denom[orow] = __float2bfloat16_rn(lse);
         linv = 1.0f / l;
       }
-      UF(5)
       if (kOut == kOutStats) continue;
       if (!c.wait_w(kOFull + sb, t >> 1)) return;
-      UF(6)
       tc_fence_after();
       if (kMerge) {
 #pragma unroll 1
@@ -597,10 +571,8 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
           st_global_v8(orow_ptr + cb * 32 + 16, pk + 8);
         }
       }
-      UF(7)
     }
   }
-  UF_STORE(row == 0 && me == 0, 8)
 }
 
 // Rows before key chunk `chunk`: every score is -1e12 (fp32 absorbs k.q), the softmax is
