@@ -31,7 +31,7 @@ def test_functions_follow_the_new_style_protocol():
 
 
 def test_note_on_gradients_that_vanish_before_each_chunk():
-    """The note SMVecMatMul.backward leaves on its results (host logic, no GPU): it holds the tensor's version counter,
+    """The note SMVecMatMul.backward leaves on its results (the native nodes' registry; no GPU): it holds the tensor's version counter,
     an in-place change voids it, and tensors that autograd derives (a sum of two gradients, a hook's replacement) do not carry
     it -- so the operator's backward falls back to the full path whenever the zeros are not guaranteed."""
     from universal_attention_triton_b200 import universal_attention_autograd as M
@@ -276,3 +276,74 @@ def test_error_of_a_backward_reaches_the_caller_with_its_type():
     shifted = torch.zeros(out.numel() + 1, dtype=out.dtype, device="cuda")[1:].view(1, 1, 2, 1, 256, 64)
     with pytest.raises(UaLibraryError, match="ua_bwd failed"):
         torch.autograd.grad([out, denom], xs, [ops.as_reference_out(shifted), torch.zeros_like(denom)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["two_consumers", "in_place_hook"])
+def test_gradients_before_each_chunk_that_join_the_merges_are_not_lost(how):
+    """In the native graph: a gradient of the operator's outputs that is more than SMVecMatMul's -- the sum with another
+    consumer's (which autograd may form in place, in the noted tensor), or an in-place change by a hook -- takes the full path.
+    Against the oracle on the gradients that really arrive, with most of their norm on the rows before the chunks."""
+    import universal_attention_triton_b200 as ua
+    from oracle import ua_oracle as O
+    from tests._util import rel_fro, valid_row_mask
+    b, h, r, L, c, d = 1, 2, 2, 512, 128, 64
+    n = L // c
+    ins = O.make_inputs(b, h, r, L, c, d, dtype=torch.bfloat16, seed=12)
+    gen = torch.Generator().manual_seed(2)
+    before = ~valid_row_mask(L, n, c)
+    extra = (torch.randn(b, h, r, L, d, n, generator=gen) * before.view(L, 1, n)).bfloat16().cuda()
+    extra_den = (torch.randn(b, h, r, L, n, generator=gen) * before).bfloat16().cuda()
+    xs = [t.cuda().requires_grad_() for t in ins]
+    out, denom = ua.UniversalAttention.apply(*xs)
+    arrived = []
+    if how == "two_consumers":
+        out.register_hook(lambda g: arrived.append(g.clone()))
+        denom.register_hook(lambda g: arrived.append(g.clone()))
+        loss = ua.SMVecMatMul.apply(out, denom).float().sum() + (out * extra).sum() + (denom * extra_den).sum()
+    else:
+        out.register_hook(lambda g: arrived.append(g.add_(extra).clone()) and None)
+        denom.register_hook(lambda g: arrived.append(g.add_(extra_den).clone()) and None)
+        loss = ua.SMVecMatMul.apply(out, denom).float().sum()
+    grads = torch.autograd.grad(loss, xs)
+    g_out = next(t for t in arrived if t.dim() == 6).float().cpu()
+    g_den = next(t for t in arrived if t.dim() == 5).float().cpu()
+    assert (g_out * before.view(L, 1, n)).norm() > 0.5 * extra.float().norm().cpu()
+    for got, want, name in zip(grads, O.ua_backward(*[t.float() for t in ins], g_out, g_den), ("dkc", "dvc", "dxq", "dsrc", "ddest")):
+        assert rel_fro(got.float().cpu(), want) <= 5e-2, (name, rel_fro(got.float().cpu(), want))
+
+
+@pytest.mark.gpu
+def test_native_node_saves_its_output_unless_switched_off():
+    """The eager path (a native node): which tensors it saves under either setting of ``set_save_output``, that an in-place change of
+    a saved output is noticed, and that both settings give the gradients of the oracle."""
+    import universal_attention_triton_b200 as ua
+    from oracle import ua_oracle as O
+    from tests._util import rel_fro
+    ins = O.make_inputs(1, 2, 2, 512, 128, 64, dtype=torch.bfloat16, seed=9)
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    try:
+        for on in (True, False):
+            ua.set_save_output(on)
+            xs = [t.cuda().requires_grad_() for t in ins]
+            packed = []
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(tuple(t.shape)) or t, lambda t: t):
+                out, denom = ua.UniversalAttention.apply(*xs)
+            assert packed.count(tuple(out.shape)) == int(on), packed
+            for x in xs:
+                assert tuple(x.shape) in packed
+            g_out = torch.randn(out.shape, generator=gen, device="cuda").to(out.dtype)
+            g_den = torch.randn(denom.shape, generator=gen, device="cuda").to(denom.dtype)
+            want = O.ua_backward(*[t.float() for t in ins], g_out.float().cpu(), g_den.float().cpu())
+            for got, ref, name in zip(torch.autograd.grad([out, denom], xs, [g_out, g_den]), want, ("dkc", "dvc", "dxq", "dsrc", "ddest")):
+                assert rel_fro(got.float().cpu(), ref) <= 5e-2, (on, name)
+            out, denom = ua.UniversalAttention.apply(*xs)
+            with torch.no_grad():
+                out.mul_(2)
+            if on:
+                with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                    torch.autograd.grad([out, denom], xs, [g_out, g_den])
+            else:
+                torch.autograd.grad([out, denom], xs, [g_out, g_den])
+    finally:
+        ua.set_save_output(True)

@@ -318,9 +318,10 @@ using torch::autograd::variable_list;
 
 bool g_strict_masked_grads = true;      // universal_attention_autograd.set_strict_masked_grads
 
-// Notes on gradient tensors whose part for the rows before each chunk is exactly zero (see _mark_masked_zero there): the tensor
-// itself, by weak reference, and its version counter, so that an in-place change voids the note and a tensor that autograd
-// builds from it does not carry it.  The last 64 are kept; a note that fell out only costs the shortcut.
+// Notes on gradient tensors whose part for the rows before each chunk is exactly zero, for the nodes below and for the Python
+// Functions (_mark_masked_zero there): the tensor itself, by weak reference, and its version counter, so that an in-place change
+// voids the note and a tensor that autograd builds from it does not carry it.  The last 64 are kept; a note that fell out only
+// costs the shortcut.
 class MaskedZeroNotes {
  public:
   void add(const Tensor& t) {
@@ -681,6 +682,8 @@ auto outside_functorch(R (*f)(A...)) {
 PYBIND11_MODULE(_ua_torch, m) {
   m.def("bind", [](py::object error, py::object unwrap) { g_error = error.release(); g_unwrap = unwrap.release(); });
   m.def("set_strict_masked_grads", [](bool on) { g_strict_masked_grads = on; });
+  m.def("mark_masked_zero", [](const Tensor& t) { notes().add(t); });
+  m.def("masked_zero", [](const Tensor& t) { return notes().has(t); });
   m.def("ua_apply", &ua_apply);
   m.def("merge_apply", &merge_apply);
   m.def("merged_apply", outside_functorch(&merged_apply));

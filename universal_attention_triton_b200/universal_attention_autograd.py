@@ -128,16 +128,15 @@ def _setup_context(ctx, inputs, outputs):
 
 def _mark_masked_zero(*tensors):
     """Notes on gradient tensors that their part for the rows before each chunk is exactly zero (``SMVecMatMul.backward``
-    produces such tensors: the merge weight of a fully masked block is exp(-1e12 - lse) = 0).  The note holds the tensor's
-    version counter, so that an in-place change of the tensor voids it; a tensor that autograd builds from it (a sum with
-    another gradient, a hook's replacement) does not carry it."""
+    produces such tensors: the merge weight of a fully masked block is exp(-1e12 - lse) = 0).  One registry for these Functions and
+    for the native nodes; a note holds the tensor's version counter, so that an in-place change of the tensor voids it, and a tensor
+    that autograd builds from it (a sum with another gradient, a hook's replacement) does not carry it."""
     for t in tensors:
-        t._ua_masked_zero = t._version
+        _lib.native().mark_masked_zero(t)
 
 
 def _masked_zero(t) -> bool:
-    v = getattr(t, "_ua_masked_zero", None)
-    return v is not None and v == t._version
+    return _lib.native().masked_zero(t)
 
 
 def _default_merge_modes() -> bool:
