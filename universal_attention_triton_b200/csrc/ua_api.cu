@@ -844,7 +844,11 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     // The kernels' producers copy rows of lse / g_denom with 16-byte bulk copies: 16-byte aligned, and fp32 but for the sweep that
     // takes its row term from the output tiles, which widens a bf16 g_denom by itself.  For wide chunks the table is a copy in which
     // the row term is formed.
-    const bool out_tiles = !wide && s.D == 64 && out_cm && aligned16(out_cm);
+    // The row term comes from the output tiles where the caller hands them over (its choice: faster, but the outputs' rounding enters
+    // the gradients), for the one chunk length at which it always could; everything else sums P dP over the keys in fp32.  Chunks of
+    // 64 keys, gradients of the operator's own outputs, B2 H8 R4 L1024: dK / dQ / d src / d dest 2.2 / 2.3 / 1.7 / 2.6e-3 from 64-bit
+    // values with the sums, 3.8 / 3.5 / 4.9 / 4.7e-3 with the tiles.
+    const bool out_tiles = !wide && ks.C == 128 && s.D == 64 && out_cm && aligned16(out_cm);
     const float* gd32 = static_cast<const float*>(g_denom_cm);
     if (g_denom_dtype != UA_F32 && (!out_tiles || (masked && ks.C == 128) || !aligned16(g_denom_cm))) {
       if ((e = launch_widen(g_denom_cm, at(w.off_gd), rows, st))) return e;

@@ -31,8 +31,8 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
       if (mode == 3) kern = bwd2_kernel<D, kC, TG, 3, true>;
       if (mode == 4) kern = bwd2_kernel<D, kC, TG, 4, true>;
     }
-    // the forward's output tiles at hand (per-chunk form, head_dim 64): the row term comes from them
-    if constexpr (Cfg::kOutTiles) {
+    // the forward's output tiles at hand (chunks of 128 keys, per-chunk form, head_dim 64): the row term comes from them
+    if constexpr (Cfg::kOutTiles && kC == 128) {
       if (mode == 1 && p.out_tiles != nullptr) {
         if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
         kern = bwd2_kernel<D, kC, TG, 1, true, true>;
