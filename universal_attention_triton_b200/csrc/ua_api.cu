@@ -884,6 +884,7 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
     qp.g_denom = gd32; qp.g_denom16 = gd32 ? nullptr : static_cast<const bf16*>(g_denom_cm);
     qp.lse = lse; qp.carry = carry_tab; qp.m = m;
     qp.acc_dk = acc_dk; qp.acc_dq = acc_dq; qp.acc_dt = nullptr; qp.acc_dkr = at(w.off_dkr);
+    if (ks.C == 64) qp.dt_cols = at(w.off_dt);
     qp.dv_chunk = dv_chunk; qp.dv_chunk_stride = (s.D + 3) * s.D; qp.dv_scale = 1.0f / (float)s.C;
     qp.dvc = static_cast<bf16*>(dvc); qp.dss = dstatic_src; qp.status = reinterpret_cast<int*>(ws);
     qp.out_tiles = out_tiles ? out_cm : nullptr;

@@ -64,7 +64,8 @@ int launch_finish_t(const Shape& s, const void* kc, const Bwd2Params& p, void* d
   const size_t dq_vec = (size_t)rows * s.R * D / 8;
   using bf16 = __nv_bfloat16;
   bwd_finish_kernel<D, TG><<<(unsigned)(row_blocks + (dq_vec + 255) / 256), 256, 0, st>>>(
-      static_cast<const bf16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dq, p.acc_dv, p.acc_ds, static_cast<bf16*>(dkc),
+      static_cast<const bf16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dq, p.acc_dv, p.acc_ds, p.dt_cols,
+      static_cast<bf16*>(dkc),
       static_cast<bf16*>(dxq), static_cast<bf16*>(dvc), static_cast<TG*>(dss), static_cast<TG*>(ddest), rows, row_blocks, dq_vec);
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }

@@ -64,6 +64,7 @@ struct Bwd2Params {
   float* acc_dk;             // (b*h, L, D) fp32, zeroed (or holding the masked-block part)
   float* acc_dq;             // (b*h, r, L, D) fp32, likewise
   float* acc_dt;             // (b*h, Lr) fp32: d static_dest is ADDED here (by row_side_finish_kernel, after the sweep)
+  float* dt_cols;            // [kC = 64] (b*h, L) fp32, zeroed: per row, sum over the keys of dell a / (a - 1), from which d static_dest is taken
   float* acc_dkr;            // (b*h, L, D) fp32 scratch, zeroed: the row-side dK_j = dG^T K_i of all chunks (see there)
   const float* dv_chunk;     // optional: row dv_chunk[chunk * dv_chunk_stride + d] * dv_scale is added to every key's dV_i (the
   int dv_chunk_stride;       // masked-block part when it comes from the kernels of the rows before a chunk)
@@ -846,7 +847,12 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
             if (qbase + 2 * x <= key) dl.x = 0.f;
             if (qbase + 2 * x + 1 <= key) dl.y = 0.f;
           }
-          dsa = ffma2(dl, f1[x], dsa);
+          if (kC == 64) {                          // (kept for the sums over the keys below)
+            f1[x] = fmul2(dl, f1[x]);
+            dsa = fadd2(dsa, f1[x]);
+          } else {
+            dsa = ffma2(dl, f1[x], dsa);
+          }
           const float2 dg = fmul2(fmul2(dl, s32k), f2[x]);
           __nv_bfloat162 h = __floats2bfloat162_rn(dg.x, dg.y);
           pk[x] = *reinterpret_cast<uint32_t*>(&h);
@@ -857,9 +863,21 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       ds_acc += dsa.x + dsa.y;
       const int db = w++ % Cfg::kRing;
       store_row(c.smem + Cfg::oDs + db * 16384, pk);
-      // (d static_dest needs no sum over the keys here: it is taken from dK_j afterwards, see row_side_finish_kernel)
       fence_proxy_async();
       c.arrive_w(qDsReady + db);
+      // d static_dest: with chunks of 128 keys it is taken from dK_j afterwards (see row_side_finish_kernel), which costs nothing here
+      // but is formed from the bf16 dG; chunks of 64 keys have always had it from fp32 sums over the keys, two warps per column.
+      if constexpr (kC == 64) {
+        float e[CG];
+#pragma unroll
+        for (int x = 0; x < H2; ++x) {
+          const float2 ev = fmul2(f1[x], s32);
+          e[2 * x] = ev.x;
+          e[2 * x + 1] = ev.y;
+        }
+        const float part = warp_colsum(e, lane);
+        if (helper) atomicAdd(p.dt_cols + (size_t)c.bh * L + c.row0_of(ht) + col0 + lane, part);
+      }
     }
   }
 
@@ -1089,13 +1107,13 @@ row_side_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restric
 }
 
 // ... and, for a whole sequence, everything that is left to do in one launch: blocks [0, row_blocks): one warp per row of K as
-// above, with dK (accumulator + row side), d static_dest and, where the sweep added them up in fp32, dV and d static_src leaving
+// above, with dK (accumulator + row side), d static_dest (chunks of 64 keys: from the sweep's sums over the keys, dt_cols) and, where the sweep added them up in fp32, dV and d static_src leaving
 // in their own types; the other blocks: dQ, eight elements per thread.
 template <int D, typename TG>
 __global__ void __launch_bounds__(256)
 bwd_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restrict__ sdest, const float* __restrict__ dkr,
                   const float* __restrict__ acc_dk, const float* __restrict__ acc_dq, const float* __restrict__ acc_dv,
-                  const float* __restrict__ acc_ds, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dq,
+                  const float* __restrict__ acc_ds, const float* __restrict__ dt_cols, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dq,
                   __nv_bfloat16* __restrict__ dv, TG* __restrict__ ds, TG* __restrict__ dt, int rows, int row_blocks, size_t dq_vec) {
   auto pack2 = [](float a, float b) -> uint32_t {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -1127,7 +1145,9 @@ bwd_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restrict__ s
     *reinterpret_cast<uint2*>(dv + at) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
   }
   if (sub == 0) {
-    Num<TG>::st(dt + row, dot != 0.f ? 0.5f * dot / Num<TG>::ld(sdest + row) : 0.f);
+    // (d a / d t = a / (3 t))
+    const float num = dt_cols ? dt_cols[row] * (1.0f / 3.0f) : 0.5f * dot;
+    Num<TG>::st(dt + row, num != 0.f ? num / Num<TG>::ld(sdest + row) : 0.f);
     if (acc_ds) Num<TG>::st(ds + row, acc_ds[row]);
   }
 }
