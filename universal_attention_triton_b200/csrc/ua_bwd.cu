@@ -101,9 +101,14 @@ int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* 
   if (!make_rows_map(&tmQ, xq, BH * s.R * p.Lr, D) || !make_rows_map(&tmG, g_out, BH * (s.N / p.m) * s.R * p.Lr, D) ||
       !make_f32_rows_map(&tmDQ, acc_dq, BH * s.R * p.Lr, D))
     return UA_ERR_CUDA;
-  // Row tiles per work item.  An item pays for its start-up once and adds to dQ where the groups at work share L2, so it should be
-  // neither short nor long: about 32 (tile, head) steps, but 16 tiles at most (B4 H8 R4 L4096 D64, 4 / 8 / 16 / 32 tiles: 466 / 438 / 471 /
-  // 564 us; B1 H16 R1 L4096 D128: 320 / 242 / 215 / 217 us), and fewer where that would leave SMs without one.
+  // Row tiles per work item.  An item pays for its start-up and for each chunk's N / w / u once, and adds to dQ where the groups at work share
+  // L2, so it should be neither short nor long: 16 tiles with one to three query heads, 8 with four or more, and fewer where that would
+  // leave SMs without an item.  Sweep times in us for 2 / 4 / 8 / 16 / 32 tiles, L4096:
+  //   head_dim 64   B4 H8 R1 259 / 170 / 141 / 136 / 154    R2 340 / 250 / 221 / 224 / 273    R4 493 / 398 / 375 / 405 / 505
+  //                 B4 H4 R8 405 / 362 / 371 / 444 / 613    B1 H4 R16 188 / 178 / 323 / 632 / 1199 (the grid's limit leaves 2: 189)
+  //   head_dim 128  B1 H16 R1 502 / 301 / 224 / 198 / 199   H8 R4 451 / 350 / 319 / 345 / 420   H8 R8 705 / 599 / 589 / 654 / 808
+  //                 H4 R16 627 / 607 / 587 / 703 / 1085
+  // (4 tiles would win 3 to 10 % with eight or more heads of head_dim 64 and lose 2 to 3 % at 128.)
   const int last = (s.N - 1) / p.m * p.m, jcap = (last < p.j_end) ? last : p.j_end;      // no row tile at or after the last chunk is before any chunk
   for (p.jp = s.R >= 4 ? 8 : 16;; p.jp /= 2) {
     p.items_per_bh = 0;
