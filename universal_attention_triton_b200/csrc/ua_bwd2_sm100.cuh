@@ -31,7 +31,7 @@
 // never read) leave as TMA reduce-adds into fp32 accumulators.  Rows BEFORE the chunk are not handled here.
 //
 // kC = 64: the keys are TMEM lanes 0..63; lanes 64..127 compute on what lies behind the 64 rows in shared memory and are
-// never read, sums over the keys take 64 of them.
+// never read, sums over the keys take 64 of them.  Row terms and d static_dest are such sums, in fp32 (no output tiles, dt_cols).
 // Segments (p.seg > 0): where one block per chunk leaves the chip idle, a sweep is cut into blocks of p.seg half tiles, each
 // with a zero reverse carry; every gradient is linear in that carry, so the correction pass (the same kernel without heads)
 // adds what the rows after a segment induce, from the totals that the segments leave (see ua_split.h for when).

@@ -74,10 +74,13 @@ _SAVE_OUTPUT = True
 
 def set_save_output(on: bool) -> None:
     """When on (default), the Functions also save their own output ``out`` for backward (chunk-major layout only).  The
-    tensor-core backward then takes the softmax gradient's row term ``sum_k P dP`` as ``out . g_out`` per row instead of
-    summing over the keys (the backward kernel then takes 2.15 ms instead of 2.55 at B4 H8 R4 L4096 D64).  ``out`` stays alive until backward has run -- which
-    it does anyway whenever ``SMVecMatMul`` (or any node that saves its input) consumes it -- and, like every saved
-    tensor, must not be modified in place before backward.  Off: exactly the reference's set of saved inputs plus the two
+    tensor-core backward of chunks of 128 keys at head_dim 64 then takes the softmax gradient's row term ``sum_k P dP`` as
+    ``out . g_out`` per row instead of summing over the keys: its kernel takes 1.70 ms instead of 2.03 at B4 H8 R4 L4096.  What it
+    costs is accuracy, as the rounding of the bf16 ``out`` enters the gradients: for gradients of the operator's own outputs
+    (B1 H8 R4 L1024, unit keys, against 64 bits) dk / dq / d src / d dest 3.6 / 3.4 / 4.1 / 4.5e-3 with it and 2.2 / 2.4 / 1.7 /
+    2.6e-3 without, with ``SMVecMatMul`` behind the operator 3.1 / 3.1 / 3.0 / 3.4e-3 and 3.0 / 3.0 / 3.0 / 3.2e-3.  (Other shapes
+    sum over the keys either way.)  ``out`` stays alive until backward has run -- which it does anyway whenever ``SMVecMatMul``
+    (or any node that saves its input) consumes it -- and, like every saved tensor, must not be modified in place before backward.  Off: exactly the reference's set of saved inputs plus the two
     small by-products."""
     global _SAVE_OUTPUT
     _SAVE_OUTPUT = bool(on)
