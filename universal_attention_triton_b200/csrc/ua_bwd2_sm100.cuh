@@ -180,37 +180,6 @@ struct Bwd2Ctx {
   __device__ __forceinline__ int srow0_of(int ht) const { return r0 + row0_of(ht) - jb * 128; }
 };
 
-// Four tcgen05.mma of one accumulation chain from ONE asm statement: what limits a single issuing thread is the
-// instruction count per MMA (descriptor arithmetic, predicate set-up), so the chain shares one predicate set-up and
-// advances the 64-bit descriptors by immediate-like steps (in 16-byte units of the descriptor's address field).
-__device__ __forceinline__ void mma4_ss(uint32_t d, uint64_t a, uint64_t b, uint64_t sa, uint64_t sb, uint32_t idesc, uint32_t acc_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\tsetp.eq.u32 q, 1, 1;\n\t"
-      "add.s64 a1, %1, %3;\n\tadd.s64 b1, %2, %4;\n\tadd.s64 a2, a1, %3;\n\tadd.s64 b2, b1, %4;\n\t"
-      "add.s64 a3, a2, %3;\n\tadd.s64 b3, b2, %4;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %5, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %5, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %5, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %5, q;\n\t}" ::"r"(d),
-      "l"(a), "l"(b), "l"(sa), "l"(sb), "r"(idesc), "r"(acc_first)
-      : "memory");
-}
-// ... with the A operand in TMEM at four given column addresses
-__device__ __forceinline__ void mma4_ts(uint32_t d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint64_t b, uint64_t sb,
-                                        uint32_t idesc, uint32_t acc_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 b1, b2, b3;\n\t"
-      "setp.ne.b32 p, %8, 0;\n\tsetp.eq.u32 q, 1, 1;\n\t"
-      "add.s64 b1, %5, %6;\n\tadd.s64 b2, b1, %6;\n\tadd.s64 b3, b2, %6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %5, %7, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], b1, %7, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], b2, %7, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%4], b3, %7, q;\n\t}" ::"r"(d),
-      "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(b), "l"(sb), "r"(idesc), "r"(acc_first)
-      : "memory");
-}
-
 // ------------------------------------------------------------- TMA producer --
 template <int D, int kC, typename TG, int kMode, bool kOutDelta>
 __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params& p, const CUtensorMap* tmK, const CUtensorMap* tmV,

@@ -16,15 +16,23 @@
 //   S_r  = Q_rj K_i^T    tcgen05.mma  M = rows, N = keys   (rows on TMEM lanes)
 //   O_r  = P_r  V_i      tcgen05.mma  A = P (bf16, TMEM), B = V_i (MN-major smem)
 //
-// Warp roles (512 threads):
-//   warp 0      TMA producer: K_i, V_i once; K_j and Q_rj tiles through mbarrier rings
-//   warp 1      MMA issuer (one elected thread issues every tcgen05.mma / commit)
+// Warp roles (512 threads; 48 / 112 / 176 registers for the roles, the decay group and the softmax groups):
+//   warp 0      TMA producer: K_i, V_i once; K_j and Q_rj tiles through a ring of two slots
+//   warp 1      issues G and S, warp 2 P V (one elected thread each, so that no product waits behind one whose operands are not there yet)
+//   warp 3      writes the rows before a chunk
 //   warps 4-7   decay group: thread = key.  Reads G from TMEM, computes the
 //               log-retention, scans it along the rows in registers (carry kept
 //               across tiles), writes the prefix C^T[row][key] to shared memory.
-//   warps 8-15  two softmax groups alternating over (tile, r): thread = row.
-//               S + C, row max / sum in registers (no shuffles), P -> TMEM as
-//               bf16, then the epilogue O / l -> out and m + log l -> lse.
+//   warps 8-15  two softmax groups alternating over (tile, r): thread = row.  The row of scores is read into registers once (S is free for
+//               the other group then), S + C, row max / sum in registers (no shuffles), P -> TMEM as bf16 in a buffer of the group's own,
+//               m + log l -> lse.  O / l of a head is written while the next head's P is formed, so no group waits for a product.
+//
+// What bounds it: the exponentials and logarithms (XU pipe, half of the cycles at R = 4), issue slots (half), and instruction fetch.  The
+// loops of the decay and the softmax warps run side by side on every scheduler, and beyond some 800 instructions together they stall on
+// fetching them: rows per pass of the decay loop, loops left rolled (unroll 1) and the length of a wait's slow path are chosen for that.  At B4 H8 R4
+// L4096 D64: 0.50 of three active warps waits for instructions; 1.4 of them did with 64 rows per pass of the decay loop (730 -> 860 us).
+// B4 H8 R4 L4096 D64 935 -> 730 us, B1 H8 R4 L8192 D128 1295 -> 1045, B1 H16 R1 L4096 D128 315 -> 279, against the form with two
+// passes over TMEM per head, outputs written from registers and one issuing thread.
 //
 // The two reductions of the operator run along perpendicular axes of the tile
 // (scan along rows per key, softmax along keys per row); putting keys on lanes
@@ -117,33 +125,32 @@ struct FwdCfg {
   static constexpr int kTileBytes = 128 * D * 2;   // one [128][D] bf16 tile
   static constexpr int kBoxBytes = 128 * 128;      // one TMA box: 128 rows x 64 elements
   static constexpr int kBoxes = D / 64;
-  static constexpr bool kOneSlot = (D == 128);      // K_j and Q tiles share one slot
-  static constexpr int kKjStages = kOneSlot ? 0 : 2;
-  static constexpr int kQStages = kOneSlot ? 1 : 2;
   static constexpr int kOBufs = (D == 64) ? 2 : 1;
   static constexpr int oKi = 0;
   static constexpr int oVi = oKi + kTileBytes;
-  static constexpr int oKj = oVi + kTileBytes;
-  static constexpr int oQ = oKj + kKjStages * kTileBytes;
-  // The decay prefix crosses from keys-on-lanes to rows-on-lanes through 64 KB fp32 tiles C^T[row][key]; with two of them the decay
-  // group is a tile ahead of the softmax groups.  At head_dim 128 that leaves shared memory for ONE 32 KB slot, which K_j and Q
-  // tiles pass through in the order of their products (each is read for 0.3 us, and the next one is needed 2 us later); with two
-  // slots for Q, one for K_j and a single C^T tile the groups took turns: B1 H8 R4 L8192 D128 1523 -> 1312 us.
-  static constexpr int kCBufs = 2;
-  static constexpr int oCs = oQ + kQStages * kTileBytes;
-  static constexpr int oT3 = oCs + kCBufs * 65536;
-  static constexpr int oBar = oT3 + 1024;
+  // two slots that K_j and Q tiles pass through in the order of their products
+  static constexpr int oSlot = oVi + kTileBytes;
+  // The decay prefix crosses from keys-on-lanes to rows-on-lanes through fp32 tiles C^T[128 rows][128 keys] of 64 KB.  With two of them the decay
+  // group is a tile ahead of the softmax groups.  head_dim 128 has room for one, which is handed over in halves of 64 rows: a half
+  // is written while the softmax groups, done with the prefix of the tile before it, form the exponentials of its last heads.
+  static constexpr bool kHalves = (D == 128);
+  static constexpr int kCBufs = kHalves ? 1 : 2;
+  static constexpr int oCs = oSlot + 2 * kTileBytes;
+  // 4 KB per softmax warp, from which 64 columns of its 32 output rows leave as one TMA store
+  static constexpr int oStage = oCs + kCBufs * 65536;
+  static constexpr int oT3 = oStage + 8 * 4096;
+  static constexpr int oBar = oT3 + 1536;
   static constexpr int oMisc = oBar + 256;
-  static constexpr int oFill = oMisc + 64;                // bf16[D]: value of a fully masked output row
-  static constexpr int kSmemBytes = oFill + 256 + 1024;  // + slack to align the base to 1024 B
+  static constexpr int oFill = oMisc + 64;               // 1 KB: rows of a fully masked tile
+  static constexpr int kSmemBytes = oFill + 1024;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
-  static constexpr uint32_t tG = 0, tS0 = 128, tS1 = 256, tO0 = 384, tO1 = 384 + D;
+  static constexpr uint32_t tG = 0, tS = 128, tP = 256, tO = 384;      // (two P buffers of 64 columns; O: kOBufs buffers of D)
 };
 
 enum FwdBar {
-  // (kCReady / kCFree: one barrier per C^T buffer, so that no waiter can fall two phases behind on a shared one)
-  kKvFull = 0, kKjFull = 1, kKjEmpty = 3, kQFull = 5, kQEmpty = 7, kGFull = 9, kGFree = 10, kCReady = 11, kCFree = 13,
-  kSFull = 15, kPReady = 17, kOFull = 19, kOFree = 21, kT3Ready = 23, kNumBars = 24
+  // (kCReady / kCFree: per C^T buffer or half buffer; kSFull .. kOFree: one per softmax group, so that no waiter can fall two phases behind)
+  kKvFull = 0, kSlotFull = 1, kSlotEmpty = 3, kGFull = 5, kGFree = 6, kT3Ready = 7, kCReady = 8, kCFree = 10,
+  kSFull = 12, kSFree = 14, kPReady = 16, kOFull = 18, kOFree = 20, kNumBars = 22
 };
 
 template <int D>
@@ -175,124 +182,96 @@ __device__ __forceinline__ void fwd_producer(const FwdCtx<D>& c, const FwdParams
     tma_load_2d(sbase + Cfg::oKi + b * Cfg::kBoxBytes, tmK, b * 64, krow, c.bar(kKvFull));
     if (!kCarryOnly) tma_load_2d(sbase + Cfg::oVi + b * Cfg::kBoxBytes, tmV, b * 64, krow, c.bar(kKvFull));
   }
-  int use = 0;                          // of the one slot (head_dim 128)
-  auto load_slot = [&](const CUtensorMap* tm, int y) -> bool {
-    if (use >= 1 && !c.wait(kQEmpty, use - 1)) return false;
-    mbar_expect_tx(c.bar(kQFull), Cfg::kTileBytes);
-    for (int b = 0; b < Cfg::kBoxes; ++b) tma_load_2d(sbase + Cfg::oQ + b * Cfg::kBoxBytes, tm, b * 64, y, c.bar(kQFull));
+  int use = 0;
+  auto load = [&](const CUtensorMap* tm, int y) -> bool {
+    const int sl = use & 1;
+    if (use >= 2 && !c.wait(kSlotEmpty + sl, (use >> 1) - 1)) return false;
+    mbar_expect_tx(c.bar(kSlotFull + sl), Cfg::kTileBytes);
+    for (int b = 0; b < Cfg::kBoxes; ++b)
+      tma_load_2d(sbase + Cfg::oSlot + sl * Cfg::kTileBytes + b * Cfg::kBoxBytes, tm, b * 64, y, c.bar(kSlotFull + sl));
     ++use;
     return true;
   };
-  auto load_kj = [&](int T) -> bool {
-    if constexpr (Cfg::kOneSlot) return load_slot(tmK, c.bh * L + c.row0 + T * 128);
-    const int ks = T & 1, u = T >> 1;
-    if (u >= 1 && !c.wait(kKjEmpty + ks, u - 1)) return false;
-    mbar_expect_tx(c.bar(kKjFull + ks), Cfg::kTileBytes);
-    for (int b = 0; b < Cfg::kBoxes; ++b)
-      tma_load_2d(sbase + Cfg::oKj + ks * Cfg::kTileBytes + b * Cfg::kBoxBytes, tmK, b * 64, c.bh * L + c.row0 + T * 128,
-                  c.bar(kKjFull + ks));
+  const int krow0 = c.bh * L + c.row0;
+  if (!load(tmK, krow0)) return;
+#pragma unroll 1
+  for (int T = 0; T < c.ntiles; ++T)
+    for (int r = 0; r < (kCarryOnly ? 1 : R); ++r) {
+      if (!kCarryOnly && !load(tmQ, (c.bh * R + r) * p.Lr + c.srow0 + T * 128)) return;
+      if (r == 0 && T + 1 < c.ntiles && !load(tmK, krow0 + (T + 1) * 128)) return;
+    }
+}
+
+// --------------------------------------------------------------- MMA issuers --
+// Two threads, so that no product waits behind one whose operands are not there yet: G and S (everything that needs loaded tiles only)
+// come from one, P V from the other.
+// D[128 x 128] = A[128][D] * B[128][D]^T, both K-major: a k-step of 16 elements is +32 B (2 in the descriptor's units of
+// 16 bytes), the second 64-element box of a tile +16384 B (1024)
+template <int D>
+__device__ __forceinline__ void issue_kmajor(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+  mma4_ss(d_tmem, desc_from_lo(a_lo), desc_from_lo(b_lo), 2, 2, idesc, 0);
+  if (D == 128) mma4_ss(d_tmem, desc_from_lo(a_lo + 1024), desc_from_lo(b_lo + 1024), 2, 2, idesc, 1);
+}
+
+template <int D, int kC, bool kCarryOnly>
+__device__ __forceinline__ void fwd_mma_scores(const FwdCtx<D>& c, const FwdParams& p) {
+  using Cfg = FwdCfg<D>;
+  const uint32_t sbase = smem_u32(c.smem);
+  constexpr uint32_t idesc_g = idesc_bf16(128, 128, 0, 0), idesc_s = idesc_bf16(128, kC, 0, 0);
+  const uint32_t kKi = desc_lo(sbase + Cfg::oKi, 16), kSlot = desc_lo(sbase + Cfg::oSlot, 16);
+  int use = 0;
+  auto slot_full = [&]() -> bool { return c.wait(kSlotFull + (use & 1), use >> 1); };
+  auto slot = [&]() -> uint32_t { return kSlot + (use & 1) * (Cfg::kTileBytes >> 4); };
+  auto slot_done = [&]() { tc_commit(c.bar(kSlotEmpty + (use++ & 1))); };
+  auto issue_g = [&](int T) -> bool {
+    if (!slot_full()) return false;
+    if (T >= 1 && !c.wait(kGFree, T - 1)) return false;
+    tc_fence_after();
+    issue_kmajor<D>(c.tmem + Cfg::tG, kKi, slot(), idesc_g);
+    tc_commit(c.bar(kGFull));
+    slot_done();
     return true;
   };
-  if (!load_kj(0)) return;
-  if (kCarryOnly) {
-    for (int T = 1; T < c.ntiles; ++T)
-      if (!load_kj(T)) return;
-    return;
-  }
+  if (!c.wait(kKvFull, 0)) return;
+  if (!issue_g(0)) return;
   int t = 0;
+#pragma unroll 1
   for (int T = 0; T < c.ntiles; ++T) {
-    for (int r = 0; r < R; ++r, ++t) {
-      if constexpr (Cfg::kOneSlot) {
-        if (!load_slot(tmQ, (c.bh * R + r) * p.Lr + c.srow0 + T * 128)) return;
-        if (r == 0 && T + 1 < c.ntiles && !load_kj(T + 1)) return;
-        continue;
+    for (int r = 0; r < (kCarryOnly ? 1 : p.s.R); ++r, ++t) {
+      if (!kCarryOnly) {
+        if (!slot_full()) return;
+        if (t >= 1 && !c.wait(kSFree + ((t - 1) & 1), (t - 1) >> 1)) return;
+        tc_fence_after();
+        issue_kmajor<D>(c.tmem + Cfg::tS, slot(), kKi, idesc_s);
+        tc_commit(c.bar(kSFull + (t & 1)));
+        slot_done();
       }
-      const int qs = t & 1, u = t >> 1;
-      if (u >= 1 && !c.wait(kQEmpty + qs, u - 1)) return;
-      mbar_expect_tx(c.bar(kQFull + qs), Cfg::kTileBytes);
-      for (int b = 0; b < Cfg::kBoxes; ++b)
-        tma_load_2d(sbase + Cfg::oQ + qs * Cfg::kTileBytes + b * Cfg::kBoxBytes, tmQ, b * 64,
-                    (c.bh * R + r) * p.Lr + c.srow0 + T * 128, c.bar(kQFull + qs));
-      if (r == 0 && T + 1 < c.ntiles && !load_kj(T + 1)) return;
+      // (the decay group gives G back shortly before the prefix of tile T is complete, without which no other head of the tile can go on)
+      if (r == 0 && T + 1 < c.ntiles && !issue_g(T + 1)) return;
     }
   }
 }
 
-// ---------------------------------------------------------------- MMA issuer --
-template <int D, int kC, bool kCarryOnly, int kOut>
-__device__ __forceinline__ void fwd_mma(const FwdCtx<D>& c, const FwdParams& p) {
+template <int D, int kC>
+__device__ __forceinline__ void fwd_mma_pv(const FwdCtx<D>& c, const FwdParams& p) {
   using Cfg = FwdCfg<D>;
-  const int R = p.s.R;
-  const uint32_t sbase = smem_u32(c.smem);
-  constexpr uint32_t idesc_g = idesc_bf16(128, 128, 0, 0), idesc_s = idesc_bf16(128, kC, 0, 0);
   constexpr uint32_t idesc_pv = idesc_bf16(128, D, 0, 1);
-  const uint32_t tS[2] = {c.tmem + Cfg::tS0, c.tmem + Cfg::tS1};
-  const uint32_t tO[2] = {c.tmem + Cfg::tO0, c.tmem + (Cfg::kOBufs == 2 ? Cfg::tO1 : Cfg::tO0)};
-
-  // D[128 x 128] = A[128][D] * B[128][D]^T, both K-major.  Operands are passed as descriptor low words
-  // (built once: shared-memory addresses never change); a k-step of 16 elements is +32 B (>>4 = 2), the
-  // second 64-element box of a tile +16384 B (>>4 = 1024).
-  auto issue_kmajor = [&](uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
-    mma_ss_c<false>(d_tmem, desc_from_lo(a_lo), desc_from_lo(b_lo), idesc);
-#pragma unroll
-    for (int ks = 1; ks < D / 16; ++ks) {
-      const uint32_t off = (ks >> 2) * 1024 + (ks & 3) * 2;
-      mma_ss_c<true>(d_tmem, desc_from_lo(a_lo + off), desc_from_lo(b_lo + off), idesc);
-    }
-  };
-  const uint32_t kKi = desc_lo(sbase + Cfg::oKi, 16);
-  const uint32_t mVi = desc_lo(sbase + Cfg::oVi, Cfg::kBoxBytes);
-  int use = 0;                          // of the one slot (head_dim 128)
-  auto issue_g = [&](int T) -> bool {
-    const int ks = T & 1, u = T >> 1;
-    if (Cfg::kOneSlot ? !c.wait(kQFull, use++) : !c.wait(kKjFull + ks, u)) return false;
-    if (T >= 1 && !c.wait(kGFree, T - 1)) return false;
-    tc_fence_after();
-    issue_kmajor(c.tmem + Cfg::tG, kKi, desc_lo(sbase + (Cfg::kOneSlot ? Cfg::oQ : Cfg::oKj + ks * Cfg::kTileBytes), 16), idesc_g);
-    tc_commit(c.bar(kGFull));
-    tc_commit(c.bar(Cfg::kOneSlot ? kQEmpty : kKjEmpty + ks));
-    return true;
-  };
-  auto issue_pv = [&](int tt) -> bool {
-    const int sb = tt & 1, ob = tt % Cfg::kOBufs;
-    if (!c.wait(kPReady + sb, tt >> 1)) return false;       // (statistics only: the group is done with the S buffer)
-    if (kOut == kOutStats) return true;
-    // the O buffer must have been drained by the epilogue that used it last
-    // (barriers are per softmax group so that each waiter sees consecutive phases)
-    if (Cfg::kOBufs == 2) {
-      if (tt >= 2 && !c.wait(kOFree + sb, (tt >> 1) - 1)) return false;
-    } else {
-      if (tt >= 1 && !c.wait(kOFree + ((tt - 1) & 1), (tt - 1) >> 1)) return false;
-    }
-    tc_fence_after();
-    mma_ts_c<false>(tO[ob], tS[sb], desc_from_lo(mVi), idesc_pv);
-#pragma unroll
-    for (int ks = 1; ks < kC / 16; ++ks) mma_ts_c<true>(tO[ob], tS[sb] + ks * 8, desc_from_lo(mVi + ks * 128), idesc_pv);
-    tc_commit(c.bar(kOFull + sb));
-    return true;
-  };
-
+  const uint32_t mVi = desc_lo(smem_u32(c.smem) + Cfg::oVi, Cfg::kBoxBytes);
+  const int heads = c.ntiles * p.s.R;
   if (!c.wait(kKvFull, 0)) return;
-  if (!issue_g(0)) return;
-  if (kCarryOnly) {
-    for (int T = 1; T < c.ntiles; ++T)
-      if (!issue_g(T)) return;
-    return;
+#pragma unroll 1
+  for (int t = 0; t < heads; ++t) {
+    const int sb = t & 1;
+    const uint32_t tP = c.tmem + Cfg::tP + sb * 64, tO = c.tmem + Cfg::tO + (t % Cfg::kOBufs) * D;
+    if (!c.wait(kPReady + sb, t >> 1)) return;
+    // (two O buffers: a group drains its own before it hands over its next P)
+    if (Cfg::kOBufs == 1 && t >= 1 && !c.wait(kOFree + (sb ^ 1), (t - 1) >> 1)) return;
+    tc_fence_after();
+#pragma unroll
+    for (int ks = 0; ks < kC / 16; ks += 4)
+      mma4_ts(tO, tP + ks * 8, tP + ks * 8 + 8, tP + ks * 8 + 16, tP + ks * 8 + 24, desc_from_lo(mVi + ks * 128), 128, idesc_pv, ks > 0);
+    tc_commit(c.bar(kOFull + sb));
   }
-  int t = 0;
-  for (int T = 0; T < c.ntiles; ++T) {
-    for (int r = 0; r < R; ++r, ++t) {
-      const int qs = Cfg::kOneSlot ? 0 : t & 1;
-      if (!c.wait(kQFull + qs, Cfg::kOneSlot ? use++ : t >> 1)) return;
-      tc_fence_after();
-      issue_kmajor(tS[t & 1], desc_lo(sbase + Cfg::oQ + qs * Cfg::kTileBytes, 16), kKi, idesc_s);
-      tc_commit(c.bar(kSFull + (t & 1)));
-      tc_commit(c.bar(kQEmpty + qs));
-      if (t >= 1 && !issue_pv(t - 1)) return;
-      if (r == 0 && T + 1 < c.ntiles && !issue_g(T + 1)) return;
-    }
-  }
-  if (t >= 1) issue_pv(t - 1);
 }
 
 // --------------------------------------------------------------- decay group --
@@ -308,7 +287,6 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
   auto gate_at = [&](int T) -> float { return (kC == 128 || c.row0 + T * 128 + k < L) ? Num<TG>::ld(sd + T * 128) : 0.f; };
   const bool live = k < kC;              // kC = 64: warps 6-7 hold no key and only fetch gates
   const float s3 = live ? cbrtf(Num<TG>::ld(ss + c.i * kC + k)) : 0.f;
-  float raw_next = gate_at(0);           // the gate value of the next tile is fetched one pass ahead: its latency hides behind the pass
   float* sT3 = reinterpret_cast<float*>(c.smem + Cfg::oT3);
   uint8_t* sCs = c.smem + Cfg::oCs;
   const size_t chunk_id = (size_t)c.bh * p.s.N + c.i, key_id = chunk_id * 128 + k;
@@ -322,13 +300,23 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     carry = sum;
   };
   if (live)
+#pragma unroll 1
     for (int T = 0; T < c.t0; ++T) add_to_carry(carry_lo + p.tile_totals[(chunk_id * p.tiles + T) * 128 + k]);
+  // static_dest^(1/3) of a tile's rows is formed a tile ahead (its gate value fetched another one before), so that the barrier behind which all
+  // four warps may read it is long complete when it is looked at.  Three buffers: a warp may still read tile T - 1's while another writes T + 1's.
+  sT3[k] = cbrtf(gate_at(0));
+  c.arrive_w(kT3Ready);
+  float raw_next = c.ntiles > 1 ? gate_at(1) : 0.f;
+  const uint32_t cst = smem_u32(c.smem + Cfg::oCs) + 4 * k;
+#pragma unroll 1
   for (int T = 0; T < c.ntiles; ++T) {
-    float* t3buf = sT3 + (T & 1) * 128;
-    t3buf[k] = cbrtf(raw_next);
-    if (T + 1 < c.ntiles) raw_next = gate_at(T + 1);
-    c.arrive_w(kT3Ready);
+    const float* t3buf = sT3 + T % 3 * 128;
     if (!c.wait_w(kT3Ready, T)) return;
+    if (T + 1 < c.ntiles) {
+      sT3[(T + 1) % 3 * 128 + k] = cbrtf(raw_next);
+      c.arrive_w(kT3Ready);
+      if (T + 2 < c.ntiles) raw_next = gate_at(T + 2);
+    }
     if (!live) continue;
     if (!c.wait_w(kGFull, T)) return;
     tc_fence_after();
@@ -336,132 +324,228 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     float* carry_row = p.carry ? p.carry + (chunk_id * (L / 64) + (c.row0 + T * 128) / 64) * 128 + k : nullptr;
     if (carry_row) carry_row[0] = carry;
     // The prefix inside a tile is  carry + (carry_lo + sum of the totals of earlier 32-row blocks + scan inside the block).
-    float tprev = carry_lo, cval = carry;
-#pragma unroll 1
-    for (int cb = 0; cb < 4; ++cb) {
-      uint32_t g[32];
-      tmem_ld32(c.tmem + Cfg::tG + lane_base + cb * 32, g);
-      tc_wait_ld();
-      if (cb == 3) {
-        tc_fence_before();
-        c.arrive_w(kGFree);
-      }
-      if (cb == 2 && carry_row && (kC == 128 || c.row0 + T * 128 + 64 < L)) carry_row[128] = cval;      // prefix after the first 64 rows of the tile
-      float v[32], t3r[32];
+    float tprev = carry_lo, cval = carry, local = 0.f;
+    const uint32_t cdst = cst + T % Cfg::kCBufs * 65536;
+    // Sixteen rows at a time, two at once with packed fp32 arithmetic, in two stages: retention() = 1 - min(a, hi) of the rows,
+    // prefix() = its logarithm, the scan, and C^T.  One stage of a block runs beside the other of the block before it: a warp alone on its
+    // scheduler would otherwise wait for the chain of three logarithms and exponentials at the end of every block.
+    auto retention = [&](uint32_t* g, int q0) {
+      const float2 k23 = make_float2(2.0f / 3.0f, 2.0f / 3.0f), s32 = make_float2(s3, s3), one2 = make_float2(1.0f, 1.0f),
+                   mone2 = make_float2(-1.0f, -1.0f);
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        const float4 t4 = reinterpret_cast<const float4*>(t3buf + cb * 32)[x];
-        t3r[4 * x] = t4.x; t3r[4 * x + 1] = t4.y; t3r[4 * x + 2] = t4.z; t3r[4 * x + 3] = t4.w;
-      }
-      float local = 0.f;
-      // (the diagonal tile is the only one with masked pairs: its tests are compiled into a path of its own)
-      auto scan32 = [&](auto on_diag) {
-        constexpr bool kDiag = decltype(on_diag)::value;
-        const float2 k23 = make_float2(2.0f / 3.0f, 2.0f / 3.0f), s32 = make_float2(s3, s3), one2 = make_float2(1.0f, 1.0f),
-                     mone2 = make_float2(-1.0f, -1.0f), ln2 = make_float2(0.6931471805599453f, 0.6931471805599453f);
+      for (int x = 0; x < 16; x += 4) {
+        const float4 t4 = reinterpret_cast<const float4*>(t3buf + q0)[x / 4];
 #pragma unroll
-        for (int x = 0; x < 32; x += 2) {
-          // two rows at a time with packed fp32 arithmetic: relu(g)^(2/3) through lg2(max(g, 0)) = -inf for g <= 0
-          const float2 lg = make_float2(lg2(fmaxf(__uint_as_float(g[x]), 0.f)), lg2(fmaxf(__uint_as_float(g[x + 1]), 0.f)));
+        for (int y = 0; y < 4; y += 2) {
+          // relu(g)^(2/3) through lg2(max(g, 0)) = -inf for g <= 0
+          const float2 lg = make_float2(lg2(fmaxf(__uint_as_float(g[x + y]), 0.f)), lg2(fmaxf(__uint_as_float(g[x + y + 1]), 0.f)));
           const float2 e23 = fmul2(lg, k23);
           const float2 pw = make_float2(ex2(e23.x), ex2(e23.y));
-          const float2 a = fmul2(fmul2(pw, s32), make_float2(t3r[x], t3r[x + 1]));
+          const float2 a = fmul2(fmul2(pw, s32), y ? make_float2(t4.z, t4.w) : make_float2(t4.x, t4.y));
           const float2 om = ffma2(make_float2(fminf(a.x, clamp_hi()), fminf(a.y, clamp_hi())), mone2, one2);
-          const float2 el = fmul2(make_float2(lg2(om.x), lg2(om.y)), ln2);
-          const int q = cb * 32 + x;
-          float2 run;
-          run.x = local + (kDiag && q <= k ? 0.f : el.x);
-          run.y = local = run.x + (kDiag && q + 1 <= k ? 0.f : el.y);
-          const float2 cv = fadd2(make_float2(carry, carry), fadd2(make_float2(tprev, tprev), run));
-          cval = cv.y;
-          v[x] = (kDiag && q < k) ? mask_value() : cv.x;
-          v[x + 1] = (kDiag && q + 1 < k) ? mask_value() : cv.y;
-        }
-      };
-      if (diag) scan32(std::true_type{});
-      else scan32(std::false_type{});
-      tprev += local;
-      if (!kCarryOnly) {
-        if (cb == 0 && T >= Cfg::kCBufs && !c.wait_w(kCFree + T % Cfg::kCBufs, T / Cfg::kCBufs - 1)) return;
-#pragma unroll
-        for (int x = 0; x < 32; ++x) {
-          const int q = cb * 32 + x;
-          *reinterpret_cast<float*>(sCs + (T % Cfg::kCBufs) * 65536 + q * 512 + ((((k >> 2) ^ (q & 7)) & 31) << 4) + (k & 3) * 4) = v[x];
+          g[x + y] = __float_as_uint(om.x);
+          g[x + y + 1] = __float_as_uint(om.y);
         }
       }
-    }
+    };
+    // (the diagonal tile is the only one with masked pairs: its tests are compiled into a path of their own)
+    auto prefix = [&](const uint32_t* om, int q0, auto on_diag) {
+      constexpr bool kDiag = decltype(on_diag)::value;
+      const float2 ln2 = make_float2(0.6931471805599453f, 0.6931471805599453f);
+#pragma unroll
+      for (int x = 0; x < 16; x += 2) {
+        const float2 el = fmul2(make_float2(lg2(__uint_as_float(om[x])), lg2(__uint_as_float(om[x + 1]))), ln2);
+        const int q = q0 + x;
+        float2 run;
+        run.x = local + (kDiag && q <= k ? 0.f : el.x);
+        run.y = local = run.x + (kDiag && q + 1 <= k ? 0.f : el.y);
+        const float2 cv = fadd2(make_float2(carry, carry), fadd2(make_float2(tprev, tprev), run));
+        cval = cv.y;
+        if (!kCarryOnly) {
+          st_shared_f1((cdst ^ ((x & 7) << 4)) + q * 512, (kDiag && q < k) ? mask_value() : cv.x);
+          st_shared_f1((cdst ^ (((x + 1) & 7) << 4)) + (q + 1) * 512, (kDiag && q + 1 < k) ? mask_value() : cv.y);
+        }
+      }
+    };
+    const uint32_t tg = c.tmem + Cfg::tG + lane_base;
+    auto tile = [&](auto on_diag) -> bool {
+      uint32_t ga[16], gb[16];
+      tmem_ld16(tg, ga);
+      tmem_ld16(tg + 16, gb);
+      if (!kCarryOnly && T >= Cfg::kCBufs && !c.wait_w(kCFree + T % Cfg::kCBufs, T / Cfg::kCBufs - 1)) return false;      // (halves: the first one)
+      tc_wait_ld();
+      retention(ga, 0);
+#pragma unroll 1
+      for (int cb = 0; cb < 4; ++cb) {
+        retention(gb, cb * 32 + 16);
+        prefix(ga, cb * 32, on_diag);
+        if (cb < 3) {
+          tmem_ld16(tg + cb * 32 + 32, ga);
+          tc_wait_ld();
+          retention(ga, cb * 32 + 32);
+        }
+        prefix(gb, cb * 32 + 16, on_diag);
+        if (cb < 3) {
+          tmem_ld16(tg + cb * 32 + 48, gb);
+          tc_wait_ld();
+        }
+        if (cb == 2) {
+          tc_fence_before();
+          c.arrive_w(kGFree);
+        }
+        if (Cfg::kHalves && !kCarryOnly && cb == 1) {
+          c.arrive_w(kCReady);
+          if (T >= 1 && !c.wait_w(kCFree + 1, T - 1)) return false;
+        }
+        tprev += local;
+        local = 0.f;
+        if (cb == 1 && carry_row && (kC == 128 || c.row0 + T * 128 + 64 < L)) carry_row[128] = cval;      // prefix after the first 64 rows of the tile
+      }
+      return true;
+    };
+    if (!(diag ? tile(std::true_type{}) : tile(std::false_type{}))) return;
     add_to_carry(tprev);      // (tprev = carry_lo + the tile's total)
-    if (!kCarryOnly) c.arrive_w(kCReady + T % Cfg::kCBufs);
+    if (!kCarryOnly) c.arrive_w(kCReady + (Cfg::kHalves ? 1 : T % Cfg::kCBufs));
   }
   if (p.total_out) p.total_out[key_id] = carry;
 }
 
 // ------------------------------------------------------------ softmax groups --
+// What a group keeps of a head until its PV product is there: the output is written while the NEXT head's probabilities are formed.
+struct FwdPending {
+  size_t row;        // (chunk, head, row) of the slab, or (b, h, r, row) in merged-output mode
+  float scale;       // 1 / l, or the chunk's weight in the row's softmax over all keys
+  bool in_range;
+};
+
+// 64 columns of the output on their way into registers (thread = row)
+template <int D>
+__device__ __forceinline__ void fwd_out_load(const FwdCtx<D>& c, int me, int cb, uint32_t* o) {
+  const uint32_t tO = c.tmem + FwdCfg<D>::tO + (FwdCfg<D>::kOBufs == 2 ? me * D : 0) + ((uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16) + cb * 64;
+#pragma unroll
+  for (int x = 0; x < 4; ++x) tmem_ld16(tO + 16 * x, o + 16 * x);
+}
+
+// o: the first 64 columns.  The warp's 32 rows leave as TMA stores from its 4 KB of shared memory (stored from registers, row by row or in whole
+// lines behind shuffles, they kept the load-store unit busy that the decay prefix passes through: B1 H8 R4 L8192 D128 6.7k of 21k cycles per tile, now 3.1k of 17k).
+template <int D, int kOut>
+__device__ __forceinline__ void fwd_out_store(const FwdCtx<D>& c, const FwdParams& p, const CUtensorMap* tmO, int me, uint32_t* o, const FwdPending& w) {
+  using Cfg = FwdCfg<D>;
+  const int lane = threadIdx.x & 31;
+  auto drained = [&]() {
+    if (Cfg::kOBufs == 1) {
+      tc_fence_before();
+      c.arrive_w(kOFree + me);
+    }
+  };
+  if constexpr (kOut == kOutMerged) {
+    const uint32_t tO = c.tmem + Cfg::tO + (Cfg::kOBufs == 2 ? me * D : 0) + ((uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16);
+    float* dst = p.merged_acc + w.row * D;
+#pragma unroll 1
+    for (int cb = 0; cb < D / 32; ++cb) {
+      uint32_t v[32];
+      tmem_ld32(tO + cb * 32, v);
+      tc_wait_ld();
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        red_add_v4(dst + cb * 32 + 4 * u, __uint_as_float(v[4 * u]) * w.scale, __uint_as_float(v[4 * u + 1]) * w.scale,
+                   __uint_as_float(v[4 * u + 2]) * w.scale, __uint_as_float(v[4 * u + 3]) * w.scale);
+    }
+    drained();
+    return;
+  }
+  const uint32_t stage = smem_u32(c.smem + Cfg::oStage) + ((threadIdx.x >> 5) - 8) * 4096, mine = stage + lane * 128 + ((lane & 7) << 4);
+  const float2 scale2 = make_float2(w.scale, w.scale);
+#pragma unroll 1
+  for (int cb = 0; cb < D / 64; ++cb) {
+    if (lane == 0) bulk_wait_read<0>();                    // the store before has read the 4 KB
+    __syncwarp();
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      uint32_t pk[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 ov = fmul2(make_float2(__uint_as_float(o[8 * x + 2 * u]), __uint_as_float(o[8 * x + 2 * u + 1])), scale2);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(ov.x, ov.y);
+        pk[u] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      st_shared_v4(mine ^ (x << 4), pk);
+    }
+    if (cb + 1 < D / 64) fwd_out_load<D>(c, me, cb + 1, o);
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0 && w.in_range) {                         // (chunks of 64 keys: half a tile at the end of the sequence, whole warps of it)
+      tma_store_2d(tmO, cb * 64, (int)w.row, stage);
+      bulk_commit_group();
+    }
+    if (cb + 1 < D / 64) {
+      tc_wait_ld();
+      drained();                                           // (D <= 128)
+    }
+  }
+}
+
 template <int D, int kC, int kOut>
-__device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams& p, int me) {
+__device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams& p, const CUtensorMap* tmO, int me) {
   constexpr bool kMerge = (kOut == kOutMerged);
   using Cfg = FwdCfg<D>;
   const int R = p.s.R, N = p.s.N;
   const int row = threadIdx.x & 127;
   const uint32_t lane_base = (uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16;
-  const uint8_t* sCrow0 = c.smem + Cfg::oCs + row * 512;
+  const uint32_t crow0 = smem_u32(c.smem + Cfg::oCs) + row * 512 + ((row & 7) << 4);      // (16-byte piece x of a row lies at piece x ^ (row % 8))
   const size_t chunk_id = (size_t)c.bh * N + c.i;
   const float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+  const uint32_t tS = c.tmem + Cfg::tS + lane_base, tP = c.tmem + Cfg::tP + me * 64 + lane_base;
+  constexpr int kEarly = 3;        // quarters of a head's exponentials before the loads of the last head's output
+  FwdPending pend;
+  int n = 0;                       // heads this group has taken
   int t = 0;
+#pragma unroll 1
   for (int T = 0; T < c.ntiles; ++T) {
     // Every softmax thread observes every phase of c_ready and arrives on c_free exactly
     // once per tile (after its last read of C in that tile), whether or not its group has
     // a head to process in this tile; parity waits stay within one phase of the barrier.
-    const int cbuf = T % Cfg::kCBufs;
-    const uint8_t* sCrow = sCrow0 + cbuf * 65536;
+    const int cbuf = Cfg::kHalves ? row >> 6 : T % Cfg::kCBufs;      // (its barriers; halves: of the one that holds the warp's rows)
+    const uint32_t crow = crow0 + (T % Cfg::kCBufs) * 65536;
     if (!c.wait_w(kCReady + cbuf, T / Cfg::kCBufs)) return;
     int last_r = -1;
+#pragma unroll 1
     for (int r = R - 1; r >= 0; --r)
       if (((T * R + r) & 1) == me) { last_r = r; break; }
     if (last_r < 0) c.arrive_w(kCFree + cbuf);
+#pragma unroll 1
     for (int r = 0; r < R; ++r, ++t) {
       if ((t & 1) != me) continue;
-      const int sb = t & 1, ob = t % Cfg::kOBufs;
-      const uint32_t tS = c.tmem + (sb ? Cfg::tS1 : Cfg::tS0) + lane_base;
-      const uint32_t tO = c.tmem + ((Cfg::kOBufs == 2 && ob) ? Cfg::tO1 : Cfg::tO0) + lane_base;
-      if (!c.wait_w(kSFull + sb, t >> 1)) return;
+      if (!c.wait_w(kSFull + me, n)) return;
       tc_fence_after();
-      // pass 1: s = S + C (written back to TMEM), row max.  64 columns per round trip: the two loads are in flight together.
-      float m = -INFINITY;
-#pragma unroll 1
-      for (int cb = 0; cb < kC / 64; ++cb) {
-        uint32_t s[64];
-        tmem_ld32(tS + cb * 64, s);
-        tmem_ld32(tS + cb * 64 + 32, s + 32);
-        tc_wait_ld();
+      // the kC scores of the row stay in registers until their exponentials are formed; the S buffer is free for the other group at once
+      uint32_t s[kC];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int chunk = cb * 16 + u;
-          const float4 cv = *reinterpret_cast<const float4*>(sCrow + (((chunk ^ (row & 7)) & 31) << 4));
-          const float2 a01 = fadd2(make_float2(__uint_as_float(s[u * 4 + 0]), __uint_as_float(s[u * 4 + 1])), make_float2(cv.x, cv.y));
-          const float2 a23 = fadd2(make_float2(__uint_as_float(s[u * 4 + 2]), __uint_as_float(s[u * 4 + 3])), make_float2(cv.z, cv.w));
-          m = fmax3(m, fmax3(a01.x, a01.y, a23.x), a23.y);
-          s[u * 4 + 0] = __float_as_uint(a01.x); s[u * 4 + 1] = __float_as_uint(a01.y);
-          s[u * 4 + 2] = __float_as_uint(a23.x); s[u * 4 + 3] = __float_as_uint(a23.y);
-        }
-        tmem_st32(tS + cb * 64, s);
-        tmem_st32(tS + cb * 64 + 32, s + 32);
+      for (int x = 0; x < kC / 16; ++x) tmem_ld16(tS + x * 16, s + x * 16);
+      tc_wait_ld();
+      tc_fence_before();
+      c.arrive_w(kSFree + me);
+      // s = S + C, row max
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int u = 0; u < kC / 4; ++u) {
+        const float4 cv = ld_shared_f4((crow ^ ((u & 7) << 4)) + (u >> 3) * 128);
+        const float2 a01 = fadd2(make_float2(__uint_as_float(s[u * 4 + 0]), __uint_as_float(s[u * 4 + 1])), make_float2(cv.x, cv.y));
+        const float2 a23 = fadd2(make_float2(__uint_as_float(s[u * 4 + 2]), __uint_as_float(s[u * 4 + 3])), make_float2(cv.z, cv.w));
+        m4[u & 3] = fmax3(fmax3(m4[u & 3], a01.x, a01.y), a23.x, a23.y);
+        s[u * 4 + 0] = __float_as_uint(a01.x); s[u * 4 + 1] = __float_as_uint(a01.y);
+        s[u * 4 + 2] = __float_as_uint(a23.x); s[u * 4 + 3] = __float_as_uint(a23.y);
       }
-      tc_wait_st();
+      const float m = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       if (r == last_r) c.arrive_w(kCFree + cbuf);
-      // pass 2: P = exp(s - m) as bf16 into the first 64 columns of the S buffer
+      // P = exp(s - m) as bf16
       const float mb = m * kLog2e;
       const float2 kL2 = make_float2(kLog2e, kLog2e), nmb2 = make_float2(-mb, -mb);
       float2 l2 = make_float2(0.f, 0.f);
-#pragma unroll 1
-      for (int cb = 0; cb < kC / 64; ++cb) {
-        uint32_t s[64];
-        tmem_ld32(tS + cb * 64, s);
-        tmem_ld32(tS + cb * 64 + 32, s + 32);
-        tc_wait_ld();
-        uint32_t pk[32];
+      uint32_t pk[kC / 2], o[64];
+      auto exponentials = [&](int u0, int u1) {
 #pragma unroll
-        for (int u = 0; u < 32; ++u) {
+        for (int u = u0; u < u1; ++u) {
           const float2 arg = ffma2(make_float2(__uint_as_float(s[2 * u]), __uint_as_float(s[2 * u + 1])), kL2, nmb2);
           const float2 pe = make_float2(ex2(arg.x), ex2(arg.y));
           __nv_bfloat162 h = __floats2bfloat162_rn(pe.x, pe.y);
@@ -470,145 +554,120 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
           l2 = fadd2(l2, pe);
           pk[u] = *reinterpret_cast<uint32_t*>(&h);
         }
-        if (kOut != kOutStats) tmem_st32(tS + cb * 32, pk);
+      };
+      exponentials(0, kC * kEarly / 8);
+      // The head before this one leaves: its product, issued half a head ago, comes out of TMEM behind the second half of the
+      // exponentials (a load takes some 450 cycles beside running products); with it the P buffer is free as well.
+      if (kOut != kOutStats) {
+        if (n >= 1 && !c.wait_w(kOFull + me, n - 1)) return;
+        tc_fence_after();
+        if (kOut == kOutTiles) fwd_out_load<D>(c, me, 0, o);      // (before the first head: loads that nothing looks at)
       }
-      if (kOut != kOutStats) tc_wait_st();
-      tc_fence_before();
-      c.arrive_w(kPReady + sb);
+      exponentials(kC * kEarly / 8, kC / 2);
+      if (kOut != kOutStats) {
+        // (with the next P the next product may overwrite the group's O: what it holds has to be in registers, or added, by then)
+        if (kMerge && n >= 1) fwd_out_store<D, kOut>(c, p, tmO, me, o, pend);
+        tc_wait_ld();
+#pragma unroll
+        for (int cb = 0; cb < kC / 32; ++cb) tmem_st16(tP + cb * 16, pk + cb * 16);
+        tc_wait_st();
+        tc_fence_before();
+        c.arrive_w(kPReady + me);
+        if (!kMerge && n >= 1) fwd_out_store<D, kOut>(c, p, tmO, me, o, pend);
+      }
       const int qg = c.srow0 + T * 128 + row;                       // row index inside the slab
-      const bool in_range = kC == 128 || qg < p.Lr;                 // (kC = 64: the last tile may be half a tile)
       const float l = l2.x + l2.y;
-      const float lse = m + lg2(l) * kLn2;
       const size_t orow = (chunk_id * R + r) * p.Lr + qg;
-      const size_t mrow = ((size_t)c.bh * R + r) * p.Lr + qg;       // the row in (b,h,r,L) order (merged-output mode)
-      float linv;
+      pend.in_range = kC == 128 || qg < p.Lr;                       // (kC = 64: the last tile may be half a tile)
       if (kMerge) {
         // exp(lse - row_lse) / l = exp(m - row_lse): weight of this chunk in the row's softmax over all keys, applied
-        // to the unnormalised P~ V (the load's latency runs under the wait for the PV product)
-        linv = ex2((m - p.row_lse[mrow]) * kLog2e);
+        // to the unnormalised P~ V
+        pend.row = ((size_t)c.bh * R + r) * p.Lr + qg;
+        pend.scale = ex2((m - p.row_lse[pend.row]) * kLog2e);
       } else {
-        if (in_range) p.lse[orow] = lse;
-        if (p.denom && in_range) p.denom[orow] = __float2bfloat16_rn(lse);
-        linv = 1.0f / l;
+        const float lse = m + lg2(l) * kLn2;
+        if (pend.in_range) p.lse[orow] = lse;
+        if (p.denom && pend.in_range) p.denom[orow] = __float2bfloat16_rn(lse);
+        pend.row = orow;
+        pend.scale = 1.0f / l;
       }
-      if (kOut == kOutStats) continue;
-      if (!c.wait_w(kOFull + sb, t >> 1)) return;
-      tc_fence_after();
-      if (kMerge) {
-#pragma unroll 1
-        for (int cb = 0; cb < D / 32; ++cb) {
-          uint32_t o[32];
-          tmem_ld32(tO + cb * 32, o);
-          tc_wait_ld();
-          if (cb == D / 32 - 1) {
-            tc_fence_before();
-            c.arrive_w(kOFree + sb);
-          }
-          float* dst = p.merged_acc + mrow * D + cb * 32;
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            red_add_v4(dst + 4 * u, __uint_as_float(o[4 * u]) * linv, __uint_as_float(o[4 * u + 1]) * linv,
-                       __uint_as_float(o[4 * u + 2]) * linv, __uint_as_float(o[4 * u + 3]) * linv);
-        }
-      } else if constexpr (D == 128) {
-        // head_dim 128: rows leave as whole 128-byte lines, eight rows per store instruction: O is loaded in the fragment order, in
-        // which a quad of threads holds a row, and regrouped to 32 contiguous bytes per thread.  Against the form below: B1 H16 R1 L4096
-        // 331 -> 314 us, 2 x (8 x 2) heads of L1536 87 -> 76 us, B1 H8 R4 L8192 1312 -> 1301 us (at head_dim 64, with half as
-        // much to store per score, the shuffles cost 1 % more than they give).
-        const int lane = threadIdx.x & 31;
-        __nv_bfloat16* out0 = p.out + (orow - lane) * D;      // the warp's first row
-#pragma unroll 1
-        for (int piece = 0; piece < 2 * D / 64; ++piece) {
-          const int hh = piece & 1, cb = piece >> 1;          // 16 of the warp's 32 rows, 64 of the columns
-          uint32_t o[32];
-          tmem_ld_16x64(tO + ((uint32_t)(hh * 16) << 16) + cb * 64, o);
-          const int ra = hh * 16 + (lane >> 2);
-          const float la = __shfl_sync(0xffffffffu, linv, ra), lb = __shfl_sync(0xffffffffu, linv, ra + 8);
-          tc_wait_ld();
-          if (piece == 2 * D / 64 - 1) {
-            tc_fence_before();
-            c.arrive_w(kOFree + sb);
-          }
-          if (!in_range) continue;
-          uint32_t wa[8], wb[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float2 va = fmul2(make_float2(__uint_as_float(o[4 * j]), __uint_as_float(o[4 * j + 1])), make_float2(la, la));
-            const float2 vb = fmul2(make_float2(__uint_as_float(o[4 * j + 2]), __uint_as_float(o[4 * j + 3])), make_float2(lb, lb));
-            const __nv_bfloat162 ha = __floats2bfloat162_rn(va.x, va.y), hb = __floats2bfloat162_rn(vb.x, vb.y);
-            wa[j] = *reinterpret_cast<const uint32_t*>(&ha);
-            wb[j] = *reinterpret_cast<const uint32_t*>(&hb);
-          }
-          quad_gather(wa, lane);
-          quad_gather(wb, lane);
-          __nv_bfloat16* dst = out0 + (size_t)ra * D + cb * 64 + (lane & 3) * 16;
-          st_global_v8(dst, wa);
-          st_global_v8(dst + 8 * D, wb);
-        }
-      } else {
-        // 32 bytes per thread and row: with 16-byte stores every one of a warp's 32 rows got half a sector at a time, and the way from
-        // L1 to L2 was busy half of the time with them (B4 H8 R4 L4096 970 -> 935 us)
-        __nv_bfloat16* orow_ptr = p.out + orow * D;
-#pragma unroll 1
-        for (int cb = 0; cb < D / 32; ++cb) {
-          uint32_t o[32];
-          tmem_ld32(tO + cb * 32, o);
-          tc_wait_ld();
-          if (cb == D / 32 - 1) {
-            tc_fence_before();
-            c.arrive_w(kOFree + sb);
-          }
-          if (!in_range) continue;
-          uint32_t pk[16];
-          const float2 linv2 = make_float2(linv, linv);
-#pragma unroll
-          for (int u = 0; u < 16; ++u) {
-            const float2 ov = fmul2(make_float2(__uint_as_float(o[2 * u]), __uint_as_float(o[2 * u + 1])), linv2);
-            __nv_bfloat162 h = __floats2bfloat162_rn(ov.x, ov.y);
-            pk[u] = *reinterpret_cast<uint32_t*>(&h);
-          }
-          st_global_v8(orow_ptr + cb * 32, pk);
-          st_global_v8(orow_ptr + cb * 32 + 16, pk + 8);
-        }
-      }
+      ++n;
     }
   }
+  if (kOut != kOutStats && n >= 1) {
+    uint32_t o[64];
+    if (!c.wait_w(kOFull + me, n - 1)) return;
+    tc_fence_after();
+    if (kOut == kOutTiles) fwd_out_load<D>(c, me, 0, o);
+    tc_wait_ld();
+    fwd_out_store<D, kOut>(c, p, tmO, me, o, pend);
+  }
+  if (kOut == kOutTiles && (threadIdx.x & 31) == 0) bulk_wait_all();      // (shared memory is read until then)
 }
 
 // Rows before key chunk `chunk`: every score is -1e12 (fp32 absorbs k.q), the softmax is
 // uniform, so out = sum_k bf16(1/kC) V_k and lse = -1e12 (universal_attention_autograd.py:28,
-// :154).  Pure HBM writes of the slab rows [row_lo, row_hi), done by warps 2-3 while the others
-// compute.  A block of a whole sweep writes its own chunk's rows (chunks with many of them have
-// few tiles to compute); a block of a segment of chunk i writes the same tiles' share of the
-// rows before chunk n-1-i, which has as many tiles to write as chunk i has to compute.
+// :154).  Pure HBM writes of the slab rows [row_lo, row_hi), done by warp 3 while the others
+// compute.  A block that sweeps tiles of chunk i writes their share of the rows before chunk n-1-i, which has
+// as many tiles to write as chunk i has to compute.  Copies of one 1 KB of shared memory: as stores of the warp, whole lines each, they
+// held up the load-store unit for the warps beside it (B4 H8 R4 L4096 D64: tiles of 12.4k cycles took 13.9k).
 template <int D, int kC>
-__device__ __forceinline__ void fwd_fill_rows(const FwdCtx<D>& c, const FwdParams& p, __nv_bfloat16* vmean, int chunk, int row_lo, int row_hi) {
+__device__ __forceinline__ void fwd_fill_rows(const FwdCtx<D>& c, const FwdParams& p, int chunk, int row_lo, int row_hi) {
+  using Cfg = FwdCfg<D>;
   if (row_lo >= row_hi) return;
-  const int t = threadIdx.x - 64;                      // 0..63
+  const int t = threadIdx.x & 31;
   const int L = p.s.L, R = p.s.R, N = p.s.N;
   const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.vc) + ((size_t)c.bh * L + (size_t)chunk * kC) * D;
   const float w = 1.0f / kC;
-  for (int d = t; d < D; d += 64) {
+  float mean[D / 32];                                  // columns t, t + 32, ..
+#pragma unroll
+  for (int x = 0; x < D / 32; ++x) {
     float acc = 0.f;
 #pragma unroll 16
-    for (int k = 0; k < kC; ++k) acc = fmaf(w, __bfloat162float(v[(size_t)k * D + d]), acc);
-    vmean[d] = __float2bfloat16_rn(acc);
+    for (int k = 0; k < kC; ++k) acc = fmaf(w, __bfloat162float(v[(size_t)k * D + x * 32 + t]), acc);
+    mean[x] = acc;
   }
-  named_bar_sync(2, 64);
+  constexpr int kVecPerRow = D / 16, kRows = 512 / D;  // 32-byte pieces of a row; rows in 1 KB
+  const int piece = t % kVecPerRow;
+  uint32_t mine[8];
+#pragma unroll
+  for (int x = 0; x < 8; ++x) {
+    float lo = 0.f, hi = 0.f;
+#pragma unroll
+    for (int y = 0; y < D / 32; ++y) {                 // column 16 piece + z is held by lane (16 piece + z) % 32
+      const float a = __shfl_sync(0xffffffffu, mean[y], (piece & 1) * 16 + 2 * x), b = __shfl_sync(0xffffffffu, mean[y], (piece & 1) * 16 + 2 * x + 1);
+      if (y == piece >> 1) { lo = a; hi = b; }
+    }
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    mine[x] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  const uint32_t src = smem_u32(c.smem + Cfg::oFill);
+  st_shared_v4(src + t * 32, mine);
+  st_shared_v4(src + t * 32 + 16, mine + 4);
+  fence_proxy_async();
+  __syncwarp();
   const size_t chunk_id = (size_t)c.bh * N + chunk;
-  const int rows = row_hi - row_lo;
-  constexpr int kVecPerRow = D / 8;                    // 16-byte vectors
-  const uint4 mine = reinterpret_cast<const uint4*>(vmean)[t % kVecPerRow];   // 64 % kVecPerRow == 0: fixed per thread
-  for (int r = 0; r < R; ++r) {
-    const size_t first = (chunk_id * R + r) * p.Lr + row_lo;
-    uint4* o = reinterpret_cast<uint4*>(p.out + first * D);
-    const size_t nvec = (size_t)rows * kVecPerRow;
-    for (size_t e = t; e < nvec; e += 64) o[e] = mine;
-    for (int q = t; q < rows; q += 64) {
-      p.lse[first + q] = mask_value();
-      if (p.denom) p.denom[first + q] = __float2bfloat16_rn(mask_value());
+  const int rows = row_hi - row_lo;                    // (a multiple of 64)
+#pragma unroll 1
+  for (int q0 = 0; q0 < rows; q0 += 64) {
+    for (int r = 0; r < R; ++r) {
+      const size_t first = (chunk_id * R + r) * p.Lr + row_lo + q0;
+      if (t == 0) {
+        __nv_bfloat16* o = p.out + first * D;
+#pragma unroll 1
+        for (int q = 0; q < 64; q += kRows) bulk_store_1d(o + q * D, src, 1024);
+        bulk_commit_group();
+        bulk_wait_read<1>();
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = t; q < 64; q += 32) {
+        p.lse[first + q] = mask_value();
+        if (p.denom) p.denom[first + q] = __float2bfloat16_rn(mask_value());
+      }
     }
   }
+  if (t == 0) bulk_wait_all();
 }
 
 // ------------------------------------------------------- log-retention of a tile --
@@ -620,8 +679,7 @@ template <int D, int kC, typename TG>
 __global__ void __launch_bounds__(512)
 tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles, const void* ssrc, const void* sdest, float* total, int* status) {
   constexpr int kTile = 128 * D * 2, kBoxes = D / 64;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];
   float* t3 = reinterpret_cast<float*>(smem + 2 * kTile);
   float* part = t3 + 128;                                // [3][128]
   uint32_t* misc = reinterpret_cast<uint32_t*>(part + 384);      // [0] tmem base, [1] abort flag, [2..5] two barriers
@@ -700,10 +758,9 @@ tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles
 template <int D, int kC, typename TG, bool kCarryOnly, int kOut = kOutTiles>
 __global__ void __launch_bounds__(512, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-           const __grid_constant__ CUtensorMap tmQ, FwdParams p) {
+           const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmO, FwdParams p) {
   using Cfg = FwdCfg<D>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);   // [0] tmem base, [1] abort flag
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = p.s.B * p.s.H;
@@ -727,9 +784,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
       c.row0 = c.i * kC;
       c.ntiles = (p.s.L - c.row0 + 127) / 128;
     }
-    fill_chunk = c.i;
+    fill_chunk = p.s.N - 1 - c.i;
     fill_lo = p.r0;
-    fill_hi = p.r0 + (kC == 128 ? ((c.i < p.j_end ? c.i : p.j_end) - p.j_begin) * 128 : c.i * kC);
+    fill_hi = p.r0 + (kC == 128 ? ((fill_chunk < p.j_end ? fill_chunk : p.j_end) - p.j_begin) * 128 : fill_chunk * kC);
   } else {
     int nt;
     for (c.i = 0;; ++c.i) {
@@ -753,15 +810,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
       uint32_t count = 1;
       // one arrival per warp of the group that signals
       if (b == kGFree || b == kCReady || b == kCReady + 1) count = kC / 32;
-      if (b == kT3Ready) count = 4;
-      if (b == kCFree || b == kCFree + 1) count = 8;
-      if (b == kPReady || b == kPReady + 1 || b == kOFree || b == kOFree + 1) count = 4;
+      if (b == kT3Ready || b == kSFree || b == kSFree + 1 || b == kPReady || b == kPReady + 1 || b == kOFree || b == kOFree + 1) count = 4;
+      if (b == kCFree || b == kCFree + 1) count = Cfg::kHalves ? 4 : 8;
       mbar_init(c.bar(b), count);
     }
     mbar_init_fence();
     prefetch_tmap(&tmK);
     prefetch_tmap(&tmV);
     prefetch_tmap(&tmQ);
+    if (kOut == kOutTiles && !kCarryOnly) prefetch_tmap(&tmO);
   }
   if (warp == 0) {
     tmem_alloc(smem_u32(misc), 512);
@@ -772,19 +829,29 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   tc_fence_after();
   c.tmem = misc[0];
 
-  if (warp == 0) {
-    if (lane == 0 && c.ntiles > 0) fwd_producer<D, kC, kCarryOnly>(c, p, &tmK, &tmV, &tmQ);
-  } else if (warp == 1) {
-    if (lane == 0 && c.ntiles > 0) fwd_mma<D, kC, kCarryOnly, kOut>(c, p);
-  } else if (warp >= 4 && warp < 8) {
+  // Registers move from the single-thread roles to the softmax warpgroups, whose threads hold a whole row of scores.
+  constexpr int kRoleRegs = 48, kDecayRegs = 112, kSoftmaxRegs = 176;
+  static_assert(128 * (kRoleRegs + kDecayRegs + 2 * kSoftmaxRegs) <= 65536, "register pool");
+  if (warp < 4) {
+    if (!kCarryOnly) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
+    if (warp == 0) {
+      if (lane == 0 && c.ntiles > 0) fwd_producer<D, kC, kCarryOnly>(c, p, &tmK, &tmV, &tmQ);
+    } else if (warp == 1) {
+      if (lane == 0 && c.ntiles > 0) fwd_mma_scores<D, kC, kCarryOnly>(c, p);
+    } else if (warp == 2) {
+      if (lane == 0 && c.ntiles > 0 && !kCarryOnly && kOut != kOutStats) fwd_mma_pv<D, kC>(c, p);
+    } else if (!kCarryOnly && p.fill_masked) {
+      fwd_fill_rows<D, kC>(c, p, fill_chunk, fill_lo, fill_hi);
+    }
+  } else if (warp < 8) {
+    if (!kCarryOnly) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDecayRegs));
     if (c.ntiles > 0) fwd_decay<D, kC, TG, kCarryOnly>(c, p);
     else if (p.total_out)      // no row of the range sees this chunk: its prefix does not move
       p.total_out[((size_t)c.bh * p.s.N + c.i) * 128 + (threadIdx.x & 127)] =
           p.carry_in ? p.carry_in[((size_t)c.bh * p.s.N + c.i) * 128 + (threadIdx.x & 127)] : 0.f;
-  } else if (warp >= 8 && !kCarryOnly) {
-    if (c.ntiles > 0) fwd_softmax<D, kC, kOut>(c, p, (warp - 8) >> 2);
-  } else if ((warp == 2 || warp == 3) && !kCarryOnly && p.fill_masked) {
-    fwd_fill_rows<D, kC>(c, p, reinterpret_cast<__nv_bfloat16*>(smem + Cfg::oFill), fill_chunk, fill_lo, fill_hi);
+  } else if (!kCarryOnly) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    if (c.ntiles > 0) fwd_softmax<D, kC, kOut>(c, p, &tmO, (warp - 8) >> 2);
   }
 
   tc_fence_before();

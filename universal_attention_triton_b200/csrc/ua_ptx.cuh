@@ -49,31 +49,31 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
   return done != 0;
 }
 
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+// low half of the nanosecond clock: differences of less than four seconds
+__device__ __forceinline__ uint32_t globaltimer_lo() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
   return t;
 }
 
 constexpr uint32_t kWaitHintNs = 20000;      // per poll; completion of the phase ends the suspension at once
+constexpr uint32_t kWaitLimitNs = 2000000000u;
 
-// Bounded wait: gives up after about `limit_ns` of wall time (or when
+// Bounded wait: gives up after about two seconds of wall time (or when
 // *abort_flag in shared memory is already set); on giving up it sets the flag so
 // that every other waiter of the block leaves as well.  Returns true when the
-// phase completed.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          uint64_t limit_ns = 2000000000ull) {
+// phase completed.  (Short on purpose: there are dozens of waits in a kernel, all inlined, and the loops around them have to stay in the
+// instruction cache.)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait_hint(bar, parity, kWaitHintNs)) return true;
-    if ((it & 63u) == 0u) {
-      if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > limit_ns) break;
+  const uint32_t t0 = globaltimer_lo();
+#pragma unroll 1
+  while (!mbar_try_wait_hint(bar, parity, kWaitHintNs))
+    if (*abort_flag || globaltimer_lo() - t0 > limit_ns) {
+      *abort_flag = 1;
+      return false;
     }
-  }
-  *abort_flag = 1;
-  return false;
+  return true;
 }
 
 // Warp-collective variants (all 32 lanes must call them).  One arrival per warp instead
@@ -83,19 +83,16 @@ __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                               uint64_t limit_ns = 2000000000ull) {
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  const uint64_t t0 = globaltimer_ns();
-  for (uint32_t it = 1;; ++it) {
-    if (__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity, kWaitHintNs))) return true;
-    if ((it & 63u) == 0u) {
-      const bool give_up = (*abort_flag != 0) || (globaltimer_ns() - t0 > limit_ns);
-      if (__any_sync(0xffffffffu, give_up)) break;
+  const uint32_t t0 = globaltimer_lo();
+#pragma unroll 1
+  while (!__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity, kWaitHintNs)))
+    if (__any_sync(0xffffffffu, *abort_flag != 0 || globaltimer_lo() - t0 > limit_ns)) {
+      *abort_flag = 1;
+      return false;
     }
-  }
-  *abort_flag = 1;
-  return false;
+  return true;
 }
 
 // --------------------------------------------------------------------- TMA ----
@@ -115,6 +112,13 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+}
+// 1-D bulk copy shared -> global (16-byte aligned addresses, size a multiple of 16 bytes)
+__device__ __forceinline__ void bulk_store_1d(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
 // Adds a [128 rows][32 floats] 128-byte-swizzled shared-memory box into global memory (fp32 tensor map); completion is
 // tracked by the issuing thread's bulk async-groups.
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
@@ -125,6 +129,9 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x,
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // every committed group has finished READING its shared-memory source
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// at most kLeft of the committed groups have yet to finish reading their sources
+template <int kLeft>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kLeft) : "memory"); }
 // every committed group is complete (its global writes included)
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
@@ -158,46 +165,43 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Same with the accumulate flag known at compile time (no predicate computation at issue time)
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ss_c(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
-  if (kAccumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 1, 1;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 1, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc)
-        : "memory");
-  }
-}
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc) {
-  if (kAccumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 1, 1;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 1, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc)
-        : "memory");
-  }
-}
-
 // D[tmem] (+)= A[tmem] * B[smem desc]
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// Four tcgen05.mma of one accumulation chain from ONE asm statement: what limits a single issuing thread is the
+// instruction count per MMA (descriptor arithmetic, predicate set-up), so the chain shares one predicate set-up and
+// advances the 64-bit descriptors by immediate-like steps (in 16-byte units of the descriptor's address field).
+__device__ __forceinline__ void mma4_ss(uint32_t d, uint64_t a, uint64_t b, uint64_t sa, uint64_t sb, uint32_t idesc, uint32_t acc_first) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\tsetp.eq.u32 q, 1, 1;\n\t"
+      "add.s64 a1, %1, %3;\n\tadd.s64 b1, %2, %4;\n\tadd.s64 a2, a1, %3;\n\tadd.s64 b2, b1, %4;\n\t"
+      "add.s64 a3, a2, %3;\n\tadd.s64 b3, b2, %4;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %5, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %5, q;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %5, q;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %5, q;\n\t}" ::"r"(d),
+      "l"(a), "l"(b), "l"(sa), "l"(sb), "r"(idesc), "r"(acc_first)
+      : "memory");
+}
+// ... with the A operand in TMEM at four given column addresses
+__device__ __forceinline__ void mma4_ts(uint32_t d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint64_t b, uint64_t sb,
+                                        uint32_t idesc, uint32_t acc_first) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 b1, b2, b3;\n\t"
+      "setp.ne.b32 p, %8, 0;\n\tsetp.eq.u32 q, 1, 1;\n\t"
+      "add.s64 b1, %5, %6;\n\tadd.s64 b2, b1, %6;\n\tadd.s64 b3, b2, %6;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %5, %7, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], b1, %7, q;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], b2, %7, q;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%4], b3, %7, q;\n\t}" ::"r"(d),
+      "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(b), "l"(sb), "r"(idesc), "r"(acc_first)
       : "memory");
 }
 
@@ -213,27 +217,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-// 16 lanes x 64 consecutive 32-bit columns in the fragment order of 16 x 8 tiles: r[4 j + {0, 1}] = columns 8 j + 2 (t % 4) + {0, 1} of
-// lane t / 4, r[4 j + {2, 3}] = the same columns of lane t / 4 + 8 (t = thread of the warp)
-__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
-        "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]),
-        "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-      "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
-      "r"(r[31])
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 // 32 lanes x 16 consecutive 32-bit columns
@@ -246,33 +234,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
-// 32 bytes in one store (32-byte aligned address): a thread that owns a row of a tile writes whole sectors
-__device__ __forceinline__ void st_global_v8(void* addr, const uint32_t* r) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]),
-               "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
 }
 
-// The four threads of a quad hold word j = 0..7 (two columns each) of the same row; afterwards thread q of the quad holds the row's
-// words of blocks 2 q and 2 q + 1 in column order, i.e. 32 contiguous bytes.  Eight shuffles.
-__device__ __forceinline__ void quad_gather(uint32_t (&w)[8], int lane) {
-  const bool b1 = lane & 2, b0 = lane & 1;
-  uint32_t lo[4], hi[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t keep = b1 ? w[4 + i] : w[i], got = __shfl_xor_sync(0xffffffffu, b1 ? w[i] : w[4 + i], 2);
-    lo[i] = b1 ? got : keep;
-    hi[i] = b1 ? keep : got;
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const uint32_t kl = b0 ? lo[2 + i] : lo[i], gl = __shfl_xor_sync(0xffffffffu, b0 ? lo[i] : lo[2 + i], 1);
-    const uint32_t kh = b0 ? hi[2 + i] : hi[i], gh = __shfl_xor_sync(0xffffffffu, b0 ? hi[i] : hi[2 + i], 1);
-    w[4 * i] = b0 ? gl : kl;
-    w[4 * i + 1] = b0 ? kl : gl;
-    w[4 * i + 2] = b0 ? gh : kh;
-    w[4 * i + 3] = b0 ? kh : gh;
-  }
+__device__ __forceinline__ void st_shared_f1(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t* v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
 
 // four floats added to global memory in one instruction (16-byte aligned address)

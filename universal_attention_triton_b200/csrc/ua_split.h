@@ -106,7 +106,7 @@ int make_split(const Shape& s) {
   if (BH * tiles > 1.3 * kSms * sweep_tiles(s, 0) || BH * tiles > 8192) return 0;
   int split = 0;
   if (!kBackward) {
-    const double start = 9.0, cost = narrow * (s.D == 64 ? 3.8 + 0.8 * R : 3.2 + 1.35 * R), totals = 3.0 + BH * tiles * (s.D == 64 ? 0.01 : 0.018);
+    const double start = 6.5, cost = narrow * (s.D == 64 ? 3.1 + 0.73 * R : 2.95 + 1.5 * R), totals = 3.0 + BH * tiles * (s.D == 64 ? 0.01 : 0.018);
     auto len = [&](int i) { return sweep_tiles(s, i); };
     double best = 0.95 * play(s, len, 0, 0, start, cost, std::numeric_limits<double>::infinity());
     for (int t = 1; t < len(0); t *= 2) {
