@@ -538,7 +538,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   constexpr int kWorkers = kC * NG;
   constexpr int kGateQuad = kC / 64;             // the quadrant whose warps fetch the gates of the next half tile
   const int L = p.s.L, R = kHeads ? p.heads : 0, N = p.s.N;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int g = (warp - 8) >> 2;                 // column group: columns [CG g, CG g + CG) of a half tile
   const int quad = warp & 3;                     // TMEM lane quadrant this warp may touch; also its helper duty inside the group
   const int key = quad * 32 + lane;
@@ -574,13 +574,18 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     }
   };
 
-  // this thread's CG columns of row `key` of a [128 keys][64 rows] bf16 tile (128-byte swizzled rows)
-  auto store_row = [&](uint8_t* base, const uint32_t* v) {
+  // this thread's CG columns of row `key` of ring buffer `ring`, a [128 keys][64 rows] bf16 tile (128-byte swizzled rows)
+  uint32_t row_at[CG / 8];
 #pragma unroll
-    for (int x = 0; x < CG / 8; ++x) {
-      const uint32_t ch = (uint32_t)((CG / 8) * g + x);
-      *reinterpret_cast<uint4*>(base + key * 128 + (((ch ^ swz) & 7) << 4)) = make_uint4(v[4 * x], v[4 * x + 1], v[4 * x + 2], v[4 * x + 3]);
-    }
+  for (int x = 0; x < CG / 8; ++x) row_at[x] = smem_u32(c.smem + Cfg::oDs) + key * 128 + ((((uint32_t)((CG / 8) * g + x) ^ swz) & 7) << 4);
+  int ring = 0;                                  // the buffer that the next gradient goes to
+  auto store_row = [&](const uint32_t* v) {
+#pragma unroll
+    for (int x = 0; x < CG / 8; ++x) st_shared_v4(row_at[x] + ring * 16384, v + 4 * x);
+  };
+  auto hand_over = [&]() {
+    c.arrive_w(qDsReady + ring);
+    ring = ring + 1 == Cfg::kRing ? 0 : ring + 1;
   };
 
   // ---- prologue: static_dest^(1/3) of the first half tile ----
@@ -591,7 +596,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     for (int q = 0; q < c.segment; ++q) suffix += p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + q) * 128 + key];
   named_bar_sync(kBarAll, kWorkers);
 
-  int u = 0, hc = 0, w = 0;                       // units, heads, gradients handed over so far
+  int u = 0, hc = 0;                             // units and heads so far
   for (int ht = 0; ht < c.nht; ++ht) {
     const int rel = c.row0_of(ht) - c.i * kC;
     const bool diag = rel < kC;                    // rows at positions of the chunk's own keys
@@ -721,16 +726,15 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
           pk[x] = *reinterpret_cast<uint32_t*>(&hp);
           dk[x] = *reinterpret_cast<uint32_t*>(&hd);
         }
-        store_row(c.smem + Cfg::oDs + w % Cfg::kRing * 16384, dk);
+        store_row(dk);
         // P^T (rows CG g + 2x, 2x + 1 as one 32-bit column).  With a ring of two, its free buffer says that the product with the
         // probabilities of two heads ago is done as well; with three it does not.
         if (Cfg::kRing > 2 && hc >= 2 && !c.wait_w(qPtFree + (hc & 1), (hc >> 1) - 1)) return;
         tmem_st8(c.tmem + Cfg::tPT + 32 * (hc & 1) + col0 / 2 + lane_base, pk);
-        ++w;
         tc_wait_st();
         fence_proxy_async();
         tc_fence_before();
-        c.arrive_w(qDsReady + (w - 1) % Cfg::kRing);
+        hand_over();
       }
     }
 
@@ -830,10 +834,9 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       if (diag) decay_grad(std::true_type{});
       else decay_grad(std::false_type{});
       ds_acc += dsa.x + dsa.y;
-      const int db = w++ % Cfg::kRing;
-      store_row(c.smem + Cfg::oDs + db * 16384, pk);
+      store_row(pk);
       fence_proxy_async();
-      c.arrive_w(qDsReady + db);
+      hand_over();
       // d static_dest: with chunks of 128 keys it is taken from dK_j afterwards (see row_side_finish_kernel), which costs nothing here
       // but is formed from the bf16 dG; chunks of 64 keys have always had it from fp32 sums over the keys, two warps per column.
       if constexpr (kC == 64) {
@@ -927,7 +930,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);      // [0] TMEM base, [1] abort flag, [2] failure note
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int BH = p.s.B * p.s.H;
 
   Bwd2Ctx c;
@@ -985,7 +988,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  c.tmem = misc[0];
+  c.tmem = uniform(misc[0]);
 
   // Register reallocation between the warpgroups: the single-thread roles and the drain warps need few registers, the
   // workers (who keep a half tile's decay prefix, its gradient and a head's probabilities in registers) many.  The block

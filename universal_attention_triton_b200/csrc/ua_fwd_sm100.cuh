@@ -158,6 +158,7 @@ struct FwdCtx {
   uint8_t* smem;
   uint32_t bars;      // shared address of barrier 0
   uint32_t tmem;
+  uint32_t lane_base;  // the TMEM lanes of the warp's quadrant, in address position
   volatile int* abort_flag;
   int i, bh, ntiles;
   int row0, srow0;    // first row of the block's first tile: in the sequence, and inside the slabs of row-indexed tensors
@@ -280,7 +281,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
   using Cfg = FwdCfg<D>;
   const int L = p.s.L;
   const int k = threadIdx.x & 127;
-  const uint32_t lane_base = (uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16;
+  const uint32_t lane_base = c.lane_base;
   const TG* ss = static_cast<const TG*>(p.ssrc) + (size_t)c.bh * L;
   const TG* sd = static_cast<const TG*>(p.sdest) + (size_t)c.bh * p.Lr + c.srow0 + k;
   // (gate of row k of tile T; with chunks of 64 keys the last tile may reach beyond the sequence)
@@ -421,7 +422,7 @@ struct FwdPending {
 // 64 columns of the output on their way into registers (thread = row)
 template <int D>
 __device__ __forceinline__ void fwd_out_load(const FwdCtx<D>& c, int me, int cb, uint32_t* o) {
-  const uint32_t tO = c.tmem + FwdCfg<D>::tO + (FwdCfg<D>::kOBufs == 2 ? me * D : 0) + ((uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16) + cb * 64;
+  const uint32_t tO = c.tmem + FwdCfg<D>::tO + (FwdCfg<D>::kOBufs == 2 ? me * D : 0) + c.lane_base + cb * 64;
 #pragma unroll
   for (int x = 0; x < 4; ++x) tmem_ld16(tO + 16 * x, o + 16 * x);
 }
@@ -439,7 +440,7 @@ __device__ __forceinline__ void fwd_out_store(const FwdCtx<D>& c, const FwdParam
     }
   };
   if constexpr (kOut == kOutMerged) {
-    const uint32_t tO = c.tmem + Cfg::tO + (Cfg::kOBufs == 2 ? me * D : 0) + ((uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16);
+    const uint32_t tO = c.tmem + Cfg::tO + (Cfg::kOBufs == 2 ? me * D : 0) + c.lane_base;
     float* dst = p.merged_acc + w.row * D;
 #pragma unroll 1
     for (int cb = 0; cb < D / 32; ++cb) {
@@ -491,7 +492,7 @@ __device__ __forceinline__ void fwd_softmax(const FwdCtx<D>& c, const FwdParams&
   using Cfg = FwdCfg<D>;
   const int R = p.s.R, N = p.s.N;
   const int row = threadIdx.x & 127;
-  const uint32_t lane_base = (uint32_t)((threadIdx.x >> 5) & 3) * 32u << 16;
+  const uint32_t lane_base = c.lane_base;
   const uint32_t crow0 = smem_u32(c.smem + Cfg::oCs) + row * 512 + ((row & 7) << 4);      // (16-byte piece x of a row lies at piece x ^ (row % 8))
   const size_t chunk_id = (size_t)c.bh * N + c.i;
   const float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
@@ -762,7 +763,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   using Cfg = FwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);   // [0] tmem base, [1] abort flag
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int BH = p.s.B * p.s.H;
 
   FwdCtx<D> c;
@@ -827,7 +828,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  c.tmem = misc[0];
+  c.tmem = uniform(misc[0]);
+  c.lane_base = (uint32_t)(warp & 3) * 32u << 16;
 
   // Registers move from the single-thread roles to the softmax warpgroups, whose threads hold a whole row of scores.
   constexpr int kRoleRegs = 48, kDecayRegs = 112, kSoftmaxRegs = 176;
