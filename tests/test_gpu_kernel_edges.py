@@ -183,3 +183,33 @@ def test_forward_sweeps_of_several_tiles_with_odd_and_even_heads(shape):
     out_sm, lse_sm, _ = ops.forward_cm(*cu, flags=_lib.FLAG_FORCE_SIMT)
     assert ((out.float() - out_sm.float()).abs() <= 2e-2 + 2.0 ** -7 * out_sm.float().abs()).all()
     assert ((lse - lse_sm).abs() <= 2e-2 + 1e-5 * lse_sm.abs()).all()
+
+
+@pytest.mark.parametrize("B,H,R,chunk,t", [(16, 16, 4, 64, 230), (40, 4, 1, 128, 511), (20, 8, 8, 128, 400), (8, 20, 3, 128, 640)])
+def test_decode_blocks_that_take_several_chunks(B, H, R, chunk, t):
+    """More chunks than resident blocks (head_dim 128): against fp32 arithmetic on the same values, at the bars of the bf16 kernels; a second
+    step from the state that the first one left."""
+    from universal_attention_triton_b200 import ops
+    D, cap = 128, (t // chunk + 2) * chunk
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    k = rnd(B, H, cap, D)
+    k = (k / k.norm(dim=-1, keepdim=True)).bfloat16()
+    v, src, dest = rnd(B, H, cap, D).bfloat16(), torch.sigmoid(rnd(B, H, cap)).bfloat16(), torch.sigmoid(rnd(B, H)).bfloat16()
+    state = -0.01 * torch.rand(B, H, cap, generator=gen, device="cuda")
+    ref_state = state.double()
+    for step in (t, t + 1):
+        q = rnd(B, H, R, D).bfloat16()
+        out, lse = ops.decode_step(step, k, v, src, q, dest, state, chunk)
+        n = step + 1
+        g = (k[:, :, :n].double() @ k[:, :, step].double().unsqueeze(-1)).squeeze(-1)
+        a = g.clamp_min(0).pow(2 / 3) * (src[:, :, :n].double() * dest.double().unsqueeze(-1)).pow(1 / 3)
+        ref_state[:, :, :n] += torch.log1p(-a.clamp(0, 1 - 1e-6))
+        ref_state[:, :, step] = 0
+        assert (state[:, :, :n].double() - ref_state[:, :, :n]).abs().max() <= 1e-5
+        for i in range(step // chunk + 1):
+            sl = slice(i * chunk, min(n, (i + 1) * chunk))
+            s = q.double() @ k[:, :, sl].double().transpose(-1, -2) + ref_state[:, :, sl].unsqueeze(2)
+            assert (lse[..., i].double() - torch.logsumexp(s, -1)).abs().max() <= 1e-4
+            ref = torch.softmax(s, -1) @ v[:, :, sl].double()
+            assert ((out[..., i].double() - ref).abs() - 2.0 ** -7 * ref.abs()).max() <= 2e-2

@@ -32,6 +32,11 @@ struct Params {
 
 constexpr int kMaxR = 8;
 
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 template <typename T, typename TG>
 __global__ void step_kernel(Params p) {
   extern __shared__ float sm[];
@@ -130,22 +135,209 @@ __global__ void step_kernel(Params p) {
   }
 }
 
-// ---- bf16, head_dim 64 / 128, chunks of 64 / 128 / 256 keys ----------------------------------------------------------
-// Bound by the one read of the caches; what it needs is bytes in flight.  One block of 2 C threads per (b, h, chunk): every
-// thread issues its 16-byte pieces of K AND of V (128 bytes of each at head_dim 128) before anything else, so that a
-// resident block keeps its whole chunk (64 KB at C = 128, D = 128) on the way.  K goes to registers, V through cp.async to the
-// thread's own places in shared memory (only the thread that fetched a piece reads it: no barrier), so that four such blocks fit
-// an SM; with V in registers as well two did (97 -> 86 us below).
+// ---- bf16, head_dim 128, chunks of 64 / 128 keys ---------------------------------------------------------------------
+// Bound by the one read of the caches; what it needs is bytes in flight at all times.  Blocks of 2 C threads stay on their SM and take one
+// (b, h, chunk) after another; K and V of a chunk are on their way through cp.async while the chunk before is worked on: the next K is asked for
+// as soon as the scores of this one are formed, the next V as soon as P V is.
 //   scores  mma.sync m16n8k16: the rows are 16 keys of a warp, the columns are the new row's key and its queries (1 + R <= 9:
 //           one or two column tiles, the rest zero).  The contraction index is permuted so that a thread's A pieces are 16
-//           contiguous bytes of a key row; no shuffles, exact bf16 products, fp32 sums.  (Eight columns are too few for tcgen05:
-//           an instruction there is 128 keys x 16 columns at the least and wants its operands in shared memory first.)
+//           contiguous bytes of a key row, which it fetches itself to places of its own: no shuffles, no barrier, exact bf16 products, fp32
+//           sums.  (Eight columns are too few for tcgen05: an instruction there is 128 keys x 16 columns at the least.)
 //   state   thread = key.   softmax  warp = query head: shuffles only.
-//   P V     thread = (8 columns of V, every 2C*8/D-th key), partial sums over the keys through shuffles and shared memory.
-// Against the kernel above (one thread per key row, V one 2-byte element at a time): B16 H8 R4 D128 at t = 6150 (418 MB of
-// caches) 332 -> 86 us = 4.9 TB/s; B1 H8 R4 D64 at t = 300 13.8 -> 3.7 us.
+//   P V     mma.sync as well: the rows are the query heads, a warp takes columns of V (ldmatrix from swizzled rows), all keys of the
+//           chunk: no sums across warps.
+// Against one block per chunk that issues its reads and then waits for them (P V on the CUDA cores, partial sums through shared memory):
+// B16 H8 R4 D128 at t = 6150 (418 MB of caches) 86 -> 76 us = 5.5 TB/s, R1 81 -> 73, R8 142 -> 104, chunks of 64 keys 78 -> 70; with items in the
+// order of the memory (chunks of a (b, h) one after the other) instead of 2 MB apart 82 -> 78 of it, with one cube root instead of a power and two 78 -> 76.
 template <int D, int C, int RT>
 struct StepCfg {
+  static constexpr int kThreads = 2 * C, kWarps = kThreads / 32;
+  static constexpr int kTPR = D / 8;                     // 16-byte pieces per row
+  static constexpr int kGroups = kThreads / kTPR;        // rows of V per pass of the fetch
+  static constexpr int kVLoads = C / kGroups;
+  static constexpr int kKLoads = D / 32;                 // 16-byte pieces of each of the two key rows of a thread
+  static constexpr int kNT = RT == 8 ? 2 : 1;            // column tiles of the score product
+  static constexpr int kSW = 8 * kNT + 1;                // row stride of the score tile (odd: thread = key reads a column)
+  static constexpr int kVT = D / 8 / kWarps;             // column tiles of P V per warp
+  static_assert(kVT >= 1, "a column tile for every warp");
+  static constexpr int kPW = C + 8;                      // row stride of P, in elements (conflict-free fragments)
+  static constexpr int oK = 0, oV = oK + C * D * 2, oS = oV + C * D * 2, oC = oS + C * kSW * 4, oP = (oC + C * 4 + 15) / 16 * 16;
+  static constexpr int kSmemBytes = oP + RT * kPW * 2;
+  // blocks per SM: what shared memory holds (1 KB per block is the system's), within the threads of an SM at 80 registers each
+  static constexpr int kBySmem = 233472 / (kSmemBytes + 1024), kByRegs = 65536 / (80 * kThreads);
+  static constexpr int kBlocks = kBySmem < kByRegs ? kBySmem : kByRegs;
+};
+
+template <int D, int C, int RT, typename TG>
+__global__ void __launch_bounds__(2 * C, StepCfg<D, C, RT>::kBlocks) step_mma_kernel(Params p, int items) {
+  using Cfg = StepCfg<D, C, RT>;
+  extern __shared__ __align__(16) uint8_t sm_step[];
+  float *s_s = reinterpret_cast<float*>(sm_step + Cfg::oS), *s_c = reinterpret_cast<float*>(sm_step + Cfg::oC);
+  __nv_bfloat16* s_p = reinterpret_cast<__nv_bfloat16*>(sm_step + Cfg::oP);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nt = p.t / C + 1, R = p.R;
+  const __nv_bfloat16 *kcache = static_cast<const __nv_bfloat16*>(p.kcache), *vcache = static_cast<const __nv_bfloat16*>(p.vcache);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const int kr0 = warp * 16 + (lane >> 2), kr1 = kr0 + 8, c8 = (lane & 3) * 8;
+  const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(sm_step), my_k = s0 + Cfg::oK + tid * 16;
+  const int vg = tid / Cfg::kTPR, vc = tid % Cfg::kTPR;
+  auto live_keys = [&](int i) { return min(C, p.t - i * C + 1); };      // what lies behind them in the caches is not read
+  auto cp16 = [&](uint32_t dst, const void* src, bool live) {           // (a piece beyond the live keys is filled with zeros)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+  };
+  auto fetch_k = [&](int item) {
+    if (item < items) {
+      const int bh = item / nt, i = item % nt, nkeys = live_keys(i);
+      const __nv_bfloat16* row = kcache + ((size_t)bh * p.Lcap + (size_t)i * C) * D + c8;
+#pragma unroll
+      for (int x = 0; x < Cfg::kKLoads; ++x) {
+        cp16(my_k + 2 * x * Cfg::kThreads * 16, row + (size_t)(kr0 < nkeys ? kr0 : 0) * D + x * 32, kr0 < nkeys);
+        cp16(my_k + (2 * x + 1) * Cfg::kThreads * 16, row + (size_t)(kr1 < nkeys ? kr1 : 0) * D + x * 32, kr1 < nkeys);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto fetch_v = [&](int item) {
+    if (item < items) {
+      const int bh = item / nt, i = item % nt, nkeys = live_keys(i);
+      const __nv_bfloat16* row = vcache + ((size_t)bh * p.Lcap + (size_t)i * C) * D + vc * 8;
+#pragma unroll
+      for (int x = 0; x < Cfg::kVLoads; ++x) {
+        const int k = vg + x * Cfg::kGroups;
+        cp16(s0 + Cfg::oV + k * D * 2 + (vc ^ (k & 7)) * 16, row + (size_t)(k < nkeys ? k : 0) * D, k < nkeys);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint4 bq[Cfg::kNT][Cfg::kKLoads];      // the new key and the queries, as columns of the score product
+  auto fetch_q = [&](int bh) {
+#pragma unroll
+    for (int n = 0; n < Cfg::kNT; ++n) {
+      const int col = n * 8 + (lane >> 2);                 // 0: the new key, 1 + r: query head r
+      const __nv_bfloat16* row = col == 0 ? kcache + ((size_t)bh * p.Lcap + p.t) * D : static_cast<const __nv_bfloat16*>(p.q) + ((size_t)bh * R + col - 1) * D;
+#pragma unroll
+      for (int x = 0; x < Cfg::kKLoads; ++x) bq[n][x] = col <= R ? __ldg(reinterpret_cast<const uint4*>(row + c8 + x * 32)) : zero;
+    }
+  };
+  // (per-key values of the state update; a thread beyond the live keys reads nothing)
+  float src = 0.f, dst = 0.f, old = 0.f;
+  auto fetch_state = [&](int bh, int i) {
+    if (tid < live_keys(i) && i * C + tid < p.t) {
+      const size_t at = (size_t)bh * p.Lcap + (size_t)i * C + tid;
+      src = Num<TG>::ld(static_cast<const TG*>(p.src) + at);
+      dst = Num<TG>::ld(static_cast<const TG*>(p.dest) + bh);
+      old = p.state[at];
+    }
+  };
+
+  int item = blockIdx.x;
+  fetch_k(item);
+  fetch_v(item);
+  fetch_q(item / nt);
+  fetch_state(item / nt, item % nt);
+  for (; item < items; item += gridDim.x) {
+    const int bh = item / nt, i = item % nt, nkeys = live_keys(i), next = item + gridDim.x;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");      // K (V of the chunk may be on its way)
+    uint4 a0[Cfg::kKLoads], a1[Cfg::kKLoads];
+#pragma unroll
+    for (int x = 0; x < Cfg::kKLoads; ++x) {
+      a0[x] = *reinterpret_cast<const uint4*>(sm_step + Cfg::oK + (2 * x * Cfg::kThreads + tid) * 16);
+      a1[x] = *reinterpret_cast<const uint4*>(sm_step + Cfg::oK + ((2 * x + 1) * Cfg::kThreads + tid) * 16);
+    }
+#pragma unroll
+    for (int n = 0; n < Cfg::kNT; ++n) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int x = 0; x < Cfg::kKLoads; ++x) {
+        mma_16816(d, a0[x].x, a1[x].x, a0[x].y, a1[x].y, bq[n][x].x, bq[n][x].y);
+        mma_16816(d, a0[x].z, a1[x].z, a0[x].w, a1[x].w, bq[n][x].z, bq[n][x].w);
+      }
+      const int cc = n * 8 + (lane & 3) * 2;
+      s_s[kr0 * Cfg::kSW + cc] = d[0]; s_s[kr0 * Cfg::kSW + cc + 1] = d[1];
+      s_s[kr1 * Cfg::kSW + cc] = d[2]; s_s[kr1 * Cfg::kSW + cc + 1] = d[3];
+    }
+    fetch_k(next);                       // (over pieces that only this thread reads, and has read)
+    if (next < items && next / nt != bh) fetch_q(next / nt);
+    __syncthreads();
+    if (tid < C) {
+      float cstate = 0.f;
+      if (tid < nkeys && i * C + tid < p.t) {
+        const float g = s_s[tid * Cfg::kSW];
+        // relu(g)^(2/3) src^(1/3) dest^(1/3) as one cube root
+        const float a = g > 0.f ? cbrtf(g * g * (src * dst)) : 0.f;
+        cstate = old + log1pf(-fminf(fmaxf(a, 0.f), clamp_hi()));
+      }
+      if (tid < nkeys) p.state[(size_t)bh * p.Lcap + (size_t)i * C + tid] = cstate;
+      s_c[tid] = cstate;
+    }
+    if (next < items) fetch_state(next / nt, next % nt);
+    __syncthreads();
+    // (a chunk of 64 keys has four warps: with eight heads a warp takes two)
+    for (int r = warp; r < RT; r += Cfg::kWarps) {
+      float e[C / 32], m = -INFINITY, z = 0.f;
+#pragma unroll
+      for (int x = 0; x < C / 32; ++x) {
+        const int k = x * 32 + lane;
+        e[x] = k < nkeys ? s_s[k * Cfg::kSW + 1 + r] + s_c[k] : -INFINITY;
+        m = fmaxf(m, e[x]);
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+      for (int x = 0; x < C / 32; ++x) {
+        e[x] = x * 32 + lane < nkeys ? __expf(e[x] - m) : 0.f;
+        z += e[x];
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+      // the reference rounds the normalised probabilities to the input dtype before the product with V (:159)
+#pragma unroll
+      for (int x = 0; x < C / 32; ++x) s_p[r * Cfg::kPW + x * 32 + lane] = __float2bfloat16_rn(e[x] / z);
+      if (lane == 0 && r < R) p.lse[((size_t)bh * nt + i) * R + r] = m + logf(z);
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");      // V (the next K may be on its way)
+    __syncthreads();
+    {
+      float acc[Cfg::kVT][4];
+#pragma unroll
+      for (int n = 0; n < Cfg::kVT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+      const int head = lane >> 2;
+      const uint32_t* prow = reinterpret_cast<const uint32_t*>(s_p + head * Cfg::kPW) + (lane & 3);
+#pragma unroll 4
+      for (int k = 0; k < C; k += 16) {
+        const uint32_t x0 = head < RT ? prow[k / 2] : 0u, x2 = head < RT ? prow[k / 2 + 4] : 0u;      // (rows 8..15 of the tile: none)
+        const int krow = k + (lane & 15);
+#pragma unroll
+        for (int n = 0; n < Cfg::kVT; ++n) {
+          uint32_t y0, y1;
+          asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(y0), "=r"(y1)
+                       : "r"(s0 + Cfg::oV + krow * D * 2 + ((warp * Cfg::kVT + n) ^ (krow & 7)) * 16));
+          mma_16816(acc[n], x0, 0u, x2, 0u, y0, y1);
+        }
+      }
+      if (head < R) {
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + (((size_t)bh * nt + i) * R + head) * D + warp * Cfg::kVT * 8 + (lane & 3) * 2;
+#pragma unroll
+        for (int n = 0; n < Cfg::kVT; ++n) {
+          Num<__nv_bfloat16>::st(out + n * 8, acc[n][0]);
+          Num<__nv_bfloat16>::st(out + n * 8 + 1, acc[n][1]);
+        }
+      }
+    }
+    if (next < items) __syncthreads();      // V, the scores and P have been read
+    fetch_v(next);
+  }
+}
+
+// ---- the same with one block per (b, h, chunk) ---------------------------------------------------------------------
+// For head_dim 64 and for chunks of 256 keys (see launch_step_mma): every thread issues its 16-byte pieces of K AND of V before anything else, so
+// that a resident block keeps its whole chunk on the way; K goes to registers, V through cp.async to the thread's own places in shared
+// memory (only the thread that fetched a piece reads it: no barrier).  Scores and state as above; P V on the CUDA cores: thread = (8 columns
+// of V, every 2C*8/D-th key), partial sums over the keys through shuffles and shared memory.
+// At head_dim 128 the blocks follow the memory (chunks of a (b, h) one after the other: C256 R4 109 -> 104 us, R2 93 -> 88); at 64 the (b, h)s of a
+// chunk do (the other way 59.7 -> 61.6 at B8 H16 R2 t8000, 30.8 -> 28.7 at B16 H4 R1 t7000).
+template <int D, int C, int RT>
+struct OnceCfg {
   static constexpr int kThreads = 2 * C, kWarps = kThreads / 32;
   static constexpr int kTPR = D / 8;                     // threads per row of V
   static constexpr int kGroups = kThreads / kTPR;        // rows of V per pass
@@ -161,12 +353,13 @@ struct StepCfg {
 };
 
 template <int D, int C, int RT, typename TG>
-__global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
-  using Cfg = StepCfg<D, C, RT>;
+__global__ void __launch_bounds__(2 * C) step_once_kernel(Params p) {
+  using Cfg = OnceCfg<D, C, RT>;
   extern __shared__ __align__(16) float sm[];
   float *s_s = sm + Cfg::oS, *s_c = sm + Cfg::oC, *s_p = sm + Cfg::oP, *s_acc = sm + Cfg::oAcc;
-  const int bh = blockIdx.x, i = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nt = p.t / C + 1, R = p.R;
+  const int bh = D == 64 ? blockIdx.x % p.BH : blockIdx.x / nt, i = D == 64 ? blockIdx.x / p.BH : blockIdx.x % nt;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nkeys = min(C, p.t - i * C + 1);             // live keys of the chunk; what lies behind them in the caches is not read
   const __nv_bfloat16* kc = static_cast<const __nv_bfloat16*>(p.kcache) + (size_t)bh * p.Lcap * D;
   const __nv_bfloat16* vrow = static_cast<const __nv_bfloat16*>(p.vcache) + ((size_t)bh * p.Lcap + (size_t)i * C) * D;
@@ -212,14 +405,10 @@ __global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
 #pragma unroll
   for (int n = 0; n < Cfg::kNT; ++n) {
     float d[4] = {0.f, 0.f, 0.f, 0.f};
-    auto mma = [&](uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, uint32_t y0, uint32_t y1) {
-      asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                   : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y0), "r"(y1));
-    };
 #pragma unroll
     for (int x = 0; x < Cfg::kKLoads; ++x) {
-      mma(a0[x].x, a1[x].x, a0[x].y, a1[x].y, bq[n][x].x, bq[n][x].y);
-      mma(a0[x].z, a1[x].z, a0[x].w, a1[x].w, bq[n][x].z, bq[n][x].w);
+      mma_16816(d, a0[x].x, a1[x].x, a0[x].y, a1[x].y, bq[n][x].x, bq[n][x].y);
+      mma_16816(d, a0[x].z, a1[x].z, a0[x].w, a1[x].w, bq[n][x].z, bq[n][x].w);
     }
     const int cc = n * 8 + (lane & 3) * 2;
     s_s[kr0 * Cfg::kSW + cc] = d[0]; s_s[kr0 * Cfg::kSW + cc + 1] = d[1];
@@ -311,14 +500,31 @@ __global__ void __launch_bounds__(2 * C) step_mma_kernel(Params p) {
 }
 
 template <int D, int C, int RT, typename TG>
-inline bool launch_step_mma(const Params& p, int nt, cudaStream_t st) {
-  using Cfg = StepCfg<D, C, RT>;
+inline bool launch_step_once(const Params& p, int nt, cudaStream_t st) {
+  using Cfg = OnceCfg<D, C, RT>;
   constexpr int smem = Cfg::kSmemFloats * 4;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(step_mma_kernel<D, C, RT, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      cudaFuncSetAttribute(step_once_kernel<D, C, RT, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return false;
-  step_mma_kernel<D, C, RT, TG><<<dim3((unsigned)p.BH, (unsigned)nt), Cfg::kThreads, smem, st>>>(p);
+  step_once_kernel<D, C, RT, TG><<<(unsigned)(p.BH * nt), Cfg::kThreads, smem, st>>>(p);
   return true;
+}
+template <int D, int C, int RT, typename TG>
+inline bool launch_step_mma(const Params& p, int nt, cudaStream_t st) {
+  // Blocks that stay pay where a chunk is long enough to hide their work and several of them fit an SM.  At t = 6150, B16 H8, staying / one
+  // chunk per block in us: D128 C128 R1 73 / 80, R4 76 / 86, R8 104 / 142, C64 R4 70 / 78; but C256 R2 117 / 93, R4 118 / 109 (one block of
+  // 150 KB per SM), and D64 R2 58 / 47 (half the bytes for the same chain of scores, softmax and P V).
+  if constexpr (D == 64 || C == 256) {
+    return launch_step_once<D, C, RT, TG>(p, nt, st);
+  } else {
+    using Cfg = StepCfg<D, C, RT>;
+    if (Cfg::kSmemBytes > 48 * 1024 &&
+        cudaFuncSetAttribute(step_mma_kernel<D, C, RT, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
+      return false;
+    const int items = p.BH * nt, grid = items < 148 * Cfg::kBlocks ? items : 148 * Cfg::kBlocks;
+    step_mma_kernel<D, C, RT, TG><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmemBytes, st>>>(p, items);
+    return true;
+  }
 }
 template <int D, int C, typename TG>
 inline bool launch_step_mma_r(const Params& p, int nt, cudaStream_t st) {
