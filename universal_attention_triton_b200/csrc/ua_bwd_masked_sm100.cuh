@@ -17,6 +17,9 @@
 // MN-major B operand of N = 128.  The terms in gd stay on the CUDA cores, in fp32: four warps accumulate
 // w_c += gd_c^T Q_rj from the Q tile in shared memory, and the drain warps add gd_c (x) ksum_c / 128 to Y on its way out.
 // head_dim 128 runs as two blocks per work item, one per 64-wide half of the output columns of Y / lanes of Nt.
+// An item goes head by head through its row tiles, so that every chunk's gradient is read in the order of the memory (row tile by row tile
+// it jumped by L rows); asking tiles into L2 ahead of the ring, and keeping the TMEM base in vector registers, cost 2 to 6 %: B4 H8 R4 L4096 D64
+// 362 -> 354 us, R1 131 -> 123, B1 H16 R1 D128 197 -> 188.  The loads alone, nothing done with them, take 232 us of the 354.
 // A work item is (batch*head, group of G chunks, range of row tiles); partial N / w / u leave as fp32 global adds.
 // Chunks of m * 128 keys come as m neighbouring "chunks" of 128 here (p.m): vbar and the weight 1 / (128 m) are the whole
 // chunk's, and all m read the same gradient rows, those before the whole chunk.
@@ -53,7 +56,6 @@ struct MkCfg {
   static constexpr int kUnits = kG / kPer;                 // slots per step when every chunk of the group is active
   static constexpr int kSlots = 3;
   static constexpr int kDoBytes = kKB * 16384;
-  static constexpr int kAhead = (D == 64) ? 12 : 6;        // gradient tiles requested into L2 ahead of the ring
   static constexpr int kMtBytes = kKB * 8192;              // one half (64 rows d') of a chunk's M^T image
   static constexpr int oSlot = 0;
   static constexpr int oQ = oSlot + kSlots * 32768;        // 2 x Q [128][64]
@@ -248,7 +250,8 @@ __global__ void __launch_bounds__(256) masked_finish_kernel(const __nv_bfloat16*
   }
   const uint32_t aV = smem_u32(sV) + 2 * ((lane & 15) * Dn::kStride + (lane >> 4) * 8);
   const float* nrow = nacc + (size_t)(n0 + (lane >> 2)) * D + (lane & 3) * 2;       // N^T[d'][d]
-#pragma unroll 2
+  constexpr int kDeep = D == 128 ? 8 : 2;          // pieces of N^T under way (head_dim 128: 45 -> 40 us for 512 chunks; at 64 the code costs more than it gives)
+#pragma unroll kDeep
   for (int k = 0; k < D; k += 16) {
     uint32_t b[kNW][3][2];
 #pragma unroll
@@ -321,24 +324,10 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
                    p.mt + ((size_t)c.bh * N + c.i0 + cc) * (size_t)(D * D * 2) + (size_t)c.h * Cfg::kMtBytes, Cfg::kMtBytes,
                    c.bar(mMtFull));
   }
-  // The gradient tiles are asked into L2 kAhead tiles before their turn in the shared-memory ring: the ring alone (a few
-  // tiles per SM) does not cover the latency of HBM at full bandwidth.
-  int pj = c.jlo, pr = 0, pc = c.clo(c.jlo);
-  auto prefetch_next = [&]() {
-    if (pj >= c.jhi) return;
-#pragma unroll
-    for (int b = 0; b < Cfg::kKB; ++b)
-      tma_prefetch_2d(tmG, 64 * b, (int)(((c.out_chunk(N, pc)) * R + pr) * L + (size_t)c.srow(pj)));
-    if (++pc >= c.chi) {
-      if (++pr >= R) { pr = 0; ++pj; }
-      pc = c.clo(pj);
-    }
-  };
-  for (int x = 0; x < Cfg::kAhead; ++x) prefetch_next();
   int s = 0, uc = 0;
-  for (int j = c.jlo; j < c.jhi; ++j) {
-    const int c0 = c.clo(j);
-    for (int r = 0; r < R; ++r, ++s) {
+  for (int r = 0; r < R; ++r)
+    for (int j = c.jlo; j < c.jhi; ++j, ++s) {
+      const int c0 = c.clo(j);
       const int qs = s & 1;
       if (s >= 2 && !c.wait(mQFree + qs, s / 2 - 1)) return;
       mbar_expect_tx(c.bar(mQFull + qs), 16384u + (uint32_t)(c.chi - c0) * 512u);
@@ -358,11 +347,9 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
           for (int b = 0; b < Cfg::kKB; ++b)
             tma_load_2d(sb + Cfg::oSlot + sl * 32768 + (cc - u * Cfg::kPer) * Cfg::kDoBytes + b * 16384, tmG, 64 * b,
                         (int)((c.out_chunk(N, cc) * R + r) * L + (size_t)c.srow(j)), c.bar(mSlotFull + sl));
-          prefetch_next();
         }
       }
     }
-  }
 }
 
 template <int D, bool kWide>
@@ -373,9 +360,9 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
   constexpr uint32_t id_y = idesc_bf16(128, 64, 0, 0);       // rows x 64: A K-major, B K-major
   if (!c.wait(mMtFull, 0)) return;
   int s = 0, uc = 0;
-  for (int j = c.jlo; j < c.jhi; ++j) {
-    const int c0 = c.clo(j);
-    for (int r = 0; r < R; ++r, ++s) {
+  for (int r = 0; r < R; ++r)
+    for (int j = c.jlo; j < c.jhi; ++j, ++s) {
+      const int c0 = c.clo(j);
       const int qs = s & 1;
       const uint32_t q_addr = sb + Cfg::oQ + qs * 16384;
       if (!c.wait(mQFull + qs, s / 2)) return;
@@ -413,7 +400,6 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
       tc_commit(c.bar(mYFull + qs));
       tc_commit(c.bar(mQFree + qs));
     }
-  }
   tc_commit(c.bar(mDone));
 }
 
@@ -430,9 +416,9 @@ __device__ __forceinline__ void mk_gate_sums(const MkCtx<kWide>& c, const Masked
 #pragma unroll
   for (int x = 0; x < Cfg::kG * 16; ++x) acc[x] = 0.f;
   int s = 0;
-  for (int j = c.jlo; j < c.jhi; ++j) {
-    const int c0 = c.clo(j);
-    for (int r = 0; r < R; ++r, ++s) {
+  for (int r = 0; r < R; ++r)
+    for (int j = c.jlo; j < c.jhi; ++j, ++s) {
+      const int c0 = c.clo(j);
       const int qs = s & 1;
       if (!c.wait_w(mQFull + qs, s / 2)) return;
       const uint8_t* q = c.smem + Cfg::oQ + qs * 16384;
@@ -461,7 +447,6 @@ __device__ __forceinline__ void mk_gate_sums(const MkCtx<kWide>& c, const Masked
       }
       c.arrive_w(mQFree + qs);
     }
-  }
   const int c0 = c.clo(c.jlo);
 #pragma unroll
   for (int grp = 0; grp < Cfg::kG / 2; ++grp) {
@@ -478,7 +463,7 @@ template <int D, bool kWide>
 __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedParams& p, const CUtensorMap* tmDQ) {
   using Cfg = MkCfg<D>;
   const int L = p.Lr, R = p.s.R, N = p.s.N;      // (L: rows per slab of the row-indexed tensors)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int row = (warp & 3) * 32 + lane;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const bool leader = (warp == 4 && lane == 0);
@@ -486,9 +471,9 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
   uint8_t* stage = c.smem + Cfg::oStage;
   const float* ks = reinterpret_cast<const float*>(c.smem + Cfg::oKs);
   int s = 0;
-  for (int j = c.jlo; j < c.jhi; ++j) {
-    const int c0 = c.clo(j);
-    for (int r = 0; r < R; ++r, ++s) {
+  for (int r = 0; r < R; ++r)
+    for (int j = c.jlo; j < c.jhi; ++j, ++s) {
+      const int c0 = c.clo(j);
       const int qs = s & 1;
       if (!c.wait_w(mYFull + qs, s / 2)) return;
       tc_fence_after();
@@ -535,7 +520,6 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
         bulk_commit_group();
       }
     }
-  }
   if (!c.wait_w(mDone, 0)) {
     if (leader) bulk_wait_all();
     return;
@@ -585,7 +569,7 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);      // [0] TMEM base, [1] abort flag, [2] failure note
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int N = p.s.N;
 
   MkCtx<kWide> c;
@@ -657,7 +641,7 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  c.tmem = misc[0];
+  c.tmem = uniform(misc[0]);
 
   if (warp == 0) {
     if (lane == 0) mk_producer<D, kWide>(c, p, &tmQ, &tmG);

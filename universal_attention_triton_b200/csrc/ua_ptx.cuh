@@ -113,10 +113,6 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
                "r"(bytes), "r"(bar)
                : "memory");
 }
-// L2 prefetch of a tile that a later TMA load will fetch (no shared memory involved)
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
-}
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
 }
