@@ -30,9 +30,9 @@
 // What bounds it: the exponentials and logarithms (XU pipe, half of the cycles at R = 4), issue slots (half), and instruction fetch.  The
 // loops of the decay and the softmax warps run side by side on every scheduler, and beyond some 800 instructions together they stall on
 // fetching them: rows per pass of the decay loop, loops left rolled (unroll 1) and the length of a wait's slow path are chosen for that.  At B4 H8 R4
-// L4096 D64: 0.50 of three active warps waits for instructions; 1.4 of them did with 64 rows per pass of the decay loop (730 -> 860 us).
-// B4 H8 R4 L4096 D64 935 -> 730 us, B1 H8 R4 L8192 D128 1295 -> 1045, B1 H16 R1 L4096 D128 315 -> 279, against the form with two
-// passes over TMEM per head, outputs written from registers and one issuing thread.
+// L4096 D64: 0.4 warps wait for instructions per instruction issued; 1.4 did with 64 rows per pass of the decay loop (730 -> 860 us).
+// B4 H8 R4 L4096 D64 935 -> 706 us, R1 574 -> 455, B1 H8 R4 L8192 D128 1295 -> 1045, L4096 356 -> 304, B1 H16 R1 L4096 D128 315 -> 270, against
+// the form with two passes over TMEM per head, outputs written from registers and one issuing thread.
 //
 // The two reductions of the operator run along perpendicular axes of the tile
 // (scan along rows per key, softmax along keys per row); putting keys on lanes
