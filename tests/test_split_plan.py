@@ -86,3 +86,47 @@ def test_plan_is_the_play_through_and_cheap(tmp_path):
     # microseconds for one direction of a length not seen before: 3 at the most on an idle host, where playing block by
     # block took 930 for both directions (the bound leaves room for a busy host)
     assert float(slowest) < 60.0, slowest
+
+
+CHOICES = r"""
+#include <cstdio>
+#include "ua_split.h"
+using namespace ua::sm100;
+int main() {
+  int way, C, D, R, BH, N;
+  while (std::scanf("%d %d %d %d %d %d", &way, &C, &D, &R, &BH, &N) == 6) {
+    const ua::Shape s{1, BH, R, N, C, D, N * C};
+    std::printf("%d\n", way ? make_split<true>(s) : make_split<false>(s));
+  }
+  return 0;
+}
+"""
+
+
+def test_plan_against_measured_segment_lengths(tmp_path):
+    """The segment length that the plan takes, against the shortest of all that were timed (profiles/segment_lengths.csv)."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")
+    if not os.path.exists(os.path.join(include, "cuda_bf16.h")):
+        pytest.skip("no CUDA headers")
+    shapes, times = [], []
+    with open(os.path.join(ROOT, "profiles", "segment_lengths.csv")) as table:
+        for line in table:
+            if not line.startswith("#"):
+                way, *rest = line.strip().split(",")
+                shapes.append((int(way == "backward"), *map(int, rest[:5])))
+                times.append({int(k): float(v) for k, v in (x.split(":") for x in rest[5:])})
+    src, exe = tmp_path / "choices.cpp", tmp_path / "choices"
+    src.write_text(CHOICES)
+    subprocess.run(["g++", "-O3", "-std=c++17", "-isystem", include, "-I", os.path.join(ROOT, "universal_attention_triton_b200", "csrc"),
+                    str(src), "-o", str(exe)], check=True, capture_output=True, text=True)
+    out = subprocess.run([str(exe)], input="\n".join(" ".join(map(str, s)) for s in shapes), check=True, capture_output=True, text=True,
+                         timeout=300).stdout.split()
+    assert len(out) == len(shapes) > 3000
+    behind = {}
+    for shape, t, seg in zip(shapes, times, map(int, out)):
+        behind.setdefault(shape[:2], []).append(t[seg] / min(t.values()))
+    # (way, keys per chunk): shapes more than 5 % behind the best length, and the farthest
+    got = {key: (sum(x > 1.05 for x in v), max(v)) for key, v in behind.items()}
+    for key, (most, farthest) in {(0, 64): (3, 1.08), (0, 128): (5, 1.10), (1, 128): (12, 1.10), (1, 64): (42, 1.36)}.items():
+        assert got[key][0] <= most and got[key][1] <= farthest, got

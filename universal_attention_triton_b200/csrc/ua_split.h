@@ -3,9 +3,11 @@
 // One block per chunk lasts as long as the longest sweep, whatever the chip has idle; many short blocks pay their start-up each.
 // Both are reckoned here: the launch is played through on 148 SMs with a block time of start + cost * tiles, for whole sweeps and
 // for segments of 1, 2, 4 .. tiles, and the shortest wins (whole sweeps unless another is at least 5 % shorter).  The constants are
-// microseconds, fitted to forwards and backwards of 1 to 4 query heads at head_dim 64 and 128 on one to 64 (batch, head) units (more heads:
-// the same straight line, not measured); of the shapes measured, with every segment length tried, the choice is the best one or
-// within 5 % of it.
+// microseconds, fitted to launches of 2360 shapes forward and 752 backward (one to 32 (batch, head) units, one to eight query heads, 2 to 44
+// chunks) with every segment length timed (profiles/segment_lengths.csv).  Forward: of those shapes 8 are more than 5 % behind the best
+// length, by 9.5 % at the most; of 300 others, drawn at random and timed afterwards, none is (3 % at the most).  Chunks of 64 keys have a
+// line of their own: as 0.7 of the other's, with constants that fitted neither, 163 of the shapes were further behind than 5 %, up to 37 %.
+// Backward: at chunks of 128 keys 12 of 376 are, up to 10 %; at chunks of 64, where the line is still the scaled one, 42 of 376, up to 36 %.
 //
 // A program whose lengths change from call to call pays for a plan in each of them, so a plan has to cost a small part of a launch:
 // only the direction asked for is reckoned, the blocks of a chunk's units are alike and are dealt out to SMs that come free at the same time
@@ -99,14 +101,18 @@ double play(const Shape& s, Len len, int seg, int skip, double start, double cos
 // Row tiles per block of the forward (kBackward: half tiles per block of the backward); 0: a block sweeps its whole chunk.
 template <bool kBackward>
 int make_split(const Shape& s) {
-  const double BH = (double)s.B * s.H, R = s.R, narrow = s.C == 64 ? 0.7 : 1.0;
+  const double BH = (double)s.B * s.H, R = s.R;
   double tiles = 0;
   for (int i = 0; i < s.N; ++i) tiles += sweep_tiles(s, i);
   // enough work for every SM behind the longest sweep: nothing to gain, and nothing to play through
   if (BH * tiles > 1.3 * kSms * sweep_tiles(s, 0) || BH * tiles > 8192) return 0;
   int split = 0;
   if (!kBackward) {
-    const double start = 6.5, cost = narrow * (s.D == 64 ? 3.1 + 0.73 * R : 2.95 + 1.5 * R), totals = 3.0 + BH * tiles * (s.D == 64 ? 0.01 : 0.018);
+    struct Line { double start, tile, head, totals, total_tile; };      // of a block, per tile, per tile and head; the totals kernel, per tile
+    static constexpr Line lines[2][2] = {{{7.3, 3.2, 0.50, 1.2, 0.017}, {8.0, 3.3, 1.15, 1.2, 0.016}},       // chunks of 64: head_dim 64, 128
+                                         {{7.3, 2.7, 1.00, 1.1, 0.017}, {10.1, 2.2, 1.50, 2.9, 0.013}}};     // chunks of 128
+    const Line& l = lines[s.C != 64][s.D != 64];
+    const double start = l.start, cost = l.tile + l.head * R, totals = l.totals + l.total_tile * BH * tiles;
     auto len = [&](int i) { return sweep_tiles(s, i); };
     double best = 0.95 * play(s, len, 0, 0, start, cost, std::numeric_limits<double>::infinity());
     for (int t = 1; t < len(0); t *= 2) {
@@ -114,6 +120,7 @@ int make_split(const Shape& s) {
       if (est < best) { best = est; split = t; }
     }
   } else {
+    const double narrow = s.C == 64 ? 0.7 : 1.0;
     const double start = 12.0, cost = narrow * (s.D == 64 ? 3.3 + 0.9 * R : 3.4 + 1.9 * R), corr_start = 6.0, corr = narrow * (s.D == 64 ? 2.2 : 2.6);
     auto len = [&](int i) { return sweep_halves(s, i); };
     double best = 0.95 * play(s, len, 0, 0, start, cost, std::numeric_limits<double>::infinity());
