@@ -213,3 +213,40 @@ def test_decode_blocks_that_take_several_chunks(B, H, R, chunk, t):
             assert (lse[..., i].double() - torch.logsumexp(s, -1)).abs().max() <= 1e-4
             ref = torch.softmax(s, -1) @ v[:, :, sl].double()
             assert ((out[..., i].double() - ref).abs() - 2.0 ** -7 * ref.abs()).max() <= 2e-2
+
+
+def _decode_reference(k, v, src, q, dest, state, t, chunk):
+    """Row t in 64 bits: per chunk the probabilities and V of the live keys, log-sum-exp, and the state of keys 0..t."""
+    n = t + 1
+    kd = k[:, :, :n].double()
+    g = (kd @ kd[:, :, t].unsqueeze(-1)).squeeze(-1).clamp_min(0)
+    a = g.pow(2 / 3) * src[:, :, :n].double().pow(1 / 3) * dest.double().unsqueeze(-1).pow(1 / 3)
+    new = state[:, :, :n].double() + torch.log1p(-a.clamp(0, 1 - 1e-6))
+    new[:, :, t] = 0
+    chunks = []
+    for i in range(t // chunk + 1):
+        sl = slice(i * chunk, min(n, (i + 1) * chunk))
+        s = q.double() @ kd[:, :, sl].transpose(-1, -2) + new[:, :, sl].unsqueeze(2)
+        chunks.append((torch.softmax(s, -1), v[:, :, sl].double(), torch.logsumexp(s, -1)))
+    return new, chunks
+
+
+@pytest.mark.parametrize("D,chunk", [(128, 128), (128, 64), (64, 128), (128, 256)])
+def test_decode_affinity_of_long_keys_and_closed_gates(D, chunk):
+    """Keys whose Gram entry has no square in fp32, with gates that are zero or that bring the affinity back to ordinary sizes."""
+    from universal_attention_triton_b200 import ops
+    B, H, R, t = 1, 2, 2, chunk + 40
+    cap = 2 * chunk
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    k = (torch.rand(B, H, cap, D, generator=gen, device="cuda") * 1e10).bfloat16()
+    v = torch.randn(B, H, cap, D, generator=gen, device="cuda").bfloat16()
+    src = torch.full((B, H, cap), 1e-24, device="cuda")
+    src[:, :, ::3], src[:, :, 1::3] = 0, 1e-30
+    q, dest = (torch.randn(B, H, R, D, generator=gen, device="cuda") * 1e-11).bfloat16(), torch.full((B, H), 1e-22, device="cuda")
+    state = torch.zeros(B, H, cap, device="cuda")
+    new, chunks = _decode_reference(k, v, src, q, dest, state, t, chunk)
+    out, lse = ops.decode_step(t, k, v, src, q, dest, state, chunk)
+    assert (state[:, :, :t + 1].double() - new).abs().max() <= 1e-5
+    for i, (p, vi, l) in enumerate(chunks):
+        assert (lse[..., i].double() - l).abs().max() <= 1e-4
+        assert ((out[..., i].double() - p @ vi).abs() <= 2.0 ** -8 * (p @ vi.abs() + (p @ vi).abs()) + 1e-5).all()

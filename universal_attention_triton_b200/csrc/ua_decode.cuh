@@ -263,8 +263,9 @@ __global__ void __launch_bounds__(2 * C, StepCfg<D, C, RT>::kBlocks) step_mma_ke
       float cstate = 0.f;
       if (tid < nkeys && i * C + tid < p.t) {
         const float g = s_s[tid * Cfg::kSW];
-        // relu(g)^(2/3) src^(1/3) dest^(1/3) as one cube root
-        const float a = g > 0.f ? cbrtf(g * g * (src * dst)) : 0.f;
+        // relu(g)^(2/3) src^(1/3) dest^(1/3) as one cube root.  Each gate (at most 1) brings its own factor g down before the two meet: g * g
+        // of long keys leaves fp32, src * dst of closed gates falls below it, and infinity times zero is no affinity
+        const float a = g > 0.f ? cbrtf((g * src) * (g * dst)) : 0.f;
         cstate = old + log1pf(-fminf(fmaxf(a, 0.f), clamp_hi()));
       }
       if (tid < nkeys) p.state[(size_t)bh * p.Lcap + (size_t)i * C + tid] = cstate;
