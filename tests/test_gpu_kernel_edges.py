@@ -231,6 +231,34 @@ def _decode_reference(k, v, src, q, dest, state, t, chunk):
     return new, chunks
 
 
+@pytest.mark.parametrize("B,H,R,chunk,D,t,gates", [(16, 16, 4, 64, 128, 230, torch.bfloat16), (40, 4, 1, 128, 128, 511, torch.float32),
+                                                   (20, 8, 8, 128, 128, 400, torch.bfloat16), (8, 20, 3, 128, 128, 640, torch.float32),
+                                                   (8, 8, 4, 128, 64, 300, torch.bfloat16), (4, 8, 2, 256, 128, 700, torch.float32)])
+def test_decode_reads_live_keys_alone_and_does_not_depend_on_the_batch(B, H, R, chunk, D, t, gates):
+    """What lies behind the live keys is NaN and stays as it is.  Rounding P and the result to bf16 (eight significant bits: at
+    most 2^-8 of the value each) moves an output by at most 2^-8 (sum_k P_k |v_k| + |out|) (1e-5 for the fp32 sums); a conversation gives the same bits alone, where no block takes a second chunk."""
+    from universal_attention_triton_b200 import ops
+    cap = (t // chunk + 2) * chunk
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    k = rnd(B, H, cap, D)
+    k = (k / k.norm(dim=-1, keepdim=True)).bfloat16()
+    v, src, dest = rnd(B, H, cap, D).bfloat16(), torch.sigmoid(rnd(B, H, cap)).to(gates), torch.sigmoid(rnd(B, H)).to(gates)
+    q, state = rnd(B, H, R, D).bfloat16(), -0.01 * torch.rand(B, H, cap, generator=gen, device="cuda")
+    for x in (k, v, src, state):
+        x[:, :, t + 1:] = float("nan")
+    new, chunks = _decode_reference(k, v, src, q, dest, state, t, chunk)
+    alone = state[-1:].clone()
+    out, lse = ops.decode_step(t, k, v, src, q, dest, state, chunk)
+    assert (state[:, :, :t + 1].double() - new).abs().max() <= 1e-5 and torch.isnan(state[:, :, t + 1:]).all()
+    for i, (p, vi, l) in enumerate(chunks):
+        ref = p @ vi
+        assert (lse[..., i].double() - l).abs().max() <= 1e-4
+        assert ((out[..., i].double() - ref).abs() <= 2.0 ** -8 * (p @ vi.abs() + ref.abs()) + 1e-5).all()
+    out1, lse1 = ops.decode_step(t, k[-1:].contiguous(), v[-1:].contiguous(), src[-1:].contiguous(), q[-1:], dest[-1:], alone, chunk)
+    assert torch.equal(out1, out[-1:]) and torch.equal(lse1, lse[-1:]) and torch.equal(alone[:, :, :t + 1], state[-1:, :, :t + 1])
+
+
 @pytest.mark.parametrize("D,chunk", [(128, 128), (128, 64), (64, 128), (128, 256)])
 def test_decode_affinity_of_long_keys_and_closed_gates(D, chunk):
     """Keys whose Gram entry has no square in fp32, with gates that are zero or that bring the affinity back to ordinary sizes."""
