@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256) widen_bf16_kernel(const bf16* __restrict_
 }
 int launch_widen(const void* src, float* dst, size_t n, cudaStream_t st) {
   const size_t n8 = aligned16(src) && aligned16(dst) ? n / 8 : 0, work = n8 ? n8 : n;
-  const unsigned blocks = (unsigned)std::min<size_t>((work + 255) / 256, 148 * 16);
+  const unsigned blocks = (unsigned)std::min<size_t>((work + 255) / 256, ua::kSms * 16);
   widen_bf16_kernel<<<blocks, 256, 0, st>>>(static_cast<const bf16*>(src), dst, n8, n);
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }
@@ -190,12 +190,12 @@ int launch_convert(const float* src, void* dst, size_t n, cudaStream_t st) {
   if (n % 8 == 0 && n >= 8 && aligned16(src) && aligned16(dst)) {
     const size_t n8 = n / 8;
     int blocks = (int)((n8 + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
+    if (blocks > ua::kSms * 8) blocks = ua::kSms * 8;
     ua::simt::convert8_kernel<T><<<blocks, 256, 0, st>>>(reinterpret_cast<const float4*>(src), static_cast<T*>(dst), n8);
     return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
   }
   int blocks = (int)((n + 1023) / 1024);
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks > ua::kSms * 16) blocks = ua::kSms * 16;
   if (blocks < 1) blocks = 1;
   ua::simt::convert_kernel<T><<<blocks, 256, 0, st>>>(src, static_cast<T*>(dst), n);
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
@@ -836,7 +836,7 @@ int ua_bwd_saved(const UaDims* dims, int dtype, int gate_dtype, const void* kc, 
       if (!lse) {
         lse = at(w.off_lse);
         if (wide) {
-          group_lse_kernel<<<148 * 8, 256, 0, st>>>(fp.lse, at(w.off_lse), (size_t)s.B * s.H * s.N, (size_t)s.R * s.L, s.L, s.N, s.C, m);
+          group_lse_kernel<<<ua::kSms * 8, 256, 0, st>>>(fp.lse, at(w.off_lse), (size_t)s.B * s.H * s.N, (size_t)s.R * s.L, s.L, s.N, s.C, m);
           if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
         }
       }
@@ -1177,7 +1177,7 @@ int ua_fwd_merged(const UaDims* dims, int dtype, int gate_dtype, const void* kc,
   ua::sm100::whole_sequence(fp);
   if ((e = ua::sm100::launch_fwd(s, gate_dtype, kc, vc, xq, fp, false, nullptr, st))) return e;
   // the row's log-sum-exp over all key chunks
-  row_lse_kernel<<<148 * 8, 256, 0, st>>>(lse_cm, row_lse, BH, s.N, s.R, s.L);
+  row_lse_kernel<<<ua::kSms * 8, 256, 0, st>>>(lse_cm, row_lse, BH, s.N, s.R, s.L);
   if (cudaGetLastError() != cudaSuccess) return UA_ERR_CUDA;
   // pass 2: every (chunk, row tile, head) adds exp(m - row_lse) P~ V to the fp32 merged accumulator
   fp.lse = nullptr; fp.carry = nullptr; fp.merged_acc = acc; fp.row_lse = row_lse;

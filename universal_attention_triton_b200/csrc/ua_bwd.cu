@@ -117,7 +117,7 @@ int launch_masked_t(const Shape& s, const void* kc, const void* vc, const void* 
       if (jmax > jcap) jmax = jcap;
       if (jmax > p.j_begin) p.items_per_bh += (jmax - p.j_begin + p.jp - 1) / p.jp;
     }
-    if (p.jp <= 2 || BH * p.items_per_bh * Cfg::kKB >= 148) break;
+    if (p.jp <= 2 || BH * p.items_per_bh * Cfg::kKB >= kSms) break;
   }
   if (p.items_per_bh == 0) return UA_OK;
   const auto* k16 = static_cast<const __nv_bfloat16*>(kc);

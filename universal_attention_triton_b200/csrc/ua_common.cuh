@@ -11,6 +11,8 @@ __device__ __forceinline__ float mask_value() { return -1e12f; }
 __device__ __forceinline__ float clamp_hi() { return 0.999999f; }   // fp32 rounding of 1 - 1e-6
 __device__ __forceinline__ float clamp_lo_bwd() { return 1e-6f; }
 
+constexpr int kSms = 148;      // what grids, and the play-through of cut sweeps, are laid out for
+
 struct Shape {
   int B, H, R, N, C, D, L;
 };

@@ -7,8 +7,11 @@
 //     state[t]  = 0
 // and the new row's outputs are, per key chunk i of `chunk` keys (only the chunks that hold keys <= t exist),
 //     lse[r][i] = logsumexp_k (k_k . q_r + state[k]),     out[r][i][:] = sum_k softmax_k(...) v_k
-// exactly row t of the full forward.  O(t * d) work and cache reads per step: HBM-bound, one block per (b, h, chunk),
-// one thread per key of the chunk, fp32 CUDA-core arithmetic (no tile is large enough for the tensor cores).
+// exactly row t of the full forward.  O(t * d) work and cache reads per step: HBM-bound.  Three kernels:
+//   step_mma_kernel   bf16, head_dim 128, chunks of 64 / 128 keys: blocks that stay and take one (b, h, chunk) after another
+//   step_once_kernel  bf16, head_dim 64, and chunks of 256 keys: a block per (b, h, chunk), the whole chunk in flight at once
+//   step_kernel       fp32, other head_dims and chunks, unaligned queries: a block per (b, h, chunk), thread = key, CUDA cores
+// The first two form scores (the first P V as well) with mma.sync; eight columns are too few for tcgen05.
 #pragma once
 #include "ua_aux.cuh"
 #include "ua_common.cuh"
@@ -515,6 +518,10 @@ inline bool launch_step_mma(const Params& p, int nt, cudaStream_t st) {
   // Blocks that stay pay where a chunk is long enough to hide their work and several of them fit an SM.  At t = 6150, B16 H8, staying / one
   // chunk per block in us: D128 C128 R1 73 / 80, R4 76 / 86, R8 104 / 142, C64 R4 70 / 78; but C256 R2 117 / 93, R4 118 / 109 (one block of
   // 150 KB per SM), and D64 R2 58 / 47 (half the bytes for the same chain of scores, softmax and P V).
+  // With fewer chunks than resident blocks no block takes a second one, and the form is still the shorter chain (P V without sums across
+  // warps).  B1 H8, GPU time per step at t = 300 / 1000 / 3000, staying / one chunk per block: C128 R1 4.0 / 4.4 / 6.1, 5.0 / 5.2 / 6.3; R4 4.4 / 4.5 / 6.3,
+  // 5.0 / 5.0 / 6.7; R8 4.8 / 4.8 / 6.9, 6.1 / 6.2 / 9.1; C64 R1 3.7 / 4.0 / 5.5, 4.9 / 5.1 / 6.0; R4 3.7 / 4.1 / 5.6, 4.4 / 4.6 / 6.3.  Chunks of 128 keys then
+  // need the opt-in to more than 48 KB, a driver call of 0.08 us per step (remembering it per context saves half of that).
   if constexpr (D == 64 || C == 256) {
     return launch_step_once<D, C, RT, TG>(p, nt, st);
   } else {
@@ -522,7 +529,7 @@ inline bool launch_step_mma(const Params& p, int nt, cudaStream_t st) {
     if (Cfg::kSmemBytes > 48 * 1024 &&
         cudaFuncSetAttribute(step_mma_kernel<D, C, RT, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
       return false;
-    const int items = p.BH * nt, grid = items < 148 * Cfg::kBlocks ? items : 148 * Cfg::kBlocks;
+    const int items = p.BH * nt, grid = items < kSms * Cfg::kBlocks ? items : kSms * Cfg::kBlocks;
     step_mma_kernel<D, C, RT, TG><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmemBytes, st>>>(p, items);
     return true;
   }
@@ -538,8 +545,8 @@ inline bool launch_step_mma_c(const Params& p, int nt, cudaStream_t st) {
   if (p.C == 64) return launch_step_mma_r<D, 64, TG>(p, nt, st);
   return p.C == 128 ? launch_step_mma_r<D, 128, TG>(p, nt, st) : launch_step_mma_r<D, 256, TG>(p, nt, st);
 }
-// What the kernel above takes: its tiles are whole 16-byte pieces of 64- or 128-wide bf16 rows, and chunks whose threads
-// (two per key) make whole warps and at most 512 of them.  Everything else (fp32, other widths) runs on step_kernel.
+// What the two mma.sync kernels take between them: tiles of whole 16-byte pieces of 64- or 128-wide bf16 rows, chunks whose threads
+// (two per key) are 512 at the most.  Everything else (fp32, other widths) runs on step_kernel.
 inline bool step_mma_takes(const Params& p, bool bf16_in) {
   return bf16_in && (p.D == 64 || p.D == 128) && (p.C == 64 || p.C == 128 || p.C == 256) &&
          (reinterpret_cast<uintptr_t>(p.q) & 15u) == 0;

@@ -27,10 +27,11 @@
 //               the other group then), S + C, row max / sum in registers (no shuffles), P -> TMEM as bf16 in a buffer of the group's own,
 //               m + log l -> lse.  O / l of a head is written while the next head's P is formed, so no group waits for a product.
 //
-// What bounds it: the exponentials and logarithms (XU pipe, half of the cycles at R = 4), issue slots (half), and instruction fetch.  The
-// loops of the decay and the softmax warps run side by side on every scheduler, and beyond some 800 instructions together they stall on
-// fetching them: rows per pass of the decay loop, loops left rolled (unroll 1) and the length of a wait's slow path are chosen for that.  At B4 H8 R4
-// L4096 D64: 0.4 warps wait for instructions per instruction issued; 1.4 did with 64 rows per pass of the decay loop (730 -> 860 us).
+// What bounds it: the exponentials and logarithms (XU pipe, half of the cycles at R = 4) and issue slots (half).  The loops of the decay and
+// the softmax warps run side by side on every scheduler, and how long they may be is bounded by instruction fetch: with 32 rows per pass of the
+// decay loop 0.4 warps wait for instructions per instruction issued, with 64 rows 1.4 (730 -> 860 us at B4 H8 R4 L4096 D64); rows per pass, loops
+// left rolled (unroll 1) and the length of a wait's slow path are chosen for that.  (The form before this one waited for instructions as little,
+// 0.4; what it had more of was waiting for TMEM loads, 2.8 against 1.5, and instructions, 27.7 against 24.5 million.)
 // B4 H8 R4 L4096 D64 935 -> 706 us, R1 574 -> 455, B1 H8 R4 L8192 D128 1295 -> 1045, L4096 356 -> 304, B1 H16 R1 L4096 D128 315 -> 270, against
 // the form with two passes over TMEM per head, outputs written from registers and one issuing thread.
 //
@@ -60,7 +61,7 @@ struct FwdParams {
   float* lse;            // (b,h,n,r,L)
   __nv_bfloat16* denom;  // (b,h,n,r,L) or null
   int* status;           // device word: 0 = ok, otherwise a role-specific timeout code
-  int fill_masked;       // write the rows before the key chunk (uniform softmax) from the two otherwise idle warps
+  int fill_masked;       // write the rows before the key chunk (uniform softmax) from warp 3
   // Row range (sequence sharding): this call computes row tiles [j_begin, j_end) only.  xq, static_dest, out,
   // lse and denom then hold just those Lr = (j_end - j_begin) * 128 rows; keys, values and static_src are whole.
   int j_begin, j_end, Lr;  // Lr: rows per (chunk, head) slab of the row-indexed tensors

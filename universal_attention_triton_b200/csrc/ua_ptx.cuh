@@ -39,9 +39,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return done != 0;
 }
 
-// The same test with a suspend-time hint: the hardware may park the thread until the phase completes or about `hint_ns`
-// have passed, instead of returning at once.  A waiter that polls with this form issues a few instructions per hint
-// period rather than a tight loop's worth, which matters when it shares a scheduler with warps that do the real work.
+// The same test with a suspend-time hint.  Measured, a poll ends when the phase completes or after about 8400 cycles, whatever the hint
+// says; so a waiter that shares a scheduler with warps that do the real work issues a few instructions per 8400 cycles.
 __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
   uint32_t done;
   asm volatile(
@@ -61,7 +60,7 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
   return t;
 }
 
-constexpr uint32_t kWaitHintNs = 20000;      // per poll; completion of the phase ends the suspension at once
+constexpr uint32_t kWaitHintNs = 20000;
 constexpr uint32_t kWaitLimitNs = 2000000000u;
 
 // Bounded wait: gives up after about two seconds of wall time (or when
@@ -166,14 +165,6 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 
 // Four tcgen05.mma of one accumulation chain from ONE asm statement: what limits a single issuing thread is the
 // instruction count per MMA (descriptor arithmetic, predicate set-up), so the chain shares one predicate set-up and
@@ -273,16 +264,7 @@ __device__ __forceinline__ float warp_transpose_reduce(float* v, int lane) {
 //   MN-major operand ([rows = K][64 elements of M or N], 128-byte rows):
 //       sbo = 1024 (8 K-rows), lbo = byte distance between 64-element groups
 //       of M/N; advance 16 K-rows = +2048 bytes.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
+//
 // The descriptor splits into a high word that is the same for every 128-byte-swizzled operand
 // (sbo = 1024, version, swizzle mode) and a low word (address >> 4, lbo >> 4) that the issuing
 // thread can advance with one 32-bit add.

@@ -23,8 +23,6 @@
 namespace ua {
 namespace sm100 {
 
-constexpr int kSms = 148;
-
 // 128-row tiles in the sweep of chunk i (chunks of 64 keys start a tile at their own first row)
 inline int sweep_tiles(const Shape& s, int i) { return (s.L - i * s.C + 127) / 128; }
 // ... and 64-row half tiles, the backward's unit

@@ -17,7 +17,7 @@ void leave(const Leave& v, bool f32, bool gates_f32, cudaStream_t st) {
   size_t most = 0;
   for (size_t n : v.n) most = n > most ? n : most;
   unsigned blocks = (unsigned)((most / 4 + kThreads - 1) / kThreads);
-  if (blocks > 148 * 8) blocks = 148 * 8;
+  if (blocks > kSms * 8) blocks = kSms * 8;
   if (f32) leave_kernel<float, float><<<blocks, kThreads, 0, st>>>(v);
   else if (gates_f32) leave_kernel<__nv_bfloat16, float><<<blocks, kThreads, 0, st>>>(v);
   else leave_kernel<__nv_bfloat16, __nv_bfloat16><<<blocks, kThreads, 0, st>>>(v);
