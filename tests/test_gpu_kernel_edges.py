@@ -151,7 +151,8 @@ def test_merge_of_few_and_of_many_chunks(dtype, vec_dtype, N, D):
 @pytest.mark.parametrize("shape", [(1, 2, 4, 12, 64, 64), (1, 4, 1, 9, 64, 64), (1, 2, 2, 8, 64, 128)])
 def test_gradients_of_chunks_of_64_keys_lose_no_more_than_their_roundings(shape):
     """Gradients of the operator's own outputs through the Function's default path, against 64 bits: what is rounded to bf16 are the
-    operands P, dS, dG of the products and the results, each by at most 2^-9, independently: sqrt(2) 2^-9 in the 2-norm.  (Row terms
+    operands P, dS, dG of the products and the results, each by less than 2^-9 in the 2-norm (a value by 2^-8 at the most, over all
+    mantissas 0.38 of that), independently: sqrt(2) 2^-9 together.  (Row terms
     from the bf16 output tiles were twice that.)  d static_dest is an fp32 sum over the keys: the result's rounding alone."""
     from universal_attention_triton_b200 import UniversalAttention
     B, H, R, n, c, D = shape
