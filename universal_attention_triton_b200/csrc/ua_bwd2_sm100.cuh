@@ -216,6 +216,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
   // in sweep order: K_j of half tile ht, then the (Q, dO) pairs of its heads (with the log-sum-exp and g_denom rows of
   // the head); a slot is refilled as soon as the MMAs that read it have completed
   int hc = 0;
+#pragma unroll 1
   for (int ht = 0; ht < c.nht; ++ht) {
     const int row0 = c.row0_of(ht), srow0 = c.srow0_of(ht);
     {
@@ -227,6 +228,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
         tma_load_2d(sb + Cfg::oKj + sl * Cfg::kHalf + b * 8192, tmK, b * 64, c.bh * L + row0, c.bar(qKjFull + sl));
     }
     if (ht + 1 < c.nht && !load_tables(ht + 1)) return;
+#pragma unroll 1
     for (int r = 0; r < Rh; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, use = hc / Cfg::kNS;
       if (use >= 1 && !c.wait(qInFree + sl, use - 1)) return;
@@ -301,12 +303,14 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
 
   if (!c.wait(qKvFull, 0)) return;
   int hc = 0;
+#pragma unroll 1
   for (int ht = 0; ht < c.nht; ++ht) {
     if (!c.wait(qKjFull + ht % Cfg::kKj, ht / Cfg::kKj)) return;
     // (the workers read the tables of the next half tile before this one is over)
     if (kMode != 4 && R > 0 && ht + 1 < c.nht && !c.wait(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
     if (R > 0 && !unit_g(ht)) return;                               // G for the decay recomputation (none without heads)
     if (kMode == 4) tc_commit(c.bar(qKjFree + ht % Cfg::kKj));      // (no back issuers: the tiles are free once these products are done)
+#pragma unroll 1
     for (int r = 0; r < R; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, b = u % Cfg::kNB;
       if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
@@ -348,7 +352,9 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
     if (kC == 128) mma4_ss(Y, t_mn + 512, k + 512, 128, 128, id_tn, 1);
   };
   if (!c.wait(qKvFull, 0)) return;
+#pragma unroll 1
   for (int ht = 0; ht < c.nht; ++ht) {
+#pragma unroll 1
     for (int r = 0; r < R; ++r, ++hc, ++w) {
       const int sl = hc % Cfg::kNS, db = w % Cfg::kRing;
       const uint32_t dsb = sb + Cfg::oDs + db * 16384;
@@ -371,6 +377,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
         tc_commit(c.bar(qInFree + sl));
         tc_commit(c.bar(qDsFree + db));
       } else {
+#pragma unroll 1
         for (int cb = 0; cb < D / 64; ++cb, ++yc) {
           if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
           tc_fence_after();
@@ -392,6 +399,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
       tc_commit(c.bar(qKjFree + ht % Cfg::kKj));
       tc_commit(c.bar(qDsFree + gb));
     } else {
+#pragma unroll 1
       for (int cb = 0; cb < D / 64; ++cb, ++yc) {
         if (yc >= 1 && !c.wait(qYFree, yc - 1)) return;
         tc_fence_after();
@@ -451,7 +459,9 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
   const uint32_t swz = (uint32_t)(row & 7);
   uint8_t* sStage = c.smem + Cfg::oStage;
   int yc = 0;
+#pragma unroll 1
   for (int ht = 0; ht < c.nht; ++ht) {
+#pragma unroll 1
     for (int z = 0; z < (Rh + 1) * (D / 64); ++z, ++yc) {
       const int r = z / (D / 64), cb = z % (D / 64);
       if (!c.wait_w(qYFull, yc)) return;
@@ -510,6 +520,7 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
   const int row = (warp - 6) * 32 + lane;               // 0..63
   const uint32_t swz = (uint32_t)(row & 7);
   const int total = c.nht * p.heads;
+#pragma unroll 1
   for (int hc = 0; hc < total; ++hc) {
     const int sl = hc % Cfg::kNS;
     const uint8_t* go = c.smem + Cfg::oSlot + sl * Cfg::kSlot + Cfg::kHalf + row * 128;
@@ -593,10 +604,12 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   if (helper && quad == kGateQuad) sT3[col0 + lane] = t3_from_table(0);
   float suffix = p.suffix_in ? p.suffix_in[((size_t)c.bh * N + c.i) * 128 + key] : 0.f, ds_acc = 0.f;
   if (!kHeads && p.seg)                          // what the segments of later rows leave
+#pragma unroll 4
     for (int q = 0; q < c.segment; ++q) suffix += p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + q) * 128 + key];
   named_bar_sync(kBarAll, kWorkers);
 
   int u = 0, hc = 0;                             // units and heads so far
+#pragma unroll 1
   for (int ht = 0; ht < c.nht; ++ht) {
     const int rel = c.row0_of(ht) - c.i * kC;
     const bool diag = rel < kC;                    // rows at positions of the chunk's own keys
@@ -666,6 +679,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     float2 dc[H2];
 #pragma unroll
     for (int x = 0; x < H2; ++x) dc[x] = make_float2(0.f, 0.f);
+#pragma unroll 1
     for (int r = 0; r < R; ++r, hc += (kMode == 4 ? 0 : 1)) {
       const int b = u % Cfg::kNB, sl = hc % Cfg::kNS;
       float* tabL = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512);      // lse[64] of the head's rows (raw)
@@ -948,6 +962,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     c.nht = c.htop - (kC == 128 ? 2 * (c.i > p.j_begin ? c.i : p.j_begin) : c.i);
   } else {
     int nht;
+#pragma unroll 1
     for (c.i = 0;; ++c.i) {
       nht = (p.s.L - c.i * kC) / 64;
       const int ns = (nht + p.seg - 1) / p.seg;
@@ -965,18 +980,18 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     return;
   }
 
-  if (threadIdx.x == 0) {
+  if (const int b = (int)threadIdx.x - 32; b >= 0 && b < qNumBars) {      // (a thread per barrier: one after the other they take 2 to 3 us)
+    uint32_t count = 1;
+    if (b == qLdDone || b == qLdDone + 1 || (b >= qDsReady && b < qDsReady + 3) || b == qTabDone) count = kC / 32 * NG;   // one arrival per worker warp
+    if (kMode == 4 && b >= qInFree && b < qInFree + 4) count = kC / 32 * NG;
+    if (b == qYFree || (b >= qDelta && b < qDelta + 4)) count = 2;                                          // the two draining warps
+    if ((b >= qDsFree && b < qDsFree + 3) || b == qFinal || b == qSFull || b == qSFull + 1) count = 2;      // both back issuers; commit and front issuer
+    mbar_init(c.bar(b), count);
+    mbar_init_fence();
+  }
+  if (threadIdx.x == 96) {
     misc[1] = 0;
     misc[2] = 0;
-    for (int b = 0; b < qNumBars; ++b) {
-      uint32_t count = 1;
-      if (b == qLdDone || b == qLdDone + 1 || (b >= qDsReady && b < qDsReady + 3) || b == qTabDone) count = kC / 32 * NG;   // one arrival per worker warp
-      if (kMode == 4 && b >= qInFree && b < qInFree + 4) count = kC / 32 * NG;
-      if (b == qYFree || (b >= qDelta && b < qDelta + 4)) count = 2;                                                                                  // the two draining warps
-      if ((b >= qDsFree && b < qDsFree + 3) || b == qFinal || b == qSFull || b == qSFull + 1) count = 2;      // both back issuers; commit and front issuer
-      mbar_init(c.bar(b), count);
-    }
-    mbar_init_fence();
     prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmQ); prefetch_tmap(&tmG);
     prefetch_tmap(&tmDQ); prefetch_tmap(&tmDK);
     if (kOutDelta) prefetch_tmap(&tmO);
@@ -1006,7 +1021,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   // warps 0-3: the four single-thread roles; warps 4-5: drain warps (6-7 complete their warpgroup); warps 8..: workers
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
-    if (lane == 0) {
+    if (elect_one()) {
       if (warp == 0) bwd2_front<D, kMode, kOutDelta>(c, p);
       else if (kMode == 4 && warp != 2) {}      // (the row-term pass has nothing for the back issuers and the drain warps)
       else if (warp == 1) bwd2_back<D, kC>(c, p, 0);
@@ -1029,6 +1044,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     if (threadIdx.x == 0) {
       if (atomicExch(p.status, 3) == 0) p.status[1] = (int)misc[2];
     }
+#pragma unroll 1
     for (int it = 0; it < 64; ++it) __nanosleep(2000);
     __syncthreads();
   }

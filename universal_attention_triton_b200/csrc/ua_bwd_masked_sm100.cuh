@@ -608,16 +608,16 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     c.chi = min(Cfg::kG, N - c.i0);
   }
 
-  if (threadIdx.x == 0) {
+  if (const int b = (int)threadIdx.x - 32; b >= 0 && b < mNumBars) {      // (a thread per barrier)
+    uint32_t count = 1;
+    if (b == mYFree || b == mYFree + 1) count = 4;     // one arrival per draining warp
+    if (b == mQFree || b == mQFree + 1) count = 9;     // the issuer's commit, the four gate-sum warps, the four draining warps
+    mbar_init(c.bar(b), count);
+    mbar_init_fence();
+  }
+  if (threadIdx.x == 64) {
     misc[1] = 0;
     misc[2] = 0;
-    for (int b = 0; b < mNumBars; ++b) {
-      uint32_t count = 1;
-      if (b == mYFree || b == mYFree + 1) count = 4;     // one arrival per draining warp
-      if (b == mQFree || b == mQFree + 1) count = 9;     // the issuer's commit, the four gate-sum warps, the four draining warps
-      mbar_init(c.bar(b), count);
-    }
-    mbar_init_fence();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmG); prefetch_tmap(&tmDQ);
   }
   if (warp == 0) {
@@ -644,9 +644,9 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   c.tmem = uniform(misc[0]);
 
   if (warp == 0) {
-    if (lane == 0) mk_producer<D, kWide>(c, p, &tmQ, &tmG);
+    if (elect_one()) mk_producer<D, kWide>(c, p, &tmQ, &tmG);
   } else if (warp == 1) {
-    if (lane == 0) mk_issuer<D, kWide>(c, p);
+    if (elect_one()) mk_issuer<D, kWide>(c, p);
   } else if (warp >= 4 && warp < 8) {
     mk_drain<D, kWide>(c, p, &tmDQ);
   } else if (warp >= 8) {

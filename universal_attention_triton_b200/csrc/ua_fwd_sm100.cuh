@@ -806,17 +806,17 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   }
   c.srow0 = p.r0 + c.row0 - p.j_begin * 128;
 
-  if (threadIdx.x == 0) {
-    misc[1] = 0;
-    for (int b = 0; b < kNumBars; ++b) {
-      uint32_t count = 1;
-      // one arrival per warp of the group that signals
-      if (b == kGFree || b == kCReady || b == kCReady + 1) count = kC / 32;
-      if (b == kT3Ready || b == kSFree || b == kSFree + 1 || b == kPReady || b == kPReady + 1 || b == kOFree || b == kOFree + 1) count = 4;
-      if (b == kCFree || b == kCFree + 1) count = Cfg::kHalves ? 4 : 8;
-      mbar_init(c.bar(b), count);
-    }
+  if (const int b = (int)threadIdx.x - 32; b >= 0 && b < kNumBars) {      // (a thread per barrier)
+    uint32_t count = 1;
+    // one arrival per warp of the group that signals
+    if (b == kGFree || b == kCReady || b == kCReady + 1) count = kC / 32;
+    if (b == kT3Ready || b == kSFree || b == kSFree + 1 || b == kPReady || b == kPReady + 1 || b == kOFree || b == kOFree + 1) count = 4;
+    if (b == kCFree || b == kCFree + 1) count = Cfg::kHalves ? 4 : 8;
+    mbar_init(c.bar(b), count);
     mbar_init_fence();
+  }
+  if (threadIdx.x == 64) {
+    misc[1] = 0;
     prefetch_tmap(&tmK);
     prefetch_tmap(&tmV);
     prefetch_tmap(&tmQ);
@@ -838,11 +838,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
   if (warp < 4) {
     if (!kCarryOnly) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
     if (warp == 0) {
-      if (lane == 0 && c.ntiles > 0) fwd_producer<D, kC, kCarryOnly>(c, p, &tmK, &tmV, &tmQ);
+      if (c.ntiles > 0 && elect_one()) fwd_producer<D, kC, kCarryOnly>(c, p, &tmK, &tmV, &tmQ);
     } else if (warp == 1) {
-      if (lane == 0 && c.ntiles > 0) fwd_mma_scores<D, kC, kCarryOnly>(c, p);
+      if (c.ntiles > 0 && elect_one()) fwd_mma_scores<D, kC, kCarryOnly>(c, p);
     } else if (warp == 2) {
-      if (lane == 0 && c.ntiles > 0 && !kCarryOnly && kOut != kOutStats) fwd_mma_pv<D, kC>(c, p);
+      if (c.ntiles > 0 && elect_one() && !kCarryOnly && kOut != kOutStats) fwd_mma_pv<D, kC>(c, p);
     } else if (!kCarryOnly && p.fill_masked) {
       fwd_fill_rows<D, kC>(c, p, fill_chunk, fill_lo, fill_hi);
     }

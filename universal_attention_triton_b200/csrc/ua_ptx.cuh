@@ -16,6 +16,17 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // B4 H8 R4 L4096 D64 730 -> 706 us, one query head 474 -> 455; backward B1 H16 R1 L4096 D128 724 -> 685.)
 __device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
+// One lane of a converged warp, the same one each time.  The single-thread roles run behind this and not behind `lane == 0`: the compiler then
+// knows that one lane at the most is active and forms descriptors, barrier and TMEM addresses where the instructions take them from, instead of
+// moving every operand through vector registers.  What that saves is code (backward 79 -> 68 KB at head_dim 64, 79 -> 64 at 128; sweep of the
+// rows before a chunk 69 -> 47), and with it waiting for instructions: warps stalled for them per instruction issued 1.0 -> 0.29 in the backward.
+// Backward B4 H8 R4 L4096 D64 1751 -> 1689 us, one query head 1186 -> 1057, B1 H16 R1 L4096 D128 671 -> 618, rows before a chunk 510 -> 380.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier ----
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -85,7 +96,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // outcome is agreed by vote so that a warp never splits on a timeout.
 __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
   __syncwarp();
-  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+  if (elect_one()) mbar_arrive(bar);
 }
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t limit_ns = kWaitLimitNs) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
