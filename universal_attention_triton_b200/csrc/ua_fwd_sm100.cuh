@@ -132,8 +132,10 @@ struct FwdCfg {
   // two slots that K_j and Q tiles pass through in the order of their products
   static constexpr int oSlot = oVi + kTileBytes;
   // The decay prefix crosses from keys-on-lanes to rows-on-lanes through fp32 tiles C^T[128 rows][128 keys] of 64 KB.  With two of them the decay
-  // group is a tile ahead of the softmax groups.  head_dim 128 has room for one, which is handed over in halves of 64 rows: a half
-  // is written while the softmax groups, done with the prefix of the tile before it, form the exponentials of its last heads.
+  // group is a tile ahead of the softmax groups.  head_dim 128 has room for one.  There the prefix of a tile is formed in TMEM, in the place of G,
+  // while the softmax groups work on the tile before, and copied (0.9k cycles) when they are done with that one's; written as it was formed it
+  // could start only then, and a tile took the 7 to 8k cycles of the decay group plus the 8k for which four heads need it: B1 H8 R4 L8192 1060 ->
+  // 965 us, B2 H8 R2 L1536 80 -> 75, B1 H4 R4 L3072 145 -> 138; one query head the same (269).  It is handed over in halves of 64 rows.
   static constexpr bool kHalves = (D == 128);
   static constexpr int kCBufs = kHalves ? 1 : 2;
   static constexpr int oCs = oSlot + 2 * kTileBytes;
@@ -280,6 +282,7 @@ __device__ __forceinline__ void fwd_mma_pv(const FwdCtx<D>& c, const FwdParams& 
 template <int D, int kC, typename TG, bool kCarryOnly>
 __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p) {
   using Cfg = FwdCfg<D>;
+  constexpr bool kHold = Cfg::kHalves && !kCarryOnly;      // the prefix stays in TMEM until C^T is free
   const int L = p.s.L;
   const int k = threadIdx.x & 127;
   const uint32_t lane_base = c.lane_base;
@@ -351,7 +354,8 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
       }
     };
     // (the diagonal tile is the only one with masked pairs: its tests are compiled into a path of their own)
-    auto prefix = [&](const uint32_t* om, int q0, auto on_diag) {
+    const uint32_t tg = c.tmem + Cfg::tG + lane_base;
+    auto prefix = [&](uint32_t* om, int q0, auto on_diag) {
       constexpr bool kDiag = decltype(on_diag)::value;
       const float2 ln2 = make_float2(0.6931471805599453f, 0.6931471805599453f);
 #pragma unroll
@@ -363,18 +367,22 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
         run.y = local = run.x + (kDiag && q + 1 <= k ? 0.f : el.y);
         const float2 cv = fadd2(make_float2(carry, carry), fadd2(make_float2(tprev, tprev), run));
         cval = cv.y;
-        if (!kCarryOnly) {
-          st_shared_f1((cdst ^ ((x & 7) << 4)) + q * 512, (kDiag && q < k) ? mask_value() : cv.x);
-          st_shared_f1((cdst ^ (((x + 1) & 7) << 4)) + (q + 1) * 512, (kDiag && q + 1 < k) ? mask_value() : cv.y);
+        const float c0 = (kDiag && q < k) ? mask_value() : cv.x, c1 = (kDiag && q + 1 < k) ? mask_value() : cv.y;
+        if (kHold) {
+          om[x] = __float_as_uint(c0);
+          om[x + 1] = __float_as_uint(c1);
+        } else if (!kCarryOnly) {
+          st_shared_f1((cdst ^ ((x & 7) << 4)) + q * 512, c0);
+          st_shared_f1((cdst ^ (((x + 1) & 7) << 4)) + (q + 1) * 512, c1);
         }
       }
+      if (kHold) tmem_st16(tg + q0, om);
     };
-    const uint32_t tg = c.tmem + Cfg::tG + lane_base;
     auto tile = [&](auto on_diag) -> bool {
       uint32_t ga[16], gb[16];
       tmem_ld16(tg, ga);
       tmem_ld16(tg + 16, gb);
-      if (!kCarryOnly && T >= Cfg::kCBufs && !c.wait_w(kCFree + T % Cfg::kCBufs, T / Cfg::kCBufs - 1)) return false;      // (halves: the first one)
+      if (!kCarryOnly && !kHold && T >= Cfg::kCBufs && !c.wait_w(kCFree + T % Cfg::kCBufs, T / Cfg::kCBufs - 1)) return false;
       tc_wait_ld();
       retention(ga, 0);
 #pragma unroll 1
@@ -391,13 +399,9 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
           tmem_ld16(tg + cb * 32 + 48, gb);
           tc_wait_ld();
         }
-        if (cb == 2) {
+        if (!kHold && cb == 2) {
           tc_fence_before();
           c.arrive_w(kGFree);
-        }
-        if (Cfg::kHalves && !kCarryOnly && cb == 1) {
-          c.arrive_w(kCReady);
-          if (T >= 1 && !c.wait_w(kCFree + 1, T - 1)) return false;
         }
         tprev += local;
         local = 0.f;
@@ -407,7 +411,26 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     };
     if (!(diag ? tile(std::true_type{}) : tile(std::false_type{}))) return;
     add_to_carry(tprev);      // (tprev = carry_lo + the tile's total)
-    if (!kCarryOnly) c.arrive_w(kCReady + (Cfg::kHalves ? 1 : T % Cfg::kCBufs));
+    if (kHold) {
+      tc_wait_st();
+#pragma unroll 1
+      for (int hb = 0; hb < 2; ++hb) {
+        uint32_t v[64];
+        tmem_ld32(tg + hb * 64, v);
+        tmem_ld32(tg + hb * 64 + 32, v + 32);
+        if (T >= 1 && !c.wait_w(kCFree + hb, T - 1)) return;
+        tc_wait_ld();
+        if (hb == 1) {
+          tc_fence_before();
+          c.arrive_w(kGFree);
+        }
+#pragma unroll
+        for (int q = 0; q < 64; ++q) st_shared_f1((cdst ^ ((q & 7) << 4)) + (hb * 64 + q) * 512, __uint_as_float(v[q]));
+        c.arrive_w(kCReady + hb);
+      }
+    } else if (!kCarryOnly) {
+      c.arrive_w(kCReady + T % Cfg::kCBufs);
+    }
   }
   if (p.total_out) p.total_out[key_id] = carry;
 }
