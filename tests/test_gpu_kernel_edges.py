@@ -279,3 +279,43 @@ def test_decode_affinity_of_long_keys_and_closed_gates(D, chunk):
     for i, (p, vi, l) in enumerate(chunks):
         assert (lse[..., i].double() - l).abs().max() <= 1e-4
         assert ((out[..., i].double() - p @ vi).abs() <= 2.0 ** -8 * (p @ vi.abs() + (p @ vi).abs()) + 1e-5).all()
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 4, 5, 128, 64), (1, 1, 2, 13, 64, 128), (1, 1, 1, 24, 128, 128), (8, 16, 2, 3, 128, 64)])
+def test_overlapping_launches_under_capture(shape, monkeypatch):
+    """The kernels of a call may overlap (totals and forward, sweep and correction pass, sweep and finish): captured, and replayed back to back
+    on inputs that change in between, they leave what separate calls leave.  Forward bit for bit; the gradients are sums in an order that
+    changes from run to run, so within a rounding of bf16 (2^-8 of a value, and 2^-8 in the 2-norm at the most)."""
+    from universal_attention_triton_b200 import ops
+    monkeypatch.delenv("UA_CHECK_STATUS", raising=False)      # (reading the status word synchronises)
+    B, H, R, n, c, D = shape
+    sets = [[t.cuda() for t in _inputs(*shape, seed=s)] for s in (3, 4, 5)]
+    cu = [t.clone() for t in sets[0]]
+    g_out = torch.randn(B, H, n, R, n * c, D, device="cuda", dtype=torch.bfloat16)
+    g_lse = torch.randn(B, H, n, R, n * c, device="cuda")
+
+    def call():
+        out, lse, denom, carry = ops.forward_cm(*cu, keep_carry=True)
+        return (out, lse, denom, *ops.backward_cm(*cu, g_out, g_lse, carry=carry, lse=lse, out_cm=out))
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = call()
+    got = []
+    for ins in sets:
+        for a, b in zip(cu, ins):
+            a.copy_(b)
+        graph.replay()
+        graph.replay()
+        got.append([t.clone() for t in held])
+    for ins, res in zip(sets, got):
+        for a, b in zip(cu, ins):
+            a.copy_(b)
+        want = call()
+        assert all(torch.equal(a, b) for a, b in zip(res[:3], want[:3]))
+        for a, b, key in zip(res[3:], want[3:], GRADS):
+            assert rel_fro(a.float().cpu(), b.float().cpu()) <= 2.0 ** -8, key

@@ -45,7 +45,12 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
     per = 0;
     for (int i = 0; i < s.N; ++i) per += ((s.L - i * kC) / 64 + p.seg - 1) / p.seg;
   }
-  kern<<<(unsigned)BH * per, threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
+  // (the correction pass of cut sweeps overlaps the end of the pass with heads, launched just before)
+  if (p.heads == 0 && p.seg) {
+    if (int e = launch_dependent(kern, (unsigned)BH * per, threads, Cfg::kSmemBytes, st, tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p)) return e;
+  } else {
+    kern<<<(unsigned)BH * per, threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
+  }
   if (p.acc_dt && mode != 4) {
     // row ranges: the row-side dK joins the accumulator; d static_dest of the range's rows comes out of it
     const int row_begin = p.j_begin * 128, row_end = p.j_end * 128;
@@ -63,11 +68,10 @@ int launch_finish_t(const Shape& s, const void* kc, const Bwd2Params& p, void* d
   const int rows = s.B * s.H * s.L, row_blocks = (rows + 8 * 128 / D - 1) / (8 * 128 / D);
   const size_t dq_vec = (size_t)rows * s.R * D / 8;
   using bf16 = __nv_bfloat16;
-  bwd_finish_kernel<D, TG><<<(unsigned)(row_blocks + (dq_vec + 255) / 256), 256, 0, st>>>(
-      static_cast<const bf16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dq, p.acc_dv, p.acc_ds, p.dt_cols,
-      static_cast<bf16*>(dkc),
-      static_cast<bf16*>(dxq), static_cast<bf16*>(dvc), static_cast<TG*>(dss), static_cast<TG*>(ddest), rows, row_blocks, dq_vec);
-  return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+  return launch_dependent(bwd_finish_kernel<D, TG>, (unsigned)(row_blocks + (dq_vec + 255) / 256), 256, 0, st,
+                          static_cast<const bf16*>(kc), static_cast<const TG*>(p.sdest), p.acc_dkr, p.acc_dk, p.acc_dq, p.acc_dv, p.acc_ds, p.dt_cols,
+                          static_cast<bf16*>(dkc), static_cast<bf16*>(dxq), static_cast<bf16*>(dvc), static_cast<TG*>(dss), static_cast<TG*>(ddest),
+                          rows, row_blocks, dq_vec);
 }
 
 }  // namespace

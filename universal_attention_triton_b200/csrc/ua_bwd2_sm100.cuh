@@ -603,6 +603,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   if (!c.wait_w(qTabFull, 0)) return;
   if (helper && quad == kGateQuad) sT3[col0 + lane] = t3_from_table(0);
   float suffix = p.suffix_in ? p.suffix_in[((size_t)c.bh * N + c.i) * 128 + key] : 0.f, ds_acc = 0.f;
+  if (!kHeads) dependency_wait();                // (launched to overlap the pass with heads; its sums commute, its totals are needed here)
   if (!kHeads && p.seg)                          // what the segments of later rows leave
 #pragma unroll 4
     for (int q = 0; q < c.segment; ++q) suffix += p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + q) * 128 + key];
@@ -945,6 +946,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);      // [0] TMEM base, [1] abort flag, [2] failure note
   const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  dependents_may_start();                      // (once every block runs: the next kernel may take the SMs that this one leaves idle)
   const int BH = p.s.B * p.s.H;
 
   Bwd2Ctx c;
@@ -962,17 +964,21 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     c.nht = c.htop - (kC == 128 ? 2 * (c.i > p.j_begin ? c.i : p.j_begin) : c.i);
   } else {
     int nht;
+    const int log_seg = 31 - __clz(p.seg);     // (a power of two: divisions here delayed every block of a late chunk by up to a microsecond)
 #pragma unroll 1
     for (c.i = 0;; ++c.i) {
       nht = (p.s.L - c.i * kC) / 64;
-      const int ns = (nht + p.seg - 1) / p.seg;
+      const int ns = (nht + p.seg - 1) >> log_seg;
       if (x < ns) break;
       x -= ns;
     }
     c.segment = x;
     c.htop = p.s.L / 64 - x * p.seg;
     c.nht = nht - x * p.seg < p.seg ? nht - x * p.seg : p.seg;
-    if (!kHeads && x == 0) return;             // no rows after the last segment
+    if (!kHeads && x == 0) {                   // no rows after the last segment
+      dependency_wait();                       // (no block ends before the kernel that this one overlaps)
+      return;
+    }
   }
   if (c.nht <= 0) {
     // no row of the range sees this chunk (sequence sharding only): nothing to add anywhere
@@ -1103,6 +1109,7 @@ bwd_finish_kernel(const __nv_bfloat16* __restrict__ kc, const TG* __restrict__ s
                   const float* __restrict__ acc_dk, const float* __restrict__ acc_dq, const float* __restrict__ acc_dv,
                   const float* __restrict__ acc_ds, const float* __restrict__ dt_cols, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dq,
                   __nv_bfloat16* __restrict__ dv, TG* __restrict__ ds, TG* __restrict__ dt, int rows, int row_blocks, size_t dq_vec) {
+  dependency_wait();
   auto pack2 = [](float a, float b) -> uint32_t {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);

@@ -39,6 +39,7 @@ int launch_t(const Shape& s, const void* kc, const void* vc, const void* xq, Fwd
   }
   auto kern = fwd_kernel<D, kC, TG, kCarryOnly, kOut>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
+  if (p.seg) return launch_dependent(kern, blocks, 512, Cfg::kSmemBytes, st, tmK, tmV, tmQ, tmO, p);
   kern<<<blocks, 512, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmO, p);
   return cudaGetLastError() == cudaSuccess ? UA_OK : UA_ERR_CUDA;
 }

@@ -304,9 +304,21 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     carry_lo = (carry - (sum - bb)) + (tile - bb);
     carry = sum;
   };
-  if (live)
+  // A segment starts from the totals of the tiles before it.  The kernel that forms them may still be running (see launch_dependent): what does not
+  // need them is done first.  Four loads at a time: each is some 700 cycles away.
+  auto start_of_segment = [&]() {
+    dependency_wait();
+    const float* tot = p.tile_totals + (size_t)chunk_id * p.tiles * 128 + k;
 #pragma unroll 1
-    for (int T = 0; T < c.t0; ++T) add_to_carry(carry_lo + p.tile_totals[(chunk_id * p.tiles + T) * 128 + k]);
+    for (int T = 0; T < c.t0; T += 4) {
+      float v[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) v[x] = T + x < c.t0 ? tot[(T + x) * 128] : 0.f;
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (T + x < c.t0) add_to_carry(carry_lo + v[x]);
+    }
+  };
   // static_dest^(1/3) of a tile's rows is formed a tile ahead (its gate value fetched another one before), so that the barrier behind which all
   // four warps may read it is long complete when it is looked at.  Three buffers: a warp may still read tile T - 1's while another writes T + 1's.
   sT3[k] = cbrtf(gate_at(0));
@@ -325,6 +337,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     if (!live) continue;
     if (!c.wait_w(kGFull, T)) return;
     tc_fence_after();
+    if (T == 0 && c.t0 > 0) start_of_segment();
     const bool diag = (c.row0 + T * 128 == c.i * kC);
     float* carry_row = p.carry ? p.carry + (chunk_id * (L / 64) + (c.row0 + T * 128) / 64) * 128 + k : nullptr;
     if (carry_row) carry_row[0] = carry;
@@ -433,6 +446,7 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     }
   }
   if (p.total_out) p.total_out[key_id] = carry;
+  dependency_wait();                           // (no block ends before the kernel that this one overlaps)
 }
 
 // ------------------------------------------------------------ softmax groups --
@@ -708,6 +722,7 @@ tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles
   float* t3 = reinterpret_cast<float*>(smem + 2 * kTile);
   float* part = t3 + 128;                                // [3][128]
   uint32_t* misc = reinterpret_cast<uint32_t*>(part + 384);      // [0] tmem base, [1] abort flag, [2..5] two barriers
+  dependents_may_start();                                // (the forward needs the totals in its decay warps only)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, BH = shp.B * shp.H, L = shp.L;
   const int bh = blockIdx.x % BH;
   int x = blockIdx.x / BH, i = 0;
@@ -814,9 +829,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUte
     fill_hi = p.r0 + (kC == 128 ? ((fill_chunk < p.j_end ? fill_chunk : p.j_end) - p.j_begin) * 128 : fill_chunk * kC);
   } else {
     int nt;
+    const int log_seg = 31 - __clz(p.seg);     // (a power of two)
     for (c.i = 0;; ++c.i) {
       nt = (p.s.L - c.i * kC + 127) / 128;
-      const int ns = (nt + p.seg - 1) / p.seg;
+      const int ns = (nt + p.seg - 1) >> log_seg;
       if (x < ns) break;
       x -= ns;
     }

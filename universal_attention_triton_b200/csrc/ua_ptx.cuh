@@ -110,6 +110,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return true;
 }
 
+// ------------------------------------------------- launches that overlap ----
+// A kernel launched as dependent (see launch_dependent) may start once every block of the kernel before it has said so or has ended;
+// what that kernel writes is there behind dependency_wait.  Both do nothing in a kernel launched otherwise.
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // --------------------------------------------------------------------- TMA ----
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(

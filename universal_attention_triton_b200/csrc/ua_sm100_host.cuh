@@ -57,6 +57,22 @@ inline bool make_f32_rows_map(CUtensorMap* map, const void* base, uint64_t rows,
   return r == CUDA_SUCCESS;
 }
 
+// Launches a kernel that may start while the one before it in the stream still runs; it waits for that one's results itself (dependency_wait).
+template <typename... P, typename... A>
+int launch_dependent(void (*kern)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? UA_OK : UA_ERR_CUDA;
+}
+
 inline bool fwd_supported(const Shape& s, int dtype) {
   return dtype == UA_BF16 && (s.C == 128 || s.C == 64) && (s.D == 64 || s.D == 128);
 }
