@@ -215,9 +215,9 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
   if (!load_tables(0)) return;
   // in sweep order: K_j of half tile ht, then the (Q, dO) pairs of its heads (with the log-sum-exp and g_denom rows of
   // the head); a slot is refilled as soon as the MMAs that read it have completed
-  int hc = 0;
+  unsigned hc = 0;
 #pragma unroll 1
-  for (int ht = 0; ht < c.nht; ++ht) {
+  for (unsigned ht = 0; ht < (unsigned)c.nht; ++ht) {
     const int row0 = c.row0_of(ht), srow0 = c.srow0_of(ht);
     {
       const int sl = ht % Cfg::kKj, use = ht / Cfg::kKj;
@@ -278,23 +278,23 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
   const uint32_t kKi = desc_lo(sb + Cfg::oKi, 16), kVi = desc_lo(sb + Cfg::oVi, 16);
 
   // (S, dP) buffer b is free again once the workers have loaded its previous unit.
-  int u = 0;
-  auto acquire = [&](int b) -> bool {
-    const int uses = u / Cfg::kNB;                                // units before u that used buffer b = u % kNB
+  unsigned u = 0;
+  auto acquire = [&](unsigned b) -> bool {
+    const unsigned uses = u / Cfg::kNB;                                // units before u that used buffer b = u % kNB
     if (uses == 0) return true;
     return c.wait(qLdDone + b, uses - 1);
   };
   // (a head's or a half tile's gradient goes to ring buffer w % kRing, its last user's products are done)
-  int w = 0;
+  unsigned w = 0;
   auto ring_free = [&]() -> bool {
-    const int at = w++;
+    const unsigned at = w++;
     return kMode == 4 || at < Cfg::kRing || c.wait(qDsFree + at % Cfg::kRing, at / Cfg::kRing - 1);
   };
   auto unit_g = [&](int ht) -> bool {
-    const int b = u % Cfg::kNB;
+    const unsigned b = u % Cfg::kNB;
     if (!acquire(b)) return false;
     tc_fence_after();
-    mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(sb + Cfg::oKj + (ht % Cfg::kKj) * Cfg::kHalf, 16));
+    mma_kk(c.tmem + (Cfg::tS0 + 128 * b), kKi, desc_lo(sb + Cfg::oKj + (ht % Cfg::kKj) * Cfg::kHalf, 16));
     tc_commit(c.bar(qSFull + b));
     mbar_arrive(c.bar(qSFull + b));
     ++u;
@@ -302,9 +302,9 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
   };
 
   if (!c.wait(qKvFull, 0)) return;
-  int hc = 0;
+  unsigned hc = 0;
 #pragma unroll 1
-  for (int ht = 0; ht < c.nht; ++ht) {
+  for (unsigned ht = 0; ht < (unsigned)c.nht; ++ht) {
     if (!c.wait(qKjFull + ht % Cfg::kKj, ht / Cfg::kKj)) return;
     // (the workers read the tables of the next half tile before this one is over)
     if (kMode != 4 && R > 0 && ht + 1 < c.nht && !c.wait(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
@@ -312,15 +312,15 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
     if (kMode == 4) tc_commit(c.bar(qKjFree + ht % Cfg::kKj));      // (no back issuers: the tiles are free once these products are done)
 #pragma unroll 1
     for (int r = 0; r < R; ++r, ++hc) {
-      const int sl = hc % Cfg::kNS, b = u % Cfg::kNB;
+      const unsigned sl = hc % Cfg::kNS, b = u % Cfg::kNB;
       if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
       if (kOutDelta && !c.wait(qDelta + sl, hc / Cfg::kNS)) return;
       if (!acquire(b)) return;
       if (!ring_free()) return;
       tc_fence_after();
       const uint32_t slot = sb + Cfg::oSlot + sl * Cfg::kSlot;
-      mma_kk(c.tmem + (b ? Cfg::tS1 : Cfg::tS0), kKi, desc_lo(slot, 16));                    // S^T  = K_i Q^T
-      mma_kk(c.tmem + (b ? Cfg::tP1 : Cfg::tP0), kVi, desc_lo(slot + Cfg::kHalf, 16));       // dP^T = V_i dO^T
+      mma_kk(c.tmem + (Cfg::tS0 + 128 * b), kKi, desc_lo(slot, 16));                    // S^T  = K_i Q^T
+      mma_kk(c.tmem + (Cfg::tP0 + 128 * b), kVi, desc_lo(slot + Cfg::kHalf, 16));       // dP^T = V_i dO^T
       tc_commit(c.bar(qSFull + b));
       mbar_arrive(c.bar(qSFull + b));
       ++u;
@@ -343,7 +343,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   const uint32_t DV = c.tmem + Cfg::tDV, DK = c.tmem + Cfg::tDK, Y = c.tmem + Cfg::tY;
   const uint64_t mKi = desc_from_lo(desc_lo(sb + Cfg::oKi, 16384));      // K_i as [K = keys][N = D] (MN-major, 64-wide groups 16 KB apart)
   uint32_t have_dv = 0, have_dk = 0;
-  int yc = 0, hc = 0, w = 0;
+  unsigned yc = 0, hc = 0, w = 0;
   // Y[rows][D] = T^T K_i with T a [128 keys][64 rows] bf16 tile read MN-major; M = 128: lanes 64..127 come from the 16 KB
   // after the tile and are never read
   auto mma_rows_out = [&](uint64_t t_mn, int cb) {       // 64 columns of D: those of K_i's column group cb
@@ -356,7 +356,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
   for (int ht = 0; ht < c.nht; ++ht) {
 #pragma unroll 1
     for (int r = 0; r < R; ++r, ++hc, ++w) {
-      const int sl = hc % Cfg::kNS, db = w % Cfg::kRing;
+      const unsigned sl = hc % Cfg::kNS, db = w % Cfg::kRing;
       const uint32_t dsb = sb + Cfg::oDs + db * 16384;
       if (!c.wait(qDsReady + db, w / Cfg::kRing)) return;
       if (which == 0) {
@@ -387,7 +387,7 @@ __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p,
         tc_commit(c.bar(qDsFree + db));
       }
     }
-    const int gb = w % Cfg::kRing;
+    const unsigned gb = w % Cfg::kRing;
     if (!c.wait(qDsReady + gb, w / Cfg::kRing)) return;
     const uint64_t kdG = desc_from_lo(desc_lo(sb + Cfg::oDs + gb * 16384, 16)), mdG = desc_from_lo(desc_lo(sb + Cfg::oDs + gb * 16384, 16384));
     ++w;
@@ -522,7 +522,7 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
   const int total = c.nht * p.heads;
 #pragma unroll 1
   for (int hc = 0; hc < total; ++hc) {
-    const int sl = hc % Cfg::kNS;
+    const unsigned sl = (unsigned)hc % Cfg::kNS;
     const uint32_t go = sb + Cfg::oSlot + sl * Cfg::kSlot + Cfg::kHalf + row0 * 128, oo = sb + Cfg::oOut + sl * Cfg::kHalf + row0 * 128;
     if (!c.wait_w(qInFull + sl, hc / Cfg::kNS)) return;
     float* tabC = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512) + 64;
@@ -619,7 +619,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     for (int q = 0; q < c.segment; ++q) suffix += p.seg_totals[(((size_t)c.bh * N + c.i) * p.max_seg + q) * 128 + key];
   named_bar_sync(kBarAll, kWorkers);
 
-  int u = 0, hc = 0;                             // units and heads so far
+  unsigned u = 0, hc = 0;                        // units and heads so far
 #pragma unroll 1
   for (int ht = 0; ht < c.nht; ++ht) {
     const int rel = c.row0_of(ht) - c.i * kC;
@@ -631,11 +631,11 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     float2 c2[H2];
     if (kHeads) {                                  // (the correction pass has no heads: no prefix, no first G unit)
       const float carry = reinterpret_cast<const float*>(ht_table(ht))[key];
-      const int b = u % Cfg::kNB;
+      const unsigned b = u % Cfg::kNB;
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
       tc_fence_after();
       uint32_t gr[CG];
-      tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
+      tmem_ld16(c.tmem + (Cfg::tS0 + 128 * b) + lane_base + col0, gr);
       float2 t3p[H2];
       load_pairs(t3v, t3p);
       tc_wait_ld();
@@ -692,7 +692,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
     for (int x = 0; x < H2; ++x) dc[x] = make_float2(0.f, 0.f);
 #pragma unroll 1
     for (int r = 0; r < R; ++r, hc += (kMode == 4 ? 0 : 1)) {
-      const int b = u % Cfg::kNB, sl = hc % Cfg::kNS;
+      const unsigned b = u % Cfg::kNB, sl = hc % Cfg::kNS;
       float* tabL = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512);      // lse[64] of the head's rows (raw)
       float* tabC = tabL + 64;                                                         // g_denom[64] (or delta[64])
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
@@ -700,8 +700,8 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       float2 pv[H2], dp[H2];
       {
         uint32_t sr[CG], dr[CG];
-        tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, sr);
-        tmem_ld16(c.tmem + (b ? Cfg::tP1 : Cfg::tP0) + lane_base + col0, dr);
+        tmem_ld16(c.tmem + (Cfg::tS0 + 128 * b) + lane_base + col0, sr);
+        tmem_ld16(c.tmem + (Cfg::tP0 + 128 * b) + lane_base + col0, dr);
         float2 nl[H2];
         load_pairs(tabL + col0, nl);                                 // lse of the rows
         tc_wait_ld();
@@ -789,11 +789,11 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
         if (!kHeads && !c.wait_w(qTabFull + (ht + 1) % Cfg::kTab, (ht + 1) / Cfg::kTab)) return;
         if (helper) sT3[((ht + 1) & 1) * 64 + col0 + lane] = t3_from_table(ht + 1);
       }
-      const int b = u % Cfg::kNB;
+      const unsigned b = u % Cfg::kNB;
       if (!c.wait_w(qSFull + b, u / Cfg::kNB)) return;
       tc_fence_after();
       uint32_t gr[CG];
-      tmem_ld16(c.tmem + (b ? Cfg::tS1 : Cfg::tS0) + lane_base + col0, gr);
+      tmem_ld16(c.tmem + (Cfg::tS0 + 128 * b) + lane_base + col0, gr);
       float2 t3p[H2];
       load_pairs(t3v, t3p);
       tc_wait_ld();
