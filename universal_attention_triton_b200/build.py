@@ -78,7 +78,7 @@ def _build_torch_module() -> None:
     for inc in include_paths() + [cuda_inc, sysconfig.get_paths()["include"]]:
         cmd += ["-isystem", inc]
     cmd += [os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_PATH, "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-L" + torch_lib,
-            "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+            "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
     _run(cmd)
 
 

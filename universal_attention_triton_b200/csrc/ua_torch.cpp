@@ -2,6 +2,7 @@
 // libua_b200.so.  ops.py documents each function under its own name; this file holds what used to be Python there, because
 // at the small sizes the host path was the whole cost (a training step of B1 H8 R4 L1024 spent 790 us of which 318 on the GPU).
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -56,6 +57,21 @@ int code_of(at::ScalarType t) {
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
+// Uninitialised tensors on the device (and, unless another is given, of the type) of one at hand, straight from the allocator: a training step makes
+// some thirty of them, and the dispatcher would take as long again for each (0.7 of 1.3 us).
+class Fresh {
+ public:
+  explicit Fresh(const Tensor& like) : device_(like.device()), type_(like.scalar_type()) {}
+  Tensor operator()(at::IntArrayRef sizes) const { return (*this)(sizes, type_); }
+  Tensor operator()(at::IntArrayRef sizes, at::ScalarType t) const { return Tensor(at::detail::empty_cuda(sizes, t, device_, std::nullopt)); }
+  Tensor operator()(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType t) const {
+    return Tensor(at::detail::empty_strided_cuda(sizes, strides, t, device_));
+  }
+ private:
+  at::Device device_;
+  at::ScalarType type_;
+};
+
 // With UA_CHECK_STATUS=1 every call synchronises and reads the kernels' status word (a bounded device-side wait that ran
 // out): for tests and debugging.
 void check_status(const Tensor& ws, void* stream, const char* what) {
@@ -104,15 +120,15 @@ std::tuple<Tensor, Tensor, Tensor, OptTensor> forward_with(const Tensor& kc_, co
   const Problem p = problem(kc, xq);
   const c10::cuda::CUDAGuard guard(kc.device());
   const Inputs in = inputs(p, kc, plain(vc_), xq, plain(ss_), plain(sd_));
-  const auto opt = kc.options().requires_grad(false);
-  Tensor out = at::empty({p.b, p.h, p.n, p.r, p.L, p.d}, opt.dtype(p.dt));
-  Tensor lse = at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(at::kFloat));
-  Tensor denom = p.code == UA_F32 || !want_denom ? lse : at::empty({p.b, p.h, p.n, p.r, p.L}, opt.dtype(p.dt));
+  const Fresh fresh(kc);
+  Tensor out = fresh({p.b, p.h, p.n, p.r, p.L, p.d}, p.dt);
+  Tensor lse = fresh({p.b, p.h, p.n, p.r, p.L}, at::kFloat);
+  Tensor denom = p.code == UA_F32 || !want_denom ? lse : fresh({p.b, p.h, p.n, p.r, p.L}, p.dt);
   const size_t ws_bytes = std::max<size_t>(ua_fwd_workspace_bytes(&p.dims, p.code, flags), 256);
-  Tensor ws = at::empty({(int64_t)ws_bytes}, opt.dtype(at::kByte));
+  Tensor ws = fresh({(int64_t)ws_bytes}, at::kByte);
   OptTensor carry;
   if (keep_carry) {
-    if (const size_t bytes = ua_carry_bytes(&p.dims, p.code, flags)) carry = at::empty({(int64_t)(bytes / 4)}, opt.dtype(at::kFloat));
+    if (const size_t bytes = ua_carry_bytes(&p.dims, p.code, flags)) carry = fresh({(int64_t)(bytes / 4)}, at::kFloat);
   }
   void* st = stream_of(kc);
   check(ua_fwd_keep(&p.dims, p.code, code_of(in.g.src.scalar_type()), ptr(in.kc), ptr(in.vc), ptr(in.q), ptr(in.g.src), ptr(in.g.dest),
@@ -157,11 +173,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> backward_cm(const Tensor& kc_
     if (!(out.is_cuda() && out.scalar_type() == p.dt && out.is_contiguous() && out.sizes() == at::IntArrayRef({p.b, p.h, p.n, p.r, p.L, p.d})))
       out = Tensor();
   }
-  const auto opt = kc.options().requires_grad(false);
-  Tensor dk = at::empty(kc.sizes(), opt), dv = at::empty(kc.sizes(), opt), dq = at::empty(xq.sizes(), opt.dtype(p.dt));
-  Tensor dss = at::empty(ss.sizes(), opt.dtype(in.g.src.scalar_type())), dsd = at::empty(sd.sizes(), opt.dtype(in.g.src.scalar_type()));
+  const Fresh fresh(kc);
+  Tensor dk = fresh(kc.sizes()), dv = fresh(kc.sizes()), dq = fresh(xq.sizes(), p.dt);
+  Tensor dss = fresh(ss.sizes(), in.g.src.scalar_type()), dsd = fresh(sd.sizes(), in.g.src.scalar_type());
   const size_t ws_bytes = std::max<size_t>(ua_bwd_workspace_bytes(&p.dims, p.code, flags), 256);
-  Tensor ws = at::empty({(int64_t)ws_bytes}, opt.dtype(at::kByte));
+  Tensor ws = fresh({(int64_t)ws_bytes}, at::kByte);
   void* st = stream_of(kc);
   check(ua_bwd_saved(&p.dims, p.code, code_of(in.g.src.scalar_type()), ptr(in.kc), ptr(in.vc), ptr(in.q), ptr(in.g.src), ptr(in.g.dest),
                      ptr(g_out), ptr(g_denom), code_of(g_denom.scalar_type()), ptr(carry), static_cast<float*>(ptr(lse)), ptr(out), ptr(dk),
@@ -189,10 +205,10 @@ std::tuple<Tensor, OptTensor> merge_fwd_cm(const Tensor& out_, const Tensor& lse
   const UaDims dims = merge_dims(out);
   const c10::cuda::CUDAGuard guard(out.device());
   TORCH_CHECK(lse.numel() * out.size(5) == out.numel(), "log-sum-exp does not fit the outputs");
-  const auto opt = out.options().requires_grad(false);
-  Tensor merged = at::empty({out.size(0), out.size(1), out.size(3), out.size(4), out.size(5)}, opt);
+  const Fresh fresh(out);
+  Tensor merged = fresh({out.size(0), out.size(1), out.size(3), out.size(4), out.size(5)});
   OptTensor row_lse;
-  if (stats) row_lse = at::empty({out.size(0), out.size(1), out.size(3), out.size(4)}, opt.dtype(at::kFloat));
+  if (stats) row_lse = fresh({out.size(0), out.size(1), out.size(3), out.size(4)}, at::kFloat);
   check(ua_merge_fwd_typed(&dims, code_of(out.scalar_type()), code_of(lse.scalar_type()), ptr(out), ptr(lse), ptr(merged),
                            row_lse ? static_cast<float*>(ptr(*row_lse)) : nullptr, stream_of(out)), stats ? "ua_merge_fwd_stats" : "ua_merge_fwd");
   return {merged, row_lse};
@@ -204,8 +220,8 @@ std::tuple<Tensor, Tensor> merge_bwd_cm(const Tensor& out_, const Tensor& lse_, 
   const UaDims dims = merge_dims(out);
   const c10::cuda::CUDAGuard guard(out.device());
   TORCH_CHECK(lse.numel() * out.size(5) == out.numel() && g.numel() * out.size(2) == out.numel(), "gradient or log-sum-exp does not fit the outputs");
-  const auto opt = out.options().requires_grad(false);
-  Tensor g_out = at::empty(out.sizes(), opt), g_lse = at::empty(lse.sizes(), opt.dtype(lse.scalar_type()));
+  const Fresh fresh(out);
+  Tensor g_out = fresh(out.sizes()), g_lse = fresh(lse.sizes(), lse.scalar_type());
   check(ua_merge_bwd_typed(&dims, code_of(out.scalar_type()), code_of(lse.scalar_type()), ptr(out), ptr(lse), ptr(g), ptr(g_out), ptr(g_lse),
                      skip_zero_weight_blocks ? UA_FLAG_SKIP_MASKED_FILL : 0, stream_of(out)), "ua_merge_bwd");
   return {g_out, g_lse};
@@ -259,11 +275,12 @@ std::tuple<Tensor, Tensor> decode_step(int64_t t, const Tensor& k, const Tensor&
   const Tensor q = q_.contiguous();
   const int64_t nt = t / chunk + 1;
   const UaDims dims{(int)b, (int)h, (int)r, (int)(cap / chunk), (int)chunk, (int)d};
-  const auto opt = k.options().requires_grad(false);
-  Tensor out = at::empty({b, h, nt, r, d}, opt.dtype(dt)), lse = at::empty({b, h, nt, r}, opt.dtype(at::kFloat));
+  const Fresh fresh(k);
+  // stored (b, h, nt, r, d) and (b, h, nt, r), with the chunk last in the shape
+  Tensor out = fresh({b, h, r, d, nt}, {h * nt * r * d, nt * r * d, d, 1, r * d}, dt), lse = fresh({b, h, r, nt}, {h * nt * r, nt * r, 1, r}, at::kFloat);
   check(ua_decode_step(&dims, code, code_of(g.src.scalar_type()), (int)t, ptr(k), ptr(v), ptr(g.src), ptr(q), ptr(g.dest),
                        static_cast<float*>(ptr(state)), ptr(out), static_cast<float*>(ptr(lse)), stream_of(k)), "ua_decode_step");
-  return {out.permute({0, 1, 3, 4, 2}), lse.permute({0, 1, 3, 2})};
+  return {out, lse};
 }
 
 // ---- input prologue ----------------------------------------------------------------------------------------------------
@@ -277,11 +294,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor> prepare_inputs(con
   const int64_t b = qs.size(0), s = qs.size(1), n = qs.size(2), d = qs.size(3), kv = ks.size(2);
   auto must = [](bool ok) { if (!ok) raise(PyExc_AssertionError, "shapes of the projections do not fit together"); };
   must(ks.sizes() == at::IntArrayRef({b, s, kv, d}) && vs.sizes() == ks.sizes() && gs.numel() == b * s * 2 * kv && n % kv == 0 && s % chunk == 0);
-  const auto opt = qs.options().requires_grad(false);
-  Tensor xq = at::empty({b, kv, n / kv, s, d}, opt), kc = at::empty({b, kv, s / chunk, chunk, d}, opt), vc = at::empty({b, kv, s / chunk, chunk, d}, opt);
-  Tensor src = at::empty({b, kv, s / chunk, chunk}, opt), dest = at::empty({b, kv, s}, opt);
+  const Fresh fresh(qs);
+  Tensor xq = fresh({b, kv, n / kv, s, d}), kc = fresh({b, kv, s / chunk, chunk, d}), vc = fresh({b, kv, s / chunk, chunk, d});
+  Tensor src = fresh({b, kv, s / chunk, chunk}), dest = fresh({b, kv, s});
   OptTensor norm;
-  if (flags & UA_PREP_NORMALIZE_KEYS) norm = at::empty({b, kv, s}, opt.dtype(at::kFloat));
+  if (flags & UA_PREP_NORMALIZE_KEYS) norm = fresh({b, kv, s}, at::kFloat);
   check(ua_prepare_inputs((int)b, (int)s, (int)n, (int)kv, (int)d, code_of(dt), flags, ptr(qs), ptr(ks), ptr(vs), ptr(gs), ptr(xq), ptr(kc), ptr(vc),
                           ptr(src), ptr(dest), norm ? static_cast<float*>(ptr(*norm)) : nullptr, stream_of(qs)), "ua_prepare_inputs");
   return {kc, vc, xq, src, dest, norm};
@@ -294,14 +311,14 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> prepare_inputs_bwd(const OptTensor& g
   const int64_t b = kc.size(0), kv = kc.size(1), s = kc.size(2) * kc.size(3), d = kc.size(4);
   const at::ScalarType dt = kc.scalar_type();
   const c10::cuda::CUDAGuard guard(kc.device());
-  const auto opt = kc.options().requires_grad(false);
-  auto full = [&](const OptTensor& g, at::IntArrayRef shape) { return g ? plain(*g).to(dt).contiguous() : at::zeros(shape, opt); };
+  const Fresh fresh(kc);
+  auto full = [&](const OptTensor& g, at::IntArrayRef shape) { return g ? plain(*g).to(dt).contiguous() : at::zeros(shape, kc.options().requires_grad(false)); };
   const Tensor gk = full(g_kc, kc.sizes()), gv = full(g_vc, kc.sizes()), gq = full(g_xq, {b, kv, n / kv, s, d});
   const Tensor gs = full(g_src, src.sizes()), gd = full(g_dest, dest.sizes());
   require_cuda(gk, gv, gq, gs, gd);
   TORCH_CHECK(gk.numel() == kc.numel() && gv.numel() == kc.numel() && gq.numel() == b * n * s * d && gs.numel() == src.numel() && gd.numel() == dest.numel(),
               "upstream gradients do not have the outputs' shape");
-  Tensor dq = at::empty({b, s, n, d}, opt), dk = at::empty({b, s, kv, d}, opt), dv = at::empty({b, s, kv, d}, opt), dg = at::empty({b, s, 2, kv}, opt);
+  Tensor dq = fresh({b, s, n, d}), dk = fresh({b, s, kv, d}), dv = fresh({b, s, kv, d}), dg = fresh({b, s, 2, kv});
   check(ua_prepare_inputs_bwd((int)b, (int)s, (int)n, (int)kv, (int)d, code_of(dt), flags, ptr(gq), ptr(gk), ptr(gv), ptr(gs), ptr(gd), ptr(kc),
                               norm ? static_cast<float*>(ptr(plain(*norm))) : nullptr, ptr(src), ptr(dest), ptr(dq), ptr(dk), ptr(dv), ptr(dg), stream_of(kc)),
         "ua_prepare_inputs_bwd");
@@ -548,20 +565,20 @@ struct AttentionNode : torch::autograd::Node {
       const Tensor xq = c.xq.unpack();
       const int64_t b = xq.size(0), s = xq.size(3), D = xq.size(4), rep = heads / kv;
       const c10::cuda::CUDAGuard guard(xq.device());
-      const auto opt = xq.options().requires_grad(false);
+      const Fresh fresh(xq);
       Tensor g = g_[0].to(xq.scalar_type()).contiguous();
       if (rep > 1 || D != d) {
-        Tensor packed = at::empty({b, kv, rep, s, D}, opt);
+        Tensor packed = fresh({b, kv, rep, s, D});
         copy_heads({{g, packed, heads, rep}});
         g = packed;
       }
       auto [dk, dv, dq, ds, dt] = c.backward(g);
       if (rep > 1 || D != d) {
-        Tensor q = at::empty({b, heads, s, d}, opt);
+        Tensor q = fresh({b, heads, s, d});
         HeadMap mk{}, mv{};
         if (D != d) {
-          mk = HeadMap{dk.view({b, kv, s, D}), at::empty({b, kv, s, d}, opt), kv, kv};
-          mv = HeadMap{dv.view({b, kv, s, D}), at::empty({b, kv, s, d}, opt), kv, kv};
+          mk = HeadMap{dk.view({b, kv, s, D}), fresh({b, kv, s, d}), kv, kv};
+          mv = HeadMap{dv.view({b, kv, s, D}), fresh({b, kv, s, d}), kv, kv};
         }
         copy_heads({{dq, q, heads, kv}, mk, mv});
         dq = q;
@@ -582,14 +599,14 @@ Tensor attention_apply(const Tensor& q, const Tensor& k, const Tensor& v, const 
   {
     const at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard guard(q.device());
-    const auto opt = q.options().requires_grad(false);
+    const Fresh fresh(q);
     Tensor qs = q.contiguous(), ks = k.contiguous(), vs = v.contiguous();
     if (rep > 1 || D != d) {
-      Tensor packed = at::empty({b, kv, rep, s, D}, opt);
+      Tensor packed = fresh({b, kv, rep, s, D});
       HeadMap mk{}, mv{};
       if (D != d) {
-        mk = HeadMap{ks, at::empty({b, kv, s, D}, opt), kv, kv};
-        mv = HeadMap{vs, at::empty({b, kv, s, D}, opt), kv, kv};
+        mk = HeadMap{ks, fresh({b, kv, s, D}), kv, kv};
+        mv = HeadMap{vs, fresh({b, kv, s, D}), kv, kv};
       }
       copy_heads({{qs, packed, heads, rep}, mk, mv});
       qs = packed;
@@ -604,7 +621,7 @@ Tensor attention_apply(const Tensor& q, const Tensor& k, const Tensor& v, const 
     std::tie(out, lse, denom, carry) = forward_with(kc, vc, xq, ss, sd, 0, grad, false);
     o = std::get<0>(merge_fwd_cm(out, lse, false));
     if (rep > 1 || D != d) {
-      Tensor unpacked = at::empty({b, heads, s, d}, opt);
+      Tensor unpacked = fresh({b, heads, s, d});
       copy_heads({{o, unpacked, heads, kv}});
       o = unpacked;
     } else {
