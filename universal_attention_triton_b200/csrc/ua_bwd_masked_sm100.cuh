@@ -309,22 +309,27 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
   {
     const int c0 = c.clo(c.jlo);
     mbar_expect_tx(c.bar(mMtFull), (uint32_t)(c.chi - c0) * Cfg::kMtBytes);
+#pragma unroll 1
     for (int cc = c0; cc < c.chi; ++cc)
       bulk_load_1d(sb + Cfg::oMt + cc * Cfg::kMtBytes,
                    p.mt + ((size_t)c.bh * N + c.i0 + cc) * (size_t)(D * D * 2) + (size_t)c.h * Cfg::kMtBytes, Cfg::kMtBytes,
                    c.bar(mMtFull));
   }
   int s = 0, uc = 0;
+#pragma unroll 1
   for (int r = 0; r < R; ++r)
+#pragma unroll 1
     for (int j = c.jlo; j < c.jhi; ++j, ++s) {
       const int c0 = c.clo(j);
       const int qs = s & 1;
       if (s >= 2 && !c.wait(mQFree + qs, s / 2 - 1)) return;
       mbar_expect_tx(c.bar(mQFull + qs), 16384u + (uint32_t)(c.chi - c0) * 512u);
       tma_load_2d(sb + Cfg::oQ + qs * 16384, tmQ, 64 * c.h, (c.bh * R + r) * L + c.srow(j), c.bar(mQFull + qs));
+#pragma unroll 1
       for (int cc = c0; cc < c.chi; ++cc)
         bulk_load_1d(sb + Cfg::oGd + (qs * Cfg::kG + cc) * 512,
                      p.g_denom + (c.out_chunk(N, cc) * R + r) * L + (size_t)c.srow(j), 512, c.bar(mQFull + qs));
+#pragma unroll 1
       for (int u = 0; u < Cfg::kUnits; ++u) {
         const MkUnit<D> un(u, c0, c.chi);
         if (!un.active()) continue;
@@ -332,6 +337,7 @@ __device__ __forceinline__ void mk_producer(const MkCtx<kWide>& c, const MaskedP
         if (uc >= Cfg::kSlots && !c.wait(mSlotFree + sl, uc / Cfg::kSlots - 1)) return;
         ++uc;
         mbar_expect_tx(c.bar(mSlotFull + sl), (uint32_t)(un.hi - un.lo) * Cfg::kDoBytes);
+#pragma unroll 1
         for (int cc = un.lo; cc < un.hi; ++cc) {
 #pragma unroll
           for (int b = 0; b < Cfg::kKB; ++b)
@@ -350,7 +356,9 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
   constexpr uint32_t id_y = idesc_bf16(128, 64, 0, 0);       // rows x 64: A K-major, B K-major
   if (!c.wait(mMtFull, 0)) return;
   int s = 0, uc = 0;
+#pragma unroll 1
   for (int r = 0; r < R; ++r)
+#pragma unroll 1
     for (int j = c.jlo; j < c.jhi; ++j, ++s) {
       const int c0 = c.clo(j);
       const int qs = s & 1;
@@ -362,6 +370,7 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
       // [K = rows][M = the 64 columns of Q, then the 64 columns of the ones tile]
       const uint64_t mQO = desc_from_lo(desc_lo(q_addr, (sb + Cfg::oOnes) - q_addr));
       uint32_t have_y = 0;
+#pragma unroll 1
       for (int u = 0; u < Cfg::kUnits; ++u) {
         const MkUnit<D> un(u, c0, c.chi);
         if (!un.active()) continue;
@@ -370,6 +379,7 @@ __device__ __forceinline__ void mk_issuer(const MkCtx<kWide>& c, const MaskedPar
         ++uc;
         tc_fence_after();
         const uint32_t slot = sb + Cfg::oSlot + sl * 32768;
+#pragma unroll 1
         for (int cc = un.lo; cc < un.hi; ++cc) {                     // Y += g Mt_c^T
           const uint32_t g_addr = slot + (cc - u * Cfg::kPer) * Cfg::kDoBytes;
 #pragma unroll
@@ -406,7 +416,9 @@ __device__ __forceinline__ void mk_gate_sums(const MkCtx<kWide>& c, const Masked
 #pragma unroll
   for (int x = 0; x < Cfg::kG * 16; ++x) acc[x] = 0.f;
   int s = 0;
+#pragma unroll 1
   for (int r = 0; r < R; ++r)
+#pragma unroll 1
     for (int j = c.jlo; j < c.jhi; ++j, ++s) {
       const int c0 = c.clo(j);
       const int qs = s & 1;
@@ -461,7 +473,9 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
   uint8_t* stage = c.smem + Cfg::oStage;
   const float* ks = reinterpret_cast<const float*>(c.smem + Cfg::oKs);
   int s = 0;
+#pragma unroll 1
   for (int r = 0; r < R; ++r)
+#pragma unroll 1
     for (int j = c.jlo; j < c.jhi; ++j, ++s) {
       const int c0 = c.clo(j);
       const int qs = s & 1;
@@ -517,6 +531,7 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
   tc_fence_after();
   const int c0 = c.clo(c.jlo);
   if ((warp & 3) < 2) {                    // lanes 0..63: rows d' = 64 h + row of N^T
+#pragma unroll 1
     for (int cc = c0; cc < c.chi; ++cc) {
       float* nacc = p.nacc + ((size_t)c.bh * N + c.i0 + cc) * (size_t)kNaccRows<D>() * D;
 #pragma unroll 1
@@ -532,6 +547,7 @@ __device__ __forceinline__ void mk_drain(const MkCtx<kWide>& c, const MaskedPara
       }
     }
   } else if ((warp & 3) == 2 && c.h == 0) {    // lane 64 (column 0 of the ones tile): u_c = column sums of g
+#pragma unroll 1
     for (int cc = c0; cc < c.chi; ++cc) {
       float* nacc = p.nacc + ((size_t)c.bh * N + c.i0 + cc) * (size_t)kNaccRows<D>() * D + (size_t)(D + 1) * D;
 #pragma unroll 1
@@ -578,11 +594,16 @@ masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bool found = false;
     c.jb = p.j_begin; c.r0 = p.r0; c.m = p.m;
     // row tiles of the range that lie before the last chunk of group gg: [j_begin, min(j_end, last chunk of gg))
-    auto jmax_of = [&](int gg) { return min((min((gg + 1) * Cfg::kG, N) - 1) / p.m * p.m, p.j_end); };
-    for (int piece = 0; p.j_begin + piece * p.jp < min((N - 1) / p.m * p.m, p.j_end); ++piece) {
+    // (no divisions for narrow chunks: they took every block 3 us of its start)
+    auto chunk_start = [&](int x) { return kWide ? x / p.m * p.m : x; };
+    auto jmax_of = [&](int gg) { return min(chunk_start(min((gg + 1) * Cfg::kG, N) - 1), p.j_end); };
+    const int jend = min(chunk_start(N - 1), p.j_end);
+#pragma unroll 1
+    for (int piece = 0; p.j_begin + piece * p.jp < jend; ++piece) {
       const int jlo = p.j_begin + piece * p.jp;
       int cnt = 0;                                                       // groups that have row tiles of this piece before a chunk
-      for (int gg = 0; gg < groups; ++gg) cnt += (jmax_of(gg) > jlo) ? 1 : 0;
+#pragma unroll 1
+      for (int gg = groups - 1; gg >= 0 && jmax_of(gg) > jlo; --gg) ++cnt;      // (jmax_of grows with the group)
       if (idx < BH * cnt) {
         c.bh = idx / cnt;
         g = groups - 1 - idx % cnt;
