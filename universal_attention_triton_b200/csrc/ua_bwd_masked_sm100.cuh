@@ -67,7 +67,7 @@ struct MkCfg {
   static constexpr int oKs = oGd + 2 * kG * 512;           // float [64][kG]: ksum_c / 128 of this block's 64 output columns
   static constexpr int oBar = oKs + 64 * kG * 4;
   static constexpr int oMisc = oBar + 256;
-  static constexpr int kSmemBytes = oMisc + 64 + 1024;     // + slack to align the base to 1024 B
+  static constexpr int kSmemBytes = oMisc + 64;
   static constexpr uint32_t tY0 = 0, tY1 = 64, tN = 128;
   static_assert(tN + kG * D <= 512, "TMEM budget");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
@@ -572,8 +572,8 @@ __global__ void __launch_bounds__(384, 1)
 masked_sweep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                     const __grid_constant__ CUtensorMap tmDQ, MaskedParams p) {
   using Cfg = MkCfg<D>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  // (used as declared: an address rounded up at run time is no shared-memory address to the compiler, and every table access a generic one)
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + Cfg::oMisc);      // [0] TMEM base, [1] abort flag, [2] failure note
   const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int N = p.s.N;
