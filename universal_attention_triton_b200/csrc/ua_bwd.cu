@@ -8,7 +8,6 @@ namespace {
 template <int D, int kC, typename TG>
 int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, const void* xq, const void* g_out, const Bwd2Params& p,
                   cudaStream_t st) {
-  using Cfg = Bwd2Cfg<D>;
   CUtensorMap tmK, tmV, tmQ, tmG, tmDQ, tmDK;
   const uint64_t BH = (uint64_t)s.B * s.H;
   if (!make_rows_map(&tmK, kc, BH * s.L, D, 64) || !make_rows_map(&tmV, vc, BH * s.L, D, 64) ||
@@ -24,6 +23,7 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
   const int threads = 32 * (8 + 4 * NG);
   CUtensorMap tmO = tmG;
   auto kern = bwd2_kernel<D, kC, TG, 1, false>;
+  size_t smem = Bwd2Cfg<D>::kSmemBytes;
   if (p.heads > 0) {
     kern = bwd2_kernel<D, kC, TG, 1, true>;
     if constexpr (kC == 128) {
@@ -32,14 +32,15 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
       if (mode == 4) kern = bwd2_kernel<D, kC, TG, 4, true>;
     }
     // the forward's output tiles at hand (chunks of 128 keys, per-chunk form, head_dim 64): the row term comes from them
-    if constexpr (Cfg::kOutTiles && kC == 128) {
+    if constexpr (D == 64 && kC == 128) {
       if (mode == 1 && p.out_tiles != nullptr) {
         if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
         kern = bwd2_kernel<D, kC, TG, 1, true, true>;
+        smem = Bwd2Cfg<D, true>::kSmemBytes;
       }
     }
   }
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return UA_ERR_CUDA;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return UA_ERR_CUDA;
   unsigned per = (unsigned)s.N;
   if (p.seg) {
     per = 0;
@@ -47,9 +48,9 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
   }
   // (the correction pass of cut sweeps overlaps the end of the pass with heads, launched just before)
   if (p.heads == 0 && p.seg) {
-    if (int e = launch_dependent(kern, (unsigned)BH * per, threads, Cfg::kSmemBytes, st, tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p)) return e;
+    if (int e = launch_dependent(kern, (unsigned)BH * per, threads, smem, st, tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p)) return e;
   } else {
-    kern<<<(unsigned)BH * per, threads, Cfg::kSmemBytes, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
+    kern<<<(unsigned)BH * per, threads, smem, st>>>(tmK, tmV, tmQ, tmG, tmDQ, tmDK, tmO, p);
   }
   if (p.acc_dt && mode != 4) {
     // row ranges: the row-side dK joins the accumulator; d static_dest of the range's rows comes out of it

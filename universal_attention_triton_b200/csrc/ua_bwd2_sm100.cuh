@@ -96,14 +96,20 @@ struct Bwd2Params {
 // tail of a head, at head_dim 128 they are 2 % faster with one query head and level with four (measured).
 constexpr int CG = 16, NG = 64 / CG;
 
-template <int D>
+// kTiles: the build that takes the row term from the forward's output tiles (see bwd2_rowdots).
+template <int D, bool kTiles = false>
 struct Bwd2Cfg {
   static constexpr int kNB = (D == 64) ? 2 : 1;            // (S, dP) buffers in TMEM
   static constexpr int kNS = (D == 64) ? 4 : 2;            // (Q, dO) slots
   // K_j slots.  Two at head_dim 128 as well, at the price of one staging tile instead of two: with one slot every half tile began with the
   // wait for K_j, 3200 of 11600 cycles with one query head (B1 H16 R1 L4096 775 -> 668 us, B1 H8 R4 L4096 828 -> 734).
   static constexpr int kKj = 2;
-  static constexpr int kRing = (D == 64) ? 3 : 2;          // buffers that dS of the heads and dG of the half tiles take in turn
+  // Buffers that dS of the heads and dG of the half tiles take in turn.  With two, a free one says that the product with the probabilities of two
+  // heads ago is done as well, and the workers wait once less per head; what they would hold up without sums over the keys in between is worth a
+  // third (two and three buffers: with output tiles R4 1613 and 1540 us, R2 320 and 310, R1 930 and 948; with sums 1802 and 1837, 347 and 357,
+  // 1007 and 1027; chunks of 64 keys, B2 H8 R4 L768, 110.5 and 115).
+  static constexpr int kRing = kTiles ? 3 : 2;
+  static constexpr int kStages = (D == 64 && !kTiles) ? 2 : 1;      // staging tiles of the drain warps
   static constexpr int kHalf = 64 * D * 2;                 // [64][D] bf16
   static constexpr int kFull = 128 * D * 2;                // [128][D] bf16
   static constexpr int kBoxes = D / 64;
@@ -114,7 +120,7 @@ struct Bwd2Cfg {
   static constexpr int kSlot = 2 * kHalf;
   static constexpr int oDs = oSlot + kNS * kSlot;          // kRing x 16 KB [128 keys][64 rows] bf16, then the staging tile
   static constexpr int oStage = oDs + kRing * 16384;               // [64][64] fp32 as two boxes of [64][32], 128-byte swizzle
-  static constexpr int oT3 = oStage + 16384;             // float [2][64]: static_dest^(1/3) of a half tile's rows
+  static constexpr int oT3 = oStage + kStages * 16384;             // float [2][64]: static_dest^(1/3) of a half tile's rows
   // per-row tables that the producer copies next to the tiles (no global load is ever issued by a worker):
   static constexpr int oHeadTab = oT3 + 512;               // kNS x { float lse[64]; float cc[64] }: log-sum-exp and g_denom (or delta) of a head's rows
   static constexpr int kTab = 3;                           // half-tile tables in flight
@@ -124,10 +130,9 @@ struct Bwd2Cfg {
   static constexpr int oBar = oXch + 4096;
   static constexpr int oMisc = oBar + 320;      // (36 barriers of 8 bytes)
   // builds that take the row term from the forward's output tiles (head_dim 64; 128 has no room for them): kNS output half tiles
-  static constexpr bool kOutTiles = (D == 64);
   static constexpr int oOut = (oMisc + 256 + 1023) / 1024 * 1024;
   static constexpr int oGd16 = oOut + kNS * kHalf;         // kNS x bf16[64]: g_denom rows of a head before they are widened
-  static constexpr int kSmemBytes = kOutTiles ? oGd16 + kNS * 128 : oMisc + 256;
+  static constexpr int kSmemBytes = kTiles ? oGd16 + kNS * 128 : oMisc + 256;
   // TMEM columns.  The row-side results Y are 64 columns wide and taken D / 64 times per unit: at head_dim 128 that leaves room for
   // probabilities (bf16 pairs, 32 columns per head) in a buffer pair of their own.  Written over the S columns they kept the (S, dP)
   // buffer until the dV product had read them, and every head waited for two rounds of products one after the other:
@@ -135,7 +140,7 @@ struct Bwd2Cfg {
   static constexpr uint32_t tDV = 0, tDK = D, tY = 2 * D;
   static constexpr uint32_t tS0 = (D == 64) ? 192 : 384, tP0 = tS0 + 64, tS1 = tS0 + 128, tP1 = tS0 + 192;
   static constexpr uint32_t tPT = (D == 64) ? 448 : 320;
-  static_assert(D == 64 || D == 128, "head_dim 64 or 128");
+  static_assert(D == 64 || (D == 128 && !kTiles), "head_dim 64 or 128, output tiles at 64");
   static_assert(D == 64 ? (tP1 + 64 <= 512) : (tP0 + 64 <= 512), "TMEM budget");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 };
@@ -184,7 +189,7 @@ struct Bwd2Ctx {
 template <int D, int kC, typename TG, int kMode, bool kOutDelta>
 __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params& p, const CUtensorMap* tmK, const CUtensorMap* tmV,
                                               const CUtensorMap* tmQ, const CUtensorMap* tmG, const CUtensorMap* tmO) {
-  using Cfg = Bwd2Cfg<D>;
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int L = p.s.L, R = p.s.R, N = p.s.N;
   const uint32_t sb = smem_u32(c.smem);
   const int krow = c.bh * L + c.i * kC;
@@ -266,7 +271,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
 // 1675 and 775.
 template <int D, int kMode, bool kOutDelta>
 __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p) {
-  using Cfg = Bwd2Cfg<D>;
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int R = p.heads;
   const uint32_t sb = smem_u32(c.smem);
   constexpr uint32_t id_g = idesc_bf16(128, 64, 0, 0);
@@ -333,9 +338,9 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
 // which = 0: the accumulators that live for the whole sweep (dV_i += P dO, dK_i += dS Q, dK_i += dG K_j);
 // which = 1: the row-side results that leave after every unit (Y = dQ_rj = dS^T K_i, Y = dK_j = dG^T K_i).
 // MMAs into one accumulator always come from the same thread, so their order is kept.
-template <int D, int kC>
+template <int D, int kC, bool kOutDelta>
 __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p, const int which) {
-  using Cfg = Bwd2Cfg<D>;
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int R = p.heads;
   const uint32_t sb = smem_u32(c.smem);
   constexpr uint32_t id_kn = idesc_bf16(128, D, 0, 1);     // A K-major (or TMEM), B MN-major
@@ -448,9 +453,9 @@ __device__ __forceinline__ float warp_colsum(float* v, int lane) {
 // leaves as TMA reduce-adds into the fp32 accumulators (other key chunks add to the same rows), which run behind the
 // next unit; the workers never touch it.
 //
-template <int D>
+template <int D, bool kOutDelta>
 __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p, const CUtensorMap* tmDQ, const CUtensorMap* tmDK) {
-  using Cfg = Bwd2Cfg<D>;
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int L = p.s.L, R = p.s.R, Rh = p.heads;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = (warp & 3) * 32 + lane;               // 0..63
@@ -466,9 +471,9 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
       const int r = z / (D / 64), cb = z % (D / 64);
       if (!c.wait_w(qYFull, yc)) return;
       tc_fence_after();
-      if (leader) bulk_wait_read_all();                 // the reduce-add before has read the staging tile
+      if (leader) bulk_wait_read<Cfg::kStages - 1>();   // the last reduce-add from this staging tile has read it
       named_bar_sync(kBarDrain, 64);
-      uint8_t* stage = sStage;
+      uint8_t* stage = sStage + (Cfg::kStages > 1 ? (yc & 1) * 16384 : 0);
 #pragma unroll 1
       for (int hb = 0; hb < 2; ++hb) {
         uint32_t o[32];
@@ -509,7 +514,7 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
 // of 64 multiply-adds per row on unpacked values (900 of the 5100 that a head of a half tile took in all warps together).
 template <int D>
 __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params& p) {
-  using Cfg = Bwd2Cfg<D>;
+  using Cfg = Bwd2Cfg<D, true>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = (warp - 6) * 32;                     // the warp's rows: two blocks of 16
   const uint32_t sb = smem_u32(c.smem), swz = (uint32_t)(lane & 7);
@@ -554,7 +559,7 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
 // kOutDelta: the row term comes from the row-dot warps (see bwd2_rowdots).
 template <int D, int kC, typename TG, int kMode, bool kHeads, bool kOutDelta>
 __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& p) {
-  using Cfg = Bwd2Cfg<D>;
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   constexpr int H2 = CG / 2;                     // packed pairs per thread
   constexpr int kWorkers = kC * NG;
   constexpr int kGateQuad = kC / 64;             // the quadrant whose warps fetch the gates of the next half tile
@@ -950,8 +955,8 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
             const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
             const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDK,
             const __grid_constant__ CUtensorMap tmO, Bwd2Params p) {
-  static_assert(!kOutDelta || (Bwd2Cfg<D>::kOutTiles && kMode == 1 && kHeads), "output-tile builds: head_dim 64, per-chunk form");
-  using Cfg = Bwd2Cfg<D>;
+  static_assert(!kOutDelta || (D == 64 && kMode == 1 && kHeads), "output-tile builds: head_dim 64, per-chunk form");
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   // Used as declared: an address rounded up at run time is no shared-memory address to the compiler, and every table access a generic one with
   // 64-bit arithmetic (a tenth of the instructions; B4 H8 R4 L4096 D64 1633 -> 1520 us, one query head 1031 -> 950, B1 H16 R1 D128 620 -> 571).
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -1041,15 +1046,15 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     if (elect_one()) {
       if (warp == 0) bwd2_front<D, kMode, kOutDelta>(c, p);
       else if (kMode == 4 && warp != 2) {}      // (the row-term pass has nothing for the back issuers and the drain warps)
-      else if (warp == 1) bwd2_back<D, kC>(c, p, 0);
+      else if (warp == 1) bwd2_back<D, kC, kOutDelta>(c, p, 0);
       else if (warp == 2) bwd2_producer<D, kC, TG, kMode, kOutDelta>(c, p, &tmK, &tmV, &tmQ, &tmG, &tmO);
-      else bwd2_back<D, kC>(c, p, 1);
+      else bwd2_back<D, kC, kOutDelta>(c, p, 1);
     }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
     if (kMode == 4) {}
-    else if (warp < 6) bwd2_drain<D>(c, p, &tmDQ, &tmDK);
-    else if (kOutDelta) bwd2_rowdots<D>(c, p);
+    else if (warp < 6) bwd2_drain<D, kOutDelta>(c, p, &tmDQ, &tmDK);
+    else if constexpr (kOutDelta) bwd2_rowdots<D>(c, p);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
     bwd2_worker<D, kC, TG, kMode, kHeads, kOutDelta>(c, p);
