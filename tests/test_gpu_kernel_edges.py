@@ -319,3 +319,31 @@ def test_overlapping_launches_under_capture(shape, monkeypatch):
         assert all(torch.equal(a, b) for a, b in zip(res[:3], want[:3]))
         for a, b, key in zip(res[3:], want[3:], GRADS):
             assert rel_fro(a.float().cpu(), b.float().cpu()) <= 2.0 ** -8, key
+
+
+@pytest.mark.parametrize("shape,tiles", [((1, 2, 1, 1, 128, 64), True), ((1, 2, 1, 3, 128, 64), True), ((8, 20, 1, 3, 128, 64), True), ((1, 2, 2, 3, 128, 64), True),
+                                         ((1, 2, 3, 3, 128, 64), False), ((1, 2, 1, 3, 128, 128), False), ((2, 2, 2, 5, 64, 64), False), ((1, 2, 3, 4, 64, 128), False)])
+def test_decay_gradient_from_the_kept_powers(shape, tiles):
+    """The powers of the gram that the decay recomputation keeps for the decay gradient, in every build of the backward (one query head and several with
+    output tiles, sums over the keys, head_dim 128 where half of them are kept), with grams that are zero, negative and above the clamp.
+    Bound: four roundings to bf16 (2^-9 of a value, in the 2-norm, each: probabilities, score gradients, decay gradients and outputs, or the result)."""
+    from universal_attention_triton_b200 import ops
+    B, H, R, n, c, D = shape
+    gen = torch.Generator().manual_seed(11)
+    k = torch.randn(B, H, n, c, D, generator=gen)
+    k = k / k.norm(dim=-1, keepdim=True) * 0.9
+    k[..., 3::16, :] = 0                                     # gram exactly zero
+    k[..., 5::16, :] *= 8                                    # ... with one another 52 and more, above the clamp where the gates are open
+    k[..., 7::16, :] = -k[..., 6::16, :]                     # ... negative
+    ins = [x.bfloat16() for x in (k, torch.randn(B, H, n, c, D, generator=gen), torch.randn(B, H, R, n * c, D, generator=gen),
+                                  torch.rand(B, H, n, c, generator=gen) * 0.4 + 0.05, torch.rand(B, H, n * c, generator=gen) * 0.4 + 0.05)]
+    g_out = torch.randn(B, H, n, R, n * c, D, generator=gen).bfloat16()
+    g_lse = torch.randn(B, H, n, R, n * c, generator=gen)
+    few = slice(0, 1)                                        # (the oracle takes one sequence of a batch)
+    want = O.ua_backward(*[x[few].double() for x in ins], g_out[few].permute(0, 1, 3, 4, 5, 2).double(), g_lse[few].permute(0, 1, 3, 4, 2).double(),
+                         compute_dtype=torch.float64)
+    cu = [x.cuda() for x in ins]
+    out, lse, denom, carry = ops.forward_cm(*cu, keep_carry=True)
+    got = ops.backward_cm(*cu, g_out.cuda(), g_lse.cuda(), carry=carry, lse=lse, out_cm=out if tiles else None)
+    for name, a, b in zip(("dk", "dv", "dq", "dsrc", "ddest"), got, want):
+        assert ((a[few].cpu().double() - b).norm() / b.norm()).item() <= 4 * 2.0 ** -9, name

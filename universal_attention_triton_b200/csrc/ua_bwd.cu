@@ -35,8 +35,8 @@ int launch_bwd2_t(const Shape& s, int mode, const void* kc, const void* vc, cons
     if constexpr (D == 64 && kC == 128) {
       if (mode == 1 && p.out_tiles != nullptr) {
         if (!make_rows_map(&tmO, p.out_tiles, BH * s.N * s.R * p.Lr, D, 64)) return UA_ERR_CUDA;
-        kern = bwd2_kernel<D, kC, TG, 1, true, true>;
-        smem = Bwd2Cfg<D, true>::kSmemBytes;
+        kern = s.R == 1 ? bwd2_kernel<D, kC, TG, 1, true, 2> : bwd2_kernel<D, kC, TG, 1, true, 1>;
+        smem = s.R == 1 ? Bwd2Cfg<D, 2>::kSmemBytes : Bwd2Cfg<D, 1>::kSmemBytes;
       }
     }
   }

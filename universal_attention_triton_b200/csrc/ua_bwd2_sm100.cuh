@@ -96,8 +96,8 @@ struct Bwd2Params {
 // tail of a head, at head_dim 128 they are 2 % faster with one query head and level with four (measured).
 constexpr int CG = 16, NG = 64 / CG;
 
-// kTiles: the build that takes the row term from the forward's output tiles (see bwd2_rowdots).
-template <int D, bool kTiles = false>
+// kTiles: 1, 2: the builds that take the row term from the forward's output tiles (see bwd2_rowdots), for several query heads and for one.
+template <int D, int kTiles = 0>
 struct Bwd2Cfg {
   static constexpr int kNB = (D == 64) ? 2 : 1;            // (S, dP) buffers in TMEM
   static constexpr int kNS = (D == 64) ? 4 : 2;            // (Q, dO) slots
@@ -105,11 +105,20 @@ struct Bwd2Cfg {
   // wait for K_j, 3200 of 11600 cycles with one query head (B1 H16 R1 L4096 775 -> 668 us, B1 H8 R4 L4096 828 -> 734).
   static constexpr int kKj = 2;
   // Buffers that dS of the heads and dG of the half tiles take in turn.  With two, a free one says that the product with the probabilities of two
-  // heads ago is done as well, and the workers wait once less per head; what they would hold up without sums over the keys in between is worth a
-  // third (two and three buffers: with output tiles R4 1613 and 1540 us, R2 320 and 310, R1 930 and 948; with sums 1802 and 1837, 347 and 357,
-  // 1007 and 1027; chunks of 64 keys, B2 H8 R4 L768, 110.5 and 115).
-  static constexpr int kRing = kTiles ? 3 : 2;
-  static constexpr int kStages = (D == 64 && !kTiles) ? 2 : 1;      // staging tiles of the drain warps
+  // heads ago is done as well, and the workers wait once less per head; what they would hold up with output tiles and several heads is worth a
+  // third (two and three buffers, B4 H8 L4096 D64: R4 1568 and 1505 us, R2 1066 and 1040, R1 835 and 870; with sums over the keys 1802 and 1837, 347
+  // and 357, 1007 and 1027; chunks of 64 keys, B2 H8 R4 L768, 110.5 and 115).
+  static constexpr int kRing = kTiles == 1 ? 3 : 2;
+  // Pairs of g^(-1/3) per worker thread that the decay recomputation leaves in shared memory for the decay gradient, which then takes one
+  // operation of the XU pipe per element instead of three (with sixteen worker warps three take 1540 cycles of a half tile, which two phases
+  // each spent).  All eight at head_dim 64 (32 KB), four at 128, where no more room is left.  B4 H8 L4096 D64: with output tiles R4 1518 -> 1489 us,
+  // R2 1136 -> 1060, R1 956 -> 850; with sums R4 1805 -> 1723, R1 1014 -> 927; chunks of 64 keys, B2 H8 R4 L768, 113.7 -> 109.5; B1 H16 R1 L4096 D128
+  // 582 -> 558.
+  static constexpr int kStash = (D == 64) ? 8 : 4;
+  // What makes room for them with several heads and at head_dim 128: one box (64 x 32 floats) for the drain warps instead of two, two output half
+  // tiles instead of one per slot (the row-dot warps are done with them early); six pairs beside three output tiles are level.
+  static constexpr int kStageBoxes = kTiles == 2 ? 2 : (D == 64 && kTiles == 0) ? 4 : 1;
+  static constexpr int kNO = kTiles == 2 ? 3 : 2;
   static constexpr int kHalf = 64 * D * 2;                 // [64][D] bf16
   static constexpr int kFull = 128 * D * 2;                // [128][D] bf16
   static constexpr int kBoxes = D / 64;
@@ -119,8 +128,8 @@ struct Bwd2Cfg {
   static constexpr int oSlot = oKj + kKj * kHalf;          // slot: Q half tile, then dO half tile
   static constexpr int kSlot = 2 * kHalf;
   static constexpr int oDs = oSlot + kNS * kSlot;          // kRing x 16 KB [128 keys][64 rows] bf16, then the staging tile
-  static constexpr int oStage = oDs + kRing * 16384;               // [64][64] fp32 as two boxes of [64][32], 128-byte swizzle
-  static constexpr int oT3 = oStage + kStages * 16384;             // float [2][64]: static_dest^(1/3) of a half tile's rows
+  static constexpr int oStage = oDs + kRing * 16384;               // boxes of [64][32] fp32, 128-byte swizzle
+  static constexpr int oT3 = oStage + kStageBoxes * 8192;             // float [2][64]: static_dest^(1/3) of a half tile's rows
   // per-row tables that the producer copies next to the tiles (no global load is ever issued by a worker):
   static constexpr int oHeadTab = oT3 + 512;               // kNS x { float lse[64]; float cc[64] }: log-sum-exp and g_denom (or delta) of a head's rows
   static constexpr int kTab = 3;                           // half-tile tables in flight
@@ -131,8 +140,9 @@ struct Bwd2Cfg {
   static constexpr int oMisc = oBar + 320;      // (36 barriers of 8 bytes)
   // builds that take the row term from the forward's output tiles (head_dim 64; 128 has no room for them): kNS output half tiles
   static constexpr int oOut = (oMisc + 256 + 1023) / 1024 * 1024;
-  static constexpr int oGd16 = oOut + kNS * kHalf;         // kNS x bf16[64]: g_denom rows of a head before they are widened
-  static constexpr int kSmemBytes = kTiles ? oGd16 + kNS * 128 : oMisc + 256;
+  static constexpr int oGd16 = oOut + kNO * kHalf;         // kNS x bf16[64]: g_denom rows of a head before they are widened
+  static constexpr int oStash = kTiles ? oGd16 + kNS * 128 : oMisc + 256;
+  static constexpr int kSmemBytes = oStash + kStash * NG * 128 * 8;
   // TMEM columns.  The row-side results Y are 64 columns wide and taken D / 64 times per unit: at head_dim 128 that leaves room for
   // probabilities (bf16 pairs, 32 columns per head) in a buffer pair of their own.  Written over the S columns they kept the (S, dP)
   // buffer until the dV product had read them, and every head waited for two rounds of products one after the other:
@@ -140,7 +150,7 @@ struct Bwd2Cfg {
   static constexpr uint32_t tDV = 0, tDK = D, tY = 2 * D;
   static constexpr uint32_t tS0 = (D == 64) ? 192 : 384, tP0 = tS0 + 64, tS1 = tS0 + 128, tP1 = tS0 + 192;
   static constexpr uint32_t tPT = (D == 64) ? 448 : 320;
-  static_assert(D == 64 || (D == 128 && !kTiles), "head_dim 64 or 128, output tiles at 64");
+  static_assert(D == 64 || (D == 128 && kTiles == 0), "head_dim 64 or 128, output tiles at 64");
   static_assert(D == 64 ? (tP1 + 64 <= 512) : (tP0 + 64 <= 512), "TMEM budget");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 };
@@ -186,7 +196,7 @@ struct Bwd2Ctx {
 };
 
 // ------------------------------------------------------------- TMA producer --
-template <int D, int kC, typename TG, int kMode, bool kOutDelta>
+template <int D, int kC, typename TG, int kMode, int kOutDelta>
 __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params& p, const CUtensorMap* tmK, const CUtensorMap* tmV,
                                               const CUtensorMap* tmQ, const CUtensorMap* tmG, const CUtensorMap* tmO) {
   using Cfg = Bwd2Cfg<D, kOutDelta>;
@@ -237,12 +247,13 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
     for (int r = 0; r < Rh; ++r, ++hc) {
       const int sl = hc % Cfg::kNS, use = hc / Cfg::kNS;
       if (use >= 1 && !c.wait(qInFree + sl, use - 1)) return;
+      if (kOutDelta && hc >= Cfg::kNO && !c.wait(qDelta + (hc - Cfg::kNO) % Cfg::kNS, (hc - Cfg::kNO) / Cfg::kNS)) return;
       const int qrow = (c.bh * R + r) * p.Lr + srow0;
       const int grow = (kMode == 2) ? qrow : (int)((out_chunk * R + r) * p.Lr + srow0);
       const uint32_t dst = sb + Cfg::oSlot + sl * Cfg::kSlot, tab = sb + Cfg::oHeadTab + sl * 512;
       const bool gd16 = kOutDelta && p.g_denom16 != nullptr;
       mbar_expect_tx(c.bar(qInFull + sl), (kOutDelta ? 3 : 2) * Cfg::kHalf + (kMode == 4 ? 256 : gd16 ? 384 : 512));
-      if (kOutDelta) tma_load_2d(sb + Cfg::oOut + sl * Cfg::kHalf, tmO, 0, grow, c.bar(qInFull + sl));
+      if (kOutDelta) tma_load_2d(sb + Cfg::oOut + (hc % Cfg::kNO) * Cfg::kHalf, tmO, 0, grow, c.bar(qInFull + sl));
 #pragma unroll
       for (int b = 0; b < Cfg::kBoxes; ++b) {
         tma_load_2d(dst + b * 8192, tmQ, b * 64, qrow, c.bar(qInFull + sl));
@@ -269,7 +280,7 @@ __device__ __forceinline__ void bwd2_producer(const Bwd2Ctx& c, const Bwd2Params
 // probability buffer at head_dim 64: waiting for that one here holds up the scores, and costs more than the workers' wait.)
 // B4 H8 R4 L4096 D64: 2015 -> 1745 us, B1 H16 R1 L4096 D128 806 -> 782; with the factors of the decay gradient formed ahead of the barrier
 // 1675 and 775.
-template <int D, int kMode, bool kOutDelta>
+template <int D, int kMode, int kOutDelta>
 __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p) {
   using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int R = p.heads;
@@ -289,7 +300,9 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
     if (uses == 0) return true;
     return c.wait(qLdDone + b, uses - 1);
   };
-  // (a head's or a half tile's gradient goes to ring buffer w % kRing, its last user's products are done)
+  // (a head's or a half tile's gradient goes to ring buffer w % kRing, its last user's products are done; at head_dim 128 with several heads waited
+  // for behind the scores' products: R4 691 -> 680 us, but with one head 556 -> 566, and at head_dim 64 with output tiles R4 1505 -> 1513)
+  const bool wait_late = D == 128 && R > 1;
   unsigned w = 0;
   auto ring_free = [&]() -> bool {
     const unsigned at = w++;
@@ -321,12 +334,13 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
       if (!c.wait(qInFull + sl, hc / Cfg::kNS)) return;
       if (kOutDelta && !c.wait(qDelta + sl, hc / Cfg::kNS)) return;
       if (!acquire(b)) return;
-      if (!ring_free()) return;
+      if (!wait_late && !ring_free()) return;
       tc_fence_after();
       const uint32_t slot = sb + Cfg::oSlot + sl * Cfg::kSlot;
       mma_kk(c.tmem + (Cfg::tS0 + 128 * b), kKi, desc_lo(slot, 16));                    // S^T  = K_i Q^T
       mma_kk(c.tmem + (Cfg::tP0 + 128 * b), kVi, desc_lo(slot + Cfg::kHalf, 16));       // dP^T = V_i dO^T
       tc_commit(c.bar(qSFull + b));
+      if (wait_late && !ring_free()) return;
       mbar_arrive(c.bar(qSFull + b));
       ++u;
     }
@@ -338,7 +352,7 @@ __device__ __forceinline__ void bwd2_front(const Bwd2Ctx& c, const Bwd2Params& p
 // which = 0: the accumulators that live for the whole sweep (dV_i += P dO, dK_i += dS Q, dK_i += dG K_j);
 // which = 1: the row-side results that leave after every unit (Y = dQ_rj = dS^T K_i, Y = dK_j = dG^T K_i).
 // MMAs into one accumulator always come from the same thread, so their order is kept.
-template <int D, int kC, bool kOutDelta>
+template <int D, int kC, int kOutDelta>
 __device__ __forceinline__ void bwd2_back(const Bwd2Ctx& c, const Bwd2Params& p, const int which) {
   using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int R = p.heads;
@@ -453,7 +467,7 @@ __device__ __forceinline__ float warp_colsum(float* v, int lane) {
 // leaves as TMA reduce-adds into the fp32 accumulators (other key chunks add to the same rows), which run behind the
 // next unit; the workers never touch it.
 //
-template <int D, bool kOutDelta>
+template <int D, int kOutDelta>
 __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p, const CUtensorMap* tmDQ, const CUtensorMap* tmDK) {
   using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int L = p.s.L, R = p.s.R, Rh = p.heads;
@@ -471,9 +485,25 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
       const int r = z / (D / 64), cb = z % (D / 64);
       if (!c.wait_w(qYFull, yc)) return;
       tc_fence_after();
-      if (leader) bulk_wait_read<Cfg::kStages - 1>();   // the last reduce-add from this staging tile has read it
-      named_bar_sync(kBarDrain, 64);
-      uint8_t* stage = sStage + (Cfg::kStages > 1 ? (yc & 1) * 16384 : 0);
+      const CUtensorMap* tm = (r < Rh) ? tmDQ : tmDK;
+      const int y = (r < Rh) ? (c.bh * R + r) * p.Lr + c.srow0_of(ht) : c.bh * L + c.row0_of(ht);
+      auto tile_free = [&](auto pending) {              // the reduce-add that used the place has read it
+        if (leader) bulk_wait_read<decltype(pending)::value>();
+        named_bar_sync(kBarDrain, 64);
+      };
+      auto leave = [&](int first, int boxes, uint32_t from) {
+        fence_proxy_async();
+        named_bar_sync(kBarDrain, 64);
+        if (leader) {
+#pragma unroll
+          for (int bx = 0; bx < boxes; ++bx) tma_reduce_add_2d(tm, 64 * cb + 32 * (first + bx), y, from + bx * 8192);
+          bulk_commit_group();
+        }
+        __syncwarp();
+      };
+      constexpr bool kTile = Cfg::kStageBoxes == 4;     // two tiles of two boxes, or one or two boxes that leave one by one
+      uint8_t* stage = sStage + (kTile ? (yc & 1) * 16384 : 0);
+      if (kTile) tile_free(std::integral_constant<int, 1>{});
 #pragma unroll 1
       for (int hb = 0; hb < 2; ++hb) {
         uint32_t o[32];
@@ -483,21 +513,14 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
           tc_fence_before();
           c.arrive_w(qYFree);
         }
-        uint8_t* box = stage + hb * 8192 + row * 128;
+        if (!kTile) tile_free(std::integral_constant<int, Cfg::kStageBoxes - 1>{});
+        uint8_t* box = stage + (kTile || Cfg::kStageBoxes == 2 ? hb * 8192 : 0);
 #pragma unroll
         for (int x = 0; x < 8; ++x)
-          *reinterpret_cast<uint4*>(box + ((((uint32_t)x ^ swz) & 7) << 4)) = make_uint4(o[4 * x], o[4 * x + 1], o[4 * x + 2], o[4 * x + 3]);
+          *reinterpret_cast<uint4*>(box + row * 128 + ((((uint32_t)x ^ swz) & 7) << 4)) = make_uint4(o[4 * x], o[4 * x + 1], o[4 * x + 2], o[4 * x + 3]);
+        if (!kTile) leave(hb, 1, smem_u32(box));
       }
-      fence_proxy_async();
-      named_bar_sync(kBarDrain, 64);
-      if (leader) {
-        const CUtensorMap* tm = (r < Rh) ? tmDQ : tmDK;
-        const int y = (r < Rh) ? (c.bh * R + r) * p.Lr + c.srow0_of(ht) : c.bh * L + c.row0_of(ht);
-#pragma unroll
-        for (int bx = 0; bx < 2; ++bx) tma_reduce_add_2d(tm, 64 * cb + 32 * bx, y, smem_u32(stage) + bx * 8192);
-        bulk_commit_group();
-      }
-      __syncwarp();
+      if (kTile) leave(0, 2, smem_u32(stage));
     }
   }
   if (leader) bulk_wait_all();                          // the reduce-adds have landed before the block retires
@@ -512,9 +535,9 @@ __device__ __forceinline__ void bwd2_drain(const Bwd2Ctx& c, const Bwd2Params& p
 // traffic.)
 // The 64 dot products are the diagonal of O dO^T, taken from mma.sync fragments in blocks of 16 rows x 8 columns: a seventh of the instructions
 // of 64 multiply-adds per row on unpacked values (900 of the 5100 that a head of a half tile took in all warps together).
-template <int D>
+template <int D, int kOutDelta>
 __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params& p) {
-  using Cfg = Bwd2Cfg<D, true>;
+  using Cfg = Bwd2Cfg<D, kOutDelta>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = (warp - 6) * 32;                     // the warp's rows: two blocks of 16
   const uint32_t sb = smem_u32(c.smem), swz = (uint32_t)(lane & 7);
@@ -528,7 +551,7 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
 #pragma unroll 1
   for (int hc = 0; hc < total; ++hc) {
     const unsigned sl = (unsigned)hc % Cfg::kNS;
-    const uint32_t go = sb + Cfg::oSlot + sl * Cfg::kSlot + Cfg::kHalf + row0 * 128, oo = sb + Cfg::oOut + sl * Cfg::kHalf + row0 * 128;
+    const uint32_t go = sb + Cfg::oSlot + sl * Cfg::kSlot + Cfg::kHalf + row0 * 128, oo = sb + Cfg::oOut + ((unsigned)hc % Cfg::kNO) * Cfg::kHalf + row0 * 128;
     if (!c.wait_w(qInFull + sl, hc / Cfg::kNS)) return;
     float* tabC = reinterpret_cast<float*>(c.smem + Cfg::oHeadTab + sl * 512) + 64;
     const __nv_bfloat16* gd16 = reinterpret_cast<const __nv_bfloat16*>(c.smem + Cfg::oGd16 + sl * 128);
@@ -557,11 +580,13 @@ __device__ __forceinline__ void bwd2_rowdots(const Bwd2Ctx& c, const Bwd2Params&
 // kHeads = false: the correction pass (p.heads == 0).  A compile-time switch: as a run-time condition around the decay
 // recomputation it cost the whole-sequence kernel 2 % (measured).
 // kOutDelta: the row term comes from the row-dot warps (see bwd2_rowdots).
-template <int D, int kC, typename TG, int kMode, bool kHeads, bool kOutDelta>
+template <int D, int kC, typename TG, int kMode, bool kHeads, int kOutDelta>
 __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& p) {
   using Cfg = Bwd2Cfg<D, kOutDelta>;
   constexpr int H2 = CG / 2;                     // packed pairs per thread
   constexpr int kWorkers = kC * NG;
+  // pairs kept from the decay recomputation for the decay gradient (the correction pass and mode 4 have only one of the two)
+  constexpr int kKeep = (!kHeads || kMode == 4) ? 0 : Cfg::kStash * 128 / kC < H2 ? Cfg::kStash * 128 / kC : H2;
   constexpr int kGateQuad = kC / 64;             // the quadrant whose warps fetch the gates of the next half tile
   const int L = p.s.L, R = kHeads ? p.heads : 0, N = p.s.N;
   const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -604,6 +629,9 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   uint32_t row_at[CG / 8];
 #pragma unroll
   for (int x = 0; x < CG / 8; ++x) row_at[x] = smem_u32(c.smem + Cfg::oDs) + key * 128 + ((((uint32_t)((CG / 8) * g + x) ^ swz) & 7) << 4);
+  // pair x of the gram, floored as in the forward
+  auto gram_pair = [&](const uint32_t* gr, int x) -> float2 { return gram_floor2(make_float2(__uint_as_float(gr[2 * x]), __uint_as_float(gr[2 * x + 1]))); };
+  float4* const stash = reinterpret_cast<float4*>(c.smem + Cfg::oStash) + g * kC + key;
   int ring = 0;                                  // the buffer that the next gradient goes to
   auto store_row = [&](const uint32_t* v) {
 #pragma unroll
@@ -647,18 +675,19 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       tc_fence_before();
       c.arrive_w(qLdDone + b);
       ++u;
-      // log-retention in log2 units: lg2(1 - min(a, hi)), a = relu(g)^(2/3) s^(1/3) t^(1/3); relu through lg2(0) = -inf
+      // log-retention in log2 units, in the forward's bits (the log-sum-exp is from its prefix)
       float run = 0.f;
       auto ell_scan = [&](auto on_diag) {
         constexpr bool kDiag = decltype(on_diag)::value;
-        const float2 k23 = make_float2(2.0f / 3.0f, 2.0f / 3.0f), one2 = make_float2(1.0f, 1.0f);
+        const float2 ns32 = make_float2(-s3, -s3);
+        float2 kept;
 #pragma unroll
         for (int x = 0; x < H2; ++x) {
-          const float2 lg = make_float2(lg2(fmaxf(__uint_as_float(gr[2 * x]), 0.f)), lg2(fmaxf(__uint_as_float(gr[2 * x + 1]), 0.f)));
-          const float2 e23 = fmul2(lg, k23);
-          const float2 pw = make_float2(ex2(e23.x), ex2(e23.y));
-          const float2 a = fmul2(fmul2(pw, s32), t3p[x]);
-          const float2 om = ffma2(make_float2(fminf(a.x, clamp_hi()), fminf(a.y, clamp_hi())), make_float2(-1.0f, -1.0f), one2);
+          const float2 gp = gram_pair(gr, x), root = inv_cbrt2(gp), om = retention2(gp, root, ns32, t3p[x]);
+          if (x < kKeep) {
+            if (x & 1) stash[(x >> 1) * kWorkers] = make_float4(kept.x, kept.y, root.x, root.y);
+            else kept = root;
+          }
           float e0 = lg2(om.x), e1 = lg2(om.y);
           if (kDiag) {
             if (qbase + 2 * x <= key) e0 = 0.f;
@@ -807,24 +836,29 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
       ++u;
       // The decay gradient is linear in dell = (sum of dC over the later rows): what does not depend on it is formed first, while
       // the other groups' totals are on their way.
-      //   f1 = t^(1/3) g^(2/3) / (clamp(a) - 1)        d static_src += dell f1
+      // (the first kKeep pairs start from the g^(-1/3) that the decay recomputation left)
       //   f2 = t^(1/3) g^(-1/3) / (clamp(a) - 1)       dG = dell s^(1/3) (2/3) f2
-      // both zero above the clamp (it passes no gradient there) and for g <= 0; one exponential serves both powers, g^(2/3) = g g^(-1/3)
+      //   f1 = t^(1/3) g^(2/3) / (clamp(a) - 1)        d static_src += dell f1
+      // both zero above the clamp (it passes no gradient there) and for g <= 0
       float2 f1[H2], f2[H2];
       {
-        const float2 km13 = make_float2(-1.0f / 3.0f, -1.0f / 3.0f), mone2 = make_float2(-1.0f, -1.0f);
+        const float2 mone2 = make_float2(-1.0f, -1.0f);
 #pragma unroll
         for (int x = 0; x < H2; ++x) {
-          const float g0 = __uint_as_float(gr[2 * x]), g1 = __uint_as_float(gr[2 * x + 1]);
-          const float2 e13 = fmul2(make_float2(lg2(g0), lg2(g1)), km13);
-          const float2 r13 = make_float2(g0 > 0.f ? ex2(e13.x) : 0.f, g1 > 0.f ? ex2(e13.y) : 0.f);
-          const float2 pw = fmul2(make_float2(g0, g1), r13);
-          const float2 a = fmul2(fmul2(pw, s32), t3p[x]);
+          const float2 gp = gram_pair(gr, x);
+          if (x >= kKeep) {
+            f2[x] = inv_cbrt2(gp);
+          } else if ((x & 1) == 0) {
+            const float4 kept = stash[(x >> 1) * kWorkers];
+            f2[x] = make_float2(kept.x, kept.y);
+            f2[x + 1] = make_float2(kept.z, kept.w);
+          }
+          const float2 a = fmul2(fmul2(fmul2(gp, f2[x]), s32), t3p[x]);
           const float2 am = fadd2(make_float2(fmaxf(a.x, clamp_lo_bwd()), fmaxf(a.y, clamp_lo_bwd())), mone2);
-          const float2 iv = make_float2(a.x <= clamp_hi() ? rcp_approx(am.x) : 0.f, a.y <= clamp_hi() ? rcp_approx(am.y) : 0.f);
-          const float2 ivt = fmul2(iv, t3p[x]);
-          f1[x] = fmul2(ivt, pw);
-          f2[x] = fmul2(ivt, r13);
+          const float2 iv = make_float2(a.x <= clamp_hi() && gp.x > gram_floor() ? rcp_approx(am.x) : 0.f,
+                                        a.y <= clamp_hi() && gp.y > gram_floor() ? rcp_approx(am.y) : 0.f);
+          f2[x] = fmul2(fmul2(iv, t3p[x]), f2[x]);
+          f1[x] = fmul2(f2[x], gp);
         }
       }
       named_bar_sync(kBarAll, kWorkers);
@@ -949,7 +983,7 @@ __device__ __forceinline__ void bwd2_worker(const Bwd2Ctx& c, const Bwd2Params& 
   }
 }
 
-template <int D, int kC, typename TG, int kMode, bool kHeads, bool kOutDelta = false>
+template <int D, int kC, typename TG, int kMode, bool kHeads, int kOutDelta = 0>
 __global__ void __launch_bounds__(32 * (8 + 4 * (64 / CG)), 1)
 bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
             const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
@@ -1054,7 +1088,7 @@ bwd2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUt
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
     if (kMode == 4) {}
     else if (warp < 6) bwd2_drain<D, kOutDelta>(c, p, &tmDQ, &tmDK);
-    else if constexpr (kOutDelta) bwd2_rowdots<D>(c, p);
+    else if constexpr (kOutDelta) bwd2_rowdots<D, kOutDelta>(c, p);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkerRegs));
     bwd2_worker<D, kC, TG, kMode, kHeads, kOutDelta>(c, p);

@@ -79,15 +79,12 @@ struct FwdParams {
   const float* row_lse;  // (b,h,r,L) fp32: log-sum-exp of every row over all key chunks (from a statistics-only run)
 };
 
-// Gated affinity and log-retention of one (key, row) pair from the Gram value
-// (universal_attention_autograd.py:148-150), with hardware ex2/lg2.  Shared by
-// the forward, the carry pre-pass and the backward so that recomputation is
-// bit-identical.
-__device__ __forceinline__ float gram_pow23(float gv) { return gv > 0.f ? ex2(lg2(gv) * (2.0f / 3.0f)) : 0.f; }
-__device__ __forceinline__ float gated_affinity(float pw, float s3, float t3) { return pw * s3 * t3; }
-__device__ __forceinline__ float log_retention(float a) {
-  return lg2(1.0f - fminf(a, clamp_hi())) * 0.6931471805599453f;
-}
+// Retention 1 - min(a, hi) of one (key, row) pair from the Gram value, a = relu(g)^(2/3) s^(1/3) t^(1/3)
+// (universal_attention_autograd.py:148-150), with hardware ex2/lg2.  Shared by the forward, the carry pre-pass and the backward so that
+// recomputation is bit-identical.  g^(2/3) is g g^(-1/3), of which the backward takes the second factor too; the rounding of the logarithm enters
+// with a third instead of two thirds.  Gram values that are not positive count as the smallest normal number, whose power (5e-26) 1 - a does not see.
+__device__ __forceinline__ float gram_floor() { return 1.17549435e-38f; }
+__device__ __forceinline__ float retention_lo() { return 1.0f - clamp_hi(); }
 
 // packed fp32 pairs (one instruction for two lanes of work: the element-wise phases are bound by instruction issue)
 __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
@@ -108,6 +105,16 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
       : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
         "l"(reinterpret_cast<unsigned long long&>(c)));
   return d;
+}
+__device__ __forceinline__ float2 gram_floor2(float2 g) { return make_float2(fmaxf(g.x, gram_floor()), fmaxf(g.y, gram_floor())); }
+__device__ __forceinline__ float2 inv_cbrt2(float2 g) {
+  const float2 e = fmul2(make_float2(lg2(g.x), lg2(g.y)), make_float2(-1.0f / 3.0f, -1.0f / 3.0f));
+  return make_float2(ex2(e.x), ex2(e.y));
+}
+// (gram values floored; ns3: minus the key's s^(1/3))
+__device__ __forceinline__ float2 retention2(float2 g, float2 inv_root, float2 ns3, float2 t3) {
+  const float2 om = ffma2(fmul2(fmul2(g, inv_root), ns3), t3, make_float2(1.0f, 1.0f));
+  return make_float2(fmaxf(om.x, retention_lo()), fmaxf(om.y, retention_lo()));
 }
 
 // What the softmax groups produce: the per-chunk output tiles (and log-sum-exp), the merged-output contribution, or the
@@ -348,19 +355,14 @@ __device__ __forceinline__ void fwd_decay(const FwdCtx<D>& c, const FwdParams& p
     // prefix() = its logarithm, the scan, and C^T.  One stage of a block runs beside the other of the block before it: a warp alone on its
     // scheduler would otherwise wait for the chain of three logarithms and exponentials at the end of every block.
     auto retention = [&](uint32_t* g, int q0) {
-      const float2 k23 = make_float2(2.0f / 3.0f, 2.0f / 3.0f), s32 = make_float2(s3, s3), one2 = make_float2(1.0f, 1.0f),
-                   mone2 = make_float2(-1.0f, -1.0f);
+      const float2 ns32 = make_float2(-s3, -s3);
 #pragma unroll
       for (int x = 0; x < 16; x += 4) {
         const float4 t4 = reinterpret_cast<const float4*>(t3buf + q0)[x / 4];
 #pragma unroll
         for (int y = 0; y < 4; y += 2) {
-          // relu(g)^(2/3) through lg2(max(g, 0)) = -inf for g <= 0
-          const float2 lg = make_float2(lg2(fmaxf(__uint_as_float(g[x + y]), 0.f)), lg2(fmaxf(__uint_as_float(g[x + y + 1]), 0.f)));
-          const float2 e23 = fmul2(lg, k23);
-          const float2 pw = make_float2(ex2(e23.x), ex2(e23.y));
-          const float2 a = fmul2(fmul2(pw, s32), y ? make_float2(t4.z, t4.w) : make_float2(t4.x, t4.y));
-          const float2 om = ffma2(make_float2(fminf(a.x, clamp_hi()), fminf(a.y, clamp_hi())), mone2, one2);
+          const float2 gp = gram_floor2(make_float2(__uint_as_float(g[x + y]), __uint_as_float(g[x + y + 1])));
+          const float2 om = retention2(gp, inv_cbrt2(gp), ns32, y ? make_float2(t4.z, t4.w) : make_float2(t4.x, t4.y));
           g[x + y] = __float_as_uint(om.x);
           g[x + y + 1] = __float_as_uint(om.y);
         }
@@ -776,11 +778,20 @@ tile_totals_kernel(const __grid_constant__ CUtensorMap tmK, Shape shp, int tiles
     uint32_t g[32];
     tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + grp * 32, g);
     tc_wait_ld();
+    // (each logarithm by itself, as in the sweeps: a cut sweep has to start where a whole one would be.  One for the
+    // product of four moved dK by 2.5e-3 where affinities come close to the clamp.)
+    const float2 ns32 = make_float2(-s3, -s3);
 #pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      float ell = log_retention(gated_affinity(gram_pow23(__uint_as_float(g[q])), s3, t3[grp * 32 + q]));
-      if (x == 0 && grp * 32 + q <= k) ell = 0.f;      // (only the first tile of a sweep has rows at or before the key)
-      local += ell;
+    for (int q = 0; q < 32; q += 2) {
+      const float2 gp = gram_floor2(make_float2(__uint_as_float(g[q]), __uint_as_float(g[q + 1])));
+      const float2 om = retention2(gp, inv_cbrt2(gp), ns32, *reinterpret_cast<const float2*>(t3 + grp * 32 + q));
+      float e0 = lg2(om.x) * 0.6931471805599453f, e1 = lg2(om.y) * 0.6931471805599453f;
+      if (x == 0) {                                    // (only the first tile of a sweep has rows at or before the key)
+        if (grp * 32 + q <= k) e0 = 0.f;
+        if (grp * 32 + q + 1 <= k) e1 = 0.f;
+      }
+      local += e0;
+      local += e1;
     }
   }
   if (grp) part[(grp - 1) * 128 + k] = local;
